@@ -50,6 +50,8 @@ struct AdjointState {
   const GemmProb* wcc_p = nullptr;
   const GemmTile* wcc_t = nullptr;
   int n_pphh_t = 0, n_wcc_t = 0;
+  std::vector<GemmProb> pphh_probs, wcc_probs;
+  OzPlan pphh_oz, wcc_oz;
 };
 
 namespace {
@@ -98,6 +100,8 @@ imsrg_status Ctx::adjoint_prepare() {
   adj->pphh_t = reinterpret_cast<const GemmTile*>(base + o[1]);
   adj->wcc_p = reinterpret_cast<const GemmProb*>(base + o[2]);
   adj->wcc_t = reinterpret_cast<const GemmTile*>(base + o[3]);
+  adj->pphh_probs = pp;
+  adj->wcc_probs = wp;
   adj->n_pphh_t = (int)pt.size();
   adj->n_wcc_t = (int)wt.size();
   return IMSRG_OK;
@@ -108,6 +112,8 @@ void Ctx::adjoint_release() {
   for (void* p : {(void*)adj->cb, (void*)adj->lccb, (void*)adj->rccb, (void*)adj->wccb, (void*)adj->monob,
                   (void*)adj->partial, adj->tables})
     if (p) cudaFree(p);
+  oz_release(adj->pphh_oz);
+  oz_release(adj->wcc_oz);
   delete adj;
   adj = nullptr;
 }
@@ -139,8 +145,7 @@ imsrg_status Ctx::commutator_vjp(const double* Lp, int hL, const double* Rp, int
     ops.in[kOpWCC] = a.wccb; ops.in[kOpLCC] = d_lcc; ops.in[kOpRCC] = d_rcc;
     ops.out[kOpLCC] = a.lccb; ops.out[kOpRCC] = a.rccb;
     ops.hL = hL; ops.hR = hR;
-    k_gemm_fp64<<<a.n_wcc_t, 256, 0, stream>>>(a.wcc_p, a.wcc_t, ops);
-    CKA(launched("k_gemm_fp64(wcc vjp)"));
+    CKA(gemm_fp64(a.wcc_oz, a.wcc_probs, a.wcc_p, a.wcc_t, a.n_wcc_t, ops));
   }
   if (D.n_ob) {  // 221: one-body cotangent -> w1 / w2 cotangents
     k_vjp_221<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, pm, a.cb, hRES, d_w1, d_w2);
@@ -154,8 +159,7 @@ imsrg_status Ctx::commutator_vjp(const double* Lp, int hL, const double* Rp, int
     ops.in[kOpL] = Lp; ops.in[kOpR] = Rp; ops.in[kOpW1] = d_w1; ops.in[kOpW2] = d_w2;
     ops.out[kOpL] = Lb; ops.out[kOpR] = Rb;
     ops.hL = hL; ops.hR = hR;
-    k_gemm_fp64<<<a.n_pphh_t, 256, 0, stream>>>(a.pphh_p, a.pphh_t, ops);
-    CKA(launched("k_gemm_fp64(pphh vjp)"));
+    CKA(gemm_fp64(a.pphh_oz, a.pphh_probs, a.pphh_p, a.pphh_t, a.n_pphh_t, ops));
   }
   if (l.n_unique) {
     k_vjp_122<<<grid_of(l.n_unique), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);

@@ -204,6 +204,8 @@ imsrg_status Ctx::upload_tables() {
   partial_capacity = std::max(nseg, l.nblocks) + 64;
   CK(cuda(cudaMalloc(&d_partial, sizeof(double) * partial_capacity), "cudaMalloc(partials)"));
   CK(cuda(cudaMalloc(&d_scalars, sizeof(double) * 64), "cudaMalloc(scalars)"));
+  CK(cuda(cudaMemset(d_scalars, 0, sizeof(double) * 64), "memset(scalars)"));
+  d_err = reinterpret_cast<int*>(d_scalars + kErrorSlot);
   CK(cuda(cudaMallocHost(&h_scalars, sizeof(double) * 64), "cudaMallocHost(scalars)"));
   CK(cuda(cudaMalloc(&d_mono, sizeof(double) * (size_t)l.N * l.N), "cudaMalloc(monopole)"));
   return IMSRG_OK;
@@ -240,6 +242,8 @@ Ctx::~Ctx() {
   for (void* p : {(void*)d_tables, (void*)d_partial, (void*)d_scalars, (void*)d_mono, (void*)d_w1, (void*)d_w2,
                   (void*)d_lcc, (void*)d_rcc, (void*)d_wcc, (void*)d_int1, (void*)d_int2, (void*)d_ad, (void*)d_gen})
     if (p) cudaFree(p);
+  oz_release(pphh_oz);
+  oz_release(wcc_oz);
   if (h_scalars) cudaFreeHost(h_scalars);
   quads_release();
   for (auto& m : prof_marks) cudaEventDestroy(m.second);
@@ -336,8 +340,7 @@ imsrg_status Ctx::pphh(const double* Lp, int hL, const double* Rp, int hR, doubl
     ops.in[kOpL] = Lp; ops.in[kOpR] = Rp;
     ops.out[kOpW1] = w1; ops.out[kOpW2] = w2;
     ops.hL = hL; ops.hR = hR;
-    k_gemm_fp64<<<(int)pphh_tiles.size(), 256, 0, stream>>>(d_pphh_probs, d_pphh_tiles, ops);
-    CK(launched("k_gemm_fp64(pphh)"));
+    CK(gemm_fp64(pphh_oz, pphh_probs, d_pphh_probs, d_pphh_tiles, (int)pphh_tiles.size(), ops));
   }
   mark(kPhasePphhGemm);
   return pphh_accumulate(hL, hR, RES, w1, w2);
@@ -363,8 +366,7 @@ imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, doubl
     ops.in[kOpLCC] = lcc; ops.in[kOpRCC] = rcc;
     ops.out[kOpWCC] = wcc;
     ops.hL = hL; ops.hR = hR;
-    k_gemm_fp64<<<(int)wcc_tiles.size(), 256, 0, stream>>>(d_wcc_probs, d_wcc_tiles, ops);
-    CK(launched("k_gemm_fp64(wcc)"));
+    CK(gemm_fp64(wcc_oz, wcc_probs, d_wcc_probs, d_wcc_tiles, (int)wcc_tiles.size(), ops));
   }
   mark(kPhasePhGemm);
   if (L.n_unique == 0) return IMSRG_OK;

@@ -10,6 +10,7 @@
 #include "../../include/imsrg_gb300.h"
 #include "dev.cuh"
 #include "gemm.h"
+#include "gemm_oz.h"
 #include "layout.h"
 #include "tc.h"
 
@@ -50,6 +51,9 @@ enum Phase : int {
   kPhaseMirror = 11,
 };
 
+// the word of d_scalars (and of h_scalars) that holds the error of a bounded wait
+constexpr int kErrorSlot = 48;
+
 struct Ctx {
   imsrg::Layout L;
   imsrg::DevLayout D{};
@@ -86,6 +90,11 @@ struct Ctx {
   double *d_int1 = nullptr, *d_int2 = nullptr, *d_ad = nullptr;
   double* d_gen = nullptr;  // w2 generator workspace (3 slabs)
   imsrg::TcState* tc = nullptr;
+  // FP64 products on the tensor cores (gemm_oz.cu): the digit plans of the ladder and of the cross-coupled products
+  imsrg::OzPlan pphh_oz, wcc_oz;
+  int oz_sms = 0;  // SMs of the device, once a plan is ready
+  // error word of the tensor-core kernels' bounded waits (in d_scalars, read with tc_error)
+  int* d_err = nullptr;
   // limit of every bounded device wait of the tensor-core kernels (imsrg_set_wait_limit), and the
   // one-shot test switch that leaves one pipeline stage of the next GEMM launch unarmed
   unsigned long long tc_wait_ns = 2000000000ull;
@@ -189,6 +198,12 @@ struct Ctx {
   imsrg_status hf_transform_2b(double* op, int herm, const double* coefs);
   imsrg_status hf_run(double* op, int herm, int mode, int max_iter, const double* coefs_in, double* coefs_out,
                       imsrg_hf_info* info);
+
+  // grouped FP64 products, gemm_oz.cu
+  imsrg_status oz_prepare(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs);
+  void oz_release(imsrg::OzPlan& P);
+  imsrg_status gemm_fp64(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs, const imsrg::GemmProb* d_probs,
+                         const imsrg::GemmTile* d_tiles, int ntiles, const imsrg::GemmOperands& ops);
 
   // tensor-core (split-BF16, tcgen05) path, gemm_tc.cu
   imsrg_status tc_prepare(int mode);

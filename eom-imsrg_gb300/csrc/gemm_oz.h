@@ -1,0 +1,68 @@
+// FP64 grouped GEMMs on the BF16 tensor cores by exact integer digits (gemm_oz.cu): plans.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "gemm.h"
+
+namespace imsrg {
+
+constexpr int kOzSlices = 8;     // base-256 digits of an operand element
+constexpr int kOzBlockK = 32;    // K of an operand block (64 bytes of BF16 a row)
+constexpr int kOzTileM = 128;    // rows of an operand block and of an output tile
+constexpr int kOzTileN = 64;     // widest output tile
+
+// One operand: op(A) as rows of M (or op(B) as rows of N) over K, cut into blocks of 128 rows x 32 K, each block
+// holding its eight digit slices one after the other.  Element (r, k) is at off + r * rs + k * ks of array id.
+struct OzOperand {
+  int64_t off;
+  int id, rows, K, nkb;
+  int rs, ks;       // strides of a row and of K (one of the two is 1)
+  int exp0;         // first of its row exponents
+  int64_t blk0;     // first block: (row block rb, K block kb) is blk0 + rb * nkb + kb
+};
+// rows r0 .. r0 + 31 of an operand, one CTA of the split
+struct OzChunk {
+  int op, r0;
+};
+struct OzTerm {
+  int64_t a_blk, b_blk;
+  int a_exp, b_exp, nkb, alpha;
+};
+struct OzProb {
+  int64_t c_off;
+  int M, N, ldc, c_id, nterm, accum;
+  OzTerm t[kMaxTerms];
+};
+// rows m0 .. m0 + 127 and columns n0 .. n0 + w - 1 of a problem (w a multiple of 16, n0 of 64)
+struct OzTile {
+  int prob, m0, n0, w;
+};
+
+// The digit plan of a problem list; `state` 0: not prepared, 1: ready, -1: the list stays on k_gemm_fp64.
+struct OzPlan {
+  int state = 0;
+  std::vector<OzOperand> ops;
+  std::vector<OzChunk> chunks;
+  std::vector<OzProb> probs;
+  std::vector<OzTile> tiles;  // CTA by CTA
+  std::vector<int> start;     // first tile of every CTA
+  int ncta = 0;
+  int64_t blocks = 0;
+  int nexp = 0;
+  void* tables = nullptr;
+  char* buf = nullptr;   // operand blocks
+  int* exps = nullptr;   // row exponents, then the non-finite flag
+  int* flag = nullptr;
+  const OzOperand* d_ops = nullptr;
+  const OzChunk* d_chunks = nullptr;
+  const OzProb* d_probs = nullptr;
+  const OzTile* d_tiles = nullptr;
+  const int* d_start = nullptr;
+};
+
+// ncta: the CTAs of the persistent kernel
+void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P);
+
+}  // namespace imsrg

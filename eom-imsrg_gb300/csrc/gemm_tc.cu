@@ -27,6 +27,7 @@
 #include "recouple.h"
 #include "split.cuh"
 #include "tc.h"
+#include "umma.cuh"
 
 namespace imsrg {
 
@@ -35,49 +36,6 @@ namespace {
 constexpr int BM = 128;
 constexpr int TILE_BYTES = BM * 128;  // 128 rows of 128 bytes: 16 KiB, one TMA box
 constexpr int NUM_THREADS = 320;  // TMA warp, MMA warp, 8 epilogue warps
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned long long globaltimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait on a barrier phase.  Returns false (after recording `code`) when it has waited
-// more than limit_ns, or when another role has already aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err,
-                                          int code, unsigned long long limit_ns) {
-  if (mbar_test(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer();
-  while (true) {
-    if (mbar_test(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (globaltimer() - t0 > limit_ns) {
-      atomicCAS(err, 0, code);
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
@@ -130,13 +88,6 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, ui
         "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
@@ -552,7 +503,6 @@ struct TcState {
   const int* d_cc_seg = nullptr;
   const int* d_swap_row = nullptr;
   float* zbuf = nullptr;  // X, the recoupling input (FP32, wcc layout)
-  int* d_err = nullptr;
   // orbit quadruples (i<=j, k<=l) of the particle-hole recoupling, j fastest
   std::vector<uint64_t> quads;
   const uint64_t* d_quads = nullptr;
@@ -649,7 +599,6 @@ void Ctx::tc_release() {
   if (tc->buf) cudaFree(tc->buf);
   if (tc->d_mem) cudaFree(tc->d_mem);
   if (tc->zbuf) cudaFree(tc->zbuf);
-  if (tc->d_err) cudaFree(tc->d_err);
   if (tc->g122_fb) cudaFree(tc->g122_fb);
   if (tc->d_g122_tasks) cudaFree(tc->d_g122_tasks);
   if (tc->d_g122_items) cudaFree(tc->d_g122_items);
@@ -862,9 +811,7 @@ imsrg_status Ctx::tc_prepare(int mode) {
   CK_TC(cuda(cudaMemset(tc->buf, 0, std::max<size_t>(bytes, 256)), "memset(tc operands)"));
   CK_TC(cuda(cudaMalloc(&tc->zbuf, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(X)"));
   CK_TC(cuda(cudaMemset(tc->zbuf, 0, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "memset(X)"));
-  CK_TC(cuda(cudaMalloc(&tc->d_err, sizeof(int)), "cudaMalloc(err)"));
   CK_TC(cuda(cudaMalloc(&tc->g122_fb, sizeof(float2) * std::max(tc->g122_nblk2, 1)), "cudaMalloc(122 blocks)"));
-  CK_TC(cuda(cudaMemset(tc->d_err, 0, sizeof(int)), "memset(err)"));
   DevPacker pk;
   pk.add(tc->split_ops, &tc->d_split_ops);
   pk.add(tc->split_prefix, &tc->d_split_prefix);
@@ -968,7 +915,7 @@ imsrg_status Ctx::tc_gemm_on(const CUtensorMap& map, int64_t slice_rows, const T
   const int unarmed = tc_unarmed_next ? 0 : -1;  // one-shot test switch
   tc_unarmed_next = 0;
   auto go = [&](auto launcher) {
-    launcher(grid, stream, map, slice_rows, probs, tiles, ntiles, out, hL, hR, tc->d_err, tc_wait_ns, unarmed);
+    launcher(grid, stream, map, slice_rows, probs, tiles, ntiles, out, hL, hR, d_err, tc_wait_ns, unarmed);
   };
   if (tc->kind == kKindTF32)
     wmax == 256 ? go(launch_tc_gemm<2, kKindTF32, 256>) : go(launch_tc_gemm<2, kKindTF32, 128>);
@@ -1037,12 +984,12 @@ imsrg_status Ctx::tc_pphh(const double* Lp, int hL, const double* Rp, int hR, do
 }
 
 imsrg_status Ctx::tc_error() {
-  if (!tc) return IMSRG_OK;
-  int e = 0;
-  CK_TC(cuda(cudaMemcpyAsync(&e, tc->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "D2H tc error"));
+  if (!tc && !oz_sms) return IMSRG_OK;
+  int& e = *reinterpret_cast<int*>(h_scalars + kErrorSlot);
+  CK_TC(cuda(cudaMemcpyAsync(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "D2H tc error"));
   CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
   if (e) {
-    cudaMemsetAsync(tc->d_err, 0, sizeof(int), stream);
+    cudaMemsetAsync(d_err, 0, sizeof(int), stream);
     static const char* role[] = {"", "producer (stage free)", "MMA (accumulator free)", "MMA (stage loaded)",
                                  "epilogue (accumulator ready)"};
     return fail(IMSRG_ERR_TIMEOUT, std::string("tensor-core GEMM: a bounded wait ran out in the ") +

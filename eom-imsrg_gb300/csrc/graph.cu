@@ -303,7 +303,11 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
                               const StepHostIO* hio) {
   CK_TC(ensure_workspace());
   CK_TC(ensure_flow_workspace());
-  if (precision == IMSRG_PREC_FP64 && L.cc_size) CK_TC(ensure_wcc());
+  if (precision == IMSRG_PREC_FP64) {
+    if (L.cc_size) CK_TC(ensure_wcc());
+    CK_TC(oz_prepare(pphh_oz, pphh_probs));
+    CK_TC(oz_prepare(wcc_oz, wcc_probs));
+  }
   if (!sg) {
     sg = new StepGraph();
     CK_TC(cuda(cudaMalloc(&sg->d_state, sizeof(StepState)), "cudaMalloc(step state)"));

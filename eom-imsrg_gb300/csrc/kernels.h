@@ -43,7 +43,9 @@ __global__ void k_zero_runs(double* x, const int64_t* runs);
 __global__ void k_zero_runs_f(float* x, const int64_t* runs);
 __global__ void k_convert_check(const double* x, const float* y, int64_t n, float* out_f32, double* out_f64);
 
-__global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, GemmOperands ops);
+// run_if: with a flag, nothing is done unless it is set
+__global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, int ntiles, GemmOperands ops,
+                            const int* run_if);
 
 // mixed-precision companions (kernels_mixed.cu)
 void launch_pandya_tc(int S, int kind, int nchunks, cudaStream_t stream, const DevLayout& D, const PandyaChunk* chunks,

@@ -464,7 +464,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
       ops.in[kOpL] = Lp; ops.in[kOpR] = R;
       ops.out[kOpW1] = S.w1; ops.out[kOpW2] = S.w2;
       ops.hL = hL; ops.hR = hR;
-      k_gemm_fp64<<<S.n_hh_t, 256, 0, stream>>>(S.hh_p, S.hh_t, ops);
+      k_gemm_fp64<<<S.n_hh_t, 256, 0, stream>>>(S.hh_p, S.hh_t, S.n_hh_t, ops, nullptr);
       CKT(launched("k_gemm_fp64(tensor hh ladder)"));
     }
     k_axpby<<<grid_n(T.slab), 256, 0, stream>>>(T.slab, S.w1, 1.0, S.w3, 1.0, S.w1);
@@ -491,7 +491,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
         k_gemm_f32<<<nt, 256, 0, stream>>>(S.exc_p, S.exc_t, ops);
         CKT(launched("k_gemm_f32(tensor pphh, excitation)"));
       } else {
-        k_gemm_fp64<<<nt, 256, 0, stream>>>(exc ? S.exc_p : S.pphh_p, exc ? S.exc_t : S.pphh_t, ops);
+        k_gemm_fp64<<<nt, 256, 0, stream>>>(exc ? S.exc_p : S.pphh_p, exc ? S.exc_t : S.pphh_t, nt, ops, nullptr);
         CKT(launched("k_gemm_fp64(tensor pphh)"));
       }
     }
@@ -522,7 +522,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
           k_gemm_f32<<<S.x_n_t, 256, 0, stream>>>(S.x_p, S.x_t, ops);
           CKT(launched("k_gemm_f32(tensor ph, excitation)"));
         } else {
-          k_gemm_fp64<<<S.x_n_t, 256, 0, stream>>>(S.x_p, S.x_t, ops);
+          k_gemm_fp64<<<S.x_n_t, 256, 0, stream>>>(S.x_p, S.x_t, S.x_n_t, ops, nullptr);
           CKT(launched("k_gemm_fp64(tensor ph, excitation)"));
         }
       }
@@ -587,7 +587,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
         ops.in[kOpLCC] = d_lcc; ops.in[kOpRCC] = S.ccr; ops.in[kOpWCC] = S.ccx;
         ops.out[kOpW1] = S.wx; ops.out[kOpW2] = S.wy;
         ops.hL = hL; ops.hR = hR;
-        k_gemm_fp64<<<S.cb_tile_n[b], 256, 0, stream>>>(S.cb_p, S.cb_t + S.cb_tile_start[b], ops);
+        k_gemm_fp64<<<S.cb_tile_n[b], 256, 0, stream>>>(S.cb_p, S.cb_t + S.cb_tile_start[b], S.cb_tile_n[b], ops, nullptr);
         CKT(launched("k_gemm_fp64(tensor ph)"));
       }
       k_ts222ph_scatter<<<grid_n((int64_t)r1 * r2), 256, 0, stream>>>(D, T, S.wx, doy ? S.wy : nullptr, J3, J4, qa,
