@@ -1,5 +1,4 @@
-// commutator_122 (src/commutators.f90:283-396) of the mixed path, FP32, by pair-group
-// sub-blocks.  Orbits sharing (l, j, tz) form a block; in channel q the pairs (a in B1,
+// commutator_122 (src/commutators.f90:283-396) by pair-group sub-blocks, in FP32 (mixed path) or FP64.  Orbits sharing (l, j, tz) form a block; in channel q the pairs (a in B1,
 // b in B2) form a group G.  The one-body factors only mix orbits of one block, so on a
 // group-pair sub-block (G1, G2) of the ordered-pair form V_A(ab, cd) (what v_elem returns)
 // the result is four one-index products:
@@ -33,23 +32,52 @@ namespace {
 
 __device__ __forceinline__ int g122_div(int e, int m) { return (int)(((unsigned)e * (unsigned)m) >> 20); }
 
-// pre and 1 / pre of a code word
-__device__ __forceinline__ float g122_pre(unsigned w) {
+template <typename T>
+struct G122Type;
+template <>
+struct G122Type<float> {
+  using T2 = float2;
+  static constexpr float kRoot2 = 1.41421356f, kHalfRoot2 = 0.70710678f;
+  __device__ static float load(double x) { return f64_to_f32(x); }
+  __device__ static double store(float x) { return f32_to_f64(x); }
+  __device__ static float flip(float x, bool neg) { return neg ? -x : x; }
+  __device__ static float f(const DevLayout& D, const double* op, int herm, int a, int b) { return d_f_elem_f(D, op, herm, a, b); }
+};
+template <>
+struct G122Type<double> {
+  using T2 = double2;
+  static constexpr double kRoot2 = 1.4142135623730951, kHalfRoot2 = 0.70710678118654752;
+  __device__ static double load(double x) { return x; }
+  __device__ static double store(double x) { return x; }
+  __device__ static double flip(double x, bool neg) {  // an integer instruction: the FP64 pipe bounds this kernel
+    return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+  }
+  __device__ static double f(const DevLayout& D, const double* op, int herm, int a, int b) { return d_f_elem(D, op, herm, a, b); }
+};
+
+// x times the size of pre of a code word (1, sqrt 2 or 2), and x over it
+template <typename T>
+__device__ __forceinline__ T g122_mul(unsigned w, T x) {
   const unsigned m = w >> 30;
-  const float v = m == 0 ? 1.0f : (m == 1 ? 1.41421356f : 2.0f);
-  return (w >> 29) & 1u ? -v : v;
+  if (m) x *= m == 1 ? G122Type<T>::kRoot2 : (T)2;
+  return x;
 }
-__device__ __forceinline__ float g122_ipre(unsigned w) {
+template <typename T>
+__device__ __forceinline__ T g122_div_pre(unsigned w, T x) {
   const unsigned m = w >> 30;
-  const float v = m == 0 ? 1.0f : (m == 1 ? 0.70710678f : 0.5f);
-  return (w >> 29) & 1u ? -v : v;
+  if (m) x *= m == 1 ? G122Type<T>::kHalfRoot2 : (T)0.5;
+  return x;
 }
 
 // the (L, R) pair of V_A of one element from its code word and stored values
-__device__ __forceinline__ float2 g122_va(unsigned w, double l, double r, int hL, int hR) {
-  const bool sw = (w & (1u << kG122IdxBits)) != 0;
-  const float pre = g122_pre(w);
-  return make_float2(f64_to_f32(l) * ((sw && hL < 0) ? -pre : pre), f64_to_f32(r) * ((sw && hR < 0) ? -pre : pre));
+template <typename T>
+__device__ __forceinline__ typename G122Type<T>::T2 g122_va(unsigned w, double l, double r, int hL, int hR) {
+  using X = G122Type<T>;
+  const bool sw = (w & (1u << kG122IdxBits)) != 0, neg = (w >> 29) & 1u;
+  typename X::T2 v;
+  v.x = X::flip(g122_mul<T>(w, X::load(l)), (sw && hL < 0) != neg);
+  v.y = X::flip(g122_mul<T>(w, X::load(r)), (sw && hR < 0) != neg);
+  return v;
 }
 
 __device__ __forceinline__ void g122_sync(bool cta, unsigned mask) {
@@ -58,10 +86,12 @@ __device__ __forceinline__ void g122_sync(bool cta, unsigned mask) {
 
 // One task on nth threads: 8 or 32 lanes of a warp (under mask), or the whole CTA (cta).  One
 // copy of this code serves all three, so the warps of a CTA share their instructions.
+template <typename T>
 __device__ __forceinline__ void g122_run(const DevLayout& D, const G122Task& t, const unsigned* __restrict__ EC,
                                          const double* __restrict__ L, int hL, const double* __restrict__ R, int hR,
-                                         double* __restrict__ RES, int hRES, const float2* __restrict__ FB,
-                                         float2* __restrict__ X, int tid, int nth, bool cta, unsigned mask) {
+                                         double* __restrict__ RES, int hRES, const typename G122Type<T>::T2* __restrict__ FB,
+                                         typename G122Type<T>::T2* __restrict__ X, int tid, int nth, bool cta, unsigned mask) {
+  using T2 = typename G122Type<T>::T2;
   const int n0 = t.nn & 255, n1 = (t.nn >> 8) & 255, n2 = (t.nn >> 16) & 255, n3 = t.nn >> 24;
   const int nb = n0 * n1, ntot = nb * n2 * n3;
   const unsigned* C = EC + t.eoff;
@@ -72,19 +102,19 @@ __device__ __forceinline__ void g122_run(const DevLayout& D, const G122Task& t, 
     const unsigned w0 = __ldg(C + e), w1 = __ldg(C + e + nth);
     const double l0 = __ldg(L + (w0 & kIdx)), r0 = __ldg(R + (w0 & kIdx));
     const double l1 = __ldg(L + (w1 & kIdx)), r1 = __ldg(R + (w1 & kIdx));
-    X[e] = g122_va(w0, l0, r0, hL, hR);
-    X[e + nth] = g122_va(w1, l1, r1, hL, hR);
+    X[e] = g122_va<T>(w0, l0, r0, hL, hR);
+    X[e + nth] = g122_va<T>(w1, l1, r1, hL, hR);
   }
   if (e < ntot) {
     const unsigned w = __ldg(C + e);
-    X[e] = g122_va(w, __ldg(L + (w & kIdx)), __ldg(R + (w & kIdx)), hL, hR);
+    X[e] = g122_va<T>(w, __ldg(L + (w & kIdx)), __ldg(R + (w & kIdx)), hL, hR);
   }
   g122_sync(cta, mask);
   const int s1 = n0, s2 = nb, s3 = nb * n2;
-  const float2* F0 = FB + t.fb[0];
-  const float2* F1 = FB + t.fb[1];
-  const float2* F2 = FB + t.fb[2];
-  const float2* F3 = FB + t.fb[3];
+  const T2* F0 = FB + t.fb[0];
+  const T2* F1 = FB + t.fb[1];
+  const T2* F2 = FB + t.fb[2];
+  const T2* F3 = FB + t.fb[3];
   for (int e = tid; e < ntot; e += nth) {
     const int ek = g122_div(e, t.mb), eb = e - ek * nb;
     const int x1 = g122_div(eb, t.m0), x0 = eb - x1 * n0;
@@ -95,45 +125,45 @@ __device__ __forceinline__ void g122_run(const DevLayout& D, const G122Task& t, 
     const unsigned w = __ldg(C + e);
     const bool sw = (w & kSwap) != 0;
     if (sw && !(t.flags & 1)) continue;
-    float out = 0.0f;
+    T out = 0;
     {  // sum_a' f(a, a') X[a', ...]
-      const float2* f = F0 + x0 * n0;
-      const float2* xp = X + (e - x0);
+      const T2* f = F0 + x0 * n0;
+      const T2* xp = X + (e - x0);
       for (int a = 0; a < n0; ++a) {
-        const float2 fv = __ldg(f + a), xv = xp[a];
-        out = fmaf(fv.x, xv.y, out);
-        out = fmaf(-fv.y, xv.x, out);
+        const T2 fv = __ldg(f + a), xv = xp[a];
+        out = fma(fv.x, xv.y, out);
+        out = fma(-fv.y, xv.x, out);
       }
     }
     {
-      const float2* f = F1 + x1 * n1;
-      const float2* xp = X + (e - x1 * s1);
+      const T2* f = F1 + x1 * n1;
+      const T2* xp = X + (e - x1 * s1);
       for (int a = 0; a < n1; ++a) {
-        const float2 fv = __ldg(f + a), xv = xp[a * s1];
-        out = fmaf(fv.x, xv.y, out);
-        out = fmaf(-fv.y, xv.x, out);
+        const T2 fv = __ldg(f + a), xv = xp[a * s1];
+        out = fma(fv.x, xv.y, out);
+        out = fma(-fv.y, xv.x, out);
       }
     }
     {  // - sum_c' f(c', c) X[..., c', ...]
-      const float2* f = F2 + x2;
-      const float2* xp = X + (e - x2 * s2);
+      const T2* f = F2 + x2;
+      const T2* xp = X + (e - x2 * s2);
       for (int a = 0; a < n2; ++a) {
-        const float2 fv = __ldg(f + a * n2), xv = xp[a * s2];
-        out = fmaf(-fv.x, xv.y, out);
-        out = fmaf(fv.y, xv.x, out);
+        const T2 fv = __ldg(f + a * n2), xv = xp[a * s2];
+        out = fma(-fv.x, xv.y, out);
+        out = fma(fv.y, xv.x, out);
       }
     }
     {
-      const float2* f = F3 + x3;
-      const float2* xp = X + (e - x3 * s3);
+      const T2* f = F3 + x3;
+      const T2* xp = X + (e - x3 * s3);
       for (int a = 0; a < n3; ++a) {
-        const float2 fv = __ldg(f + a * n3), xv = xp[a * s3];
-        out = fmaf(-fv.x, xv.y, out);
-        out = fmaf(fv.y, xv.x, out);
+        const T2 fv = __ldg(f + a * n3), xv = xp[a * s3];
+        out = fma(-fv.x, xv.y, out);
+        out = fma(fv.y, xv.x, out);
       }
     }
-    const float v = out * g122_ipre(w);  // stored = V_A / pre
-    RES[w & kIdx] = f32_to_f64((sw && hRES < 0) ? -v : v);
+    const T v = g122_div_pre<T>(w, out);  // stored = V_A / pre
+    RES[w & kIdx] = G122Type<T>::store(G122Type<T>::flip(v, (sw && hRES < 0) != (((w >> 29) & 1u) != 0u)));
   }
   g122_sync(cta, mask);
 }
@@ -141,21 +171,26 @@ __device__ __forceinline__ void g122_run(const DevLayout& D, const G122Task& t, 
 // blocks [0, nbig): one big task each on the whole CTA; the other blocks: eight warps, each with
 // a slice of slice_f2 (L, R) pairs (four sub-slices of sub_f2 for the 8-lane groups), taking
 // runs of tasks from the counter until none is left
-__global__ void __launch_bounds__(kG122Threads, 5) k_comm122_sub(DevLayout D, const G122Task* __restrict__ tasks,
+template <typename T>
+__global__ void __launch_bounds__(kG122Threads, sizeof(T) == 4 ? 5 : 3) k_comm122_sub(DevLayout D, const G122Task* __restrict__ tasks,
                                                               const int2* __restrict__ items, int nitems, int nbig,
                                                               int* counter, const unsigned* __restrict__ EC,
                                                               int slice_f2, int sub_f2, const double* __restrict__ L,
                                                               int hL, const double* __restrict__ R, int hR,
                                                               double* __restrict__ RES, int hRES,
-                                                              const float2* __restrict__ FB) {
-  extern __shared__ float2 g122_x[];
+                                                              const typename G122Type<T>::T2* __restrict__ FB,
+                                                              const int* __restrict__ skip) {
+  using T2 = typename G122Type<T>::T2;
+  extern __shared__ __align__(16) unsigned char g122_smem[];
+  T2* g122_x = reinterpret_cast<T2*>(g122_smem);
+  if (skip && *skip) return;
   if ((int)blockIdx.x < nbig) {
     const G122Task t = tasks[blockIdx.x];
-    g122_run(D, t, EC, L, hL, R, hR, RES, hRES, FB, g122_x, threadIdx.x, kG122Threads, true, 0u);
+    g122_run<T>(D, t, EC, L, hL, R, hR, RES, hRES, FB, g122_x, threadIdx.x, kG122Threads, true, 0u);
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float2* slice = g122_x + (size_t)warp * slice_f2;
+  T2* slice = g122_x + (size_t)warp * slice_f2;
   for (;;) {
     int it = 0;
     if (lane == 0) it = atomicAdd(counter, 1);
@@ -169,7 +204,7 @@ __global__ void __launch_bounds__(kG122Threads, 5) k_comm122_sub(DevLayout D, co
     const unsigned mask = quad ? 0xFFu << (grp * 8) : 0xffffffffu;
     for (int k = grp; k < cnt; k += step) {
       const G122Task t = tasks[w.x + k];
-      g122_run(D, t, EC, L, hL, R, hR, RES, hRES, FB, slice + grp * sub_f2, lane & (nth - 1), nth, false, mask);
+      g122_run<T>(D, t, EC, L, hL, R, hR, RES, hRES, FB, slice + grp * sub_f2, lane & (nth - 1), nth, false, mask);
     }
     __syncwarp();
   }
@@ -177,32 +212,90 @@ __global__ void __launch_bounds__(kG122Threads, 5) k_comm122_sub(DevLayout D, co
 
 }  // namespace
 
+// f(x, y) of L and R on every block; also clears the work counter and the flag behind it
+template <typename T>
 __global__ void k_comm122_fb2(DevLayout D, PairGroupsDev G, int nspb, const double* __restrict__ L, int hL,
-                              const double* __restrict__ R, int hR, float2* __restrict__ FB, int* counter) {
+                              const double* __restrict__ R, int hR, typename G122Type<T>::T2* __restrict__ FB, int* counter) {
   const int B = blockIdx.x;
-  if (B == 0 && threadIdx.x == 0) *counter = 0;
+  if (B == 0 && threadIdx.x < 2) counter[threadIdx.x] = 0;
   if (B >= nspb) return;
   const int n = G.spb_n[B];
   const int* o = G.spb_orb + G.spb_start[B];
   for (int r = threadIdx.x; r < n * n; r += blockDim.x) {
     const int x = r / n, y = r - (r / n) * n;
-    FB[G.blk_off[B] + r] = make_float2(d_f_elem_f(D, L, hL, o[x], o[y]), d_f_elem_f(D, R, hR, o[x], o[y]));
+    typename G122Type<T>::T2 v;
+    v.x = G122Type<T>::f(D, L, hL, o[x], o[y]);
+    v.y = G122Type<T>::f(D, R, hR, o[x], o[y]);
+    FB[G.blk_off[B] + r] = v;
   }
 }
 
+// flag = 1 unless the lower triangles of L's and R's square arrays are herm times their upper ones: one CTA per pair of
+// 32 x 32 tiles.  Reads both operators' square arrays once (0.09 ms at eMax 10).
+__global__ void __launch_bounds__(256) k_check_mirror(DevLayout D, const int4* __restrict__ tiles, int ntiles,
+                                                      const double* __restrict__ L, int hL, const double* __restrict__ R,
+                                                      int hR, int* flag) {
+  __shared__ double X[2][32][33];
+  if ((int)blockIdx.x >= ntiles) return;
+  const int4 t = tiles[blockIdx.x];
+  if (!t.w) return;
+  const int i0 = t.y, j0 = t.z, n = D.gn1[t.x], tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t base = D.goff[t.x];
+  for (int r = ty; r < 32; r += 8) {  // the upper tile
+    const int i = i0 + tx, j = j0 + r;
+    const bool in = i < n && j < n;
+    const int64_t e = base + i + (int64_t)j * n;
+    X[0][r][tx] = in ? L[e] : 0.0;
+    X[1][r][tx] = in ? R[e] : 0.0;
+  }
+  __syncthreads();
+  bool bad = false;
+  for (int r = ty; r < 32; r += 8) {  // the lower one: (j0 + tx, i0 + r) against (i0 + r, j0 + tx)
+    const int i = j0 + tx, j = i0 + r;
+    if (i < n && j < n && i > j) {
+      const int64_t e = base + i + (int64_t)j * n;
+      bad |= !(L[e] == G122Type<double>::flip(X[0][tx][r], hL < 0)) || !(R[e] == G122Type<double>::flip(X[1][tx][r], hR < 0));
+    }
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 1;
+}
+
+template <typename T>
+void launch_comm122_fb(int nspb, cudaStream_t st, const DevLayout& D, const PairGroupsDev& G, const double* L, int hL,
+                       const double* R, int hR, void* FB, int* counter) {
+  k_comm122_fb2<T><<<std::max(nspb, 1), 64, 0, st>>>(D, G, nspb, L, hL, R, hR, static_cast<typename G122Type<T>::T2*>(FB), counter);
+}
+template <typename T>
 void launch_comm122(int grid, size_t smem, cudaStream_t st, const DevLayout& D, const G122Task* tasks,
                     const int2* items, int nitems, int nbig, int* counter, const unsigned* codes, int slice_f2, int sub_f2,
-                    const double* L, int hL, const double* R, int hR, double* RES, int hRES, const float2* FB) {
-  k_comm122_sub<<<grid, kG122Threads, smem, st>>>(D, tasks, items, nitems, nbig, counter, codes, slice_f2, sub_f2, L,
-                                                  hL, R, hR, RES, hRES, FB);
+                    const double* L, int hL, const double* R, int hR, double* RES, int hRES, const void* FB,
+                    const int* skip) {
+  k_comm122_sub<T><<<grid, kG122Threads, smem, st>>>(D, tasks, items, nitems, nbig, counter, codes, slice_f2, sub_f2, L, hL,
+                                                     R, hR, RES, hRES, static_cast<const typename G122Type<T>::T2*>(FB), skip);
 }
+template void launch_comm122_fb<float>(int, cudaStream_t, const DevLayout&, const PairGroupsDev&, const double*, int,
+                                       const double*, int, void*, int*);
+template void launch_comm122_fb<double>(int, cudaStream_t, const DevLayout&, const PairGroupsDev&, const double*, int,
+                                        const double*, int, void*, int*);
+template void launch_comm122<float>(int, size_t, cudaStream_t, const DevLayout&, const G122Task*, const int2*, int, int, int*,
+                                    const unsigned*, int, int, const double*, int, const double*, int, double*, int,
+                                    const void*, const int*);
+template void launch_comm122<double>(int, size_t, cudaStream_t, const DevLayout&, const G122Task*, const int2*, int, int, int*,
+                                     const unsigned*, int, int, const double*, int, const double*, int, double*, int,
+                                     const void*, const int*);
 
-cudaError_t g122_smem_attr(size_t smem) {
-  return cudaFuncSetAttribute(k_comm122_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
-cudaError_t g122_blocks_per_sm(size_t smem, int* n) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, k_comm122_sub, kG122Threads, smem);
+// shared memory limits and resident CTAs per SM of the FP32 ([0], smem bytes) and the FP64 kernel ([1], twice as many; 0
+// where a CTA cannot have that much)
+cudaError_t g122_occupancy(size_t smem, int* per_sm) {
+  cudaError_t e = cudaFuncSetAttribute(k_comm122_sub<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_comm122_sub<float>, kG122Threads, smem);
+  if (e != cudaSuccess) return e;
+  per_sm[1] = 0;
+  if (2 * smem > 227 * 1024) return cudaSuccess;
+  e = cudaFuncSetAttribute(k_comm122_sub<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * smem));
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_comm122_sub<double>, kG122Threads, 2 * smem);
 }
 
 size_t g122_smem_bytes(int tiny_cap, int warp_cap, int nmax4) {
@@ -296,8 +389,9 @@ std::string g122_partition(G122Plan& P, int tiny_cap, int warp_cap) {
     for (size_t k : big) P.tasks.push_back(P.all[k]);
   }
   P.nbig = (int)P.tasks.size();
-  // warp work, channel by channel: runs of up to 16 small tasks (four at a time on 8-lane
-  // groups, similar sizes together) and runs of warp tasks of about 512 elements
+  // warp work, channel by channel: four small tasks at a time on 8-lane groups (similar sizes together), or one warp
+  // task.  Longer runs saved fetches of the counter and lost more at the ends and in small bases: runs of 16 / of about 512
+  // elements took 43 us at eMax 4, 116 at eMax 8 and 425 at eMax 10 (FP32), these 25, 91 and 385.
   size_t i = 0;
   while (i < n) {
     const int q = P.all[i].q;
@@ -313,18 +407,14 @@ std::string g122_partition(G122Plan& P, int tiny_cap, int warp_cap) {
     std::stable_sort(tiny.begin(), tiny.end(), [&](size_t a, size_t b) {
       return P.elems[a] != P.elems[b] ? P.elems[a] > P.elems[b] : P.all[a].nn < P.all[b].nn;
     });
-    for (size_t k = 0; k < tiny.size(); k += 16) {
-      const size_t e = std::min(tiny.size(), k + 16);
+    for (size_t k = 0; k < tiny.size(); k += 4) {
+      const size_t e = std::min(tiny.size(), k + 4);
       P.items.push_back(make_int2((int)P.tasks.size(), (int)(e - k)));
       for (size_t m = k; m < e; ++m) P.tasks.push_back(P.all[tiny[m]]);
     }
-    for (size_t k = 0; k < warp.size();) {
-      int64_t sum = 0;
-      size_t e = k;
-      while (e < warp.size() && e - k < 4 && sum < 512) sum += P.elems[warp[e++]];
-      P.items.push_back(make_int2((int)P.tasks.size(), (int)(e - k) | 1 << 16));
-      for (size_t m = k; m < e; ++m) P.tasks.push_back(P.all[warp[m]]);
-      k = e;
+    for (size_t k : warp) {
+      P.items.push_back(make_int2((int)P.tasks.size(), 1 | 1 << 16));
+      P.tasks.push_back(P.all[k]);
     }
     i = j;
   }

@@ -1,4 +1,4 @@
-// commutator_122 of the mixed path by pair-group sub-blocks (comm122.cu): the host plan and
+// commutator_122 by pair-group sub-blocks (comm122.cu): the host plan and
 // its launch.
 #pragma once
 #include <cuda_runtime.h>
@@ -53,14 +53,18 @@ std::string build_g122_plan(const Layout& L, const PairGroups& G, G122Plan& P);
 // on a warp, larger ones on a CTA
 std::string g122_partition(G122Plan& P, int tiny_cap, int warp_cap);
 size_t g122_smem_bytes(int tiny_cap, int warp_cap, int nmax4);
-cudaError_t g122_smem_attr(size_t smem);
-cudaError_t g122_blocks_per_sm(size_t smem, int* n);  // resident CTAs of the 122 kernel per SM
+cudaError_t g122_occupancy(size_t smem, int* per_sm);
 
-// f(x, y) of L and R on every block, as (fL, fR) pairs; also clears the work counter
-__global__ void k_comm122_fb2(DevLayout D, PairGroupsDev G, int nspb, const double* L, int hL, const double* R, int hR,
-                              float2* FB, int* counter);
+// T: float (FP32 arithmetic, FB of float2) or double (FB of double2)
+template <typename T>
+void launch_comm122_fb(int nspb, cudaStream_t st, const DevLayout& D, const PairGroupsDev& G, const double* L, int hL,
+                       const double* R, int hR, void* FB, int* counter);
+template <typename T>
 void launch_comm122(int grid, size_t smem, cudaStream_t st, const DevLayout& D, const G122Task* tasks,
                     const int2* items, int nitems, int nbig, int* counter, const unsigned* codes, int slice_f2, int sub_f2,
-                    const double* L, int hL, const double* R, int hR, double* RES, int hRES, const float2* FB);
+                    const double* L, int hL, const double* R, int hR, double* RES, int hRES, const void* FB,
+                    const int* skip);
+__global__ void k_check_mirror(DevLayout D, const int4* tiles, int ntiles, const double* L, int hL, const double* R, int hR,
+                               int* flag);
 
 }  // namespace imsrg

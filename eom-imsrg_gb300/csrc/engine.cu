@@ -244,6 +244,7 @@ Ctx::~Ctx() {
     if (p) cudaFree(p);
   oz_release(pphh_oz);
   oz_release(wcc_oz);
+  gather_release();
   if (h_scalars) cudaFreeHost(h_scalars);
   quads_release();
   for (auto& m : prof_marks) cudaEventDestroy(m.second);
@@ -290,7 +291,7 @@ imsrg_status Ctx::c121(const double* Lp, int hL, const double* Rp, int hR, doubl
 
 imsrg_status Ctx::c122(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES) {
   if (L.n_unique == 0) return IMSRG_OK;
-  k_comm122<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, Lp, hL, Rp, hR, RES, hRES);
+  k_comm122<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, Lp, hL, Rp, hR, RES, hRES, nullptr);
   return launched("k_comm122");
 }
 
@@ -331,7 +332,8 @@ imsrg_status Ctx::pphh_accumulate(int hL, int hR, double* RES, const double* w1,
 
 
 
-imsrg_status Ctx::pphh(const double* Lp, int hL, const double* Rp, int hR, double* RES, double* w1, double* w2) {
+// W1, W2
+imsrg_status Ctx::pphh_products(const double* Lp, int hL, const double* Rp, int hR, double* w1, double* w2) {
   CK(pphh_clear(w1, w2));
   if (precision != IMSRG_PREC_FP64) {
     CK(tc_pphh(Lp, hL, Rp, hR, w1, w2));
@@ -343,6 +345,11 @@ imsrg_status Ctx::pphh(const double* Lp, int hL, const double* Rp, int hR, doubl
     CK(gemm_fp64(pphh_oz, pphh_probs, d_pphh_probs, d_pphh_tiles, (int)pphh_tiles.size(), ops));
   }
   mark(kPhasePphhGemm);
+  return IMSRG_OK;
+}
+
+imsrg_status Ctx::pphh(const double* Lp, int hL, const double* Rp, int hR, double* RES, double* w1, double* w2) {
+  CK(pphh_products(Lp, hL, Rp, hR, w1, w2));
   return pphh_accumulate(hL, hR, RES, w1, w2);
 }
 
@@ -358,7 +365,7 @@ imsrg_status Ctx::c221(int hL, int hR, double* RES, int hRES, const double* w1, 
   return launched("k_comm221");
 }
 
-imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, double* RES, int hRES, double* wcc) {
+imsrg_status Ctx::wcc_products(const double* lcc, int hL, const double* rcc, int hR, double* wcc) {
   // the piecewise entry point keeps the reference's FP64 WCC; the mixed-precision full
   // commutator (tc_commutator) uses the fused split-BF16 path instead
   if (!wcc_tiles.empty()) {
@@ -369,6 +376,11 @@ imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, doubl
     CK(gemm_fp64(wcc_oz, wcc_probs, d_wcc_probs, d_wcc_tiles, (int)wcc_tiles.size(), ops));
   }
   mark(kPhasePhGemm);
+  return IMSRG_OK;
+}
+
+imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, double* RES, int hRES, double* wcc) {
+  CK(wcc_products(lcc, hL, rcc, hR, wcc));
   if (L.n_unique == 0) return IMSRG_OK;
   k_comm222ph<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, wcc, hL, hR, RES, hRES);
   CK(launched("k_comm222ph"));
@@ -387,6 +399,33 @@ imsrg_status Ctx::commutator(const double* Lp, int hL, const double* Rp, int hR,
   CK(c111(Lp, hL, Rp, hR, RES));
   CK(c121(Lp, hL, Rp, hR, RES, hRES));
   mark(kPhaseOneBody);
+  if (L.slab >= kGatherMinSlab) CK(gather_prepare());
+  if (gp.state > 0 && gp.per_sm[1] > 0 && L.slab >= kGatherMinSlab) {
+    // 122 and the recoupling write the upper triangles only; the ladder update comes last (additions commute) and
+    // writes the lower triangles in the same pass
+    CK(c122_groups<double>(Lp, hL, Rp, hR, RES, hRES));
+    k_comm122<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, Lp, hL, Rp, hR, RES, hRES, gp.d_counter + 1);
+    CK(launched("k_comm122"));
+    mark(kPhase122);
+    CK(pphh_products(Lp, hL, Rp, hR, d_w1, d_w2));
+    CK(c221(hL, hR, RES, hRES, d_w1, d_w2));
+    mark(kPhase221);
+    CK(ensure_wcc());
+    CK(wcc_products(d_lcc, hL, d_rcc, hR, d_wcc));
+    const int64_t nq = (int64_t)gp.quads.size();
+    if (nq) {
+      launch_recouple_w((int)std::min<int64_t>((nq + 255) / 256, gp.num_sms * 32), stream, D, gp.d_quads, nq, gp.d_xcol, d_wcc,
+                        hL, hR, RES);
+      CK(launched("k_recouple_w"));
+    }
+    mark(kPhaseRecouple);
+    if (!upd_tiles.empty()) {
+      launch_pphh_update_mirror((int)upd_tiles.size(), stream, D, d_upd_tiles, RES, d_w1, d_w2, hL * hR, hRES);
+      CK(launched("k_pphh_update_mirror"));
+    }
+    mark(kPhasePphhUpdate);
+    return IMSRG_OK;
+  }
   CK(c122(Lp, hL, Rp, hR, RES, hRES));
   mark(kPhase122);
   CK(pphh(Lp, hL, Rp, hR, RES, d_w1, d_w2));

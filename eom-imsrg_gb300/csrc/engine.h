@@ -9,6 +9,7 @@
 
 #include "../../include/imsrg_gb300.h"
 #include "dev.cuh"
+#include "gather.h"
 #include "gemm.h"
 #include "gemm_oz.h"
 #include "layout.h"
@@ -51,6 +52,11 @@ enum Phase : int {
   kPhaseMirror = 11,
 };
 
+// From this size on the FP64 commutator takes 122 by pair groups and the recoupling by orbit quadruples; below it a thread
+// per element is as fast and the extra launches are not (122 and recoupling: eMax 4, 57 thousand elements, 24 + 24 us
+// against 32 + 29; eMax 5, 240 thousand, 61 + 37 us against 42 + 35; eMax 10 6.3 + 9.7 ms against 1.3 + 1.8).
+constexpr int64_t kGatherMinSlab = 100000;
+
 // the word of d_scalars (and of h_scalars) that holds the error of a bounded wait
 constexpr int kErrorSlot = 48;
 
@@ -90,6 +96,7 @@ struct Ctx {
   double *d_int1 = nullptr, *d_int2 = nullptr, *d_ad = nullptr;
   double* d_gen = nullptr;  // w2 generator workspace (3 slabs)
   imsrg::TcState* tc = nullptr;
+  imsrg::GatherPlan gp;  // gather kernels of the commutator (gather.cu)
   // FP64 products on the tensor cores (gemm_oz.cu): the digit plans of the ladder and of the cross-coupled products
   imsrg::OzPlan pphh_oz, wcc_oz;
   int oz_sms = 0;  // SMs of the device, once a plan is ready
@@ -129,6 +136,7 @@ struct Ctx {
   imsrg_status c121(const double* L, int hL, const double* R, int hR, double* RES, int hRES);
   imsrg_status c122(const double* L, int hL, const double* R, int hR, double* RES, int hRES);
   imsrg_status pphh(const double* L, int hL, const double* R, int hR, double* RES, double* w1, double* w2);
+  imsrg_status pphh_products(const double* L, int hL, const double* R, int hR, double* w1, double* w2);
   imsrg_status pphh_clear(double* w1, double* w2);
   imsrg_status pphh_accumulate(int hL, int hR, double* RES, const double* w1, const double* w2);
   imsrg_status c221(int hL, int hR, double* RES, int hRES, const double* w1, const double* w2);
@@ -136,6 +144,7 @@ struct Ctx {
   imsrg_status pphh_clear_f(float* w1, float* w2);
   imsrg_status c221_f(int hL, int hR, double* RES, int hRES, const float* w1, const float* w2);
   imsrg_status ensure_wcc();
+  imsrg_status wcc_products(const double* lcc, int hL, const double* rcc, int hR, double* wcc);
   imsrg_status ph(const double* lcc, int hL, const double* rcc, int hR, double* RES, int hRES, double* wcc);
   imsrg_status commutator(const double* L, int hL, const double* R, int hR, double* RES, int hRES, bool with_e0);
   imsrg_status axpby(const double* A, double ax, const double* B, double bx, double* C);
@@ -199,6 +208,13 @@ struct Ctx {
   imsrg_status hf_run(double* op, int herm, int mode, int max_iter, const double* coefs_in, double* coefs_out,
                       imsrg_hf_info* info);
 
+  // gather plan and commutator_122 by pair groups, gather.cu
+  imsrg_status gather_prepare();
+  void gather_release();
+  imsrg_status g122_set_caps(int tiny_cap, int small_cap);
+  template <typename T>
+  imsrg_status c122_groups(const double* L, int hL, const double* R, int hR, double* RES, int hRES);
+
   // grouped FP64 products, gemm_oz.cu
   imsrg_status oz_prepare(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs);
   void oz_release(imsrg::OzPlan& P);
@@ -223,7 +239,6 @@ struct Ctx {
   int tc_tile_k() const;      // K values per 128-byte tile row of the operand slices (64 BF16, 32 TF32)
   int tc_elem_bytes() const;  // bytes per operand value (2 BF16, 4 TF32)
   int tc_kind() const;        // operand type of the slices (0 BF16, 1 TF32)
-  imsrg_status tc_g122_partition(int tiny_cap, int small_cap);
   imsrg_status tc_set_tiles(const int* wmax, const bool* narrow, int order);
   imsrg_status tc_autotune(const double* L, int hL, const double* R, int hR, double* RES, imsrg_tune_info* info);
 };

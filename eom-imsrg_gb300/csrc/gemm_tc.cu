@@ -499,26 +499,12 @@ struct TcState {
   const int* d_cc_seg = nullptr;
   const int* d_swap_row = nullptr;
   float* zbuf = nullptr;  // X, the recoupling input (FP32, wcc layout)
-  // orbit quadruples (i<=j, k<=l) of the particle-hole recoupling, j fastest
-  std::vector<uint64_t> quads;
-  const uint64_t* d_quads = nullptr;
-  std::vector<int> xcol;              // X column offset of every pair and J' (recouple.cu)
   std::vector<unsigned> xmask;        // the X elements the recoupling reads (store masks, recouple.cu)
   const unsigned* d_xmask = nullptr;
-  const int* d_xcol = nullptr;
   int recouple_minb = 6;              // launch-bounds variant of k_recouple_q
   int recouple_ctas = 0;              // CTAs of k_recouple_q
   std::vector<SplitChunk> chunks;
   const SplitChunk* d_chunks = nullptr;
-  // commutator_122 by pair-group sub-blocks (comm122.cu): the plan, its launch order for the
-  // current caps (tc_g122_partition) and its device copies (tasks and runs sized for all tasks)
-  G122Plan g122;
-  G122Task* d_g122_tasks = nullptr;
-  int2* d_g122_items = nullptr;
-  const unsigned* d_g122_codes = nullptr;
-  int* d_g122_counter = nullptr;
-  PairGroupsDev g122_w{};
-  int g122_nspb = 0, g122_nblk2 = 0, g122_per_sm = 1;
   // tuned launch parameters (imsrg_autotune): GEMM tile order and shape
   int gemm_order = 0;  // 0: longest K first, 1: problem order
   // tile shape of each list: widest output tile (128 or 256 columns) and narrow last column
@@ -533,8 +519,6 @@ struct TcState {
   const TcProb* d_all_probs = nullptr;
   TcTile* d_tile_mem = nullptr;  // [pphh tiles | X tiles | merged tiles]
   size_t tile_cap_pphh = 0, tile_cap_z = 0, tile_cap_all = 0;
-  std::vector<int> g_start, g_n, g_orb, g_b1, g_b2, g_blk_off;
-  float2* g122_fb = nullptr;  // (fL, fR)(x, y) on every (l, j, tz) block
   int num_sms = 148;
 };
 
@@ -595,10 +579,6 @@ void Ctx::tc_release() {
   if (tc->buf) cudaFree(tc->buf);
   if (tc->d_mem) cudaFree(tc->d_mem);
   if (tc->zbuf) cudaFree(tc->zbuf);
-  if (tc->g122_fb) cudaFree(tc->g122_fb);
-  if (tc->d_g122_tasks) cudaFree(tc->d_g122_tasks);
-  if (tc->d_g122_items) cudaFree(tc->d_g122_items);
-  if (tc->d_g122_counter) cudaFree(tc->d_g122_counter);
   if (tc->d_tile_mem) cudaFree(tc->d_tile_mem);
   delete tc;
   tc = nullptr;
@@ -730,7 +710,8 @@ imsrg_status Ctx::tc_prepare(int mode) {
     tc->z_probs.push_back(p);
   }
   tc->total_tiles = tiles;
-  if (l.JM + 1 > 26) return fail(IMSRG_ERR_UNSUPPORTED, "mixed recoupling supports 2j <= 25 (eMax <= 12)");
+  CK_TC(gather_prepare());
+  if (gp.state < 0) return fail(IMSRG_ERR_UNSUPPORTED, gp.why);
   // ---- Pandya chunks: at most 1024 elements of one cross-coupled channel each (both operators)
   for (int q = 0; q < l.ncc; ++q) {
     const int64_t n = l.cc_off[q + 1] - l.cc_off[q];
@@ -741,59 +722,10 @@ imsrg_status Ctx::tc_prepare(int mode) {
     for (int64_t e0 = 0; e0 < n; e0 += 1024)
       tc->pandya_chunks.push_back(PandyaChunk{q, (int)e0, (int)std::min<int64_t>(1024, n - e0), m});
   }
-  // ---- commutator_122 tasks: the group pairs G1 <= G2 of each channel
-  {
-    PairGroups pg;
-    build_pair_groups(pg, l);
-    tc->g_start = pg.spb_start; tc->g_n = pg.spb_n; tc->g_orb = pg.spb_orb;
-    tc->g_b1 = pg.grp_b1; tc->g_b2 = pg.grp_b2; tc->g_blk_off = pg.blk_off;
-    tc->g122_nspb = pg.nspb;
-    tc->g122_nblk2 = pg.nblk2;
-    const std::string e = build_g122_plan(l, pg, tc->g122);
-    if (!e.empty()) return fail(IMSRG_ERR_UNSUPPORTED, e);
-  }
-  // ---- recoupling quadruples: bra (i<=j) of class c1, ket (k<=l) of class c2, with
-  //      c1 < c2, or c1 == c2 and (i,j) <= (k,l) (the unique stored elements), matching
-  //      2Tz and parity and sharing at least one J
-  {
-    const int N = l.N;
-    std::vector<std::vector<int>> by_tp(4);  // orbits grouped by (tz, l parity)
-    for (int o = 0; o < N; ++o) by_tp[((l.tz[o] + 1) / 2) * 2 + (l.ll[o] & 1)].push_back(o);
-    for (int i = 0; i < N; ++i)
-      for (int k = 0; k < N; ++k)
-        for (int ll2 = k; ll2 < N; ++ll2) {
-          const int tzj = l.tz[k] + l.tz[ll2] - l.tz[i];
-          if (tzj != -1 && tzj != 1) continue;
-          const int par = ((l.ll[k] + l.ll[ll2] - l.ll[i]) % 2 + 2) % 2;
-          const int c2 = l.con[k] + l.con[ll2];
-          const int kl_lo = std::abs(l.jj[k] - l.jj[ll2]), kl_hi = l.jj[k] + l.jj[ll2];
-          for (int j : by_tp[((tzj + 1) / 2) * 2 + par]) {
-            if (j < i) continue;
-            const int c1 = l.con[i] + l.con[j];
-            if (c1 > c2) continue;
-            if (c1 == c2 && (i > k || (i == k && j > ll2))) continue;
-            const int lo = std::max(std::abs(l.jj[i] - l.jj[j]), kl_lo), hi = std::min(l.jj[i] + l.jj[j], kl_hi);
-            if (lo > hi) continue;
-            tc->quads.push_back((uint64_t)i | ((uint64_t)j << 16) | ((uint64_t)k << 32) | ((uint64_t)ll2 << 48));
-          }
-        }
-    // within the quadruples of one orbit i, by (jj, jk, jl): neighbouring threads then share their J and J' ranges and
-    // 6j rows, so a warp's loops run with its lanes in step (the X rows read for one i are the same in any order)
-    auto shape = [&](uint64_t qd) {
-      return (l.jj[(qd >> 16) & 0xFFFF] * 64 + l.jj[(qd >> 32) & 0xFFFF]) * 64 + l.jj[(qd >> 48) & 0xFFFF];
-    };
-    for (size_t a = 0; a < tc->quads.size();) {
-      size_t b = a;
-      while (b < tc->quads.size() && (tc->quads[b] & 0xFFFF) == (tc->quads[a] & 0xFFFF)) ++b;
-      std::stable_sort(tc->quads.begin() + a, tc->quads.begin() + b,
-                       [&](uint64_t x, uint64_t y) { return shape(x) < shape(y); });
-      a = b;
-    }
-  }
   // X stores only where the recoupling reads: the masks of the 32-row column segments
   {
     std::vector<int> moff;
-    tc->xmask = build_x_read_mask(l, tc->quads, moff);
+    tc->xmask = build_x_read_mask(l, gp.quads, moff);
     for (TcProb& p : tc->z_probs)
       for (int q = 0; q < l.ncc; ++q)
         if (l.cc_rlen[q] == p.M && l.wcc_off[q] == p.c_off && moff[q] >= 0) p.xmask = moff[q] + 1;
@@ -807,7 +739,6 @@ imsrg_status Ctx::tc_prepare(int mode) {
   CK_TC(cuda(cudaMemset(tc->buf, 0, std::max<size_t>(bytes, 256)), "memset(tc operands)"));
   CK_TC(cuda(cudaMalloc(&tc->zbuf, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(X)"));
   CK_TC(cuda(cudaMemset(tc->zbuf, 0, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "memset(X)"));
-  CK_TC(cuda(cudaMalloc(&tc->g122_fb, sizeof(float2) * std::max(tc->g122_nblk2, 1)), "cudaMalloc(122 blocks)"));
   DevPacker pk;
   pk.add(tc->split_ops, &tc->d_split_ops);
   pk.add(tc->split_prefix, &tc->d_split_prefix);
@@ -824,29 +755,12 @@ imsrg_status Ctx::tc_prepare(int mode) {
   pk.add(tc->cc_nkb, &tc->d_cc_nkb);
   pk.add(tc->cc_seg, &tc->d_cc_seg);
   pk.add(tc->swap_row, &tc->d_swap_row);
-  pk.add(tc->quads, &tc->d_quads);
-  tc->xcol = build_xcol(l);
-  pk.add(tc->xcol, &tc->d_xcol);
   pk.add(tc->xmask, &tc->d_xmask);
   pk.add(tc->chunks, &tc->d_chunks);
-  pk.add(tc->g_start, &tc->g122_w.spb_start);
-  pk.add(tc->g_n, &tc->g122_w.spb_n);
-  pk.add(tc->g_orb, &tc->g122_w.spb_orb);
-  pk.add(tc->g_b1, &tc->g122_w.grp_b1);
-  pk.add(tc->g_b2, &tc->g122_w.grp_b2);
-  pk.add(tc->g_blk_off, &tc->g122_w.blk_off);
-  pk.add(tc->g122.codes, &tc->d_g122_codes);
 
   CK_TC(cuda(cudaMalloc(&tc->d_mem, pk.buf.size()), "cudaMalloc(tc tables)"));
   CK_TC(cuda(cudaMemcpy(tc->d_mem, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tc tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(tc->d_mem) + f.first;
-  CK_TC(cuda(cudaMalloc(&tc->d_g122_tasks, sizeof(G122Task) * std::max<size_t>(tc->g122.all.size(), 1)),
-             "cudaMalloc(122 tasks)"));
-  CK_TC(cuda(cudaMalloc(&tc->d_g122_items, sizeof(int2) * std::max<size_t>(tc->g122.all.size(), 1)),
-             "cudaMalloc(122 runs)"));
-  CK_TC(cuda(cudaMalloc(&tc->d_g122_counter, sizeof(int)), "cudaMalloc(122 counter)"));
-  CK_TC(cuda(cudaMemset(tc->d_g122_counter, 0, sizeof(int)), "cudaMemset(122 counter)"));
-  CK_TC(tc_g122_partition(tc->g122.tiny_cap, tc->g122.warp_cap));
   tc->recouple_ctas = tc->num_sms * 32;
   // tile lists: the most tiles come with 128-wide tiles
   tc->tile_cap_pphh = make_tiles(tc->pphh_probs, 128, false).size();
@@ -1040,17 +954,7 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
   CK_TC(c121(Lp, hL, Rp, hR, RES, hRES));
   mark(kPhaseOneBody);
   if (L.n_unique) {
-    k_comm122_fb2<<<tc->g122_nspb, 64, 0, stream>>>(D, tc->g122_w, tc->g122_nspb, Lp, hL, Rp, hR, tc->g122_fb,
-                                                     tc->d_g122_counter);
-    CK_TC(launched("k_comm122_fb2"));
-    const G122Plan& P = tc->g122;
-    // the big tasks, then enough eight-warp CTAs to fill the GPU at the occupancy the shared
-    // memory allows (the warps take the runs from the counter)
-    const int grid = P.nbig + tc->num_sms * std::max(1, tc->g122_per_sm);
-    launch_comm122(grid, P.smem_bytes, stream, D, tc->d_g122_tasks, tc->d_g122_items, (int)P.items.size(), P.nbig,
-                   tc->d_g122_counter, tc->d_g122_codes, std::max(P.warp_cap, 4 * P.tiny_cap), P.tiny_cap, Lp, hL,
-                   Rp, hR, RES, hRES, tc->g122_fb);
-    CK_TC(launched("k_comm122_sub"));
+    CK_TC(c122_groups<float>(Lp, hL, Rp, hR, RES, hRES));
   }
   mark(kPhase122);
   if (!tc->small_tiles.empty()) {  // the K = nhh products (W2) on FP32 SIMT
@@ -1068,49 +972,24 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
     CK_TC(tc_gemm(tc->d_z_probs, tc->d_z_tiles, (int)tc->z_tiles.size(), gout, hL, hR, tc->wmax[1]));
     mark(kPhasePhGemm);
   }
-  if (!tc->quads.empty()) {
-    const int64_t nq = (int64_t)tc->quads.size();
+  if (!gp.quads.empty()) {
+    const int64_t nq = (int64_t)gp.quads.size();
     const int grid = (int)std::min<int64_t>((nq + 255) / 256, tc->recouple_ctas);
-    launch_recouple_q(tc->recouple_minb, grid, stream, D, tc->d_quads, nq, tc->d_xcol, tc->zbuf, RES);
+    launch_recouple_q(tc->recouple_minb, grid, stream, D, gp.d_quads, nq, gp.d_xcol, tc->zbuf, RES);
     CK_TC(launched("k_recouple_q"));
   }
   mark(kPhaseRecouple);
   // the ladder's contribution last (additions commute), with the lower triangles of the square
   // arrays written from the updated upper ones in the same pass
   if (!upd_tiles.empty()) {
-    k_pphh_update_mirror_f<<<(int)upd_tiles.size(), 256, 0, stream>>>(D, d_upd_tiles, RES, w1f, w2f,
-                                                                     (float)(hL * hR), hRES);
-    CK_TC(launched("k_pphh_update_mirror_f"));
+    launch_pphh_update_mirror((int)upd_tiles.size(), stream, D, d_upd_tiles, RES, w1f, w2f, hL * hR, hRES);
+    CK_TC(launched("k_pphh_update_mirror"));
   }
   mark(kPhasePphhUpdate);
   return IMSRG_OK;
 }
 
 // ---------------------------------------------------------------- autotuner
-// Splits the 122 tasks into [tiny | warp | cta] runs by size, keeping channel order inside
-// each run, and uploads the list.  The caps must keep the per-CTA shared memory of the
-// 8-lane and warp kernels within the 48 KiB default.
-imsrg_status Ctx::tc_g122_partition(int tiny_cap, int small_cap) {
-  G122Plan& P = tc->g122;
-  const int bt = P.tiny_cap, bw = P.warp_cap;
-  const std::string e = g122_partition(P, tiny_cap, small_cap);
-  if (!e.empty()) {
-    g122_partition(P, bt, bw);  // keep the previous caps
-    return fail(IMSRG_ERR_INVALID_ARGUMENT, e);
-  }
-  if (!P.tasks.empty()) {
-    CK_TC(cuda(cudaMemcpyAsync(tc->d_g122_tasks, P.tasks.data(), sizeof(G122Task) * P.tasks.size(),
-                               cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(122 tasks)"));
-    if (!P.items.empty())
-      CK_TC(cuda(cudaMemcpyAsync(tc->d_g122_items, P.items.data(), sizeof(int2) * P.items.size(),
-                                 cudaMemcpyHostToDevice, stream), "cudaMemcpyAsync(122 runs)"));
-    CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(122 tasks)"));
-  }
-  CK_TC(cuda(g122_smem_attr(P.smem_bytes), "smem attr (122)"));
-  CK_TC(cuda(g122_blocks_per_sm(P.smem_bytes, &tc->g122_per_sm), "occupancy (122)"));
-  return IMSRG_OK;
-}
-
 // Tile lists of the persistent GEMMs for their tile shapes and an order: per list ([0] ladder,
 // [1] X, [2] the merged list) the widest tile wmax (128, or 256 with two slices) and narrow last
 // column tiles or not; order 0 = longest K first (LPT), 1 = problem order.  No output element
@@ -1178,14 +1057,14 @@ imsrg_status Ctx::tc_autotune(const double* Lp, int hL, const double* Rp, int hR
     best = base;
     // 122 caps
     static const int caps[][2] = {{32, 256}, {64, 256}, {32, 512}, {64, 512}, {64, 1024}};
-    int bt = tc->g122.tiny_cap, bs = tc->g122.warp_cap;
+    int bt = gp.g122.tiny_cap, bs = gp.g122.warp_cap;
     for (const auto& c : caps) {
-      if ((st = tc_g122_partition(c[0], c[1])) != IMSRG_OK) break;
+      if ((st = g122_set_caps(c[0], c[1])) != IMSRG_OK) break;
       float ms;
       if ((st = time_one(&ms)) != IMSRG_OK) break;
       if (ms < best) { best = ms; bt = c[0]; bs = c[1]; }
     }
-    if (st != IMSRG_OK || (st = tc_g122_partition(bt, bs)) != IMSRG_OK) break;
+    if (st != IMSRG_OK || (st = g122_set_caps(bt, bs)) != IMSRG_OK) break;
     // recoupling: the launch-bounds variant and the CTA count (no output depends on them)
     {
       int bm = tc->recouple_minb, bc = tc->recouple_ctas;
@@ -1248,8 +1127,8 @@ imsrg_status Ctx::tc_autotune(const double* Lp, int hL, const double* Rp, int hR
     float after = 0.0f;
     if ((st = time_one(&after)) != IMSRG_OK) break;
     if (info) {
-      info->tiny_cap = tc->g122.tiny_cap;
-      info->small_cap = tc->g122.warp_cap;
+      info->tiny_cap = gp.g122.tiny_cap;
+      info->small_cap = gp.g122.warp_cap;
       info->recouple_kind = 1;
       info->recouple_min_blocks = tc->recouple_minb;
       info->recouple_ctas = tc->recouple_ctas;
@@ -1278,7 +1157,7 @@ extern "C" imsrg_status imsrg_recouple_traffic(imsrg_ctx* ctx, int64_t* x_reads,
   if (c->precision == IMSRG_PREC_FP64) return c->fail(IMSRG_ERR_UNSUPPORTED, "the recoupling kernel runs in the mixed modes");
   if (cudaSetDevice(c->device) != cudaSuccess) return c->fail(IMSRG_ERR_CUDA, "cudaSetDevice");
   CK_TC(c->tc_prepare(c->precision));
-  const RecoupleTraffic t = recouple_traffic(c->L, c->tc->quads);
+  const RecoupleTraffic t = recouple_traffic(c->L, c->gp.quads);
   *x_reads = t.x_reads;
   *x_distinct = t.x_distinct;
   *res_elems = t.res_elems;
@@ -1298,7 +1177,7 @@ extern "C" imsrg_status imsrg_set_tuning(imsrg_ctx* ctx, const imsrg_tune_info* 
     return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "imsrg_set_tuning: value out of range");
   CK_TC(c->ensure_workspace());
   CK_TC(c->tc_prepare(c->precision));
-  CK_TC(c->tc_g122_partition(cfg->tiny_cap, cfg->small_cap));
+  CK_TC(c->g122_set_caps(cfg->tiny_cap, cfg->small_cap));
   {
     const bool m = cfg->gemm_merged != 0;
     const int wx = cfg->gemm_wmax_x ? cfg->gemm_wmax_x : cfg->gemm_wmax;

@@ -12,7 +12,9 @@
 namespace imsrg {
 
 __global__ void k_pandya(DevLayout D, const double* op, int herm, double* cc);
-__global__ void k_comm122(DevLayout D, const double* L, int hL, const double* R, int hR, double* RES, int hRES);
+// run_if: with a flag, nothing is done unless it is set
+__global__ void k_comm122(DevLayout D, const double* L, int hL, const double* R, int hR, double* RES, int hRES,
+                          const int* run_if);
 __global__ void k_pphh_update(DevLayout D, double* RES, const double* w1, const double* w2, double pm);
 __global__ void k_comm222ph(DevLayout D, const double* WCC, int hL, int hR, double* RES, int hRES);
 __global__ void k_comm111(DevLayout D, const double* L, int hL, const double* R, int hR, double* RES);
@@ -50,7 +52,10 @@ __global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, int nt
 // mixed-precision companions (kernels_mixed.cu)
 void launch_pandya_tc(int S, int kind, int nchunks, cudaStream_t stream, const DevLayout& D, const PandyaChunk* chunks,
                       const PandyaOps& ops, void* buf, int64_t slice_elems, const int* swap_row);
-__global__ void k_pphh_update_mirror_f(DevLayout D, const int4* tiles, double* RES, const float* w1, const float* w2,
-                                       float pm, int herm);
+// the ladder update with the mirror of the square arrays' lower triangles, last in a commutator
+void launch_pphh_update_mirror(int ntiles, cudaStream_t st, const DevLayout& D, const int4* tiles, double* RES,
+                               const float* w1, const float* w2, int pm, int herm);
+void launch_pphh_update_mirror(int ntiles, cudaStream_t st, const DevLayout& D, const int4* tiles, double* RES,
+                               const double* w1, const double* w2, int pm, int herm);
 
 }  // namespace imsrg

@@ -42,7 +42,8 @@ __global__ void k_pandya(DevLayout D, const double* __restrict__ op, int herm, d
 // ---------------------------------------------------------------- commutator_122
 // src/commutators.f90:283-396 -- ASSIGNS every 2b element of RES.
 __global__ void k_comm122(DevLayout D, const double* __restrict__ L, int hL, const double* __restrict__ R, int hR,
-                          double* __restrict__ RES, int hRES) {
+                          double* __restrict__ RES, int hRES, const int* __restrict__ run_if) {
+  if (run_if && !*run_if) return;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < D.n_unique; u += (int64_t)gridDim.x * blockDim.x) {
     int q, g, IX, JX;
     d_unique_decode(D, u, q, g, IX, JX);

@@ -201,15 +201,21 @@ __global__ void k_comm111f(DevLayout D, const double* __restrict__ L, int hL, co
 
 // lower triangle of every square array (pppp, phph, hhhh) = herm * upper triangle
 // The ladder update and the mirror pass in one: RES += W1 - W2 on the rectangular arrays and,
-// on the square arrays, RES(i, j) += W(i, j) - pm W(j, i) for i <= j (W = W1 - W2, FP32) with
+// on the square arrays, RES(i, j) += W(i, j) - pm W(j, i) for i <= j (W = W1 - W2, FP32 or FP64) with
 // the lower triangle then written from the updated upper one, RES(j, i) = herm RES(i, j).  It
 // runs after every other contribution to RES's two-body part (122 assigns it, the recoupling
 // adds to the upper triangles; additions commute), so RES's upper triangles are read once.
-__global__ void __launch_bounds__(256) k_pphh_update_mirror_f(DevLayout D, const int4* __restrict__ tiles,
-                                                              double* __restrict__ RES, const float* __restrict__ w1,
-                                                              const float* __restrict__ w2, float pm, int herm) {
-  __shared__ float Xa[32][33];
-  __shared__ float Xb[32][33];
+template <typename T>
+__device__ __forceinline__ double to_f64(T x) {
+  if constexpr (sizeof(T) == 4) return f32_to_f64(x);
+  else return x;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_pphh_update_mirror(DevLayout D, const int4* __restrict__ tiles,
+                                                            double* __restrict__ RES, const T* __restrict__ w1,
+                                                            const T* __restrict__ w2, T pm, int herm) {
+  __shared__ T Xa[32][33];
+  __shared__ T Xb[32][33];
   __shared__ double V[32][33];
   const int4 t = tiles[blockIdx.x];
   const int k = t.x, i0 = t.y, j0 = t.z;
@@ -221,24 +227,25 @@ __global__ void __launch_bounds__(256) k_pphh_update_mirror_f(DevLayout D, const
       const int i = i0 + tx, j = j0 + r;
       if (i < n1 && j < n2) {
         const int64_t e = base + i + (int64_t)j * n1;
-        RES[e] += f32_to_f64(w1[e] - w2[e]);
+        RES[e] += to_f64<T>(w1[e] - w2[e]);
       }
     }
     return;
   }
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + tx, j = j0 + r;
-    Xa[r][tx] = (i < n1 && j < n1) ? w1[base + i + (int64_t)j * n1] - w2[base + i + (int64_t)j * n1] : 0.0f;
+    Xa[r][tx] = (i < n1 && j < n1) ? w1[base + i + (int64_t)j * n1] - w2[base + i + (int64_t)j * n1] : (T)0;
     const int ib = j0 + tx, jb = i0 + r;
-    Xb[r][tx] = (ib < n1 && jb < n1) ? w1[base + ib + (int64_t)jb * n1] - w2[base + ib + (int64_t)jb * n1] : 0.0f;
+    Xb[r][tx] = (ib < n1 && jb < n1) ? w1[base + ib + (int64_t)jb * n1] - w2[base + ib + (int64_t)jb * n1] : (T)0;
   }
   __syncthreads();
   for (int r = ty; r < 32; r += 8) {
     const int i = i0 + tx, j = j0 + r;
     if (i < n1 && j < n1 && i <= j) {
       const int64_t e = base + i + (int64_t)j * n1;
-      const double v = RES[e] + f32_to_f64(Xa[r][tx] - Xb[tx][r] * pm);
-      RES[e] = v;
+      const double v = RES[e] + to_f64<T>(Xa[r][tx] - Xb[tx][r] * pm);
+      // FP64: the reference's sign flip of the diagonal (RES(IX,IX) = RES*herm, src/commutators.f90:914)
+      RES[e] = (sizeof(T) == 8 && i == j && herm < 0) ? -v : v;
       V[r][tx] = v;
     }
   }
@@ -252,5 +259,14 @@ __global__ void __launch_bounds__(256) k_pphh_update_mirror_f(DevLayout D, const
   }
 }
 
+
+void launch_pphh_update_mirror(int ntiles, cudaStream_t st, const DevLayout& D, const int4* tiles, double* RES,
+                               const float* w1, const float* w2, int pm, int herm) {
+  k_pphh_update_mirror<float><<<ntiles, 256, 0, st>>>(D, tiles, RES, w1, w2, (float)pm, herm);
+}
+void launch_pphh_update_mirror(int ntiles, cudaStream_t st, const DevLayout& D, const int4* tiles, double* RES,
+                               const double* w1, const double* w2, int pm, int herm) {
+  k_pphh_update_mirror<double><<<ntiles, 256, 0, st>>>(D, tiles, RES, w1, w2, (double)pm, herm);
+}
 
 }  // namespace imsrg

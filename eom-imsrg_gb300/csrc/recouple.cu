@@ -1,4 +1,4 @@
-// commutator_222_ph recoupling (src/commutators.f90:804-921) of the mixed-precision path.
+// commutator_222_ph recoupling (src/commutators.f90:804-921), one thread per orbit quadruple.
 //
 // The reference gathers, for every stored element (ij, kl; J) and every J' shared by the
 // pairs, four cross-coupled products W_{gik,rjl} etc. and sums them with 6j symbols.  Here
@@ -92,6 +92,75 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_recouple_q(DevLayout D, con
   }
 }
 
+__device__ __forceinline__ double d_flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+
+// The FP64 form, on the reference's products W = LCC RCC^T: the four W elements of each J' are folded as they are read,
+//   zd(J') = Z[(k,i),(j,l)] + phase Z[(l,j),(i,k)],  Z(r, c) = hL W(r, c) - hR W(c, r),  phase = (-1)^((ji+jj+jk+jl)/2),
+// (exchange: k and l swapped), signs by integer instructions.  Bound by the W sectors it touches (four scattered reads of
+// 8 bytes for each J').
+__global__ void __launch_bounds__(256, 3) k_recouple_w(DevLayout D, const uint64_t* __restrict__ quads, int64_t nquads,
+                                                       const int* __restrict__ xcol, const double* __restrict__ W, int hL,
+                                                       int hR, double* __restrict__ RES) {
+  const int N = D.N, NJ = D.NJ;
+  const bool nL = hL < 0, nR = hR > 0;  // the signs of the hL and of the -hR terms
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nquads;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t qd = quads[t];
+    const int i = (int)(qd & 0xFFFF), j = (int)((qd >> 16) & 0xFFFF), k = (int)((qd >> 32) & 0xFFFF),
+              l = (int)((qd >> 48) & 0xFFFF);
+    const int ji = D.jj[i], jj = D.jj[j], jk = D.jj[k], jl = D.jj[l];
+    const bool ph = ((ji + jj + jk + jl) >> 1) & 1;
+    const int dlo = max(abs(jj - jl), abs(ji - jk)), dhi = min(jj + jl, ji + jk);
+    const int elo = max(abs(ji - jl), abs(jj - jk)), ehi = min(ji + jl, jj + jk);
+    const int nd = (dhi - dlo) / 2 + 1, ne = (ehi - elo) / 2 + 1;
+    double zd[kRcMaxJp], ze[kRcMaxJp];
+    for (int term = 0; term < 2; ++term) {  // columns of (i, x) and rows of (y, j): direct x = k, y = l
+      const int x = term ? l : k, y = term ? k : l, lo = term ? elo : dlo, n = term ? ne : nd;
+      double* z = term ? ze : zd;
+      const int* cix = xcol + (i * N + x) * NJ;
+      const int* cxi = xcol + (x * N + i) * NJ;
+      const int* cjy = xcol + (j * N + y) * NJ;
+      const int* cyj = xcol + (y * N + j) * NJ;
+      const int* ryj = D.ccr_t + y * NJ * N + j;
+      const int* rix = D.ccr_t + i * NJ * N + x;
+      const int* rxi = D.ccr + (x * N + i) * NJ;
+      const int* rjy = D.ccr + (j * N + y) * NJ;
+      for (int m = 0; m < n; ++m) {
+        const int h = (lo >> 1) + m;
+        const double w1 = __ldg(W + cjy[h] + rxi[h]), w2 = __ldg(W + cix[h] + __ldg(ryj + h * N));
+        const double w3 = __ldg(W + cyj[h] + __ldg(rix + h * N)), w4 = __ldg(W + cxi[h] + rjy[h]);
+        z[m] = (d_flip(w1, nL) + d_flip(w2, nL != ph)) + (d_flip(w3, nR != ph) + d_flip(w4, nR));
+      }
+    }
+    const int nh = D.sj_nh;
+    const int kd = (((ji >> 1) * nh + (jj >> 1)) * nh + (jl >> 1)) * nh + (jk >> 1);
+    const int ke = (((ji >> 1) * nh + (jj >> 1)) * nh + (jk >> 1)) * nh + (jl >> 1);
+    const double* sjd = D.sj_val + D.sj_off[kd];
+    const double* sje = D.sj_val + D.sj_off[ke];
+    const int d3 = D.sj_j3min[kd], d6 = D.sj_j6min[kd], dn6 = D.sj_n6[kd];
+    const int e3 = D.sj_j3min[ke], e6 = D.sj_j6min[ke], en6 = D.sj_n6[ke];
+    const int C1 = D.con[i] + D.con[j], C2 = D.con[k] + D.con[l];
+    const int g = (C1 == 0) ? C2 : (C1 == 1 ? (C2 == 1 ? 3 : 5) : 4);
+    const int T = D.tz[i] + D.tz[j], P = (D.ll[i] + D.ll[j]) & 1;
+    const int Jlo = max(abs(ji - jj), abs(jk - jl)), Jhi = min(ji + jj, jk + jl);
+    for (int J = Jlo; J <= Jhi; J += 2) {
+      const double* rd = sjd + ((J - d3) >> 1) * dn6 + ((dlo - d6) >> 1);
+      const double* re = sje + ((J - e3) >> 1) * en6 + ((elo - e6) >> 1);
+      double sd = 0.0, se = 0.0;
+      for (int m = 0; m < nd; ++m) sd = fma(__ldg(rd + m), zd[m], sd);
+      for (int m = 0; m < ne; ++m) se = fma(__ldg(re + m), ze[m], se);
+      double sm = d_flip(sd, !((jl + jk + J) & 2)) + se;  // -(-1)^((jl+jk+J)/2) of the direct term
+      if (i == j) sm *= .70710678118;  // literal of src/commutators.f90:834
+      if (k == l) sm *= .70710678118;
+      const int kk = (3 * J + (T + 2) + P) * 6 + g;
+      const int IX = D.pairpos_t[(i * NJ + (J >> 1)) * N + j], JX = D.pairpos[(k * N + l) * NJ + (J >> 1)];
+      atomicAdd(RES + D.goff[kk] + IX + (int64_t)JX * D.gn1[kk], sm);
+    }
+  }
+}
+
 }  // namespace
 
 void launch_recouple_q(int min_blocks, int grid, cudaStream_t st, const DevLayout& D, const uint64_t* quads,
@@ -102,6 +171,11 @@ void launch_recouple_q(int min_blocks, int grid, cudaStream_t st, const DevLayou
     case 8: k_recouple_q<8><<<grid, 256, 0, st>>>(D, quads, nquads, xcol, X, RES); break;
     default: k_recouple_q<4><<<grid, 256, 0, st>>>(D, quads, nquads, xcol, X, RES); break;
   }
+}
+
+void launch_recouple_w(int grid, cudaStream_t st, const DevLayout& D, const uint64_t* quads, int64_t nquads, const int* xcol,
+                       const double* W, int hL, int hR, double* RES) {
+  if (nquads > 0) k_recouple_w<<<grid, 256, 0, st>>>(D, quads, nquads, xcol, W, hL, hR, RES);
 }
 
 std::vector<int> build_xcol(const Layout& L) {

@@ -1,4 +1,4 @@
-// Particle-hole recoupling of the mixed path (recouple.cu).
+// Particle-hole recoupling by orbit quadruples (recouple.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,5 +30,9 @@ RecoupleTraffic recouple_traffic(const Layout& L, const std::vector<uint64_t>& q
 // one thread per quadruple; min_blocks 4, 6 or 8 (launch-bounds variants)
 void launch_recouple_q(int min_blocks, int grid, cudaStream_t st, const DevLayout& D, const uint64_t* quads,
                        int64_t nquads, const int* xcol, const float* X, double* RES);
+
+// the FP64 form on the products W
+void launch_recouple_w(int grid, cudaStream_t st, const DevLayout& D, const uint64_t* quads, int64_t nquads, const int* xcol,
+                       const double* W, int hL, int hR, double* RES);
 
 }  // namespace imsrg
