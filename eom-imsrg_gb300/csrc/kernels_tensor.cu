@@ -45,6 +45,21 @@ __device__ double d_nine(const DevTLayout& T, int a, int b, int J1, int c, int d
   return sm;
 }
 
+// the same times sqrt((J1+1)(J2+1)(J3+1)(J4+1)), for |J1 - J2| <= rank, |J3 - J4| <= rank and the triads (a b J1), (a c J3)
+__device__ __forceinline__ double d_nine_n(const DevTLayout& T, int a, int b, int J1, int c, int d, int J2, int J3, int J4) {
+  const int nh = T.six_nh, rank = T.rank;
+  if (T.nine) {
+    const int64_t o = T.nine_off[(((a >> 1) * nh + (b >> 1)) * nh + (c >> 1)) * nh + (d >> 1)];
+    const int i1 = (J1 - abs(a - b)) >> 1, i3 = (J3 - abs(a - c)) >> 1;
+    return __ldg(T.nine + o + ((int64_t)(i1 * (rank + 1) + ((J2 - J1 + rank) >> 1)) * (min(a, c) + 1) + i3) * (rank + 1) +
+                 ((J4 - J3 + rank) >> 1));
+  }
+  return d_nine(T, a, b, J1, c, d, J2, J3, J4) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * (T.sq[J3 >> 1] * T.sq[J4 >> 1]);
+}
+__device__ __forceinline__ double d_flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+
 __device__ __forceinline__ int d_tg(int c1, int c2) {
   // (bra class, ket class) -> tgam index: pp-pp 0 pp-ph 1 pp-hh 2 ph-ph 3 hh-hh 4 ph-hh 5 hh-pp 6 ph-pp 7 hh-ph 8
   return c1 == 0 ? c2 : (c1 == 1 ? (c2 == 0 ? 7 : (c2 == 1 ? 3 : 5)) : (c2 == 0 ? 6 : (c2 == 1 ? 8 : 4)));
@@ -231,11 +246,11 @@ __global__ void k_ts121(DevLayout D, DevTLayout T, const double* __restrict__ L,
     double smx = 0.0, smy = 0.0;
     for (int J2 = abs(ji - jq); J2 <= ji + jq; J2 += 2)
       for (int J1 = abs(ja - jp); J1 <= ja + jp; J1 += 2)
-        smx += d_telem(D, T, R, hR, ak, pk, ik, qk, J1, J2) * sqrt((J1 + 1.0) * (J2 + 1.0)) * d_sgn(J1 >> 1) *
+        smx += d_telem(D, T, R, hR, ak, pk, ik, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * d_sgn(J1 >> 1) *
                d_six_t(T, J1, J2, jq, jp, ji);
     for (int J1 = abs(ji - jp); J1 <= ji + jp; J1 += 2)
       for (int J2 = abs(ja - jq); J2 <= ja + jq; J2 += 2)
-        smy += d_telem(D, T, R, hR, ik, pk, ak, qk, J1, J2) * sqrt((J1 + 1.0) * (J2 + 1.0)) * d_sgn(J1 >> 1) *
+        smy += d_telem(D, T, R, hR, ik, pk, ak, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * d_sgn(J1 >> 1) *
                d_six_t(T, J1, J2, jq, jp, ji);
     sm += L[D.off_fph + a + (int64_t)i * D.P] * (hL * smx - smy) * d_sgn((rank + jq + ji) >> 1);
   }
@@ -280,30 +295,34 @@ __global__ void k_ts211(DevLayout D, DevTLayout T, const double* __restrict__ LC
 }
 
 // ---------------------------------------------------------------- TS_commutator_221
-// src/TS_commutators.f90:809-1067: one-body traces of the tensor intermediates w1 (hole c), w2 (particle c)
-__global__ void k_ts221(DevLayout D, DevTLayout T, const double* __restrict__ w1, const double* __restrict__ w2,
-                        int pm, double* __restrict__ RES, int hRES) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+// src/TS_commutators.f90:809-1067: one-body traces of the tensor intermediates w1 (hole c), w2 (particle c).  A CTA per
+// output, threads over (c, J1): a warp per output with a lane per c took 0.40 ms at eMax 6, rank 2.
+__global__ void __launch_bounds__(256) k_ts221(DevLayout D, DevTLayout T, const double* __restrict__ w1,
+                                               const double* __restrict__ w2, int pm, double* __restrict__ RES, int hRES) {
+  __shared__ double red[8];
+  const int w = blockIdx.x, lane = threadIdx.x & 31;
   if (w >= T.n_ob) return;
   const int kind = T.ob_kind[w], p = T.ob_p[w], q = T.ob_q[w], ik = T.ob_pk[w], jk = T.ob_qk[w];
   const int ji = D.jj[ik], jj = D.jj[jk], rank = T.rank;
   double sm = 0.0;
-  for (int c = lane; c < D.N; c += 32) {
+  for (int t = threadIdx.x; t < D.N * D.NJ; t += blockDim.x) {
+    const int c = t % D.N, jc = D.jj[c], J1 = abs(jc - ji) + 2 * (t / D.N);
+    if (J1 > jc + ji) continue;
     const double* wx = D.con[c] ? w1 : w2;
-    const int jc = D.jj[c];
     double s = 0.0;
-    for (int J1 = abs(jc - ji); J1 <= jc + ji; J1 += 2) {
-      for (int J2 = abs(jc - jj); J2 <= min(J1 - 2, jc + jj); J2 += 2)
-        s -= sqrt((J1 + 1.0) * (J2 + 1.0)) * d_six_t(T, J1, J2, jj, ji, jc) *
-             d_telem(D, T, wx, 1, c, jk, c, ik, J2, J1) * d_sgn(J2 >> 1) * pm;
-      for (int J2 = max(J1, abs(jc - jj)); J2 <= jc + jj; J2 += 2)
-        s += sqrt((J1 + 1.0) * (J2 + 1.0)) * d_six_t(T, J1, J2, jj, ji, jc) *
-             d_telem(D, T, wx, 1, c, ik, c, jk, J1, J2) * d_sgn(J1 >> 1);
+    for (int J2 = max(abs(jc - jj), J1 - rank); J2 <= min(J1 + rank, jc + jj); J2 += 2) {
+      const double v = J2 < J1 ? d_telem(D, T, wx, 1, c, jk, c, ik, J2, J1) * -pm : d_telem(D, T, wx, 1, c, ik, c, jk, J1, J2);
+      s = fma(T.sq[J2 >> 1] * d_six_t(T, J1, J2, jj, ji, jc), d_flip(v, (min(J1, J2) >> 1) & 1), s);
     }
-    sm += s * d_sgn((jc + jj) >> 1);
+    sm += d_flip(s * T.sq[J1 >> 1], ((jc + jj) >> 1) & 1);
   }
   sm = wsum(sm);
-  if (lane == 0) tob_acc(D, T, RES, hRES, kind, p, q, ik, jk, sm * d_sgn(rank >> 1));
+  if (lane == 0) red[threadIdx.x >> 5] = sm;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) sm += red[k];
+    tob_acc(D, T, RES, hRES, kind, p, q, ik, jk, sm * d_sgn(rank >> 1));
+  }
 }
 
 // ---------------------------------------------------------------- TS_commutator_122 / 212
@@ -399,7 +418,7 @@ namespace {
 // one element of the tensor Pandya transform (rows (a, b) / ph columns (p, h) as k_tpandya
 // reads them); exc: zero unless the tensor element read is (pp,hh) or (hh,pp)
 __device__ __forceinline__ double tpandya_at(const DevLayout& D, const DevTLayout& T, const double* __restrict__ R,
-                                             int hR, int J3, int J4, int term, int a, int b, int p, int h, double norm,
+                                             int hR, int J3, int J4, int term, int a, int b, int p, int h, double scale,
                                              int exc) {
   const int dp = T.dpar >> 1;
   // an excitation operator has only (pp,hh) and (hh,pp) elements: the pairs (a,h) and (p,b) read
@@ -411,13 +430,14 @@ __device__ __forceinline__ double tpandya_at(const DevLayout& D, const DevTLayou
   const int ja = D.jj[a], jb = D.jj[b], jp = D.jj[p], jh = D.jj[h];
   double sm = 0.0;
   for (int Ja = abs(ja - jh); Ja <= ja + jh; Ja += 2)
-    for (int Jb = abs(jp - jb); Jb <= jp + jb; Jb += 2) {
+    for (int Jb = max(abs(jp - jb), Ja - T.rank); Jb <= min(jp + jb, Ja + T.rank); Jb += 2) {
       const double t = term == 1 ? d_telem(D, T, R, hR, a, h, p, b, Ja, Jb) : d_telem(D, T, R, hR, h, a, b, p, Ja, Jb);
       if (t == 0.0) continue;
-      const double nj = term == 1 ? d_nine(T, ja, jb, J3, jh, jp, J4, Ja, Jb) : d_nine(T, jh, jp, J3, ja, jb, J4, Ja, Jb);
-      sm -= d_sgn(Jb >> 1) * sqrt((Ja + 1.0) * (Jb + 1.0)) * nj * t;
+      const double nj = term == 1 ? d_nine_n(T, ja, jb, J3, jh, jp, J4, Ja, Jb) : d_nine_n(T, jh, jp, J3, ja, jb, J4, Ja, Jb);
+      sm = fma(d_flip(nj, !((Jb >> 1) & 1)), t, sm);
     }
-  return term == 1 ? sm * d_sgn((jh + jb + J4) >> 1) * norm : sm * d_sgn((jp + ja + J4) >> 1) * norm * d_sgn((jp + jh) >> 1);
+  const int ph = term == 1 ? (jh + jb + J4) >> 1 : ((jp + ja + J4) >> 1) + ((jp + jh) >> 1);
+  return d_flip(sm * scale, ph & 1);
 }
 
 // the block of a flattened element index (prefix counts pre[0..n], pre[0] = 0)
@@ -432,24 +452,52 @@ __device__ __forceinline__ int d_block_of(const int64_t* __restrict__ pre, int n
 }
 }  // namespace
 
-__global__ void k_tpandya(DevLayout D, DevTLayout T, const double* __restrict__ R, int hR, int J3, int J4, int qa,
-                          int qb, int term, double scale, double* __restrict__ out) {
-  const int r1 = D.cc_rlen[qa], r2 = D.cc_rlen[qb];
-  const int nb1 = D.cc_nph[qa], nb2 = D.cc_nph[qb];
-  const int64_t n = term == 1 ? (int64_t)r1 * nb2 : (int64_t)nb1 * r2;
-  const double norm = sqrt((J3 + 1.0) * (J4 + 1.0)) * scale;
+// The cross-coupled tensor blocks of a batch in one launch: per block CCR (term 2, scale 1/sqrt(J3+1)) and then CCX (term
+// 1, scale 1/sqrt(J4+1)); pre: prefix counts of their elements
+__global__ void k_tpandya(DevLayout D, DevTLayout T, const double* __restrict__ R, int hR, const PhBlock* __restrict__ blk,
+                          const int64_t* __restrict__ pre, int nblk, double* __restrict__ ccr, double* __restrict__ ccx) {
+  const int64_t n = pre[nblk];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int ib = d_block_of(pre, nblk, e);
+    const PhBlock B = blk[ib];
+    int64_t f = e - pre[ib];
+    const int qa = B.qa, qb = B.qb, r1 = D.cc_rlen[qa], r2 = D.cc_rlen[qb], nb1 = D.cc_nph[qa];
+    const int64_t n2 = B.ccr >= 0 ? (int64_t)nb1 * r2 : 0;
     int a, b, p, h;
-    if (term == 1) {
-      const int col = (int)(e / r1), row = (int)(e - (int64_t)col * r1);
-      a = D.cc_ra[D.cc_row_off[qa] + row]; b = D.cc_rb[D.cc_row_off[qa] + row];
-      p = D.cc_cp[D.cc_col_off[qb] + col]; h = D.cc_ch[D.cc_col_off[qb] + col];
-    } else {
-      const int col = (int)(e / nb1), row = (int)(e - (int64_t)col * nb1);
+    if (f < n2) {
+      const int col = (int)(f / nb1), row = (int)(f - (int64_t)col * nb1);
       p = D.cc_cp[D.cc_col_off[qa] + row]; h = D.cc_ch[D.cc_col_off[qa] + row];
       b = D.cc_ra[D.cc_row_off[qb] + col]; a = D.cc_rb[D.cc_row_off[qb] + col];
+      ccr[B.ccr + f] = tpandya_at(D, T, R, hR, B.J3, B.J4, 2, a, b, p, h, 1.0 / T.sq[B.J3 >> 1], 0);
+    } else {
+      f -= n2;
+      const int col = (int)(f / r1), row = (int)(f - (int64_t)col * r1);
+      a = D.cc_ra[D.cc_row_off[qa] + row]; b = D.cc_rb[D.cc_row_off[qa] + row];
+      p = D.cc_cp[D.cc_col_off[qb] + col]; h = D.cc_ch[D.cc_col_off[qb] + col];
+      ccx[B.ccx + f] = tpandya_at(D, T, R, hR, B.J3, B.J4, 1, a, b, p, h, 1.0 / T.sq[B.J4 >> 1], 0);
     }
-    out[e] = tpandya_at(D, T, R, hR, J3, J4, term, a, b, p, h, norm, 0);
+  }
+}
+
+// the normalised 9j table: one CTA per quadruple (a, b, c, d)
+__global__ void k_tensor_nine(DevTLayout T, double* __restrict__ out) {
+  const int nh = T.six_nh, k = T.rank + 1, rank = T.rank;
+  int q = blockIdx.x;
+  const int d = 2 * (q % nh) + 1; q /= nh;
+  const int c = 2 * (q % nh) + 1; q /= nh;
+  const int b = 2 * (q % nh) + 1, a = 2 * (q / nh) + 1;
+  const int n1 = min(a, b) + 1, n3 = min(a, c) + 1, n = n1 * k * n3 * k;
+  double* o = out + T.nine_off[blockIdx.x];
+  for (int e = threadIdx.x; e < n; e += blockDim.x) {
+    int r = e;
+    const int i4 = r % k; r /= k;
+    const int J3 = abs(a - c) + 2 * (r % n3); r /= n3;
+    const int i2 = r % k, J1 = abs(a - b) + 2 * (r / k);
+    const int J2 = J1 - rank + 2 * i2, J4 = J3 - rank + 2 * i4;
+    double v = 0.0;
+    if (J2 >= 0 && J4 >= 0 && J2 >= abs(c - d) && J2 <= c + d && J4 >= abs(b - d) && J4 <= b + d)
+      v = d_nine(T, a, b, J1, c, d, J2, J3, J4) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * (T.sq[J3 >> 1] * T.sq[J4 >> 1]);
+    o[e] = v;
   }
 }
 
@@ -466,62 +514,53 @@ __global__ void k_tpandya_exc(DevLayout D, DevTLayout T, const double* __restric
     const ExcBlock B = blk[ib];
     const int64_t f = e - pre[ib];
     const int qa = B.qa, qb = B.qb, nb1 = D.cc_nph[qa];
-    const double n34 = sqrt((B.J3 + 1.0) * (B.J4 + 1.0));
     if (f < (int64_t)nb1 * B.nx) {  // CCR
       const int c = (int)(f / nb1), row = (int)(f - (int64_t)c * nb1);
       const int col = pe[B.xs + c];
       const int p = D.cc_cp[D.cc_col_off[qa] + row], h = D.cc_ch[D.cc_col_off[qa] + row];
       const int b = D.cc_ra[D.cc_row_off[qb] + col], a = D.cc_rb[D.cc_row_off[qb] + col];
-      ccr[B.ccr + f] = tpandya_at(D, T, R, hR, B.J3, B.J4, 2, a, b, p, h, n34 / sqrt(B.J3 + 1.0), 1);
+      ccr[B.ccr + f] = tpandya_at(D, T, R, hR, B.J3, B.J4, 2, a, b, p, h, 1.0 / T.sq[B.J3 >> 1], 1);
     } else {  // CCX
       const int64_t g = f - (int64_t)nb1 * B.nx;
       const int col = (int)(g / B.ny), r = (int)(g - (int64_t)col * B.ny);
       const int row = hp[B.ys + r];
       const int a = D.cc_ra[D.cc_row_off[qa] + row], b = D.cc_rb[D.cc_row_off[qa] + row];
       const int p = D.cc_cp[D.cc_col_off[qb] + col], h = D.cc_ch[D.cc_col_off[qb] + col];
-      ccx[B.ccx + g] = tpandya_at(D, T, R, hR, B.J3, B.J4, 1, a, b, p, h, n34 / sqrt(B.J4 + 1.0), 1);
+      ccx[B.ccx + g] = tpandya_at(D, T, R, hR, B.J3, B.J4, 1, a, b, p, h, 1.0 / T.sq[B.J4 >> 1], 1);
     }
   }
 }
 
 namespace {
-// add_elem_to_tensor (src/basic_IMSRG.f90:1687-1772): a <= b, c <= d, J1 <= J2
-__device__ __forceinline__ void d_tadd(const DevLayout& D, const DevTLayout& T, double* RES, double V, int a, int b,
-                                       int c, int d, int J1, int J2) {
-  const int P = (D.ll[a] + D.ll[b]) & 1;
-  const int q = d_tblock(D, T, J1, J2, (D.tz[a] + D.tz[b]) >> 1, P);
-  if (q < 0) return;
-  const int g = d_tg(D.con[a] + D.con[b], D.con[c] + D.con[d]);
-  const int N = D.N, NJ = D.NJ;
-  const int i1 = D.pairpos[(a * N + b) * NJ + (J1 >> 1)], i2 = D.pairpos[(c * N + d) * NJ + (J2 >> 1)];
-  if (i1 < 0 || i2 < 0) return;
-  double pre = 1.0;
-  if (a == b) pre *= 1.4142135623730951;
-  if (c == d) pre *= 1.4142135623730951;
-  const int k = q * 9 + g;
-  atomicAdd(RES + T.goff[k] + i1 + (int64_t)i2 * T.n1[k], V * pre);
-}
-
 __device__ __forceinline__ bool d_odd(int J) { return ((J >> 1) & 1) == 1; }
 
-// one recoupling loop of TS_commutator_222_ph: J1 over [o1, o2], J2 over
-// [max(J1, i1, |J1 - rank|), min(i2, J1 + rank)], 9j {n1 n2 J3; n3 n4 J4; J1 J2 rank}
+// one recoupling loop of TS_commutator_222_ph: J1 over [o1, o2], J2 over [max(J1, i1), min(i2, J1 + rank)], adding
+// (-1)^neg(J1, J2) val times the normalised 9j {n1 n2 J3; n3 n4 J4; J1 J2 rank} to the tensor elements (add_elem_to_tensor,
+// src/basic_IMSRG.f90:1687-1772: a <= b, c <= d, J1 <= J2).  Signs by integer instructions, one multiplication a term: the
+// FP64 pipe and the reductions at L2 bound this kernel.
 template <class C>
 __device__ __forceinline__ void recouple_loop(const DevLayout& D, const DevTLayout& T, double* RES, int J3, int J4,
                                               int o1, int o2, int i1, int i2, bool skip_o, bool skip_i, int n1, int n2,
-                                              int n3, int n4, double p34, C coef, int a, int b, int c, int d,
-                                              int exc) {
-  if (exc) {  // only the (pp,hh) and (hh,pp) outputs are wanted
-    const int g = d_tg(D.con[a] + D.con[b], D.con[c] + D.con[d]);
-    if (g != 2 && g != 6) return;
-  }
+                                              int n3, int n4, double val, C neg, int a, int b, int c, int d, int exc) {
+  const int g = d_tg(D.con[a] + D.con[b], D.con[c] + D.con[d]);
+  if (exc && g != 2 && g != 6) return;  // only the (pp,hh) and (hh,pp) outputs are wanted
+  const int P = (D.ll[a] + D.ll[b]) & 1, tz = ((D.tz[a] + D.tz[b]) >> 1) + 1, N = D.N, NJ = D.NJ;
+  const int* pos1 = D.pairpos + (a * N + b) * NJ;
+  const int* pos2 = D.pairpos + (c * N + d) * NJ;
+  if (a == b) val *= 1.4142135623730951;
+  if (c == d) val *= 1.4142135623730951;
   for (int J1 = o1; J1 <= o2; J1 += 2) {
-    if (skip_o && d_odd(J1)) continue;
-    const double p134 = p34 * sqrt(J1 + 1.0);
-    for (int J2 = max(max(J1, i1), abs(J1 - T.rank)); J2 <= min(i2, J1 + T.rank); J2 += 2) {
+    if ((skip_o && d_odd(J1)) || J1 > 2 * D.JM) continue;
+    const int x1 = pos1[J1 >> 1];
+    if (x1 < 0) continue;
+    for (int J2 = max(J1, i1); J2 <= min(i2, J1 + T.rank); J2 += 2) {
       if (skip_i && d_odd(J2)) continue;
-      const double V = p134 * sqrt(J2 + 1.0) * d_nine(T, n1, n2, J3, n3, n4, J4, J1, J2) * coef(J1, J2);
-      d_tadd(D, T, RES, V, a, b, c, d, J1, J2);
+      const int q = T.lut[(((J1 >> 1) * (T.rank / 2 + 1) + ((J2 - J1) >> 1)) * 3 + tz) * 2 + P];
+      const int x2 = pos2[J2 >> 1];
+      if (q < 0 || x2 < 0) continue;
+      const int k = q * 9 + g;
+      atomicAdd(RES + T.goff[k] + x1 + (int64_t)x2 * T.n1[k],
+                d_flip(val * d_nine_n(T, n1, n2, J3, n3, n4, J4, J1, J2), neg(J1, J2)));
     }
   }
 }
@@ -537,37 +576,36 @@ __device__ __forceinline__ void ph_scatter_elem(const DevLayout& D, const DevTLa
                                                 int qa, int qb, int IX, int JX, double X, double Y, int hL, int hR,
                                                 double thresh, int exc) {
   const int rank = T.rank;
-  const double p34 = sqrt((J3 + 1.0) * (J4 + 1.0));
-  const double ph34 = d_sgn((J3 + J4) >> 1);
+  const bool ph34 = ((J3 + J4) >> 1) & 1, nL = hL < 0, nR = hR < 0;
   const int d = D.cc_ra[D.cc_row_off[qa] + IX], a = D.cc_rb[D.cc_row_off[qa] + IX];
   const int c = D.cc_ra[D.cc_row_off[qb] + JX], b = D.cc_rb[D.cc_row_off[qb] + JX];
   const int ja = D.jj[a], jb = D.jj[b], jc = D.jj[c], jd = D.jj[d];
-  const double pabcd = d_sgn((ja + jb + jc + jd) >> 1);
+  const bool pabcd = ((ja + jb + jc + jd) >> 1) & 1;
   if (fabs(X) > thresh) {
     const int J1min = abs(ja - jb), J1max = ja + jb, J2min = abs(jc - jd), J2max = jc + jd;
     if (b >= a) {
       if (d >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, c == d, ja, jd, jb, jc, p34,
-                      [&](int, int J2) { return d_sgn((jb + jd + J2) >> 1) * ph34 * hL * X; }, a, b, c, d, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, a == b, jd, ja, jc, jb, p34,
-                      [&](int J1, int) { return -d_sgn((jc + ja + J1 + rank) >> 1) * hR * X; }, c, d, a, b, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, c == d, ja, jd, jb, jc, X,
+                      [&](int, int J2) { return (((((jb + jd + J2) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, a, b, c, d, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, a == b, jd, ja, jc, jb, X,
+                      [&](int J1, int) { return (((((jc + ja + J1 + rank) >> 1) & 1) ^ (int)nR ^ 1) & 1) != 0; }, c, d, a, b, exc);
       } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, false, ja, jd, jb, jc, p34,
-                      [&](int, int) { return d_sgn((jb + jc) >> 1) * ph34 * hL * X; }, a, b, d, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, a == b, jd, ja, jc, jb, p34,
-                      [&](int, int) { return d_sgn((ja - jd + rank) >> 1) * hR * X; }, d, c, a, b, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, false, ja, jd, jb, jc, X,
+                      [&](int, int) { return (((((jb + jc) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, a, b, d, c, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, a == b, jd, ja, jc, jb, X,
+                      [&](int, int) { return (((((ja - jd + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, d, c, a, b, exc);
       }
     } else {
       if (d >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, c == d, ja, jd, jb, jc, p34,
-                      [&](int J1, int J2) { return d_sgn((ja + jd + J1 + J2) >> 1) * ph34 * hL * X; }, b, a, c, d, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, false, jd, ja, jc, jb, p34,
-                      [&](int J1, int J2) { return d_sgn((jc - jb + J1 + J2 + rank) >> 1) * hR * X; }, c, d, b, a, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, c == d, ja, jd, jb, jc, X,
+                      [&](int J1, int J2) { return (((((ja + jd + J1 + J2) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, b, a, c, d, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, false, jd, ja, jc, jb, X,
+                      [&](int J1, int J2) { return (((((jc - jb + J1 + J2 + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, c, d, b, a, exc);
       } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, false, ja, jd, jb, jc, p34,
-                      [&](int J1, int) { return d_sgn((ja + jc + J1) >> 1) * ph34 * hL * X; }, b, a, d, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, false, jd, ja, jc, jb, p34,
-                      [&](int, int J2) { return d_sgn((jb - jd + J2 + rank) >> 1) * hR * X; }, d, c, b, a, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, false, ja, jd, jb, jc, X,
+                      [&](int J1, int) { return (((((ja + jc + J1) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, b, a, d, c, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, false, jd, ja, jc, jb, X,
+                      [&](int, int J2) { return (((((jb - jd + J2 + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, d, c, b, a, exc);
       }
     }
   }
@@ -575,43 +613,47 @@ __device__ __forceinline__ void ph_scatter_elem(const DevLayout& D, const DevTLa
     const int J1min = abs(jd - jb), J1max = jd + jb, J2min = abs(jc - ja), J2max = jc + ja;
     if (b >= d) {
       if (a >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, p34,
-                      [&](int, int J2) { return d_sgn((jc + ja + J2) >> 1) * hL * Y; }, d, b, c, a, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, p34,
-                      [&](int J1, int) { return d_sgn((jd - jb + J1 + rank) >> 1) * ph34 * hR * Y; }, c, a, d, b, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, Y,
+                      [&](int, int J2) { return (((((jc + ja + J2) >> 1) & 1) ^ (int)nL) & 1) != 0; }, d, b, c, a, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, Y,
+                      [&](int J1, int) { return (((((jd - jb + J1 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, c, a, d, b, exc);
       } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, p34,
-                      [&](int, int) { return -hL * Y; }, d, b, a, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, b == d, ja, jd, jc, jb, p34,
-                      [&](int, int) { return pabcd * ph34 * d_sgn(rank >> 1) * hR * Y; }, a, c, d, b, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, Y,
+                      [&](int, int) { return (((int)nL ^ 1) & 1) != 0; }, d, b, a, c, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, b == d, ja, jd, jc, jb, Y,
+                      [&](int, int) { return (((int)pabcd ^ (int)ph34 ^ ((rank >> 1) & 1) ^ (int)nR) & 1) != 0; }, a, c, d, b, exc);
       }
     } else {
       if (a >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, p34,
-                      [&](int J1, int J2) { return -pabcd * d_sgn((J1 + J2) >> 1) * hL * Y; }, b, d, c, a, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, p34,
-                      [&](int J1, int J2) { return d_sgn((J1 + J2 + rank) >> 1) * ph34 * hR * Y; }, c, a, b, d, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, Y,
+                      [&](int J1, int J2) { return (((int)pabcd ^ (((J1 + J2) >> 1) & 1) ^ (int)nL ^ 1) & 1) != 0; }, b, d, c, a, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, Y,
+                      [&](int J1, int J2) { return (((((J1 + J2 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, c, a, b, d, exc);
       } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, p34,
-                      [&](int J1, int) { return d_sgn((jb + jd + J1) >> 1) * hL * Y; }, b, d, a, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, d == b, ja, jd, jc, jb, p34,
-                      [&](int, int J2) { return d_sgn((ja - jc + J2 + rank) >> 1) * ph34 * hR * Y; }, a, c, b, d, exc);
+        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, Y,
+                      [&](int J1, int) { return (((((jb + jd + J1) >> 1) & 1) ^ (int)nL) & 1) != 0; }, b, d, a, c, exc);
+        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, d == b, ja, jd, jc, jb, Y,
+                      [&](int, int J2) { return (((((ja - jc + J2 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, a, c, b, d, exc);
       }
     }
   }
 }
 }  // namespace
 
-__global__ void k_ts222ph_scatter(DevLayout D, DevTLayout T, const double* __restrict__ Wx,
-                                  const double* __restrict__ Wy, int J3, int J4, int qa, int qb, int hL, int hR,
-                                  double thresh, int exc, double* __restrict__ RES) {
-  const int r1 = D.cc_rlen[qa], r2 = D.cc_rlen[qb];
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)r1 * r2;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int JX = (int)(e / r1), IX = (int)(e - (int64_t)JX * r1);
-    const double X = Wx[e], Y = Wy ? Wy[e] : 0.0;
+// the blocks of a batch in one launch; pre: prefix counts of r1 r2
+__global__ void k_ts222ph_scatter(DevLayout D, DevTLayout T, const PhBlock* __restrict__ blk, const int64_t* __restrict__ pre,
+                                  int nblk, const double* __restrict__ Wx, const double* __restrict__ Wy, int hL, int hR,
+                                  double thresh, double* __restrict__ RES) {
+  const int64_t n = pre[nblk];
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int ib = d_block_of(pre, nblk, e);
+    const PhBlock B = blk[ib];
+    const int64_t f = e - pre[ib];
+    const int r1 = D.cc_rlen[B.qa];
+    const int JX = (int)(f / r1), IX = (int)(f - (int64_t)JX * r1);
+    const double X = B.ccr >= 0 ? Wx[B.wx + f] : 0.0, Y = B.ccx >= 0 ? Wy[B.wy + f] : 0.0;
     if (fabs(X) <= thresh && fabs(Y) <= thresh) continue;
-    ph_scatter_elem(D, T, RES, J3, J4, qa, qb, IX, JX, X, Y, hL, hR, thresh, exc);
+    ph_scatter_elem(D, T, RES, B.J3, B.J4, B.qa, B.qb, IX, JX, X, Y, hL, hR, thresh, 0);
   }
 }
 

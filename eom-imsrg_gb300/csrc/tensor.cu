@@ -35,8 +35,9 @@ __global__ void k_ts122f(DevLayout D, DevTLayout T, const double* L, int hL, con
 __global__ void k_ts212f(DevLayout D, DevTLayout T, const double* L, int hL, const double* R, int hR, double* RES,
                          ElemSegs sg);
 __global__ void k_ts_pphh_update(int64_t n, int64_t off, double* RES, const double* w1, const double* w2);
-__global__ void k_tpandya(DevLayout D, DevTLayout T, const double* R, int hR, int J3, int J4, int qa, int qb, int term,
-                          double scale, double* out);
+__global__ void k_tpandya(DevLayout D, DevTLayout T, const double* R, int hR, const PhBlock* blk, const int64_t* pre,
+                          int nblk, double* ccr, double* ccx);
+__global__ void k_tensor_nine(DevTLayout T, double* out);
 // FP32 SIMT form of k_gemm_fp64 (FP64 operands and results), gemm_tc.cu
 __global__ void k_gemm_f32(const GemmProb* probs, const GemmTile* tiles, GemmOperands ops);
 __global__ void k_tpandya_exc(DevLayout D, DevTLayout T, const double* R, int hR, const ExcBlock* blk,
@@ -44,8 +45,8 @@ __global__ void k_tpandya_exc(DevLayout D, DevTLayout T, const double* R, int hR
 __global__ void k_ts222ph_scatter_exc(DevLayout D, DevTLayout T, const ExcBlock* blk, const int64_t* pre, int nblk,
                                       const int* pe, const int* hp, const double* Wx, const double* Wy, int hL, int hR,
                                       double* RES);
-__global__ void k_ts222ph_scatter(DevLayout D, DevTLayout T, const double* Wx, const double* Wy, int J3, int J4,
-                                  int qa, int qb, int hL, int hR, double thresh, int exc, double* RES);
+__global__ void k_ts222ph_scatter(DevLayout D, DevTLayout T, const PhBlock* blk, const int64_t* pre, int nblk,
+                                  const double* Wx, const double* Wy, int hL, int hR, double thresh, double* RES);
 }  // namespace imsrg
 
 namespace {
@@ -168,41 +169,90 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
       seg_off.push_back(T.goff[(size_t)q * 9 + g] - T.goff[0]);
       seg_pre.push_back(seg_pre.back() + n);
     }
-  // per cross-coupled block: Wx = -LCC(qa) CCR and Wy = CCX LCC(qb)^T
+  // cross-coupled blocks, Wx = -LCC(qa) CCR and Wy = CCX LCC(qb)^T, in batches of at most `most` W elements: one by one
+  // (140 blocks at eMax 4, rank 2) their launches were short and mostly idle; 2 M elements fill the GPU, and a sixteenth
+  // of the whole keeps large bases to a few launches
   std::vector<GemmProb> cbp;
   std::vector<GemmTile> cbt;
-  for (size_t b = 0; b < T.cb_J3.size(); ++b) {
-    const int qa = T.cb_qa[b], qb = T.cb_qb[b];
-    const int r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb], nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
-    std::vector<GemmProb> ps;
-    if (nb1) {
-      GemmProb p{};
-      p.c_id = kOpW1; p.M = r1; p.N = r2; p.ldc = r1; p.nterm = 1;
-      GemmTerm& t = p.t[0];
-      t.a_id = kOpLCC; t.a_off = L.cc_off[qa]; t.lda = r1; t.ta = 0;
-      t.b_id = kOpRCC; t.b_off = 0; t.ldb = nb1; t.tb = 0;
-      t.K = nb1; t.alpha = kAlphaNeg | kAlphaOne;
-      ps.push_back(p);
+  std::vector<int64_t> ph_pre_p, ph_pre_s;
+  {
+    int64_t all = 0;
+    for (size_t b = 0; b < T.cb_J3.size(); ++b) all += (int64_t)L.cc_rlen[T.cb_qa[b]] * L.cc_rlen[T.cb_qb[b]];
+    const int64_t most = std::max<int64_t>((int64_t)1 << 21, all / 16);
+    int64_t occr = 0, occx = 0, ow = 0;
+    auto close = [&]() {
+      if (st->ph_batches.empty()) return;
+      PhBatch& B = st->ph_batches.back();
+      if (!B.n) return;
+      B.prob0 = (int)cbp.size();
+      B.tile0 = (int)cbt.size();
+      auto tiles = build_tiles(B.probs, 64, 64);
+      B.ntiles = (int)tiles.size();
+      cbt.insert(cbt.end(), tiles.begin(), tiles.end());
+      cbp.insert(cbp.end(), B.probs.begin(), B.probs.end());
+      st->ph_sizes[0] = std::max(st->ph_sizes[0], occr);
+      st->ph_sizes[1] = std::max(st->ph_sizes[1], occx);
+      st->ph_sizes[2] = std::max(st->ph_sizes[2], ow);
+    };
+    for (size_t b = 0; b < T.cb_J3.size(); ++b) {
+      const int qa = T.cb_qa[b], qb = T.cb_qb[b];
+      const int64_t r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb];
+      const int nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
+      const bool dox = nb1 > 0, doy = nb2 > 0 && T.cb_J3[b] != T.cb_J4[b];
+      if ((!dox && !doy) || r1 * r2 == 0) continue;
+      if (st->ph_batches.empty() || ow + r1 * r2 > most) {
+        close();
+        st->ph_batches.emplace_back();
+        st->ph_batches.back().b0 = (int)st->ph_blocks.size();
+        st->ph_batches.back().pre0 = (int)ph_pre_p.size();
+        ph_pre_p.push_back(0);
+        ph_pre_s.push_back(0);
+        occr = occx = ow = 0;
+      }
+      PhBatch& B = st->ph_batches.back();
+      PhBlock K{T.cb_J3[b], T.cb_J4[b], qa, qb, dox ? occr : -1, doy ? occx : -1, ow, ow};
+      if (dox) {
+        GemmProb p{};
+        p.c_id = kOpW1; p.c_off = ow; p.M = (int)r1; p.N = (int)r2; p.ldc = (int)r1; p.nterm = 1;
+        GemmTerm& t = p.t[0];
+        t.a_id = kOpLCC; t.a_off = L.cc_off[qa]; t.lda = (int)r1; t.ta = 0;
+        t.b_id = kOpRCC; t.b_off = occr; t.ldb = nb1; t.tb = 0;
+        t.K = nb1; t.alpha = kAlphaNeg | kAlphaOne;
+        B.probs.push_back(p);
+        occr += nb1 * r2;
+      }
+      if (doy) {
+        GemmProb p{};
+        p.c_id = kOpW2; p.c_off = ow; p.M = (int)r1; p.N = (int)r2; p.ldc = (int)r1; p.nterm = 1;
+        GemmTerm& t = p.t[0];
+        t.a_id = kOpWCC; t.a_off = occx; t.lda = (int)r1; t.ta = 0;
+        t.b_id = kOpLCC; t.b_off = L.cc_off[qb]; t.ldb = (int)r2; t.tb = 1;
+        t.K = nb2; t.alpha = kAlphaOne;
+        B.probs.push_back(p);
+        occx += r1 * nb2;
+      }
+      ow += r1 * r2;
+      B.np += (dox ? nb1 * r2 : 0) + (doy ? r1 * nb2 : 0);
+      B.ns += r1 * r2;
+      ++B.n;
+      ph_pre_p.push_back(B.np);
+      ph_pre_s.push_back(B.ns);
+      st->ph_blocks.push_back(K);
     }
-    if (nb2 && T.cb_J3[b] != T.cb_J4[b]) {
-      GemmProb p{};
-      p.c_id = kOpW2; p.M = r1; p.N = r2; p.ldc = r1; p.nterm = 1;
-      GemmTerm& t = p.t[0];
-      t.a_id = kOpWCC; t.a_off = 0; t.lda = r1; t.ta = 0;
-      t.b_id = kOpLCC; t.b_off = L.cc_off[qb]; t.ldb = r2; t.tb = 1;
-      t.K = nb2; t.alpha = kAlphaOne;
-      ps.push_back(p);
-    }
-    const int base = (int)cbp.size();
-    auto tiles = build_tiles(ps, 64, 64);
-    st->cb_tile_start.push_back((int)cbt.size());
-    st->cb_tile_n.push_back((int)tiles.size());
-    for (auto& t : tiles) {
-      t.prob += base;
-      cbt.push_back(t);
-    }
-    for (auto& p : ps) cbp.push_back(p);
+    close();
   }
+  // sqrt(J + 1), and the offsets of the 9j table where it stays within 1 GB
+  std::vector<double> sq(2 * L.JM + T.rank + 2);
+  for (size_t k = 0; k < sq.size(); ++k) sq[k] = std::sqrt(2.0 * k + 1.0);
+  std::vector<int64_t> nine_off;
+  int64_t nine_n = 0;
+  for (int a = 1; a <= L.JM; a += 2)
+    for (int b = 1; b <= L.JM; b += 2)
+      for (int c = 1; c <= L.JM; c += 2)
+        for (int e = 1; e <= L.JM; e += 2) {
+          nine_off.push_back(nine_n);
+          nine_n += (int64_t)(std::min(a, b) + 1) * (T.rank + 1) * (std::min(a, c) + 1) * (T.rank + 1);
+        }
   Pack pk;
   DevTLayout& d = st->DT;
   d.rank = T.rank; d.dpar = T.dpar; d.nblocks = T.nblocks; d.n_ob = (int)T.ob_kind.size();
@@ -223,6 +273,9 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
   pk.add(xbp, &st->x_p); pk.add(xbt, &st->x_t);
   pk.add(xblk, &st->x_blk); pk.add(xpre_p, &st->x_pre_p); pk.add(xpre_s, &st->x_pre_s);
   pk.add(cbp, &st->cb_p); pk.add(cbt, &st->cb_t);
+  pk.add(st->ph_blocks, &st->d_ph_blocks); pk.add(ph_pre_p, &st->d_ph_pre_p); pk.add(ph_pre_s, &st->d_ph_pre_s);
+  pk.add(sq, &d.sq); pk.add(nine_off, &d.nine_off);
+  st->pphh_probs = pphh; st->exc_probs = exc; st->x_probs = xbp;
   pk.add(T.seg_start, &st->seg_start); pk.add(T.seg_len, &st->seg_len); pk.add(T.seg_w, &st->seg_w);
   CKT(cuda(cudaMalloc(&st->tables, pk.buf.size()), "cudaMalloc(tensor tables)"));
   CKT(cuda(cudaMemcpy(st->tables, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tensor tables)"));
@@ -237,12 +290,19 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
     CKT(cuda(cudaMalloc(p, tb), "cudaMalloc(tensor workspace)"));
     CKT(cuda(cudaMemsetAsync(*p, 0, tb, stream), "memset(tensor workspace)"));
   }
-  const size_t xb = sizeof(double) * (size_t)std::max<int64_t>(T.cb_max_x, 1);
-  const size_t wb = sizeof(double) * (size_t)std::max<int64_t>(T.cb_max_w, 1);
-  CKT(cuda(cudaMalloc(&st->ccx, xb), "cudaMalloc(CCX tensor)"));
-  CKT(cuda(cudaMalloc(&st->ccr, xb), "cudaMalloc(CCR tensor)"));
-  CKT(cuda(cudaMalloc(&st->wx, wb), "cudaMalloc(Wx)"));
-  CKT(cuda(cudaMalloc(&st->wy, wb), "cudaMalloc(Wy)"));
+  double** ph[] = {&st->ccr, &st->ccx, &st->wx, &st->wy};
+  for (int k = 0; k < 4; ++k)
+    CKT(cuda(cudaMalloc(ph[k], sizeof(double) * (size_t)std::max<int64_t>(st->ph_sizes[std::min(k, 2)], 1)),
+             "cudaMalloc(cross-coupled tensor blocks)"));
+  d.nine = nullptr;
+  if (nine_n * (int64_t)sizeof(double) <= (int64_t)1 << 30 && cudaMalloc(&st->d_nine, sizeof(double) * (size_t)nine_n) == cudaSuccess) {
+    k_tensor_nine<<<(int)nine_off.size(), 128, 0, stream>>>(d, st->d_nine);
+    CKT(launched("k_tensor_nine"));
+    d.nine = st->d_nine;
+  } else {
+    cudaGetLastError();
+    st->d_nine = nullptr;
+  }
   *out = st.get();
   reg[key] = std::move(st);
   return IMSRG_OK;
@@ -258,8 +318,12 @@ void Ctx::tensor_release() {
     TensorState* s = it->second.get();
     for (void* p : {(void*)s->w1, (void*)s->w2, (void*)s->ccx, (void*)s->ccr, (void*)s->wx, (void*)s->wy,
                     (void*)s->bch_a, (void*)s->bch_b, s->tables, (void*)s->tc_buf, s->tc_tables, (void*)s->w3,
-                    (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3]})
+                    (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3], (void*)s->d_nine})
       if (p) cudaFree(p);
+    oz_release(s->pphh_oz);
+    oz_release(s->exc_oz);
+    oz_release(s->x_oz);
+    for (PhBatch& B : s->ph_batches) oz_release(B.oz);
     it = reg.erase(it);
   }
 }
@@ -335,47 +399,54 @@ imsrg_status Ctx::tensor_tc_prepare(TensorState& S) {
   S.ph_lcc_nchunks = (int)chunks.size() - ladder_nchunks;
   // per block: CCR (src 0, its columns, K = nb1) and CCX (src 1, its rows, K = nb2) into two
   // regions shared by all blocks, then Wx = -LCC(qa) CCR and Wy = CCX LCC(qb)^T
-  const TLayout& TT = S.T;
-  int ccr_tiles_max = 0, ccx_tiles_max = 0;
-  for (size_t b = 0; b < TT.cb_J3.size(); ++b) {
-    const int qa = TT.cb_qa[b], qb = TT.cb_qb[b];
-    const int r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb], nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
-    ccr_tiles_max = std::max(ccr_tiles_max, ((r2 + BMr - 1) / BMr) * ((nb1 + BKk - 1) / BKk));
-    ccx_tiles_max = std::max(ccx_tiles_max, ((r1 + BMr - 1) / BMr) * ((nb2 + BKk - 1) / BKk));
+  auto tiles_of = [&](int rows, int K) { return ((rows + BMr - 1) / BMr) * ((K + BKk - 1) / BKk); };
+  int most_tiles = 0;  // the batches share one region of the operand buffer
+  for (const PhBatch& B : S.ph_batches) {
+    int n = 0;
+    for (int b = B.b0; b < B.b0 + B.n; ++b) {
+      const PhBlock& K = S.ph_blocks[b];
+      if (K.ccr >= 0) n += tiles_of(L.cc_rlen[K.qb], L.cc_nph[K.qa]);
+      if (K.ccx >= 0) n += tiles_of(L.cc_rlen[K.qa], L.cc_nph[K.qb]);
+    }
+    most_tiles = std::max(most_tiles, n);
   }
-  const int ccr_base = tiles, ccx_base = tiles + ccr_tiles_max;
-  tiles += ccr_tiles_max + ccx_tiles_max;
+  const int ph_base = tiles;
+  tiles += most_tiles;
   std::vector<TcTile> tph;
   S.ph_chunk_start.clear(); S.ph_chunk_n.clear(); S.ph_tile_start.clear(); S.ph_tile_n.clear();
-  for (size_t b = 0; b < TT.cb_J3.size(); ++b) {
-    const int qa = TT.cb_qa[b], qb = TT.cb_qb[b];
-    const int r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb], nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
-    const bool dox = nb1 > 0, doy = nb2 > 0 && TT.cb_J3[b] != TT.cb_J4[b];
+  for (const PhBatch& B : S.ph_batches) {
     S.ph_chunk_start.push_back((int)chunks.size());
     S.ph_tile_start.push_back((int)(tl.size() + tph.size()));
-    auto add_prob = [&](int K, TcTermDesc t, int c_id) {
-      TcProb q{};
-      q.M = r1; q.N = r2; q.nkb = (K + BKk - 1) / BKk; q.nterm = 1; q.t[0] = t;
-      q.out_f32 = 0; q.c_id = c_id; q.c_off = 0; q.ldc = r1;
-      probs.push_back(q);
-      const int pi = (int)probs.size() - 1;
-      for (int m0 = 0; m0 < r1; m0 += BMr)
-        for (int n0 = 0; n0 < r2; n0 += BMr) tph.push_back(TcTile{pi, m0, n0, BMr});
-    };
-    if (dox && r1 && r2) {
-      TcSplitOp o{};
-      o.src = 0; o.src_off = 0; o.rows = r2; o.K = nb1; o.nkb = (nb1 + BKk - 1) / BKk; o.tile_base = ccr_base;
-      ops.push_back(o);
-      add_chunks((int)ops.size() - 1);
-      add_prob(nb1, TcTermDesc{lcc_tile[qa], ccr_base, kSignNeg}, kOpW1);
-    }
-    if (doy && r1 && r2) {
-      TcSplitOp o{};
-      o.src = 1; o.src_off = 0; o.rows = r1; o.K = nb2; o.nkb = (nb2 + BKk - 1) / BKk; o.tile_base = ccx_base;
-      o.trans = 1; o.ld = r1;
-      ops.push_back(o);
-      add_chunks((int)ops.size() - 1);
-      add_prob(nb2, TcTermDesc{ccx_base, lcc_tile[qb], 0}, kOpW2);
+    int at = ph_base;
+    for (int b = B.b0; b < B.b0 + B.n; ++b) {
+      const PhBlock& K = S.ph_blocks[b];
+      const int r1 = L.cc_rlen[K.qa], r2 = L.cc_rlen[K.qb], nb1 = L.cc_nph[K.qa], nb2 = L.cc_nph[K.qb];
+      auto add_prob = [&](int Kk, TcTermDesc t, int c_id, int64_t off) {
+        TcProb q{};
+        q.M = r1; q.N = r2; q.nkb = (Kk + BKk - 1) / BKk; q.nterm = 1; q.t[0] = t;
+        q.out_f32 = 0; q.c_id = c_id; q.c_off = off; q.ldc = r1;
+        probs.push_back(q);
+        const int pi = (int)probs.size() - 1;
+        for (int m0 = 0; m0 < r1; m0 += BMr)
+          for (int n0 = 0; n0 < r2; n0 += BMr) tph.push_back(TcTile{pi, m0, n0, BMr});
+      };
+      if (K.ccr >= 0) {
+        TcSplitOp o{};
+        o.src = 0; o.src_off = K.ccr; o.rows = r2; o.K = nb1; o.nkb = (nb1 + BKk - 1) / BKk; o.tile_base = at;
+        at += tiles_of(r2, nb1);
+        ops.push_back(o);
+        add_chunks((int)ops.size() - 1);
+        add_prob(nb1, TcTermDesc{lcc_tile[K.qa], o.tile_base, kSignNeg}, kOpW1, K.wx);
+      }
+      if (K.ccx >= 0) {
+        TcSplitOp o{};
+        o.src = 1; o.src_off = K.ccx; o.rows = r1; o.K = nb2; o.nkb = (nb2 + BKk - 1) / BKk; o.tile_base = at;
+        at += tiles_of(r1, nb2);
+        o.trans = 1; o.ld = r1;
+        ops.push_back(o);
+        add_chunks((int)ops.size() - 1);
+        add_prob(nb2, TcTermDesc{o.tile_base, lcc_tile[K.qb], 0}, kOpW2, K.wy);
+      }
     }
     S.ph_chunk_n.push_back((int)chunks.size() - S.ph_chunk_start.back());
     S.ph_tile_n.push_back((int)(tl.size() + tph.size()) - S.ph_tile_start.back());
@@ -474,7 +545,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
       CKT(launched("k_ts_pphh_update"));
     }
     if (nob) {
-      k_ts221<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
+      k_ts221<<<nob, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
       CKT(launched("k_ts221"));
     }
   } else if (pieces & 32) {
@@ -491,8 +562,8 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
         k_gemm_f32<<<nt, 256, 0, stream>>>(S.exc_p, S.exc_t, ops);
         CKT(launched("k_gemm_f32(tensor pphh, excitation)"));
       } else {
-        k_gemm_fp64<<<nt, 256, 0, stream>>>(exc ? S.exc_p : S.pphh_p, exc ? S.exc_t : S.pphh_t, nt, ops, nullptr);
-        CKT(launched("k_gemm_fp64(tensor pphh)"));
+        CKT(exc ? gemm_fp64(S.exc_oz, S.exc_probs, S.exc_p, S.exc_t, nt, ops)
+                : gemm_fp64(S.pphh_oz, S.pphh_probs, S.pphh_p, S.pphh_t, nt, ops));
       }
     }
     if (T.n2b) {
@@ -500,7 +571,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
       CKT(launched("k_ts_pphh_update"));
     }
     if (nob) {
-      k_ts221<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
+      k_ts221<<<nob, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
       CKT(launched("k_ts221"));
     }
   }
@@ -522,76 +593,39 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
           k_gemm_f32<<<S.x_n_t, 256, 0, stream>>>(S.x_p, S.x_t, ops);
           CKT(launched("k_gemm_f32(tensor ph, excitation)"));
         } else {
-          k_gemm_fp64<<<S.x_n_t, 256, 0, stream>>>(S.x_p, S.x_t, S.x_n_t, ops, nullptr);
-          CKT(launched("k_gemm_fp64(tensor ph, excitation)"));
+          CKT(gemm_fp64(S.x_oz, S.x_probs, S.x_p, S.x_t, S.x_n_t, ops));
         }
       }
       k_ts222ph_scatter_exc<<<grid_n(S.x_ns), 256, 0, stream>>>(D, T, S.x_blk, S.x_pre_s, S.x_nblk, S.d_pe, S.d_hp,
                                                                  S.x_buf[2], S.x_buf[3], hL, hR, RES);
       CKT(launched("k_ts222ph_scatter_exc"));
     }
-  } else if ((pieces & 64) && precision != IMSRG_PREC_FP64) {  // split-BF16 cross-coupled products
-    CKT(tensor_tc_prepare(S));
-    const TLayout& H = S.T;
-    CKT(tc_split_on(S.tc_ops, S.tc_chunks + S.tc_nchunks, S.ph_lcc_nchunks, d_lcc, nullptr, S.tc_buf,
-                    S.tc_slice_elems));
-    for (size_t b = 0; b < H.cb_J3.size(); ++b) {
-      const int J3 = H.cb_J3[b], J4 = H.cb_J4[b], qa = H.cb_qa[b], qb = H.cb_qb[b];
-      const int r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb], nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
-      const bool dox = nb1 > 0, doy = nb2 > 0 && J3 != J4;
-      if (!dox && !doy) continue;
-      if (dox) {
-        k_tpandya<<<grid_n((int64_t)nb1 * r2), 256, 0, stream>>>(D, T, R, hR, J3, J4, qa, qb, 2,
-                                                                 1.0 / std::sqrt(J3 + 1.0), S.ccr);
-        CKT(launched("k_tpandya"));
-      } else {
-        CKT(cuda(cudaMemsetAsync(S.wx, 0, sizeof(double) * (size_t)r1 * r2, stream), "memset(Wx)"));
-      }
-      if (doy) {
-        k_tpandya<<<grid_n((int64_t)r1 * nb2), 256, 0, stream>>>(D, T, R, hR, J3, J4, qa, qb, 1,
-                                                                 1.0 / std::sqrt(J4 + 1.0), S.ccx);
-        CKT(launched("k_tpandya"));
-      }
-      CKT(tc_split_on(S.tc_ops, S.tc_chunks + S.ph_chunk_start[b], S.ph_chunk_n[b], S.ccr, S.ccx, S.tc_buf,
-                      S.tc_slice_elems));
-      TcOut out{};
-      out.f64[kOpW1] = S.wx;
-      out.f64[kOpW2] = S.wy;
-      CKT(tc_gemm_on(S.tc_map, S.tc_slice_rows, S.tc_probs, S.tc_tiles + S.ph_tile_start[b], S.ph_tile_n[b], out, hL,
-                     hR));
-      k_ts222ph_scatter<<<grid_n((int64_t)r1 * r2), 256, 0, stream>>>(D, T, S.wx, doy ? S.wy : nullptr, J3, J4, qa,
-                                                                      qb, hL, hR, thresh, exc, RES);
-      CKT(launched("k_ts222ph_scatter"));
-    }
   } else if (pieces & 64) {
-    const TLayout& H = S.T;
-    for (size_t b = 0; b < H.cb_J3.size(); ++b) {
-      const int J3 = H.cb_J3[b], J4 = H.cb_J4[b], qa = H.cb_qa[b], qb = H.cb_qb[b];
-      const int r1 = L.cc_rlen[qa], r2 = L.cc_rlen[qb], nb1 = L.cc_nph[qa], nb2 = L.cc_nph[qb];
-      const bool dox = nb1 > 0, doy = nb2 > 0 && J3 != J4;
-      if (!dox && !doy) continue;
-      if (dox) {
-        k_tpandya<<<grid_n((int64_t)nb1 * r2), 256, 0, stream>>>(D, T, R, hR, J3, J4, qa, qb, 2,
-                                                                 1.0 / std::sqrt(J3 + 1.0), S.ccr);
-        CKT(launched("k_tpandya"));
+    const bool mixed = precision != IMSRG_PREC_FP64;  // split-BF16 cross-coupled products
+    if (mixed) {
+      CKT(tensor_tc_prepare(S));
+      CKT(tc_split_on(S.tc_ops, S.tc_chunks + S.tc_nchunks, S.ph_lcc_nchunks, d_lcc, nullptr, S.tc_buf, S.tc_slice_elems));
+    }
+    for (size_t i = 0; i < S.ph_batches.size(); ++i) {
+      PhBatch& B = S.ph_batches[i];
+      k_tpandya<<<grid_n(B.np), 256, 0, stream>>>(D, T, R, hR, S.d_ph_blocks + B.b0, S.d_ph_pre_p + B.pre0, B.n, S.ccr, S.ccx);
+      CKT(launched("k_tpandya"));
+      if (mixed) {
+        CKT(tc_split_on(S.tc_ops, S.tc_chunks + S.ph_chunk_start[i], S.ph_chunk_n[i], S.ccr, S.ccx, S.tc_buf,
+                        S.tc_slice_elems));
+        TcOut out{};
+        out.f64[kOpW1] = S.wx;
+        out.f64[kOpW2] = S.wy;
+        CKT(tc_gemm_on(S.tc_map, S.tc_slice_rows, S.tc_probs, S.tc_tiles + S.ph_tile_start[i], S.ph_tile_n[i], out, hL, hR));
       } else {
-        CKT(cuda(cudaMemsetAsync(S.wx, 0, sizeof(double) * (size_t)r1 * r2, stream), "memset(Wx)"));
-      }
-      if (doy) {
-        k_tpandya<<<grid_n((int64_t)r1 * nb2), 256, 0, stream>>>(D, T, R, hR, J3, J4, qa, qb, 1,
-                                                                 1.0 / std::sqrt(J4 + 1.0), S.ccx);
-        CKT(launched("k_tpandya"));
-      }
-      if (S.cb_tile_n[b]) {
         GemmOperands ops{};
         ops.in[kOpLCC] = d_lcc; ops.in[kOpRCC] = S.ccr; ops.in[kOpWCC] = S.ccx;
         ops.out[kOpW1] = S.wx; ops.out[kOpW2] = S.wy;
         ops.hL = hL; ops.hR = hR;
-        k_gemm_fp64<<<S.cb_tile_n[b], 256, 0, stream>>>(S.cb_p, S.cb_t + S.cb_tile_start[b], S.cb_tile_n[b], ops, nullptr);
-        CKT(launched("k_gemm_fp64(tensor ph)"));
+        CKT(gemm_fp64(B.oz, B.probs, S.cb_p + B.prob0, S.cb_t + B.tile0, B.ntiles, ops));
       }
-      k_ts222ph_scatter<<<grid_n((int64_t)r1 * r2), 256, 0, stream>>>(D, T, S.wx, doy ? S.wy : nullptr, J3, J4, qa,
-                                                                      qb, hL, hR, thresh, exc, RES);
+      k_ts222ph_scatter<<<grid_n(B.ns), 256, 0, stream>>>(D, T, S.d_ph_blocks + B.b0, S.d_ph_pre_s + B.pre0, B.n, S.wx, S.wy,
+                                                          hL, hR, thresh, RES);
       CKT(launched("k_ts222ph_scatter"));
     }
   }

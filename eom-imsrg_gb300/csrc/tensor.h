@@ -40,7 +40,6 @@ struct TLayout {
   // cross-coupled tensor blocks of TS_commutator_222_ph: (J3, J4 >= J3, Tz 0/1, PAR) and their
   // scalar cross-coupled channels qa (J3, Tz, PAR), qb (J4, Tz, PAR xor dpar/2)
   std::vector<int> cb_J3, cb_J4, cb_Tz, cb_PAR, cb_qa, cb_qb;
-  int64_t cb_max_w = 0, cb_max_x = 0, cb_max_r = 0;  // largest r1*r2, r1*nb2 / nb1*r2, r
   // Frobenius-norm segments (weight 1 for fhh, fpp and J1 == J2 blocks, 2 otherwise)
   std::vector<int64_t> seg_start;
   std::vector<int> seg_len;
@@ -102,6 +101,19 @@ struct DevTLayout {
   const int* tnb_start;
   const int* tnb_count;
   const int* tnb_list;
+  const double* sq;         // sqrt(J + 1), [J / 2] up to 4 jmax + rank
+  // {a b J1; c d J2; J3 J4 rank} sqrt((J1+1)(J2+1)(J3+1)(J4+1)) of every quadruple of j (nullptr: evaluated where used):
+  // nine[nine_off[((a/2 nh + b/2) nh + c/2) nh + d/2] + ((i1 (rank+1) + i2) n3 + i3) (rank+1) + i4], i1 = (J1-|a-b|)/2,
+  // i2 = (J2-J1+rank)/2, i3 = (J3-|a-c|)/2 < n3 = min(a,c)+1, i4 = (J4-J3+rank)/2
+  const double* nine;
+  const int64_t* nine_off;
+};
+
+// one cross-coupled tensor block of a batch of TS_commutator_222_ph: the offsets of its CCR (nb1 x r2), CCX (r1 x nb2)
+// and of its Wx / Wy (r1 x r2) in the batch's buffers (-1: no such product, its W is zero)
+struct PhBlock {
+  int J3, J4, qa, qb;
+  int64_t ccr, ccx, wx, wy;
 };
 
 }  // namespace imsrg

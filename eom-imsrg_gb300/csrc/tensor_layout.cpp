@@ -136,9 +136,6 @@ std::string build_tlayout(TLayout& T, const Layout& L, int rank, int dpar) {
           if (r1 * r2 == 0) continue;
           T.cb_J3.push_back(j3); T.cb_J4.push_back(j4); T.cb_Tz.push_back(tz); T.cb_PAR.push_back(par);
           T.cb_qa.push_back(qa); T.cb_qb.push_back(qb);
-          T.cb_max_w = std::max(T.cb_max_w, r1 * r2);
-          T.cb_max_x = std::max(T.cb_max_x, std::max(r1 * L.cc_nph[qb], (int64_t)L.cc_nph[qa] * r2));
-          T.cb_max_r = std::max(T.cb_max_r, std::max(r1, r2));
         }
 
   // Frobenius-norm segments

@@ -34,6 +34,17 @@ constexpr int kTensorExcitation = 1024;
 // output slot of the second product of a tensor ladder problem (TcOut::f64 index)
 constexpr int kTensorOpW3 = 7;
 
+// cross-coupled blocks b0 .. b0 + n - 1 of TensorState::ph_blocks
+struct PhBatch {
+  int b0 = 0, n = 0;
+  int pre0 = 0;              // its n + 1 prefix counts
+  int64_t np = 0, ns = 0;    // Pandya and W elements
+  int tile0 = 0, ntiles = 0; // of k_gemm_fp64
+  std::vector<GemmProb> probs;
+  int prob0 = 0;
+  imsrg::OzPlan oz;
+};
+
 // device state of one (rank, dpar) layout
 struct TensorState {
   TLayout T;
@@ -63,10 +74,18 @@ struct TensorState {
   int x_nblk = 0, x_n_t = 0;
   int64_t x_np = 0, x_ns = 0, x_sizes[4] = {0, 0, 0, 0};
   double* x_buf[4] = {nullptr, nullptr, nullptr, nullptr};
-  // per cross-coupled block: GEMM problems (Wx, Wy) and their tile range
+  // the cross-coupled blocks of TS_222_ph in batches: each batch is one Pandya launch, one grouped product and one
+  // scatter launch, on buffers that the batches share
+  std::vector<imsrg::PhBlock> ph_blocks;
+  std::vector<PhBatch> ph_batches;
+  const imsrg::PhBlock* d_ph_blocks = nullptr;
+  const int64_t *d_ph_pre_p = nullptr, *d_ph_pre_s = nullptr;
   const GemmProb* cb_p = nullptr;
   const GemmTile* cb_t = nullptr;
-  std::vector<int> cb_tile_start, cb_tile_n;
+  int64_t ph_sizes[3] = {0, 0, 0};  // CCR, CCX and W elements of the largest batch
+  std::vector<GemmProb> pphh_probs, exc_probs, x_probs;
+  imsrg::OzPlan pphh_oz, exc_oz, x_oz;
+  double* d_nine = nullptr;  // 9j table (DevTLayout::nine)
   const int64_t* seg_start = nullptr;
   const int* seg_len = nullptr;
   const int8_t* seg_w = nullptr;
@@ -96,7 +115,7 @@ struct TensorState {
   // are split into shared regions of the buffer and Wx = -LCC(qa) CCR, Wy = CCX LCC(qb)^T run
   // as single-term problems
   int ph_lcc_nchunks = 0;
-  std::vector<int> ph_chunk_start, ph_chunk_n, ph_tile_start, ph_tile_n;  // per block
+  std::vector<int> ph_chunk_start, ph_chunk_n, ph_tile_start, ph_tile_n;  // per batch
 };
 
 struct imsrg_tensor {
