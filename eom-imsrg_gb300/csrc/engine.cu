@@ -63,6 +63,20 @@ void Ctx::mark(int phase) {
     if (_s != IMSRG_OK) return _s;               \
   } while (0)
 
+imsrg_status Ctx::fork(int k) {
+  if (prof) return IMSRG_OK;
+  CK(cuda(cudaEventRecord(ev_fork[k], stream), "cudaEventRecord(fork)"));
+  CK(cuda(cudaStreamWaitEvent(branch_stream[k], ev_fork[k], 0), "cudaStreamWaitEvent(fork)"));
+  forked[k] = true;
+  return IMSRG_OK;
+}
+imsrg_status Ctx::join(int k) {
+  if (!forked[k]) return IMSRG_OK;
+  forked[k] = false;
+  CK(cuda(cudaEventRecord(ev_join[k], branch_stream[k]), "cudaEventRecord(join)"));
+  return cuda(cudaStreamWaitEvent(stream, ev_join[k], 0), "cudaStreamWaitEvent(join)");
+}
+
 // ---------------------------------------------------------------- device tables
 namespace {
 
@@ -254,6 +268,12 @@ Ctx::~Ctx() {
   if (ev_ext_in) cudaEventDestroy(ev_ext_in);
   if (ev_ext_out) cudaEventDestroy(ev_ext_out);
   if (stream) cudaStreamSynchronize(stream);
+  for (int k = 0; k < kBranches; ++k) {
+    if (branch_stream[k]) cudaStreamSynchronize(branch_stream[k]);
+    if (branch_stream[k]) cudaStreamDestroy(branch_stream[k]);
+    if (ev_fork[k]) cudaEventDestroy(ev_fork[k]);
+    if (ev_join[k]) cudaEventDestroy(ev_join[k]);
+  }
   for (double* p : op_pool) cudaFree(p);
   tc_release();
   graph_release();
@@ -304,18 +324,6 @@ imsrg_status Ctx::pphh_clear(double* w1, double* w2) {
   if (!zero_runs_w2.empty()) {
     k_zero_runs<<<(int)zero_runs_w2.size() / 2, 256, 0, stream>>>(w2, d_zero_runs_w2);
     CK(launched("k_zero_runs"));
-  }
-  return IMSRG_OK;
-}
-
-imsrg_status Ctx::pphh_clear_f(float* w1, float* w2) {
-  if (!zero_runs_w1.empty()) {
-    k_zero_runs_f<<<(int)zero_runs_w1.size() / 2, 256, 0, stream>>>(w1, d_zero_runs_w1);
-    CK(launched("k_zero_runs_f"));
-  }
-  if (!zero_runs_w2.empty()) {
-    k_zero_runs_f<<<(int)zero_runs_w2.size() / 2, 256, 0, stream>>>(w2, d_zero_runs_w2);
-    CK(launched("k_zero_runs_f"));
   }
   return IMSRG_OK;
 }
@@ -381,6 +389,10 @@ imsrg_status Ctx::wcc_products(const double* lcc, int hL, const double* rcc, int
 
 imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, double* RES, int hRES, double* wcc) {
   CK(wcc_products(lcc, hL, rcc, hR, wcc));
+  return ph_recouple(hL, hR, RES, hRES, wcc);
+}
+
+imsrg_status Ctx::ph_recouple(int hL, int hR, double* RES, int hRES, const double* wcc) {
   if (L.n_unique == 0) return IMSRG_OK;
   k_comm222ph<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, wcc, hL, hR, RES, hRES);
   CK(launched("k_comm222ph"));
@@ -390,28 +402,53 @@ imsrg_status Ctx::ph(const double* lcc, int hL, const double* rcc, int hR, doubl
 
 imsrg_status Ctx::commutator(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES, bool with_e0) {
   CK(ensure_workspace());
-  if (precision != IMSRG_PREC_FP64) return tc_commutator(Lp, hL, Rp, hR, RES, hRES, with_e0);
+  const imsrg_status s = precision != IMSRG_PREC_FP64 ? tc_commutator(Lp, hL, Rp, hR, RES, hRES, with_e0)
+                                                      : fp64_commutator(Lp, hL, Rp, hR, RES, hRES, with_e0);
+  for (int k = 0; k < kBranches; ++k) join(k);  // after an error: what a branch has issued is ordered all the same
+  return s;
+}
+
+imsrg_status Ctx::fp64_commutator(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES, bool with_e0) {
   mark(kPhaseStart);
+  const bool groups = L.slab >= kGatherMinSlab;
+  if (groups) CK(gather_prepare());
+  CK(ensure_wcc());
+  // three branches that meet where RES's two-body part is added to: the one-body parts and 122, the ladder's products, and
+  // (main) the cross-coupled products.  A small basis leaves most of the GPU idle in every kernel: one after the other
+  // they took 146 us at eMax 2 and 490 at eMax 6, so 71 and 347; a branch more for the second Pandya pass gave nothing and
+  // costs 8 us of host calls.
+  CK(fork(0));
+  CK(fork(1));
   CK(pandya(Rp, hR, d_rcc));
   CK(pandya(Lp, hL, d_lcc));
   mark(kPhasePandya);
-  if (with_e0) CK(e0(Lp, hL, Rp, hR, RES, nullptr));
-  CK(c111(Lp, hL, Rp, hR, RES));
-  CK(c121(Lp, hL, Rp, hR, RES, hRES));
-  mark(kPhaseOneBody);
-  if (L.slab >= kGatherMinSlab) CK(gather_prepare());
-  if (gp.state > 0 && gp.per_sm[1] > 0 && L.slab >= kGatherMinSlab) {
-    // 122 and the recoupling write the upper triangles only; the ladder update comes last (additions commute) and
-    // writes the lower triangles in the same pass
-    CK(c122_groups<double>(Lp, hL, Rp, hR, RES, hRES));
-    k_comm122<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, Lp, hL, Rp, hR, RES, hRES, gp.d_counter + 1);
-    CK(launched("k_comm122"));
+  CK(on(0, [&]() -> imsrg_status {
+    if (with_e0) CK(e0(Lp, hL, Rp, hR, RES, nullptr));
+    CK(c111(Lp, hL, Rp, hR, RES));
+    CK(c121(Lp, hL, Rp, hR, RES, hRES));
+    mark(kPhaseOneBody);
+    return IMSRG_OK;
+  }));
+  CK(on(1, [&]() { return pphh_products(Lp, hL, Rp, hR, d_w1, d_w2); }));
+  const bool by_groups = groups && gp.state > 0 && gp.per_sm[1] > 0;
+  CK(on(0, [&]() -> imsrg_status {
+    if (by_groups) {  // upper triangles only, as the recoupling: the ladder update comes last and mirrors them
+      CK(c122_groups<double>(Lp, hL, Rp, hR, RES, hRES));
+      k_comm122<<<grid_for(L.n_unique), kThreads, 0, stream>>>(D, Lp, hL, Rp, hR, RES, hRES, gp.d_counter + 1);
+      CK(launched("k_comm122"));
+    } else {
+      CK(c122(Lp, hL, Rp, hR, RES, hRES));
+    }
     mark(kPhase122);
-    CK(pphh_products(Lp, hL, Rp, hR, d_w1, d_w2));
-    CK(c221(hL, hR, RES, hRES, d_w1, d_w2));
-    mark(kPhase221);
-    CK(ensure_wcc());
-    CK(wcc_products(d_lcc, hL, d_rcc, hR, d_wcc));
+    return IMSRG_OK;
+  }));
+  CK(wcc_products(d_lcc, hL, d_rcc, hR, d_wcc));
+  CK(join(0));
+  CK(join(1));
+  CK(fork(0));
+  CK(on(0, [&]() { return c221(hL, hR, RES, hRES, d_w1, d_w2); }));
+  mark(kPhase221);
+  if (by_groups) {
     const int64_t nq = (int64_t)gp.quads.size();
     if (nq) {
       launch_recouple_w((int)std::min<int64_t>((nq + 255) / 256, gp.num_sms * 32), stream, D, gp.d_quads, nq, gp.d_xcol, d_wcc,
@@ -424,16 +461,11 @@ imsrg_status Ctx::commutator(const double* Lp, int hL, const double* Rp, int hR,
       CK(launched("k_pphh_update_mirror"));
     }
     mark(kPhasePphhUpdate);
-    return IMSRG_OK;
+  } else {
+    CK(pphh_accumulate(hL, hR, RES, d_w1, d_w2));
+    CK(ph_recouple(hL, hR, RES, hRES, d_wcc));
   }
-  CK(c122(Lp, hL, Rp, hR, RES, hRES));
-  mark(kPhase122);
-  CK(pphh(Lp, hL, Rp, hR, RES, d_w1, d_w2));
-  CK(c221(hL, hR, RES, hRES, d_w1, d_w2));
-  mark(kPhase221);
-  CK(ensure_wcc());
-  CK(ph(d_lcc, hL, d_rcc, hR, RES, hRES, d_wcc));
-  return IMSRG_OK;
+  return join(0);
 }
 
 imsrg_status Ctx::axpby(const double* A, double ax, const double* B, double bx, double* C) {
@@ -625,6 +657,11 @@ imsrg_status imsrg_ctx_create(const imsrg_basis* b, int32_t device, imsrg_ctx** 
   }
   imsrg_status s = c->cuda(cudaSetDevice(device), "cudaSetDevice");
   if (s == IMSRG_OK) s = c->cuda(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+  for (int k = 0; k < Ctx::kBranches && s == IMSRG_OK; ++k) {
+    s = c->cuda(cudaStreamCreateWithFlags(&c->branch_stream[k], cudaStreamNonBlocking), "cudaStreamCreate(branch)");
+    if (s == IMSRG_OK) s = c->cuda(cudaEventCreateWithFlags(&c->ev_fork[k], cudaEventDisableTiming), "cudaEventCreate");
+    if (s == IMSRG_OK) s = c->cuda(cudaEventCreateWithFlags(&c->ev_join[k], cudaEventDisableTiming), "cudaEventCreate");
+  }
   if (s == IMSRG_OK) s = c->cuda(cudaEventCreateWithFlags(&c->ev_ext_in, cudaEventDisableTiming), "cudaEventCreate");
   if (s == IMSRG_OK) s = c->cuda(cudaEventCreateWithFlags(&c->ev_ext_out, cudaEventDisableTiming), "cudaEventCreate");
   if (s == IMSRG_OK) s = c->upload_tables();

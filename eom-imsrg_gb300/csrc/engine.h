@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/imsrg_gb300.h"
@@ -57,6 +58,8 @@ enum Phase : int {
 // against 32 + 29; eMax 5, 240 thousand, 61 + 37 us against 42 + 35; eMax 10 6.3 + 9.7 ms against 1.3 + 1.8).
 constexpr int64_t kGatherMinSlab = 100000;
 
+// up to this size the mixed commutator runs 122 beside its GEMM (gemm_tc.cu)
+constexpr int64_t kIdleSlab = (int64_t)1 << 22;
 // the word of d_scalars (and of h_scalars) that holds the error of a bounded wait
 constexpr int kErrorSlot = 48;
 
@@ -114,6 +117,23 @@ struct Ctx {
   // kernel launches issued (cumulative) and optional per-phase CUDA-event timing
   int64_t launches = 0;
   bool prof = false;
+  // Side branches of a commutator: fork(k) makes branch k wait for the main stream's work so far, on(k, f) issues f's
+  // launches on it, join(k) makes the main stream wait for them.  Every fork is joined before the call returns, so that
+  // the main stream alone orders what the context does.  With per-phase timing everything stays on the main stream.
+  static constexpr int kBranches = 2;
+  cudaStream_t branch_stream[kBranches] = {};
+  cudaEvent_t ev_fork[kBranches] = {}, ev_join[kBranches] = {};
+  bool forked[kBranches] = {};
+  imsrg_status fork(int k);
+  imsrg_status join(int k);
+  template <class F>
+  imsrg_status on(int k, F&& f) {
+    if (!forked[k]) return f();
+    std::swap(stream, branch_stream[k]);
+    const imsrg_status s = f();
+    std::swap(stream, branch_stream[k]);
+    return s;
+  }
   std::vector<std::pair<int, cudaEvent_t>> prof_marks;
   std::vector<cudaEvent_t> prof_pool;
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
@@ -141,12 +161,13 @@ struct Ctx {
   imsrg_status pphh_accumulate(int hL, int hR, double* RES, const double* w1, const double* w2);
   imsrg_status c221(int hL, int hR, double* RES, int hRES, const double* w1, const double* w2);
   // the same on FP32 W1 / W2 (the mixed commutator's own workspaces, same element offsets)
-  imsrg_status pphh_clear_f(float* w1, float* w2);
   imsrg_status c221_f(int hL, int hR, double* RES, int hRES, const float* w1, const float* w2);
   imsrg_status ensure_wcc();
   imsrg_status wcc_products(const double* lcc, int hL, const double* rcc, int hR, double* wcc);
+  imsrg_status ph_recouple(int hL, int hR, double* RES, int hRES, const double* wcc);
   imsrg_status ph(const double* lcc, int hL, const double* rcc, int hR, double* RES, int hRES, double* wcc);
   imsrg_status commutator(const double* L, int hL, const double* R, int hR, double* RES, int hRES, bool with_e0);
+  imsrg_status fp64_commutator(const double* L, int hL, const double* R, int hR, double* RES, int hRES, bool with_e0);
   imsrg_status axpby(const double* A, double ax, const double* B, double bx, double* C);
   imsrg_status axpy_frob_async(double* Y, double a, const double* X, double scale, int slot, bool with_e0);
   imsrg_status frob_async(const double* op, double scale, int slot);

@@ -918,6 +918,16 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
                                 bool with_e0) {
   const int64_t ncc = L.cc_size;
   mark(kPhaseStart);
+  // W1 and W2 of the ladder in FP32, in the first half of the FP64 workspaces
+  float* w1f = reinterpret_cast<float*>(d_w1);
+  float* w2f = reinterpret_cast<float*>(d_w2);
+  // branch 0: what only needs L and R and keeps few SMs busy (the small products W2, E0, the one-body parts), beside the
+  // operand passes and the GEMM
+  CK_TC(fork(0));
+  // (one after the other they took 156, 292, 560 and 1718 us at eMax 4, 7, 8 and 10, so 91, 229, 482 and 1615).  In bases
+  // that leave SMs idle branch 1 takes 122, beside the GEMM: 84 and 215 us at eMax 4 and 7; at eMax 8 the same, at
+  // eMax 10, where every kernel fills the GPU, 1661.
+  const bool idle = L.slab < kIdleSlab;
   // operands of both tensor-core products: the Pandya tiles (particle-hole) and the split
   // columns of the ladder arrays; then one persistent launch computes the K = npp ladder
   // products W1 and the recoupling input X over the merged tile list
@@ -928,13 +938,46 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
     CK_TC(launched("k_pandya_tc"));
   }
   mark(kPhasePandya);
-  // W1 and W2 of the ladder in FP32, in the first half of the FP64 workspaces
-  float* w1f = reinterpret_cast<float*>(d_w1);
-  float* w2f = reinterpret_cast<float*>(d_w2);
-  CK_TC(pphh_clear_f(w1f, w2f));
+  CK_TC(on(0, [&]() -> imsrg_status {
+    if (!zero_runs_w2.empty()) {
+      k_zero_runs_f<<<(int)zero_runs_w2.size() / 2, 256, 0, stream>>>(w2f, d_zero_runs_w2);
+      CK_TC(launched("k_zero_runs_f"));
+    }
+    if (!tc->small_tiles.empty()) {  // the K = nhh products (W2) on FP32 SIMT
+      GemmOperands ops{};
+      ops.in[kOpL] = Lp; ops.in[kOpR] = Rp;
+      ops.out[kOpW1] = d_w1; ops.out[kOpW2] = d_w2;  // FP32 stores at the same element offsets
+      ops.hL = hL; ops.hR = hR;
+      k_gemm_f32_w<<<(int)tc->small_tiles.size(), 256, 0, stream>>>(tc->d_small_probs, tc->d_small_tiles, ops);
+      CK_TC(launched("k_gemm_f32_w"));
+    }
+    mark(kPhasePphhSmall);
+    if (with_e0) CK_TC(e0(Lp, hL, Rp, hR, RES, nullptr));
+    {  // commutator_111 block by block (one-body operators only couple orbits of one (l, j, tz) block)
+      const int n = L.A * L.A + L.P * L.A + L.P * L.P;
+      k_comm111f<<<(n + 255) / 256, 256, 0, stream>>>(D, Lp, hL, Rp, hR, RES);
+      CK_TC(launched("k_comm111f"));
+    }
+    CK_TC(c121(Lp, hL, Rp, hR, RES, hRES));
+    mark(kPhaseOneBody);
+    return IMSRG_OK;
+  }));
+  if (!zero_runs_w1.empty()) {
+    k_zero_runs_f<<<(int)zero_runs_w1.size() / 2, 256, 0, stream>>>(w1f, d_zero_runs_w1);
+    CK_TC(launched("k_zero_runs_f"));
+  }
   if (!tc->chunks.empty()) CK_TC(tc_split_on(tc->d_split_ops, tc->d_chunks, (int)tc->chunks.size(), Lp, Rp, tc->buf,
                                              tc->slice_elems));
   mark(kPhasePphhSplit);
+  auto c122 = [&]() -> imsrg_status {
+    if (L.n_unique) CK_TC(c122_groups<float>(Lp, hL, Rp, hR, RES, hRES));
+    mark(kPhase122);
+    return IMSRG_OK;
+  };
+  if (idle) {
+    CK_TC(fork(1));
+    CK_TC(on(1, c122));
+  }
   TcOut gout{};
   gout.w1f = w1f;
   gout.xmask = tc->d_xmask;
@@ -945,28 +988,12 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
   else
     CK_TC(tc_gemm(tc->d_pphh_probs, tc->d_pphh_tiles, (int)tc->pphh_tiles.size(), gout, hL, hR, tc->wmax[0]));
   mark(kPhasePphhGemm);
-  if (with_e0) CK_TC(e0(Lp, hL, Rp, hR, RES, nullptr));
-  {  // commutator_111 block by block (one-body operators only couple orbits of one (l, j, tz) block)
-    const int n = L.A * L.A + L.P * L.A + L.P * L.P;
-    k_comm111f<<<(n + 255) / 256, 256, 0, stream>>>(D, Lp, hL, Rp, hR, RES);
-    CK_TC(launched("k_comm111f"));
-  }
-  CK_TC(c121(Lp, hL, Rp, hR, RES, hRES));
-  mark(kPhaseOneBody);
-  if (L.n_unique) {
-    CK_TC(c122_groups<float>(Lp, hL, Rp, hR, RES, hRES));
-  }
-  mark(kPhase122);
-  if (!tc->small_tiles.empty()) {  // the K = nhh products (W2) on FP32 SIMT
-    GemmOperands ops{};
-    ops.in[kOpL] = Lp; ops.in[kOpR] = Rp;
-    ops.out[kOpW1] = d_w1; ops.out[kOpW2] = d_w2;  // FP32 stores at the same element offsets
-    ops.hL = hL; ops.hR = hR;
-    k_gemm_f32_w<<<(int)tc->small_tiles.size(), 256, 0, stream>>>(tc->d_small_probs, tc->d_small_tiles, ops);
-    CK_TC(launched("k_gemm_f32_w"));
-  }
-  mark(kPhasePphhSmall);
-  CK_TC(c221_f(hL, hR, RES, hRES, w1f, w2f));
+  if (!idle) CK_TC(c122());
+  CK_TC(join(0));
+  CK_TC(join(1));
+  // branch 0 again: the one-body part of the ladder, beside the recoupling
+  CK_TC(fork(0));
+  CK_TC(on(0, [&]() { return c221_f(hL, hR, RES, hRES, w1f, w2f); }));
   mark(kPhase221);
   if (!tc->merged) {
     CK_TC(tc_gemm(tc->d_z_probs, tc->d_z_tiles, (int)tc->z_tiles.size(), gout, hL, hR, tc->wmax[1]));
@@ -986,7 +1013,7 @@ imsrg_status Ctx::tc_commutator(const double* Lp, int hL, const double* Rp, int 
     CK_TC(launched("k_pphh_update_mirror"));
   }
   mark(kPhasePphhUpdate);
-  return IMSRG_OK;
+  return join(0);
 }
 
 // ---------------------------------------------------------------- autotuner
