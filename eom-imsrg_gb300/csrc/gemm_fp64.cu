@@ -105,4 +105,49 @@ __global__ void __launch_bounds__(256) k_gemm_fp64(const GemmProb* __restrict__ 
   }
 }
 
+// The same list in 16 x 16 output tiles, one thread an element: for small channels, where a 64 x 64 tile is mostly padding
+// (the FP64 pipe does two FMAs a clock and SM, so a padded tile costs what a full one does) and leaves SMs idle.  The next
+// 16 x 16 blocks of A and B are loaded while the present ones are multiplied.
+__global__ void __launch_bounds__(256) k_gemm_fp64_small(const GemmProb* __restrict__ probs,
+                                                         const GemmTile* __restrict__ tiles, GemmOperands ops) {
+  __shared__ double As[2][16][17];
+  __shared__ double Bs[2][16][17];
+  const GemmTile tile = tiles[blockIdx.x];
+  const GemmProb& P = probs[tile.prob];
+  const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
+  const int gm = tile.m0 + x, gn = tile.n0 + y, M = P.M, N = P.N;
+  double acc = 0.0;
+  int buf = 0;
+  for (int t = 0; t < P.nterm; ++t) {
+    const GemmTerm& T = P.t[t];
+    const double* A = ops.in[T.a_id] + T.a_off;
+    const double* B = ops.in[T.b_id] + T.b_off;
+    const double alpha = alpha_of(T.alpha, ops.hL, ops.hR);
+    const int K = T.K, lda = T.lda, ldb = T.ldb;
+    // lanes along the contiguous index of each operand
+    auto load = [&](int k0, double& a, double& b) {
+      const int am = tile.m0 + (T.ta ? y : x), ak = k0 + (T.ta ? x : y);
+      a = (am < M && ak < K) ? A[T.ta ? ak + (int64_t)am * lda : am + (int64_t)ak * lda] : 0.0;
+      const int bn = tile.n0 + (T.tb ? x : y), bk = k0 + (T.tb ? y : x);
+      b = (bn < N && bk < K) ? B[T.tb ? bn + (int64_t)bk * ldb : bk + (int64_t)bn * ldb] : 0.0;
+    };
+    double a, b;
+    load(0, a, b);
+    for (int k0 = 0; k0 < K; k0 += 16, buf ^= 1) {
+      if (T.ta) As[buf][x][y] = a; else As[buf][y][x] = a;  // [k][m]
+      if (T.tb) Bs[buf][y][x] = b; else Bs[buf][x][y] = b;  // [k][n]
+      __syncthreads();
+      if (k0 + 16 < K) load(k0 + 16, a, b);
+      const int kn = min(16, K - k0);
+      double s = 0.0;
+      for (int k = 0; k < kn; ++k) s = fma(As[buf][k][x], Bs[buf][k][y], s);
+      acc = fma(alpha, s, acc);
+    }
+  }
+  if (gm < M && gn < N) {
+    double* c = ops.out[P.c_id] + P.c_off + gm + (int64_t)gn * P.ldc;
+    *c = P.accum ? *c + acc : acc;
+  }
+}
+
 }  // namespace imsrg

@@ -481,6 +481,20 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   if (P.state) return IMSRG_OK;
   P.state = -1;
   cudaDeviceGetAttribute(&oz_sms, cudaDevAttrMultiProcessorCount, device);
+  double macs = 0.0;
+  for (const GemmProb& g : probs)
+    for (int i = 0; i < g.nterm; ++i)
+      macs += (double)((g.M + 15) / 16 * 16) * ((g.N + 15) / 16 * 16) * g.t[i].K;
+  if (macs < kOzMinMacs) {
+    const std::vector<GemmTile> t = build_tiles(probs, 16, 16);
+    if (t.empty()) return IMSRG_OK;
+    CK_TC(cuda(cudaMalloc(&P.tables, sizeof(GemmTile) * t.size()), "cudaMalloc(FP64 product tiles)"));
+    CK_TC(cuda(cudaMemcpy(P.tables, t.data(), sizeof(GemmTile) * t.size(), cudaMemcpyHostToDevice), "cudaMemcpy(FP64 product tiles)"));
+    P.d_small = static_cast<const GemmTile*>(P.tables);
+    P.nsmall = (int)t.size();
+    P.state = 2;
+    return IMSRG_OK;
+  }
   build_oz_plan(probs, oz_sms, P);
   if (P.tiles.empty()) return IMSRG_OK;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
@@ -528,6 +542,10 @@ imsrg_status Ctx::gemm_fp64(OzPlan& P, const std::vector<GemmProb>& probs, const
                             const GemmTile* d_tiles, int ntiles, const GemmOperands& ops) {
   if (!ntiles) return IMSRG_OK;
   CK_TC(oz_prepare(P, probs));
+  if (P.state == 2) {
+    k_gemm_fp64_small<<<P.nsmall, 256, 0, stream>>>(d_probs, P.d_small, ops);
+    return launched("k_gemm_fp64_small");
+  }
   if (P.state > 0) {
     CK_TC(cuda(cudaMemsetAsync(P.flag, 0, sizeof(int), stream), "memset(non-finite flag)"));
     k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, P.buf, P.exps, P.flag);

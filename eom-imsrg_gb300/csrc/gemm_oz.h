@@ -11,6 +11,10 @@ namespace imsrg {
 constexpr int kOzSlices = 8;     // base-256 digits of an operand element
 constexpr int kOzBlockK = 32;    // K of an operand block (64 bytes of BF16 a row)
 constexpr int kOzTileM = 128;    // rows of an operand block and of an output tile
+// Multiply-adds of a list, in 16 x 16 tiles, from which the digits pay: the FP64 pipe does 0.6 per ns, the digit kernels take
+// about 30 us before they have done any (ladder / cross-coupled list at eMax 4, 5 and 8 M: 56 / 30 us by digits, 32 / 20 on
+// the FP64 pipe; at eMax 5, 33 and 40 M: 74 / 43 and 86 / 74).
+constexpr double kOzMinMacs = 2e7;
 constexpr int kOzTileN = 64;     // widest output tile
 
 // One operand: op(A) as rows of M (or op(B) as rows of N) over K, cut into blocks of 128 rows x 32 K, each block
@@ -40,7 +44,8 @@ struct OzTile {
   int prob, m0, n0, w;
 };
 
-// The digit plan of a problem list; `state` 0: not prepared, 1: ready, -1: the list stays on k_gemm_fp64.
+// The digit plan of a problem list; `state` 0: not prepared, 1: ready, 2: a small list, for k_gemm_fp64_small (its tiles in
+// `tables`), -1: the list stays on k_gemm_fp64.
 struct OzPlan {
   int state = 0;
   std::vector<OzOperand> ops;
@@ -55,6 +60,8 @@ struct OzPlan {
   char* buf = nullptr;   // operand blocks
   int* exps = nullptr;   // row exponents, then the non-finite flag
   int* flag = nullptr;
+  const GemmTile* d_small = nullptr;
+  int nsmall = 0;
   const OzOperand* d_ops = nullptr;
   const OzChunk* d_chunks = nullptr;
   const OzProb* d_probs = nullptr;

@@ -48,6 +48,8 @@ __global__ void k_convert_check(const double* x, const float* y, int64_t n, floa
 // run_if: with a flag, nothing is done unless it is set
 __global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, int ntiles, GemmOperands ops,
                             const int* run_if);
+// 16 x 16 tiles
+__global__ void k_gemm_fp64_small(const GemmProb* probs, const GemmTile* tiles, GemmOperands ops);
 
 // mixed-precision companions (kernels_mixed.cu)
 void launch_pandya_tc(int S, int kind, int nchunks, cudaStream_t stream, const DevLayout& D, const PandyaChunk* chunks,
