@@ -120,7 +120,7 @@ struct Ctx {
   // Side branches of a commutator: fork(k) makes branch k wait for the main stream's work so far, on(k, f) issues f's
   // launches on it, join(k) makes the main stream wait for them.  Every fork is joined before the call returns, so that
   // the main stream alone orders what the context does.  With per-phase timing everything stays on the main stream.
-  static constexpr int kBranches = 2;
+  static constexpr int kBranches = 3;
   cudaStream_t branch_stream[kBranches] = {};
   cudaEvent_t ev_fork[kBranches] = {}, ev_join[kBranches] = {};
   bool forked[kBranches] = {};
@@ -210,6 +210,8 @@ struct Ctx {
   void tensor_release();
   imsrg_status tensor_commutator(TensorState& S, const double* L, int hL, const double* R, int hR, double* RES,
                                  int pieces);
+  imsrg_status tensor_pieces(TensorState& S, const double* L, int hL, const double* R, int hR, double* RES, int pieces);
+  imsrg_status tensor_ladder(TensorState& S, const double* L, int hL, const double* R, int hR, bool exc);
   imsrg_status tensor_frob(TensorState& S, const double* op, double scale, int slot);
   imsrg_status bch_tensor(TensorState& S, const double* G, int hG, double* HS, int max_terms, double conv, int* terms);
   // perturbative triples after the flow (triples.cu)

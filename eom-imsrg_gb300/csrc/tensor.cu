@@ -482,6 +482,50 @@ imsrg_status Ctx::tensor_tc_prepare(TensorState& S) {
 imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, const double* R, int hR, double* RES,
                                     int pieces) {
   CKT(ensure_workspace());
+  if ((pieces & 96) && precision != IMSRG_PREC_FP64 && !(pieces & kTensorExcitation)) CKT(tensor_tc_prepare(S));
+  const imsrg_status s = tensor_pieces(S, Lp, hL, R, hR, RES, pieces);
+  for (int k = 0; k < kBranches; ++k) join(k);  // after an error: what a branch has issued is ordered all the same
+  return s;
+}
+
+// W1 and W2 of TS_222_pp_hh
+imsrg_status Ctx::tensor_ladder(TensorState& S, const double* Lp, int hL, const double* R, int hR, bool exc) {
+  const DevTLayout& T = S.DT;
+  const size_t tb = sizeof(double) * (size_t)T.slab;
+  GemmOperands ops{};
+  ops.in[kOpL] = Lp; ops.in[kOpR] = R;
+  ops.out[kOpW1] = S.w1; ops.out[kOpW2] = S.w2;
+  ops.hL = hL; ops.hR = hR;
+  CKT(cuda(cudaMemsetAsync(S.w1, 0, tb, stream), "memset(tensor w1)"));
+  CKT(cuda(cudaMemsetAsync(S.w2, 0, tb, stream), "memset(tensor w2)"));
+  if (precision != IMSRG_PREC_FP64 && !exc) {  // split-BF16 products through pp pairs
+    CKT(cuda(cudaMemsetAsync(S.w3, 0, tb, stream), "memset(tensor w3)"));
+    CKT(tc_split_on(S.tc_ops, S.tc_chunks, S.tc_nchunks, Lp, R, S.tc_buf, S.tc_slice_elems));
+    TcOut out{};
+    out.f64[kOpW1] = S.w1;
+    out.f64[kTensorOpW3] = S.w3;
+    CKT(tc_gemm_on(S.tc_map, S.tc_slice_rows, S.tc_probs, S.tc_tiles, S.tc_ntiles, out, hL, hR));
+    if (S.n_hh_t) {
+      k_gemm_fp64<<<S.n_hh_t, 256, 0, stream>>>(S.hh_p, S.hh_t, S.n_hh_t, ops, nullptr);
+      CKT(launched("k_gemm_fp64(tensor hh ladder)"));
+    }
+    k_axpby<<<grid_n(T.slab), 256, 0, stream>>>(T.slab, S.w1, 1.0, S.w3, 1.0, S.w1);
+    return launched("k_axpby");
+  }
+  const int nt = exc ? S.n_exc_t : S.n_pphh_t;
+  if (!nt) return IMSRG_OK;
+  if (precision != IMSRG_PREC_FP64) {  // mixed modes: the excitation ladder in FP32
+    k_gemm_f32<<<nt, 256, 0, stream>>>(S.exc_p, S.exc_t, ops);
+    return launched("k_gemm_f32(tensor pphh, excitation)");
+  }
+  return exc ? gemm_fp64(S.exc_oz, S.exc_probs, S.exc_p, S.exc_t, nt, ops)
+             : gemm_fp64(S.pphh_oz, S.pphh_probs, S.pphh_p, S.pphh_t, nt, ops);
+}
+
+// Four branches: the one-body pieces (0), the ladder's products (1), 122 and 212 (2) and the particle-hole term (main),
+// which meet where they add to the same part of RES.  Each alone leaves most of the GPU idle in the bases that this runs
+// on (one after the other: BCH_TENSOR at eMax 4, rank 2 3.2 ms, EOM product at eMax 6 1.29 ms).
+imsrg_status Ctx::tensor_pieces(TensorState& S, const double* Lp, int hL, const double* R, int hR, double* RES, int pieces) {
   const DevTLayout& T = S.DT;
   const int hRES = -hL * hR;
   const double thresh = (pieces & (kTensorExactPh | kTensorExcitation)) ? 0.0 : 1e-6;
@@ -490,90 +534,46 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
   const int exc = (pieces & kTensorExcitation) ? 1 : 0;
   const ElemSegs segs = exc ? S.exc_segs : ElemSegs{};
   const int64_t n2out = exc ? S.exc_n2 : (int64_t)T.n2b;
-  if (L.cc_size) CKT(pandya(Lp, hL, d_lcc));
   const int nob = T.n_ob;
-  if (pieces & 1) {
-    const int64_t n1 = (int64_t)L.A * L.A + (int64_t)L.P * L.A + (int64_t)L.P * L.P;
-    k_ts111<<<grid_n(n1 * 32), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES);
-    CKT(launched("k_ts111"));
-  }
-  if ((pieces & 2) && nob) {
-    k_ts121<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, hRES);
-    CKT(launched("k_ts121"));
-  }
+  for (int k = 0; k < kBranches; ++k) CKT(fork(k));
+  if (L.cc_size) CKT(pandya(Lp, hL, d_lcc));
+  CKT(on(0, [&]() -> imsrg_status {
+    if (pieces & 1) {
+      const int64_t n1 = (int64_t)L.A * L.A + (int64_t)L.P * L.A + (int64_t)L.P * L.P;
+      k_ts111<<<grid_n(n1 * 32), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES);
+      CKT(launched("k_ts111"));
+    }
+    if ((pieces & 2) && nob) {
+      k_ts121<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, hRES);
+      CKT(launched("k_ts121"));
+    }
+    return IMSRG_OK;
+  }));
+  CKT(on(2, [&]() -> imsrg_status {
+    const bool f32 = precision != IMSRG_PREC_FP64;
+    if ((pieces & 8) && n2out) {
+      if (f32)
+        k_ts122f<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
+      else
+        k_ts122<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
+      CKT(launched("k_ts122"));
+    }
+    if ((pieces & 16) && n2out) {
+      if (f32)
+        k_ts212f<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
+      else
+        k_ts212<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
+      CKT(launched("k_ts212"));
+    }
+    return IMSRG_OK;
+  }));
+  if (pieces & 32) CKT(on(1, [&]() { return tensor_ladder(S, Lp, hL, R, hR, exc != 0); }));
   if ((pieces & 4) && nob) {
-    k_ts211<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, d_lcc, hL, R, hR, RES, hRES);
-    CKT(launched("k_ts211"));
-  }
-  if ((pieces & 8) && n2out) {
-    if (precision != IMSRG_PREC_FP64)
-      k_ts122f<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
-    else
-      k_ts122<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
-    CKT(launched("k_ts122"));
-  }
-  if ((pieces & 16) && n2out) {
-    if (precision != IMSRG_PREC_FP64)
-      k_ts212f<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
-    else
-      k_ts212<<<grid_n(n2out), 256, 0, stream>>>(D, T, Lp, hL, R, hR, RES, segs);
-    CKT(launched("k_ts212"));
-  }
-  if ((pieces & 32) && precision != IMSRG_PREC_FP64 && !exc) {  // split-BF16 products through pp pairs
-    CKT(tensor_tc_prepare(S));
-    const size_t tb = sizeof(double) * (size_t)T.slab;
-    CKT(cuda(cudaMemsetAsync(S.w1, 0, tb, stream), "memset(tensor w1)"));
-    CKT(cuda(cudaMemsetAsync(S.w2, 0, tb, stream), "memset(tensor w2)"));
-    CKT(cuda(cudaMemsetAsync(S.w3, 0, tb, stream), "memset(tensor w3)"));
-    CKT(tc_split_on(S.tc_ops, S.tc_chunks, S.tc_nchunks, Lp, R, S.tc_buf, S.tc_slice_elems));
-    TcOut out{};
-    out.f64[kOpW1] = S.w1;
-    out.f64[kTensorOpW3] = S.w3;
-    CKT(tc_gemm_on(S.tc_map, S.tc_slice_rows, S.tc_probs, S.tc_tiles, S.tc_ntiles, out, hL, hR));
-    if (S.n_hh_t) {
-      GemmOperands ops{};
-      ops.in[kOpL] = Lp; ops.in[kOpR] = R;
-      ops.out[kOpW1] = S.w1; ops.out[kOpW2] = S.w2;
-      ops.hL = hL; ops.hR = hR;
-      k_gemm_fp64<<<S.n_hh_t, 256, 0, stream>>>(S.hh_p, S.hh_t, S.n_hh_t, ops, nullptr);
-      CKT(launched("k_gemm_fp64(tensor hh ladder)"));
-    }
-    k_axpby<<<grid_n(T.slab), 256, 0, stream>>>(T.slab, S.w1, 1.0, S.w3, 1.0, S.w1);
-    CKT(launched("k_axpby"));
-    if (T.n2b) {
-      k_ts_pphh_update<<<grid_n(T.n2b), 256, 0, stream>>>(T.n2b, S.T.goff.empty() ? 0 : S.T.goff[0], RES, S.w1, S.w2);
-      CKT(launched("k_ts_pphh_update"));
-    }
-    if (nob) {
-      k_ts221<<<nob, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
-      CKT(launched("k_ts221"));
-    }
-  } else if (pieces & 32) {
-    const size_t tb = sizeof(double) * (size_t)T.slab;
-    CKT(cuda(cudaMemsetAsync(S.w1, 0, tb, stream), "memset(tensor w1)"));
-    CKT(cuda(cudaMemsetAsync(S.w2, 0, tb, stream), "memset(tensor w2)"));
-    const int nt = exc ? S.n_exc_t : S.n_pphh_t;
-    if (nt) {
-      GemmOperands ops{};
-      ops.in[kOpL] = Lp; ops.in[kOpR] = R;
-      ops.out[kOpW1] = S.w1; ops.out[kOpW2] = S.w2;
-      ops.hL = hL; ops.hR = hR;
-      if (exc && precision != IMSRG_PREC_FP64) {  // mixed modes: the excitation ladder in FP32
-        k_gemm_f32<<<nt, 256, 0, stream>>>(S.exc_p, S.exc_t, ops);
-        CKT(launched("k_gemm_f32(tensor pphh, excitation)"));
-      } else {
-        CKT(exc ? gemm_fp64(S.exc_oz, S.exc_probs, S.exc_p, S.exc_t, nt, ops)
-                : gemm_fp64(S.pphh_oz, S.pphh_probs, S.pphh_p, S.pphh_t, nt, ops));
-      }
-    }
-    if (T.n2b) {
-      k_ts_pphh_update<<<grid_n(T.n2b), 256, 0, stream>>>(T.n2b, S.T.goff.empty() ? 0 : S.T.goff[0], RES, S.w1, S.w2);
-      CKT(launched("k_ts_pphh_update"));
-    }
-    if (nob) {
-      k_ts221<<<nob, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
-      CKT(launched("k_ts221"));
-    }
+    CKT(fork(0));  // after the cross-coupled L
+    CKT(on(0, [&]() -> imsrg_status {
+      k_ts211<<<(nob * 32 + 255) / 256, 256, 0, stream>>>(D, T, d_lcc, hL, R, hR, RES, hRES);
+      return launched("k_ts211");
+    }));
   }
   if ((pieces & 64) && exc) {  // excitation mode: packed CCR / CCX of all blocks (FP32 products in mixed modes)
     if (S.x_nblk) {
@@ -596,6 +596,7 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
           CKT(gemm_fp64(S.x_oz, S.x_probs, S.x_p, S.x_t, S.x_n_t, ops));
         }
       }
+      CKT(join(2));
       k_ts222ph_scatter_exc<<<grid_n(S.x_ns), 256, 0, stream>>>(D, T, S.x_blk, S.x_pre_s, S.x_nblk, S.d_pe, S.d_hp,
                                                                  S.x_buf[2], S.x_buf[3], hL, hR, RES);
       CKT(launched("k_ts222ph_scatter_exc"));
@@ -603,7 +604,6 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
   } else if (pieces & 64) {
     const bool mixed = precision != IMSRG_PREC_FP64;  // split-BF16 cross-coupled products
     if (mixed) {
-      CKT(tensor_tc_prepare(S));
       CKT(tc_split_on(S.tc_ops, S.tc_chunks + S.tc_nchunks, S.ph_lcc_nchunks, d_lcc, nullptr, S.tc_buf, S.tc_slice_elems));
     }
     for (size_t i = 0; i < S.ph_batches.size(); ++i) {
@@ -624,12 +624,28 @@ imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, co
         ops.hL = hL; ops.hR = hR;
         CKT(gemm_fp64(B.oz, B.probs, S.cb_p + B.prob0, S.cb_t + B.tile0, B.ntiles, ops));
       }
+      CKT(join(2));
       k_ts222ph_scatter<<<grid_n(B.ns), 256, 0, stream>>>(D, T, S.d_ph_blocks + B.b0, S.d_ph_pre_s + B.pre0, B.n, S.wx, S.wy,
                                                           hL, hR, thresh, RES);
       CKT(launched("k_ts222ph_scatter"));
     }
   }
-  return IMSRG_OK;
+  CKT(join(2));
+  CKT(join(1));
+  if (pieces & 32) {
+    if (nob) {  // after the other one-body pieces, beside the two-body update
+      CKT(fork(0));
+      CKT(on(0, [&]() -> imsrg_status {
+        k_ts221<<<nob, 256, 0, stream>>>(D, T, S.w1, S.w2, hL * hR, RES, hRES);
+        return launched("k_ts221");
+      }));
+    }
+    if (T.n2b) {
+      k_ts_pphh_update<<<grid_n(T.n2b), 256, 0, stream>>>(T.n2b, S.T.goff.empty() ? 0 : S.T.goff[0], RES, S.w1, S.w2);
+      CKT(launched("k_ts_pphh_update"));
+    }
+  }
+  return join(0);
 }
 
 imsrg_status Ctx::tensor_frob(TensorState& S, const double* op, double scale, int slot) {
