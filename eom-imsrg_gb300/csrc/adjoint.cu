@@ -121,25 +121,77 @@ void Ctx::adjoint_release() {
 imsrg_status Ctx::commutator_vjp(const double* Lp, int hL, const double* Rp, int hR, int hRES, bool with_e0,
                                  const double* Cb, double* Lb, double* Rb) {
   CKA(adjoint_prepare());
+  const imsrg_status s = vjp_pieces(Lp, hL, Rp, hR, hRES, with_e0, Cb, Lb, Rb);
+  for (int k = 0; k < kBranches; ++k) join(k);  // after an error: what a branch has issued is ordered all the same
+  return s;
+}
+
+// The pieces carry the cotangent of RES backwards one after the other; what each makes of it for L and R goes on beside the
+// next: the WCC transposes and the Pandya transposes on the main stream, the ladder's on branch 1, 122, 121, 111 and E0 on
+// branch 2.  Everything that adds to Lb and Rb does so atomically.
+imsrg_status Ctx::vjp_pieces(const double* Lp, int hL, const double* Rp, int hR, int hRES, bool with_e0, const double* Cb,
+                             double* Lb, double* Rb) {
   const Layout& l = L;
   const size_t sb = sizeof(double) * (size_t)l.slab;
   AdjointState& a = *adj;
+  CKA(fork(0));
   CKA(cuda(cudaMemcpyAsync(a.cb, Cb, sb, cudaMemcpyDeviceToDevice, stream), "copy cotangent"));
   CKA(cuda(cudaMemsetAsync(d_w1, 0, sb, stream), "memset(w1b)"));
   CKA(cuda(cudaMemsetAsync(d_w2, 0, sb, stream), "memset(w2b)"));
   if (l.cc_size) {
-    CKA(cuda(cudaMemsetAsync(a.lccb, 0, sizeof(double) * l.cc_size, stream), "memset(LCCb)"));
-    CKA(cuda(cudaMemsetAsync(a.rccb, 0, sizeof(double) * l.cc_size, stream), "memset(RCCb)"));
     CKA(cuda(cudaMemsetAsync(a.wccb, 0, sizeof(double) * l.wcc_size, stream), "memset(WCCb)"));
-    // forward Pandya transforms (inputs of the WCC transposes)
-    CKA(pandya(Lp, hL, d_lcc));
-    CKA(pandya(Rp, hR, d_rcc));
+    CKA(on(0, [&]() -> imsrg_status {
+      CKA(cuda(cudaMemsetAsync(a.lccb, 0, sizeof(double) * l.cc_size, stream), "memset(LCCb)"));
+      CKA(cuda(cudaMemsetAsync(a.rccb, 0, sizeof(double) * l.cc_size, stream), "memset(RCCb)"));
+      // forward Pandya transforms (inputs of the WCC transposes)
+      CKA(pandya(Lp, hL, d_lcc));
+      return pandya(Rp, hR, d_rcc);
+    }));
   }
   const int pm = hL * hR;
   if (l.n_unique) {  // 222_ph: RES cotangent -> WCC cotangent -> LCC / RCC cotangents
     k_vjp_222ph<<<grid_of(l.n_unique), 256, 0, stream>>>(D, a.cb, hL, hR, hRES, a.wccb);
     CKA(launched("k_vjp_222ph"));
   }
+  CKA(fork(1));
+  CKA(on(1, [&]() -> imsrg_status {
+    if (D.n_ob) {  // 221: one-body cotangent -> w1 / w2 cotangents
+      k_vjp_221<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, pm, a.cb, hRES, d_w1, d_w2);
+      CKA(launched("k_vjp_221"));
+    }
+    // 222_pp_hh: RES accumulation -> W cotangents -> L / R cotangents
+    k_vjp_pphh_wbar<<<grid_of(l.slab - l.goff[0]), 256, 0, stream>>>(D, a.cb, d_w1, d_w2, (double)pm);
+    CKA(launched("k_vjp_pphh_wbar"));
+    CKA(fork(2));  // 122 clears the two-body cotangent once the ladder has read it
+    if (!a.n_pphh_t) return IMSRG_OK;
+    GemmOperands ops{};
+    ops.in[kOpL] = Lp; ops.in[kOpR] = Rp; ops.in[kOpW1] = d_w1; ops.in[kOpW2] = d_w2;
+    ops.out[kOpL] = Lb; ops.out[kOpR] = Rb;
+    ops.hL = hL; ops.hR = hR;
+    return gemm_fp64(a.pphh_oz, a.pphh_probs, a.pphh_p, a.pphh_t, a.n_pphh_t, ops);
+  }));
+  CKA(on(2, [&]() -> imsrg_status {
+    if (l.n_unique) {
+      k_vjp_122<<<grid_of(l.n_unique), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);
+      CKA(launched("k_vjp_122"));
+    }
+    if (D.n_ob) {
+      k_vjp_121<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);
+      CKA(launched("k_vjp_121"));
+    }
+    {
+      const int64_t n1 = (int64_t)l.A * l.A + (int64_t)l.P * l.A + (int64_t)l.P * l.P;
+      k_vjp_111<<<grid_of(2 * n1 * 32), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, Lb, Rb);
+      CKA(launched("k_vjp_111"));
+    }
+    if (with_e0) {
+      dim3 grid(16, l.nblocks + 1);
+      k_vjp_e0<<<grid, 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, Lb, Rb);
+      CKA(launched("k_vjp_e0"));
+    }
+    return IMSRG_OK;
+  }));
+  CKA(join(0));
   if (a.n_wcc_t) {
     GemmOperands ops{};
     ops.in[kOpWCC] = a.wccb; ops.in[kOpLCC] = d_lcc; ops.in[kOpRCC] = d_rcc;
@@ -147,45 +199,14 @@ imsrg_status Ctx::commutator_vjp(const double* Lp, int hL, const double* Rp, int
     ops.hL = hL; ops.hR = hR;
     CKA(gemm_fp64(a.wcc_oz, a.wcc_probs, a.wcc_p, a.wcc_t, a.n_wcc_t, ops));
   }
-  if (D.n_ob) {  // 221: one-body cotangent -> w1 / w2 cotangents
-    k_vjp_221<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, pm, a.cb, hRES, d_w1, d_w2);
-    CKA(launched("k_vjp_221"));
-  }
-  // 222_pp_hh: RES accumulation -> W cotangents -> L / R cotangents
-  k_vjp_pphh_wbar<<<grid_of(l.slab - l.goff[0]), 256, 0, stream>>>(D, a.cb, d_w1, d_w2, (double)pm);
-  CKA(launched("k_vjp_pphh_wbar"));
-  if (a.n_pphh_t) {
-    GemmOperands ops{};
-    ops.in[kOpL] = Lp; ops.in[kOpR] = Rp; ops.in[kOpW1] = d_w1; ops.in[kOpW2] = d_w2;
-    ops.out[kOpL] = Lb; ops.out[kOpR] = Rb;
-    ops.hL = hL; ops.hR = hR;
-    CKA(gemm_fp64(a.pphh_oz, a.pphh_probs, a.pphh_p, a.pphh_t, a.n_pphh_t, ops));
-  }
-  if (l.n_unique) {
-    k_vjp_122<<<grid_of(l.n_unique), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);
-    CKA(launched("k_vjp_122"));
-  }
-  if (D.n_ob) {
-    k_vjp_121<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);
-    CKA(launched("k_vjp_121"));
-  }
-  {
-    const int64_t n1 = (int64_t)l.A * l.A + (int64_t)l.P * l.A + (int64_t)l.P * l.P;
-    k_vjp_111<<<grid_of(2 * n1 * 32), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, Lb, Rb);
-    CKA(launched("k_vjp_111"));
-  }
-  if (with_e0) {
-    dim3 grid(16, l.nblocks + 1);
-    k_vjp_e0<<<grid, 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, Lb, Rb);
-    CKA(launched("k_vjp_e0"));
-  }
   if (l.cc_size) {
     k_pandya_vjp<<<grid_of(l.cc_size), 256, 0, stream>>>(D, hL, a.lccb, Lb);
     CKA(launched("k_pandya_vjp"));
     k_pandya_vjp<<<grid_of(l.cc_size), 256, 0, stream>>>(D, hR, a.rccb, Rb);
     CKA(launched("k_pandya_vjp"));
   }
-  return IMSRG_OK;
+  CKA(join(1));
+  return join(2);
 }
 
 imsrg_status Ctx::white_vjp(const double* H, int hH, const double* ETAb, double* Hb) {

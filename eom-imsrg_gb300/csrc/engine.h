@@ -201,6 +201,8 @@ struct Ctx {
   void adjoint_release();
   imsrg_status commutator_vjp(const double* L, int hL, const double* R, int hR, int hRES, bool with_e0,
                               const double* Cb, double* Lb, double* Rb);
+  imsrg_status vjp_pieces(const double* L, int hL, const double* R, int hR, int hRES, bool with_e0, const double* Cb,
+                          double* Lb, double* Rb);
   imsrg_status white_vjp(const double* H, int hH, const double* ETAb, double* Hb);
   imsrg_status dot(const double* A, const double* B, double* out);
 

@@ -33,7 +33,7 @@ struct GemmProb {
   int ldc;
   int c_id;
   int nterm;
-  int accum;  // 0: C = sum, 1: C += sum
+  int accum;  // 0: C = sum, 1: C += sum (atomically)
   GemmTerm t[kMaxTerms];
 };
 

@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(256) k_gemm_fp64(const GemmProb* __restrict__ 
         const int gm = tile.m0 + tx + 16 * i, gn = tile.n0 + ty + 16 * j;
         if (gm < P.M && gn < P.N) {
           double* c = C + gm + (int64_t)gn * P.ldc;
-          *c = P.accum ? *c + acc[i][j] : acc[i][j];
+          if (P.accum) atomicAdd(c, acc[i][j]);  // other kernels may add to the same elements
+          else *c = acc[i][j];
         }
       }
   }
@@ -146,7 +147,8 @@ __global__ void __launch_bounds__(256) k_gemm_fp64_small(const GemmProb* __restr
   }
   if (gm < M && gn < N) {
     double* c = ops.out[P.c_id] + P.c_off + gm + (int64_t)gn * P.ldc;
-    *c = P.accum ? *c + acc : acc;
+    if (P.accum) atomicAdd(c, acc);
+    else *c = acc;
   }
 }
 

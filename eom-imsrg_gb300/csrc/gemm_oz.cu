@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int nterm = P.nterm;
       double* C = out.out[P.c_id] + P.c_off + m + (int64_t)n * P.ldc;
       const int M = P.M, N = P.N, ldc = P.ldc, nn = N - n;
-      bool add = P.accum != 0;
+      const bool accum = P.accum != 0;
       for (int term = 0; term < nterm && ok; ++term) {
         const OzTerm& T = P.t[term];
         const int nchunk = (T.nkb + kChunkBlocks - 1) / kChunkBlocks;
@@ -341,7 +341,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int c = 0; c < nchunk && ok; ++c, ++cc) {
 #pragma unroll
           for (int d = S - 1; d >= 0; --d) {
-            if (!mbar_wait(&dfull[d], cc & 1, abort_flag, err, 4, wait_ns)) { ok = false; break; }
+            // the warp goes on or gives up as one (the TMEM loads below are the whole warp's)
+            ok = __all_sync(0xffffffffu, mbar_wait(&dfull[d], cc & 1, abort_flag, err, 4, wait_ns));
+            if (!ok) break;
             tc_fence_after();
             if (mine) {
 #pragma unroll
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (lane == 0) mbar_arrive(&dempty[d]);
           }
         }
-        if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+        if (!ok) break;
         if (!mine) continue;
         const int sel = T.alpha & 3;
         const bool neg = ((sel == kAlphaHL && out.hL < 0) || (sel == kAlphaHR && out.hR < 0)) != ((T.alpha & kAlphaNeg) != 0);
@@ -378,11 +380,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int j = 0; j < 16; ++j) {
           double v = oz_value(H[j], L[j], neg, ea + __shfl_sync(0xffffffffu, eb, j));
           if (m < M && j < nn) {
-            if (add) v += C[(int64_t)j * ldc];
-            C[(int64_t)j * ldc] = v;
+            double* c = C + (int64_t)j * ldc;
+            if (accum) {  // a reduction: other kernels may add to the same elements
+              atomicAdd(c, v);
+            } else {
+              if (term > 0) v += *c;
+              *c = v;
+            }
           }
         }
-        add = true;  // later terms add to the first
       }
     }
   }

@@ -371,8 +371,8 @@ __global__ void k_vjp_e0(DevLayout D, const double* __restrict__ L, int hL, cons
   const int64_t o = D.goff[q * 6 + 2];
   const double w = -2.0 * hR * (D.lamJ[q] + 1) * eb;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    Lb[o + t] += w * R[o + t];
-    Rb[o + t] += w * L[o + t];
+    atomicAdd(Lb + o + t, w * R[o + t]);
+    atomicAdd(Rb + o + t, w * L[o + t]);
   }
 }
 
