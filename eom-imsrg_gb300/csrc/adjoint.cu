@@ -22,7 +22,8 @@ __global__ void k_vjp_222ph(DevLayout D, double* cb, int hL, int hR, int hRES, d
 __global__ void k_vjp_221(DevLayout D, int pm, double* cb, int hRES, double* w1b, double* w2b);
 __global__ void k_vjp_pphh_wbar(DevLayout D, const double* cb, double* w1b, double* w2b, double pm);
 __global__ void k_vjp_122(DevLayout D, const double* L, int hL, const double* R, int hR, double* cb, int hRES,
-                          double* Lb, double* Rb);
+                          double* Lb, double* Rb, double* F, int nsame);
+__global__ void k_vjp_122_sum(DevLayout D, const double* F, int nsame, int hL, int hR, double* Lb, double* Rb);
 __global__ void k_vjp_121(DevLayout D, const double* L, int hL, const double* R, int hR, double* cb, int hRES,
                           double* Lb, double* Rb);
 __global__ void k_vjp_111(DevLayout D, const double* L, int hL, const double* R, int hR, const double* cb,
@@ -44,6 +45,7 @@ struct AdjointState {
   double* wccb = nullptr;   // cotangent of WCC (FP64, wcc_size)
   double* monob = nullptr;  // N x N monopole cotangents
   double* partial = nullptr;
+  double* fpart = nullptr;  // one-body cotangents of 122, a copy for each lane
   void* tables = nullptr;
   const GemmProb* pphh_p = nullptr;
   const GemmTile* pphh_t = nullptr;
@@ -78,6 +80,7 @@ imsrg_status Ctx::adjoint_prepare() {
   CKA(cuda(cudaMalloc(&adj->wccb, sizeof(double) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(WCCb)"));
   CKA(cuda(cudaMalloc(&adj->monob, sizeof(double) * (size_t)l.N * l.N), "cudaMalloc(monopole cotangents)"));
   CKA(cuda(cudaMalloc(&adj->partial, sizeof(double) * kDotBlocks), "cudaMalloc(dot partials)"));
+  CKA(cuda(cudaMalloc(&adj->fpart, sizeof(double) * 128 * l.same_list.size()), "cudaMalloc(one-body cotangents)"));
   const auto pp = build_pphh_vjp_problems(l.nblocks, l.ncls, l.goff);
   const auto pt = build_tiles(pp, 64, 64);
   const auto wp = build_wcc_vjp_problems(l.ncc, l.cc_rlen, l.cc_nph, l.cc_off, l.wcc_off);
@@ -110,7 +113,7 @@ imsrg_status Ctx::adjoint_prepare() {
 void Ctx::adjoint_release() {
   if (!adj) return;
   for (void* p : {(void*)adj->cb, (void*)adj->lccb, (void*)adj->rccb, (void*)adj->wccb, (void*)adj->monob,
-                  (void*)adj->partial, adj->tables})
+                  (void*)adj->partial, (void*)adj->fpart, adj->tables})
     if (p) cudaFree(p);
   oz_release(adj->pphh_oz);
   oz_release(adj->wcc_oz);
@@ -172,8 +175,12 @@ imsrg_status Ctx::vjp_pieces(const double* Lp, int hL, const double* Rp, int hR,
   }));
   CKA(on(2, [&]() -> imsrg_status {
     if (l.n_unique) {
-      k_vjp_122<<<grid_of(l.n_unique), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);
+      const int nsame = (int)l.same_list.size();
+      CKA(cuda(cudaMemsetAsync(a.fpart, 0, sizeof(double) * 128 * (size_t)nsame, stream), "memset(one-body cotangents)"));
+      k_vjp_122<<<grid_of(l.n_unique), 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb, a.fpart, nsame);
       CKA(launched("k_vjp_122"));
+      k_vjp_122_sum<<<(2 * l.N * 32 + 255) / 256, 256, 0, stream>>>(D, a.fpart, nsame, hL, hR, Lb, Rb);
+      CKA(launched("k_vjp_122_sum"));
     }
     if (D.n_ob) {
       k_vjp_121<<<(D.n_ob * 32 + 255) / 256, 256, 0, stream>>>(D, Lp, hL, Rp, hR, a.cb, hRES, Lb, Rb);

@@ -201,8 +201,14 @@ __global__ void k_vjp_pphh_wbar(DevLayout D, const double* __restrict__ cb, doub
 
 // ---------------------------------------------------------------- 122
 // transpose of k_comm122 (which assigns every 2b element)
+// Every term is a reduction at L2.  The one-body ones fall on the few hundred elements inside (l, j, tz) blocks, often the
+// same one for all lanes: each lane has a copy of its own of them in F, [(row or column, orbit, position in its block)][L or
+// R][lane], so that a warp's reductions are one contiguous row (k_vjp_122_sum adds the copies up).  To the elements
+// themselves they took 0.41 ms at eMax 6 (commutator_vjp 0.93 -> 0.82 ms with the copies).
 __global__ void k_vjp_122(DevLayout D, const double* __restrict__ L, int hL, const double* __restrict__ R, int hR,
-                          double* __restrict__ cb, int hRES, double* __restrict__ Lb, double* __restrict__ Rb) {
+                          double* __restrict__ cb, int hRES, double* __restrict__ Lb, double* __restrict__ Rb,
+                          double* __restrict__ F, int nsame) {
+  const int lane = threadIdx.x & 31;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < D.n_unique; u += (int64_t)gridDim.x * blockDim.x) {
     int q, g, IX, JX, a, b, c, d;
     decode_pairs(D, u, q, g, IX, JX, a, b, c, d);
@@ -220,39 +226,57 @@ __global__ void k_vjp_122(DevLayout D, const double* __restrict__ L, int hL, con
     if (s == 0.0) continue;
     const int JT = D.lamJ[q];
     // term sign * (f(L; x, y) v(R; ...) - f(R; x, y) v(L; ...))
-    auto term = [&](int fx, int fy, int va, int vb, int vc, int vd, double sign) {
+    auto term = [&](int fx, int fy, int va, int vb, int vc, int vd, double sign, int e) {
       VRef r;
       if (!d_vref(D, va, vb, vc, vd, JT, r)) return;
       const FRef f = d_fref(D, fx, fy);
       const double vR = R[r.idx] * vfac(r, hR), vL = L[r.idx] * vfac(r, hL);
       const double fL = fval(L, f, hL), fR = fval(R, f, hR);
       const double ss = sign * s;
-      atomicAdd(Lb + f.idx, ss * vR * (f.herm ? hL : 1));
+      atomicAdd(F + (int64_t)e * 64 + lane, ss * vR);
       atomicAdd(Rb + r.idx, ss * fL * vfac(r, hR));
-      atomicAdd(Rb + f.idx, -ss * vL * (f.herm ? hR : 1));
+      atomicAdd(F + (int64_t)e * 64 + 32 + lane, -ss * vL);
       atomicAdd(Lb + r.idx, -ss * fR * vfac(r, hL));
     };
     for (int t = 0, s0 = D.same_start[a], n = D.same_count[a]; t < n; ++t) {
       const int i = D.same_list[s0 + t];
-      term(a, i, i, b, c, d, 1.0);
+      term(a, i, i, b, c, d, 1.0, s0 + t);
     }
     for (int t = 0, s0 = D.same_start[b], n = D.same_count[b]; t < n; ++t) {
       const int i = D.same_list[s0 + t];
-      term(b, i, a, i, c, d, 1.0);
+      term(b, i, a, i, c, d, 1.0, s0 + t);
     }
     for (int t = 0, s0 = D.same_start[c], n = D.same_count[c]; t < n; ++t) {
       const int i = D.same_list[s0 + t];
-      term(i, c, a, b, i, d, -1.0);
+      term(i, c, a, b, i, d, -1.0, nsame + s0 + t);
     }
     for (int t = 0, s0 = D.same_start[d], n = D.same_count[d]; t < n; ++t) {
       const int i = D.same_list[s0 + t];
-      term(i, d, a, b, c, i, -1.0);
+      term(i, d, a, b, c, i, -1.0, nsame + s0 + t);
     }
   }
 }
 
 // ---------------------------------------------------------------- 121
 // transpose of k_comm121: one warp per one-body output
+// the lanes' copies into the cotangents of f: a warp per (row or column, orbit)
+__global__ void k_vjp_122_sum(DevLayout D, const double* __restrict__ F, int nsame, int hL, int hR, double* __restrict__ Lb,
+                              double* __restrict__ Rb) {
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (w >= 2 * D.N) return;
+  const bool col = w >= D.N;
+  const int x = col ? w - D.N : w;
+  for (int t = 0, s0 = D.same_start[x], n = D.same_count[x]; t < n; ++t) {
+    const int i = D.same_list[s0 + t];
+    const double* f64 = F + (int64_t)((col ? nsame : 0) + s0 + t) * 64;
+    const double gL = warp_sum(f64[lane]), gR = warp_sum(f64[32 + lane]);
+    if (lane) continue;
+    const FRef f = col ? d_fref(D, i, x) : d_fref(D, x, i);
+    atomicAdd(Lb + f.idx, gL * (f.herm ? hL : 1));
+    atomicAdd(Rb + f.idx, gR * (f.herm ? hR : 1));
+  }
+}
+
 __global__ void k_vjp_121(DevLayout D, const double* __restrict__ L, int hL, const double* __restrict__ R, int hR,
                           double* __restrict__ cb, int hRES, double* __restrict__ Lb, double* __restrict__ Rb) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
