@@ -761,7 +761,9 @@ imsrg_status Ctx::tc_prepare(int mode) {
   CK_TC(cuda(cudaMalloc(&tc->d_mem, pk.buf.size()), "cudaMalloc(tc tables)"));
   CK_TC(cuda(cudaMemcpy(tc->d_mem, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tc tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(tc->d_mem) + f.first;
-  tc->recouple_ctas = tc->num_sms * 32;
+  // CTAs of the recoupling: about one wave where the quadruples are few, many short ones where their lengths would
+  // otherwise leave a long tail (commutator at eMax 7 212 us with 32 a SM, 207 with 8; eMax 10 1606 with 32, 1579 with 128)
+  tc->recouple_ctas = tc->num_sms * (gp.quads.size() < ((size_t)1 << 20) ? 8 : 128);
   // tile lists: the most tiles come with 128-wide tiles
   tc->tile_cap_pphh = make_tiles(tc->pphh_probs, 128, false).size();
   tc->tile_cap_z = make_tiles(tc->z_probs, 128, false).size();
@@ -770,6 +772,12 @@ imsrg_status Ctx::tc_prepare(int mode) {
              "cudaMalloc(GEMM tiles)"));
   tc->d_pphh_tiles = tc->d_tile_mem;
   tc->d_z_tiles = tc->d_tile_mem + tc->tile_cap_pphh;
+  // two BF16 slices: 256-wide tiles in problem order (neighbouring tiles share operand rows in L2; bf16x3 commutator at
+  // eMax 10 1606 -> 1570 us, eMax 8 422 -> 418); three slices and TF32 are as fast or faster in 128-wide ones, longest first
+  if (S == 2 && kind == kKindBF16) {
+    for (int& w : tc->wmax) w = 256;
+    tc->gemm_order = 1;
+  }
   CK_TC(tc_set_tiles(tc->wmax, tc->narrow, tc->gemm_order));
 
   // tensor map over the whole operand buffer: rows of 64 bf16 (128 bytes), box 64 x 128
