@@ -54,7 +54,9 @@ struct HFState {
   std::vector<int> row_off, col_off;
   int nrow = 0, ncol = 0, ndp = 0;
   std::vector<int> grp_b1, grp_b2;
-  std::vector<int4> tasks;
+  std::vector<int4> tasks;  // ncta sub-blocks for a CTA each, then those for a warp each
+  int64_t ncta = 0;
+  int warp_pairs = 0;  // most orbit pairs of a warp's sub-block
   HFDev dev{};
   void* tables = nullptr;
   double* d_M = nullptr;
@@ -63,6 +65,8 @@ struct HFState {
 };
 
 namespace {
+
+constexpr int kHFWarpElems = 128;  // largest sub-block that a warp transforms by itself
 
 // ---------------------------------------------------------------- device kernels
 // M[r + nrow*c] = sum_J (J+1) v_elem(i, g, j, h, J) for row r = (i, j), column c = (g, h)
@@ -78,112 +82,155 @@ __global__ void k_hf_mean_field(DevLayout D, HFDev H, const double* op, int herm
   }
 }
 
-// out[e] = sum_a C[a + i*n] in[e + (a - i)*stride], i = (e / stride) % n: one index of the
-// four-index tensor transformed by the block's coefficient matrix C (column-major n x n)
-__device__ __forceinline__ void hf_mode(const double* __restrict__ in, double* __restrict__ out, int ntot, int n,
-                                        int stride, const double* __restrict__ C) {
-  for (int e = threadIdx.x; e < ntot; e += blockDim.x) {
-    const int i = (e / stride) % n;
+// Pair (x in block b1, y in block b2) of channel J, packed for the sub-block kernel: position
+// in its stored list, hole count of the pair, sign of the stored order (V_A(ji) =
+// -(-1)^((ji+jj-J)/2) V_A(ij)), whether the orbits are the same, and the two block indices.
+struct HFPair {
+  int pos, bits;
+  __device__ __forceinline__ int con() const { return bits & 3; }
+  __device__ __forceinline__ unsigned neg() const { return ((unsigned)bits & 4u) << 29; }
+  __device__ __forceinline__ bool same() const { return bits & 8; }
+  __device__ __forceinline__ bool twice() const { return bits & 16; }  // the same stored pair as (y, x), y < x
+  __device__ __forceinline__ int x() const { return (bits >> 5) & 0x1FFF; }
+  __device__ __forceinline__ int y() const { return bits >> 18; }
+};
+__device__ __forceinline__ HFPair hf_pair(const DevLayout& D, int oi, int oj, int x, int y, bool same_block, int J) {
+  HFPair p;
+  const bool swap = oi > oj;
+  const int lo = swap ? oj : oi, hi = swap ? oi : oj;
+  p.pos = D.pairpos[(lo * D.N + hi) * D.NJ + (J >> 1)];
+  p.bits = (D.con[lo] + D.con[hi]) | (x << 5) | (y << 18);
+  if (swap && !((((D.jj[oi] + D.jj[oj] - J) >> 1)) & 1)) p.bits |= 4;
+  if (oi == oj) p.bits |= 8;
+  if (same_block && x > y) p.bits |= 16;
+  return p;
+}
+__device__ __forceinline__ double hf_flip(double v, unsigned sign) {
+  return __hiloint2double(__double2hiint(v) ^ (int)sign, __double2loint(v));
+}
+// arrays of a channel by the hole counts of bra and ket: pp,pp 0 | pp,ph 1 | pp,hh 2 | ph,ph 3 | hh,hh 4 | ph,hh 5
+__device__ __forceinline__ int hf_array(int c1, int c2) { return c1 == 0 ? c2 : (c1 == 1 ? (c2 == 1 ? 3 : 5) : 4); }
+
+template <int T>
+__device__ __forceinline__ void hf_sync() {
+  if constexpr (T == 32)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// One index of the four-index tensor of a sub-block transformed by its block's coefficients C
+// (column-major n x n): out[e] = sum_a C[a + i*n] in[e + (a - i)*stride], i the index of e.
+template <int T, typename Index>
+__device__ __forceinline__ void hf_mode(double*& in, double*& out, int ntot, int n, int stride,
+                                        const double* __restrict__ C, int t, Index index) {
+  if (n == 1 && C[0] == 1.0) return;  // the same for every thread of the task
+  for (int e = t; e < ntot; e += T) {
+    const int i = index(e);
     const double* src = in + e - i * stride;
     const double* c = C + i * n;
     double s = 0.0;
     for (int a = 0; a < n; ++a) s += c[a] * src[a * stride];
     out[e] = s;
   }
+  hf_sync<T>();
+  double* const swap = in;
+  in = out;
+  out = swap;
 }
 
-// pair (x in block b1, y in block b2) of channel J: stored orbit order, phase, 1/sqrt(1+d)
-__device__ __forceinline__ void hf_stored_pair(const DevLayout& D, int oi, int oj, int J, int& lo, int& hi,
-                                               double& f) {
-  if (oi <= oj) {
-    lo = oi; hi = oj;
-    f = (oi == oj) ? 0.70710678118654752 : 1.0;
-  } else {  // V_A(ji) = -(-1)^((ji+jj-J)/2) V_A(ij)
-    lo = oj; hi = oi;
-    f = d_sgn(1 + ((D.jj[oi] + D.jj[oj] - J) >> 1));
-  }
-}
-
-__device__ __forceinline__ void hf_write(const DevLayout& D, double* op, int q, int J, int lo1, int hi1, int lo2,
-                                         int hi2, double w) {
-  const int C1 = D.con[lo1] + D.con[hi1], C2 = D.con[lo2] + D.con[hi2];
-  if (C1 > C2) return;  // the transposed element is stored instead
-  const int g = (C1 == 0) ? C2 : (C1 == 1 ? (C2 == 1 ? 3 : 5) : 4);
-  const int k = q * 6 + g;
-  const int NJ = D.NJ, N = D.N;
-  const int i1 = D.pairpos[(lo1 * N + hi1) * NJ + (J >> 1)];
-  const int i2 = D.pairpos[(lo2 * N + hi2) * NJ + (J >> 1)];
-  op[D.goff[k] + i1 + (int64_t)i2 * D.gn1[k]] = w;
-}
-
-// one CTA per (channel, pair group G1 <= G2): gather V_A over the four orbit blocks, apply
-// the coefficients index by index, write back every stored element of G1 x G2 and G2 x G1
-__global__ void k_hf_transform_2b(DevLayout D, HFDev H, double* op, int herm, const double* __restrict__ dp,
-                                  int nmax4) {
+// One sub-block (channel, pair group G1 <= G2) per T threads: gather V_A over the four orbit
+// blocks, apply the coefficients index by index, write back every stored element of G1 x G2
+// and G2 x G1.
+//
+// Most sub-blocks are small: at eMax 8 they average 31 elements and 96% have 128 or fewer, so
+// a CTA of 128 threads for each left most lanes idle and waited at six barriers for a chain of
+// dependent loads.  Up to kHFWarpElems elements a warp takes one; larger ones keep the CTA.
+// The orbit pairs of both groups are looked up once per sub-block (at most n^2 of them) and
+// an element needs one multiplication for its place, instead of the full index search of
+// v_elem for the read and again for each write; phases are sign flips, since FP64 runs at 2
+// operations a clock per SM.  eMax 8, start to end of the entry point: 419 -> 215 us (limits
+// of 32, 64 and 256 elements 222, 216 and 223), eMax 9 823 -> 444, eMax 4 34 -> 24.
+template <int T>
+__global__ void __launch_bounds__(128)
+    k_hf_transform_2b(DevLayout D, HFDev H, int64_t ntask, double* op, int herm, const double* __restrict__ dp, int cap,
+                      int pcap) {
   extern __shared__ double hf_sm[];
-  double* X = hf_sm;
-  double* Y = hf_sm + nmax4;
-  const int4 t = H.tasks[blockIdx.x];
-  const int q = t.x, G1 = t.y, G2 = t.z;
-  const int b[4] = {H.grp_b1[G1], H.grp_b2[G1], H.grp_b1[G2], H.grp_b2[G2]};
-  const int n0 = H.spb_n[b[0]], n1 = H.spb_n[b[1]], n2 = H.spb_n[b[2]], n3 = H.spb_n[b[3]];
-  const int* o0 = H.spb_orb + H.spb_start[b[0]];
-  const int* o1 = H.spb_orb + H.spb_start[b[1]];
-  const int* o2 = H.spb_orb + H.spb_start[b[2]];
-  const int* o3 = H.spb_orb + H.spb_start[b[3]];
+  const int t = threadIdx.x % T, w = threadIdx.x / T;
+  const int64_t task = blockIdx.x * (int64_t)(128 / T) + w;
+  if (task >= ntask) return;  // a whole warp (T = 32); never with T = 128
+  double* X = hf_sm + (size_t)w * (2 * cap + pcap);
+  double* Y = X + cap;
+  HFPair* bra = (HFPair*)(Y + cap);
+  const int4 tk = H.tasks[task];
+  const int q = tk.x, G1 = tk.y, G2 = tk.z;
+  const int b0 = H.grp_b1[G1], b1 = H.grp_b2[G1], b2 = H.grp_b1[G2], b3 = H.grp_b2[G2];
+  const int n0 = H.spb_n[b0], n1 = H.spb_n[b1], n2 = H.spb_n[b2], n3 = H.spb_n[b3];
+  const int* o0 = H.spb_orb + H.spb_start[b0];
+  const int* o1 = H.spb_orb + H.spb_start[b1];
+  const int* o2 = H.spb_orb + H.spb_start[b2];
+  const int* o3 = H.spb_orb + H.spb_start[b3];
   const int J = D.lamJ[q];
-  const int ntot = n0 * n1 * n2 * n3;
-  for (int e = threadIdx.x; e < ntot; e += blockDim.x) {
-    int r = e;
-    const int x0 = r % n0; r /= n0;
-    const int x1 = r % n1; r /= n1;
-    const int x2 = r % n2;
-    const int x3 = r / n2;
-    X[e] = d_v_elem(D, op, herm, o0[x0], o1[x1], o2[x2], o3[x3], J);
+  const int nbra = n0 * n1, nket = n2 * n3, ntot = nbra * nket;
+  HFPair* ket = bra + nbra;
+  for (int k = t; k < nbra + nket; k += T) {
+    if (k < nbra) {
+      const int y = k / n0, x = k - y * n0;
+      bra[k] = hf_pair(D, o0[x], o1[y], x, y, b0 == b1, J);
+    } else {
+      const int y = (k - nbra) / n2, x = k - nbra - y * n2;
+      bra[k] = hf_pair(D, o2[x], o3[y], x, y, b2 == b3, J);
+    }
   }
-  __syncthreads();
-  hf_mode(X, Y, ntot, n0, 1, dp + H.dp_off[b[0]]);
-  __syncthreads();
-  hf_mode(Y, X, ntot, n1, n0, dp + H.dp_off[b[1]]);
-  __syncthreads();
-  hf_mode(X, Y, ntot, n2, n0 * n1, dp + H.dp_off[b[2]]);
-  __syncthreads();
-  hf_mode(Y, X, ntot, n3, n0 * n1 * n2, dp + H.dp_off[b[3]]);
-  __syncthreads();
+  hf_sync<T>();
+  // e = (bra pair) + nbra (ket pair); the quotient by nbra as a product with 2^32 / nbra,
+  // rounded up: exact while e * nbra < 2^32
+  const unsigned rcp = nbra > 1 ? 0xFFFFFFFFu / (unsigned)nbra + 1u : 0u;
+  auto ket_of = [&](int e) { return nbra > 1 ? (int)__umulhi((unsigned)e, rcp) : e; };
+  const int64_t* goff = D.goff + q * 6;
+  const int* gn1 = D.gn1 + q * 6;
+  for (int e = t; e < ntot; e += T) {
+    const int ek = ket_of(e);
+    const HFPair p = bra[e - ek * nbra], s = ket[ek];
+    const bool tr = p.con() > s.con();
+    const int g = tr ? hf_array(s.con(), p.con()) : hf_array(p.con(), s.con());
+    const int i1 = tr ? s.pos : p.pos, i2 = tr ? p.pos : s.pos;
+    double v = op[goff[g] + i1 + (int64_t)i2 * gn1[g]];
+    if (p.same() || s.same()) v *= p.same() && s.same() ? 1.4142135623730951 * 1.4142135623730951 : 1.4142135623730951;
+    X[e] = hf_flip(v, p.neg() ^ s.neg() ^ (tr && herm < 0 ? 0x80000000u : 0u));
+  }
+  hf_sync<T>();
+  hf_mode<T>(X, Y, ntot, n0, 1, dp + H.dp_off[b0], t, [&](int e) { return bra[e - ket_of(e) * nbra].x(); });
+  hf_mode<T>(X, Y, ntot, n1, n0, dp + H.dp_off[b1], t, [&](int e) { return bra[e - ket_of(e) * nbra].y(); });
+  hf_mode<T>(X, Y, ntot, n2, nbra, dp + H.dp_off[b2], t, [&](int e) { return ket[ket_of(e)].x(); });
+  hf_mode<T>(X, Y, ntot, n3, nbra * n2, dp + H.dp_off[b3], t, [&](int e) { return ket[ket_of(e)].y(); });
   // stored pairs of each group: x <= y inside one block, every (x, y) across two blocks
-  const bool same1 = b[0] == b[1], same2 = b[2] == b[3];
-  const int nbra = same1 ? n0 * (n0 + 1) / 2 : n0 * n1;
-  const int nket = same2 ? n2 * (n2 + 1) / 2 : n2 * n3;
-  for (int e = threadIdx.x; e < nbra * nket; e += blockDim.x) {
-    const int eb = e % nbra, ek = e / nbra;
-    int x0, x1, x2, x3;
-    if (same1) {
-      x1 = 0;
-      while ((x1 + 1) * (x1 + 2) / 2 <= eb) ++x1;
-      x0 = eb - x1 * (x1 + 1) / 2;
-    } else {
-      x0 = eb % n0;
-      x1 = eb / n0;
+  for (int e = t; e < ntot; e += T) {
+    const int ek = ket_of(e);
+    const HFPair p = bra[e - ek * nbra], s = ket[ek];
+    if (p.twice() || s.twice()) continue;
+    double v = X[e];
+    if (p.same()) v *= 0.70710678118654752;
+    if (s.same()) v *= 0.70710678118654752;
+    v = hf_flip(v, p.neg() ^ s.neg());
+    if (p.con() <= s.con()) {
+      const int g = hf_array(p.con(), s.con());
+      op[goff[g] + p.pos + (int64_t)s.pos * gn1[g]] = v;
     }
-    if (same2) {
-      x3 = 0;
-      while ((x3 + 1) * (x3 + 2) / 2 <= ek) ++x3;
-      x2 = ek - x3 * (x3 + 1) / 2;
-    } else {
-      x2 = ek % n2;
-      x3 = ek / n2;
+    if (G1 != G2 && s.con() <= p.con()) {
+      const int g = hf_array(s.con(), p.con());
+      op[goff[g] + s.pos + (int64_t)p.pos * gn1[g]] = herm < 0 ? -v : v;
     }
-    int lo1, hi1, lo2, hi2;
-    double f1, f2;
-    hf_stored_pair(D, o0[x0], o1[x1], J, lo1, hi1, f1);
-    hf_stored_pair(D, o2[x2], o3[x3], J, lo2, hi2, f2);
-    const double v = X[x0 + n0 * (x1 + n1 * (x2 + n2 * x3))] * f1 * f2;
-    hf_write(D, op, q, J, lo1, hi1, lo2, hi2, v);
-    if (G1 != G2) hf_write(D, op, q, J, lo2, hi2, lo1, hi1, herm * v);
   }
 }
 
 // ---------------------------------------------------------------- host helpers
+// shared memory of a CTA's sub-block: two copies of the elements and the orbit pairs
+size_t hf_cta_smem(int nmax) {
+  const size_t n2 = (size_t)nmax * nmax;
+  return sizeof(double) * (2 * n2 * n2 + 2 * n2);
+}
+
 // C = A^T B A for n x n column-major matrices
 std::vector<double> sandwich(int n, const std::vector<double>& A, const std::vector<double>& B) {
   std::vector<double> BA((size_t)n * n, 0.0), C((size_t)n * n, 0.0);
@@ -310,6 +357,11 @@ imsrg_status Ctx::hf_prepare() {
   for (int q = 0; q < L.nblocks; ++q)
     for (int G2 = PG.grp_first[q]; G2 < PG.grp_first[q + 1]; ++G2)
       for (int G1 = PG.grp_first[q]; G1 <= G2; ++G1) S->tasks.push_back(make_int4(q, G1, G2, 0));
+  auto pairs = [&](int G1) { return PG.spb_n[PG.grp_b1[G1]] * PG.spb_n[PG.grp_b2[G1]]; };
+  const auto warps = std::stable_partition(S->tasks.begin(), S->tasks.end(),
+                                           [&](const int4& t) { return PG.elems(t.y, t.z) > kHFWarpElems; });
+  S->ncta = warps - S->tasks.begin();
+  for (auto t = warps; t != S->tasks.end(); ++t) S->warp_pairs = std::max(S->warp_pairs, pairs(t->y) + pairs(t->z));
   S->prefix = L.off_fph + (int64_t)L.P * L.A;
   // one device allocation for the integer tables
   std::vector<char> buf;
@@ -349,10 +401,9 @@ imsrg_status Ctx::hf_prepare() {
   CKH(cuda(cudaMalloc(&S->d_M, sizeof(double) * std::max<int64_t>((int64_t)S->nrow * S->ncol, 1)),
            "cudaMalloc(HF mean-field tensor)"));
   CKH(cuda(cudaMalloc(&S->d_dp, sizeof(double) * std::max(S->ndp, 1)), "cudaMalloc(HF coefficients)"));
-  const int nmax4 = S->nmax * S->nmax * S->nmax * S->nmax;
-  const size_t smem = sizeof(double) * 2 * (size_t)nmax4;
-  if (smem > 48 * 1024)
-    CKH(cuda(cudaFuncSetAttribute(k_hf_transform_2b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+  const size_t smem = hf_cta_smem(S->nmax);
+  if (S->ncta && smem > 48 * 1024)
+    CKH(cuda(cudaFuncSetAttribute(k_hf_transform_2b<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
              "cudaFuncSetAttribute(k_hf_transform_2b)"));
   return IMSRG_OK;
 }
@@ -392,14 +443,21 @@ imsrg_status Ctx::hf_transform_2b(double* op, int herm, const double* coefs) {
   CKH(cuda(cudaMemcpyAsync(S.d_dp, dp.data(), sizeof(double) * S.ndp, cudaMemcpyHostToDevice, stream),
            "cudaMemcpyAsync(HF coefficients)"));
   if (S.tasks.empty()) return cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(HF)");
-  const int nmax4 = S.nmax * S.nmax * S.nmax * S.nmax;
-  const size_t smem = sizeof(double) * 2 * (size_t)nmax4;
-  const int64_t ntask = (int64_t)S.tasks.size();
-  for (int64_t t0 = 0; t0 < ntask; t0 += 2147483647LL) {  // grid.x limit
-    const int nb = (int)std::min<int64_t>(ntask - t0, 2147483647LL);
+  const int64_t nwarp = (int64_t)S.tasks.size() - S.ncta;
+  for (int64_t t0 = 0; t0 < S.ncta; t0 += 2147483647LL) {  // grid.x limit
+    const int64_t n = std::min<int64_t>(S.ncta - t0, 2147483647LL);
     HFDev dv = S.dev;
     dv.tasks += t0;
-    k_hf_transform_2b<<<nb, 128, smem, stream>>>(D, dv, op, herm, S.d_dp, nmax4);
+    k_hf_transform_2b<128><<<(int)n, 128, hf_cta_smem(S.nmax), stream>>>(
+        D, dv, n, op, herm, S.d_dp, S.nmax * S.nmax * S.nmax * S.nmax, 2 * S.nmax * S.nmax);
+    CKH(launched("k_hf_transform_2b"));
+  }
+  for (int64_t t0 = 0; t0 < nwarp; t0 += 4 * 2147483647LL) {
+    const int64_t n = std::min<int64_t>(nwarp - t0, 4 * 2147483647LL);
+    HFDev dv = S.dev;
+    dv.tasks += S.ncta + t0;
+    k_hf_transform_2b<32><<<(int)((n + 3) / 4), 128, 4 * sizeof(double) * (2 * kHFWarpElems + S.warp_pairs), stream>>>(
+        D, dv, n, op, herm, S.d_dp, kHFWarpElems, S.warp_pairs);
     CKH(launched("k_hf_transform_2b"));
   }
   // the host copy of the coefficients must outlive the copy
