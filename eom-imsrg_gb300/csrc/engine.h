@@ -228,7 +228,7 @@ struct Ctx {
   // Hartree-Fock and normal ordering (hf.cu)
   imsrg_status hf_prepare();
   void hf_release();
-  imsrg_status hf_mean_field(const double* op, int herm, std::vector<double>& M);
+  imsrg_status hf_mean_field(const double* op, int herm);
   imsrg_status hf_transform_2b(double* op, int herm, const double* coefs);
   imsrg_status hf_run(double* op, int herm, int mode, int max_iter, const double* coefs_in, double* coefs_out,
                       imsrg_hf_info* info);
