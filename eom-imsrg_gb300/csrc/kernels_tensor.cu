@@ -531,109 +531,81 @@ __global__ void k_tpandya_exc(DevLayout D, DevTLayout T, const double* __restric
   }
 }
 
-namespace {
-__device__ __forceinline__ bool d_odd(int J) { return ((J >> 1) & 1) == 1; }
-
-// one recoupling loop of TS_commutator_222_ph: J1 over [o1, o2], J2 over [max(J1, i1), min(i2, J1 + rank)], adding
-// (-1)^neg(J1, J2) val times the normalised 9j {n1 n2 J3; n3 n4 J4; J1 J2 rank} to the tensor elements (add_elem_to_tensor,
-// src/basic_IMSRG.f90:1687-1772: a <= b, c <= d, J1 <= J2).  Signs by integer instructions, one multiplication a term: the
-// FP64 pipe and the reductions at L2 bound this kernel.
-template <class C>
-__device__ __forceinline__ void recouple_loop(const DevLayout& D, const DevTLayout& T, double* RES, int J3, int J4,
-                                              int o1, int o2, int i1, int i2, bool skip_o, bool skip_i, int n1, int n2,
-                                              int n3, int n4, double val, C neg, int a, int b, int c, int d, int exc) {
-  const int g = d_tg(D.con[a] + D.con[b], D.con[c] + D.con[d]);
-  if (exc && g != 2 && g != 6) return;  // only the (pp,hh) and (hh,pp) outputs are wanted
-  const int P = (D.ll[a] + D.ll[b]) & 1, tz = ((D.tz[a] + D.tz[b]) >> 1) + 1, N = D.N, NJ = D.NJ;
-  const int* pos1 = D.pairpos + (a * N + b) * NJ;
-  const int* pos2 = D.pairpos + (c * N + d) * NJ;
-  if (a == b) val *= 1.4142135623730951;
-  if (c == d) val *= 1.4142135623730951;
-  for (int J1 = o1; J1 <= o2; J1 += 2) {
-    if ((skip_o && d_odd(J1)) || J1 > 2 * D.JM) continue;
-    const int x1 = pos1[J1 >> 1];
-    if (x1 < 0) continue;
-    for (int J2 = max(J1, i1); J2 <= min(i2, J1 + T.rank); J2 += 2) {
-      if (skip_i && d_odd(J2)) continue;
-      const int q = T.lut[(((J1 >> 1) * (T.rank / 2 + 1) + ((J2 - J1) >> 1)) * 3 + tz) * 2 + P];
-      const int x2 = pos2[J2 >> 1];
-      if (q < 0 || x2 < 0) continue;
-      const int k = q * 9 + g;
-      atomicAdd(RES + T.goff[k] + x1 + (int64_t)x2 * T.n1[k],
-                d_flip(val * d_nine_n(T, n1, n2, J3, n3, n4, J4, J1, J2), neg(J1, J2)));
-    }
-  }
-}
-}  // namespace
-
 // ---------------------------------------------------------------- TS_commutator_222_ph
 // src/TS_commutators.f90:1529-1843 for one cross-coupled tensor block: every element of
 // Wx (and Wy) above thresh in size recouples into the two-body tensor elements it feeds (ACCUMULATES);
 // TS_commutator_222_ph uses thresh = 1e-6 (src/TS_commutators.f90:1562, 1714), the EOM product 0
 namespace {
-// the recouplings of one (Wx, Wy) element pair, rows (d, a) of qa and (c, b) of qb
+// The recouplings of one (Wx, Wy) element pair, rows (d, a) of qa and (c, b) of qb: two sums of X and two of Y, each over J1 of
+// the pair (p, q) and J2 of (r, t), J1 <= J2, adding (-1)^neg(J1, J2) val times a normalised 9j to the tensor elements
+// (add_elem_to_tensor, src/basic_IMSRG.f90:1687-1772), whose pairs are stored in ascending order: a swap of p and q is a phase
+// 1 + (jp + jq + J1) / 2.  Signs by integer instructions, one multiplication a term.
+//
+// One loop for the four sums and for every order of the orbits, its signs linear in J1 / 2 and J2 / 2: written out, the sixteen
+// cases took the warps through sixteen copies of the loop and past the instruction cache, 55% of the time between two issues
+// (first term of the eMax 4 observable: before 704 us).
 __device__ __forceinline__ void ph_scatter_elem(const DevLayout& D, const DevTLayout& T, double* RES, int J3, int J4,
                                                 int qa, int qb, int IX, int JX, double X, double Y, int hL, int hR,
                                                 double thresh, int exc) {
-  const int rank = T.rank;
-  const bool ph34 = ((J3 + J4) >> 1) & 1, nL = hL < 0, nR = hR < 0;
+  const int rank = T.rank, N = D.N, NJ = D.NJ;
+  const int ph34 = (J3 + J4) >> 1, nL = hL < 0, nR = hR < 0;
   const int d = D.cc_ra[D.cc_row_off[qa] + IX], a = D.cc_rb[D.cc_row_off[qa] + IX];
   const int c = D.cc_ra[D.cc_row_off[qb] + JX], b = D.cc_rb[D.cc_row_off[qb] + JX];
   const int ja = D.jj[a], jb = D.jj[b], jc = D.jj[c], jd = D.jj[d];
-  const bool pabcd = ((ja + jb + jc + jd) >> 1) & 1;
-  if (fabs(X) > thresh) {
-    const int J1min = abs(ja - jb), J1max = ja + jb, J2min = abs(jc - jd), J2max = jc + jd;
-    if (b >= a) {
-      if (d >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, c == d, ja, jd, jb, jc, X,
-                      [&](int, int J2) { return (((((jb + jd + J2) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, a, b, c, d, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, a == b, jd, ja, jc, jb, X,
-                      [&](int J1, int) { return (((((jc + ja + J1 + rank) >> 1) & 1) ^ (int)nR ^ 1) & 1) != 0; }, c, d, a, b, exc);
-      } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, a == b, false, ja, jd, jb, jc, X,
-                      [&](int, int) { return (((((jb + jc) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, a, b, d, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, a == b, jd, ja, jc, jb, X,
-                      [&](int, int) { return (((((ja - jd + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, d, c, a, b, exc);
-      }
+#pragma unroll 1
+  for (int s = 0; s < 4; ++s) {
+    double val = s < 2 ? X : Y;
+    if (!(fabs(val) > thresh)) continue;
+    // X: pairs (a, b) and (c, d), then the other way round; Y: (d, b) and (c, a), then (c, a) and (d, b)
+    const bool odd = s & 1, y = s & 2;
+    int p = y ? d : a, q = b, r = c, t = y ? a : d;
+    int jp = y ? jd : ja, jq = jb, jr = jc, jt = y ? ja : jd;
+    // 9j {n1 n2 J3; n3 n4 J4; J1 J2 rank}: rows of the first sum, their entries swapped in the second
+    const int n1 = odd ? jt : jp, n2 = odd ? jp : jt, n3 = odd ? jr : jq, n4 = odd ? jq : jr;
+    int neg, f1 = 0, f2 = 0;  // parity of the sign: neg + f1 J1 / 2 + f2 J2 / 2
+    if (!odd) {
+      neg = y ? ((jc + ja) >> 1) + nL : ((jb + jd) >> 1) + ph34 + nL;
+      f2 = 1;
     } else {
-      if (d >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, c == d, ja, jd, jb, jc, X,
-                      [&](int J1, int J2) { return (((((ja + jd + J1 + J2) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, b, a, c, d, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == d, false, jd, ja, jc, jb, X,
-                      [&](int J1, int J2) { return (((((jc - jb + J1 + J2 + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, c, d, b, a, exc);
-      } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, false, false, ja, jd, jb, jc, X,
-                      [&](int J1, int) { return (((((ja + jc + J1) >> 1) & 1) ^ (int)ph34 ^ (int)nL) & 1) != 0; }, b, a, d, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, false, false, jd, ja, jc, jb, X,
-                      [&](int, int J2) { return (((((jb - jd + J2 + rank) >> 1) & 1) ^ (int)nR) & 1) != 0; }, d, c, b, a, exc);
-      }
+      neg = y ? ((jd - jb + rank) >> 1) + ph34 + nR : ((jc + ja + rank) >> 1) + nR + 1;
+      f1 = 1;
+      int k = p; p = r; r = k;
+      k = q; q = t; t = k;
+      k = jp; jp = jr; jr = k;
+      k = jq; jq = jt; jt = k;
     }
-  }
-  if (fabs(Y) > thresh) {
-    const int J1min = abs(jd - jb), J1max = jd + jb, J2min = abs(jc - ja), J2max = jc + ja;
-    if (b >= d) {
-      if (a >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, Y,
-                      [&](int, int J2) { return (((((jc + ja + J2) >> 1) & 1) ^ (int)nL) & 1) != 0; }, d, b, c, a, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, Y,
-                      [&](int J1, int) { return (((((jd - jb + J1 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, c, a, d, b, exc);
-      } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, d == b, c == a, jd, ja, jb, jc, Y,
-                      [&](int, int) { return (((int)nL ^ 1) & 1) != 0; }, d, b, a, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, b == d, ja, jd, jc, jb, Y,
-                      [&](int, int) { return (((int)pabcd ^ (int)ph34 ^ ((rank >> 1) & 1) ^ (int)nR) & 1) != 0; }, a, c, d, b, exc);
-      }
-    } else {
-      if (a >= c) {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, Y,
-                      [&](int J1, int J2) { return (((int)pabcd ^ (((J1 + J2) >> 1) & 1) ^ (int)nL ^ 1) & 1) != 0; }, b, d, c, a, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, c == a, b == d, ja, jd, jc, jb, Y,
-                      [&](int J1, int J2) { return (((((J1 + J2 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, c, a, b, d, exc);
-      } else {
-        recouple_loop(D, T, RES, J3, J4, J1min, J1max, J2min, J2max, b == d, a == c, jd, ja, jb, jc, Y,
-                      [&](int J1, int) { return (((((jb + jd + J1) >> 1) & 1) ^ (int)nL) & 1) != 0; }, b, d, a, c, exc);
-        recouple_loop(D, T, RES, J3, J4, J2min, J2max, J1min, J1max, a == c, d == b, ja, jd, jc, jb, Y,
-                      [&](int, int J2) { return (((((ja - jc + J2 + rank) >> 1) & 1) ^ (int)ph34 ^ (int)nR) & 1) != 0; }, a, c, b, d, exc);
+    if (p > q) {
+      neg += 1 + ((jp + jq) >> 1);
+      f1 ^= 1;
+      const int k = p; p = q; q = k;
+    }
+    if (r > t) {
+      neg += 1 + ((jr + jt) >> 1);
+      f2 ^= 1;
+      const int k = r; r = t; t = k;
+    }
+    const int g = d_tg(D.con[p] + D.con[q], D.con[r] + D.con[t]);
+    if (exc && g != 2 && g != 6) continue;  // only the (pp,hh) and (hh,pp) outputs are wanted
+    const int P = (D.ll[p] + D.ll[q]) & 1, tz = ((D.tz[p] + D.tz[q]) >> 1) + 1;
+    const int* pos1 = D.pairpos + (p * N + q) * NJ;
+    const int* pos2 = D.pairpos + (r * N + t) * NJ;
+    if (p == q) val *= 1.4142135623730951;
+    if (r == t) val *= 1.4142135623730951;
+    // orbits that are the same couple to even J / 2 only
+    const int dJ1 = p == q ? 4 : 2, dJ2 = r == t ? 4 : 2;
+    const int J1max = min(jp + jq, 2 * D.JM), J2lo = abs(jr - jt), J2hi = jr + jt;
+    for (int J1 = abs(jp - jq); J1 <= J1max; J1 += dJ1) {
+      const int x1 = pos1[J1 >> 1];
+      if (x1 < 0) continue;
+      int J2 = max(J1, J2lo);
+      if (r == t) J2 = (J2 + 2) & ~3;
+      for (const int J2max = min(J2hi, J1 + rank); J2 <= J2max; J2 += dJ2) {
+        const int k2 = T.lut[(((J1 >> 1) * (rank / 2 + 1) + ((J2 - J1) >> 1)) * 3 + tz) * 2 + P];
+        const int x2 = pos2[J2 >> 1];
+        if (k2 < 0 || x2 < 0) continue;
+        const int k = k2 * 9 + g;
+        atomicAdd(RES + T.goff[k] + x1 + (int64_t)x2 * T.n1[k],
+                  d_flip(val * d_nine_n(T, n1, n2, J3, n3, n4, J4, J1, J2), ((neg + f1 * (J1 >> 1) + f2 * (J2 >> 1)) & 1) != 0));
       }
     }
   }
