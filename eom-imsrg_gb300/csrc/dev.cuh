@@ -68,6 +68,28 @@ struct DevLayout {
 __device__ __forceinline__ bool d_tri(int a, int b, int J) { return J <= a + b && J >= abs(a - b); }
 __device__ __forceinline__ double d_sgn(int n) { return (n & 1) ? -1.0 : 1.0; }
 
+// Phases and small factors without FP64 instructions where that can be done: the FP64 pipe takes 2 operations a clock per SM,
+// and the gather kernels spent more of them on factors of one than on the sums (same values; commutator at eMax 6
+// 351 -> 325 us, at eMax 10 8.73 -> 8.40 ms, its adjoint at eMax 6 813 -> 765 us, the eMax 4 observable 1969 -> 1832 us).
+__device__ __forceinline__ double d_flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+// 2^(nsq/2) with a sign, nsq = 0, 1 or 2: the swap phases of an element's pairs and sqrt(2) for each pair of equal orbits
+// (the product of two rounded sqrt(2) is an ulp above 2)
+__device__ __forceinline__ double d_pair_factor(bool neg, int nsq) {
+  return d_flip(nsq == 0 ? 1.0 : (nsq == 1 ? 1.4142135623730951 : 1.4142135623730951 * 1.4142135623730951), neg);
+}
+// x times such a factor: +-1 flips the sign
+__device__ __forceinline__ double d_times(double x, double factor) {
+  const int hi = __double2hiint(factor);
+  return (hi & 0x7FFFFFFF) == 0x3FF00000 ? d_flip(x, hi < 0) : x * factor;
+}
+// n as double, 1 <= n < 2^20
+__device__ __forceinline__ double d_int(int n) {
+  const int e = 31 - __clz(n);
+  return __hiloint2double(((1023 + e) << 20) | ((n << (20 - e)) & 0xFFFFF), 0);
+}
+
 // 6j symbol {j1 j2 j3; j4 j5 j6} (j1,j2,j4,j5 odd, j3,j6 even; doubled units)
 __device__ __forceinline__ double d_sixj(const DevLayout& D, int j1, int j2, int j3, int j4, int j5, int j6) {
   if (!(d_tri(j1, j2, j3) && d_tri(j4, j5, j3) && d_tri(j1, j5, j6) && d_tri(j4, j2, j6))) return 0.0;
@@ -81,7 +103,7 @@ __device__ __forceinline__ double d_f_elem(const DevLayout& D, const double* op,
   const int c1 = D.con[a], c2 = D.con[b];
   if (c1 + c2 == 0) return op[D.off_fpp + D.loc[a] + (int64_t)D.loc[b] * D.P];
   if (c1 + c2 == 2) return op[D.off_fhh + D.loc[a] + (int64_t)D.loc[b] * D.A];
-  if (c1 > c2) return op[D.off_fph + D.loc[b] + (int64_t)D.loc[a] * D.P] * herm;
+  if (c1 > c2) return d_flip(op[D.off_fph + D.loc[b] + (int64_t)D.loc[a] * D.P], herm < 0);
   return op[D.off_fph + D.loc[a] + (int64_t)D.loc[b] * D.P];
 }
 
@@ -92,6 +114,7 @@ struct VRef {
   int64_t idx;
   double pre;
   bool herm;
+  __device__ __forceinline__ double factor(int h) const { return d_flip(pre, herm && h < 0); }
 };
 __device__ __forceinline__ bool d_vref(const DevLayout& D, int a, int b, int c, int d, int J, VRef& r) {
   const int ja = D.jj[a], jb = D.jj[b], jc = D.jj[c], jd = D.jj[d];
@@ -106,20 +129,20 @@ __device__ __forceinline__ bool d_vref(const DevLayout& D, int a, int b, int c, 
   const int lo = C1 < C2 ? C1 : C2, hi = C1 < C2 ? C2 : C1;
   const int g = (lo == 0) ? hi : (lo == 1 ? (hi == 1 ? 3 : 5) : 4);
   const int NJ = D.NJ, N = D.N;
-  double pre = 1.0;
+  int neg = 0, nsq = 0;
   int i1, i2;
   if (a > b) {
     i1 = D.pairpos[(b * N + a) * NJ + (J >> 1)];
-    pre = d_sgn(1 + ((ja + jb - J) >> 1));
+    neg = 1 + ((ja + jb - J) >> 1);
   } else {
-    if (a == b) pre = 1.4142135623730951;
+    nsq = a == b;
     i1 = D.pairpos[(a * N + b) * NJ + (J >> 1)];
   }
   if (c > d) {
     i2 = D.pairpos[(d * N + c) * NJ + (J >> 1)];
-    pre *= d_sgn(1 + ((jc + jd - J) >> 1));
+    neg += 1 + ((jc + jd - J) >> 1);
   } else {
-    if (c == d) pre *= 1.4142135623730951;
+    nsq += c == d;
     i2 = D.pairpos[(c * N + d) * NJ + (J >> 1)];
   }
   const int k = q * 6 + g;
@@ -131,7 +154,7 @@ __device__ __forceinline__ bool d_vref(const DevLayout& D, int a, int b, int c, 
     r.idx = D.goff[k] + i1 + (int64_t)i2 * n1;
     r.herm = false;
   }
-  r.pre = pre;
+  r.pre = d_pair_factor(neg & 1, nsq);
   return true;
 }
 
@@ -273,7 +296,7 @@ __device__ __forceinline__ double d_v_elem(const DevLayout& D, const double* op,
                                            int J) {
   VRef r;
   if (!d_vref(D, a, b, c, d, J, r)) return 0.0;
-  return op[r.idx] * (r.herm ? herm * r.pre : r.pre);
+  return d_times(op[r.idx], r.factor(herm));
 }
 
 // (q, g, IX, JX) of unique 2b element u (upper triangle incl. diagonal for square arrays,

@@ -20,12 +20,12 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ double vfac(const VRef& r, int herm) { return r.herm ? herm * r.pre : r.pre; }
+__device__ __forceinline__ double vfac(const VRef& r, int herm) { return r.factor(herm); }
 
 __device__ __forceinline__ void d_vadd(const DevLayout& D, double* bar, int herm, int a, int b, int c, int d, int J,
                                        double g) {
   VRef r;
-  if (d_vref(D, a, b, c, d, J, r)) atomicAdd(bar + r.idx, g * vfac(r, herm));
+  if (d_vref(D, a, b, c, d, J, r)) atomicAdd(bar + r.idx, d_times(g, vfac(r, herm)));
 }
 
 // slab position f_elem(a,b) reads, and whether the operator's herm multiplies it
@@ -230,13 +230,13 @@ __global__ void k_vjp_122(DevLayout D, const double* __restrict__ L, int hL, con
       VRef r;
       if (!d_vref(D, va, vb, vc, vd, JT, r)) return;
       const FRef f = d_fref(D, fx, fy);
-      const double vR = R[r.idx] * vfac(r, hR), vL = L[r.idx] * vfac(r, hL);
+      const double vR = d_times(R[r.idx], vfac(r, hR)), vL = d_times(L[r.idx], vfac(r, hL));
       const double fL = fval(L, f, hL), fR = fval(R, f, hR);
       const double ss = sign * s;
       atomicAdd(F + (int64_t)e * 64 + lane, ss * vR);
-      atomicAdd(Rb + r.idx, ss * fL * vfac(r, hR));
+      atomicAdd(Rb + r.idx, d_times(ss * fL, vfac(r, hR)));
       atomicAdd(F + (int64_t)e * 64 + 32 + lane, -ss * vL);
-      atomicAdd(Lb + r.idx, -ss * fR * vfac(r, hL));
+      atomicAdd(Lb + r.idx, d_times(-ss * fR, vfac(r, hL)));
     };
     for (int t = 0, s0 = D.same_start[a], n = D.same_count[a]; t < n; ++t) {
       const int i = D.same_list[s0 + t];
@@ -296,14 +296,14 @@ __global__ void k_vjp_121(DevLayout D, const double* __restrict__ L, int hL, con
     VRef r;
     for (int JT = abs(ji - jq); JT <= ji + jq; JT += 2) {
       if (d_vref(D, ak, pk, ik, qk, JT, r)) {
-        smx += R[r.idx] * vfac(r, hR) * (JT + 1);
-        smx2 += L[r.idx] * vfac(r, hL) * (JT + 1);
+        smx += d_times(R[r.idx], vfac(r, hR)) * (JT + 1);
+        smx2 += d_times(L[r.idx], vfac(r, hL)) * (JT + 1);
         atomicAdd(Rb + r.idx, sb * lph * hL * (JT + 1) * vfac(r, hR));
         atomicAdd(Lb + r.idx, -sb * rph * hR * (JT + 1) * vfac(r, hL));
       }
       if (d_vref(D, ik, pk, ak, qk, JT, r)) {
-        smy += R[r.idx] * vfac(r, hR) * (JT + 1);
-        smy2 += L[r.idx] * vfac(r, hL) * (JT + 1);
+        smy += d_times(R[r.idx], vfac(r, hR)) * (JT + 1);
+        smy2 += d_times(L[r.idx], vfac(r, hL)) * (JT + 1);
         atomicAdd(Rb + r.idx, -sb * lph * (JT + 1) * vfac(r, hR));
         atomicAdd(Lb + r.idx, sb * rph * (JT + 1) * vfac(r, hL));
       }

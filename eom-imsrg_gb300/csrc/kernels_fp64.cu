@@ -10,6 +10,10 @@ namespace imsrg {
 // calculate_cross_coupled (src/cross_coupled.f90:1190-1300): one thread per CCX element,
 // CCX(q) column-major (rlen x nph), threads consecutive in the row index.
 __global__ void k_pandya(DevLayout D, const double* __restrict__ op, int herm, double* __restrict__ cc) {
+  constexpr int kSq = 64;
+  __shared__ double sq[kSq];  // sqrt(JC + 1): a square root costs as much as the sum of an element
+  for (int k = threadIdx.x; k < kSq; k += blockDim.x) sq[k] = sqrt(2.0 * k + 1.0);
+  __syncthreads();
   const int64_t total = D.cc_size;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int lo = 0, hi = D.ncc;
@@ -32,8 +36,8 @@ __global__ void k_pandya(DevLayout D, const double* __restrict__ op, int herm, d
       const int Jmin = max(abs(jp - jb), abs(ja - jh)), Jmax = min(jp + jb, ja + jh);
       double sm = 0.0;
       for (int JT = Jmin; JT <= Jmax; JT += 2)
-        sm += d_sgn(JT >> 1) * (JT + 1) * d_sixj(D, jp, jh, JC, ja, jb, JT) * d_v_elem(D, op, herm, h, a, p, b, JT);
-      val = sm * d_sgn((jh + jb + JC) >> 1) * sqrt(JC + 1.0);
+        sm += d_flip(d_int(JT + 1) * d_sixj(D, jp, jh, JC, ja, jb, JT), (JT >> 1) & 1) * d_v_elem(D, op, herm, h, a, p, b, JT);
+      val = d_flip(sm, ((jh + jb + JC) >> 1) & 1) * (JC >> 1 < kSq ? sq[JC >> 1] : sqrt(JC + 1.0));
     }
     cc[e] = val;
   }
@@ -59,7 +63,7 @@ __global__ void k_comm122(DevLayout D, const double* __restrict__ L, int hL, con
       for (int t = 0; t < n; ++t) {
         const int i = D.same_list[s0 + t];
         if (d_vref(D, i, b, c, d, JT, r)) {
-          const double vR = R[r.idx] * (r.herm ? hR * r.pre : r.pre), vL = L[r.idx] * (r.herm ? hL * r.pre : r.pre);
+          const double vR = d_times(R[r.idx], r.factor(hR)), vL = d_times(L[r.idx], r.factor(hL));
           sm += d_f_elem(D, L, hL, a, i) * vR - d_f_elem(D, R, hR, a, i) * vL;
         }
       }
@@ -69,7 +73,7 @@ __global__ void k_comm122(DevLayout D, const double* __restrict__ L, int hL, con
       for (int t = 0; t < n; ++t) {
         const int i = D.same_list[s0 + t];
         if (d_vref(D, a, i, c, d, JT, r)) {
-          const double vR = R[r.idx] * (r.herm ? hR * r.pre : r.pre), vL = L[r.idx] * (r.herm ? hL * r.pre : r.pre);
+          const double vR = d_times(R[r.idx], r.factor(hR)), vL = d_times(L[r.idx], r.factor(hL));
           sm += d_f_elem(D, L, hL, b, i) * vR - d_f_elem(D, R, hR, b, i) * vL;
         }
       }
@@ -79,7 +83,7 @@ __global__ void k_comm122(DevLayout D, const double* __restrict__ L, int hL, con
       for (int t = 0; t < n; ++t) {
         const int i = D.same_list[s0 + t];
         if (d_vref(D, a, b, i, d, JT, r)) {
-          const double vR = R[r.idx] * (r.herm ? hR * r.pre : r.pre), vL = L[r.idx] * (r.herm ? hL * r.pre : r.pre);
+          const double vR = d_times(R[r.idx], r.factor(hR)), vL = d_times(L[r.idx], r.factor(hL));
           sm += -d_f_elem(D, L, hL, i, c) * vR + d_f_elem(D, R, hR, i, c) * vL;
         }
       }
@@ -89,7 +93,7 @@ __global__ void k_comm122(DevLayout D, const double* __restrict__ L, int hL, con
       for (int t = 0; t < n; ++t) {
         const int i = D.same_list[s0 + t];
         if (d_vref(D, a, b, c, i, JT, r)) {
-          const double vR = R[r.idx] * (r.herm ? hR * r.pre : r.pre), vL = L[r.idx] * (r.herm ? hL * r.pre : r.pre);
+          const double vR = d_times(R[r.idx], r.factor(hR)), vL = d_times(L[r.idx], r.factor(hL));
           sm += -d_f_elem(D, L, hL, i, d) * vR + d_f_elem(D, R, hR, i, d) * vL;
         }
       }
@@ -326,12 +330,12 @@ __global__ void k_comm121(DevLayout D, const double* __restrict__ L, int hL, con
     VRef r;
     for (int JT = abs(ji - jq); JT <= ji + jq; JT += 2) {
       if (d_vref(D, ak, pk, ik, qk, JT, r)) {
-        smx += R[r.idx] * (r.herm ? hR * r.pre : r.pre) * (JT + 1);
-        smx2 += L[r.idx] * (r.herm ? hL * r.pre : r.pre) * (JT + 1);
+        smx += d_times(R[r.idx], r.factor(hR)) * (JT + 1);
+        smx2 += d_times(L[r.idx], r.factor(hL)) * (JT + 1);
       }
       if (d_vref(D, ik, pk, ak, qk, JT, r)) {
-        smy += R[r.idx] * (r.herm ? hR * r.pre : r.pre) * (JT + 1);
-        smy2 += L[r.idx] * (r.herm ? hL * r.pre : r.pre) * (JT + 1);
+        smy += d_times(R[r.idx], r.factor(hR)) * (JT + 1);
+        smy2 += d_times(L[r.idx], r.factor(hL)) * (JT + 1);
       }
     }
     const double lph = L[D.off_fph + a + (int64_t)i * D.P], rph = R[D.off_fph + a + (int64_t)i * D.P];

@@ -56,9 +56,6 @@ __device__ __forceinline__ double d_nine_n(const DevTLayout& T, int a, int b, in
   }
   return d_nine(T, a, b, J1, c, d, J2, J3, J4) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * (T.sq[J3 >> 1] * T.sq[J4 >> 1]);
 }
-__device__ __forceinline__ double d_flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
-}
 
 __device__ __forceinline__ int d_tg(int c1, int c2) {
   // (bra class, ket class) -> tgam index: pp-pp 0 pp-ph 1 pp-hh 2 ph-ph 3 hh-hh 4 ph-hh 5 hh-pp 6 ph-pp 7 hh-ph 8
@@ -79,11 +76,11 @@ struct TRef {
 __device__ bool d_tref(const DevLayout& D, const DevTLayout& T, int herm, int ax, int bx, int cx, int dx, int J1x,
                        int J2x, TRef& r) {
   int a = ax, b = bx, c = cx, d = dx, J1 = J1x, J2 = J2x;
-  double phase = 1.0;
+  int neg = 0, nsq = 0;
   if (J1x > J2x) {
     a = cx; b = dx; c = ax; d = bx;
     J1 = J2x; J2 = J1x;
-    phase = d_sgn((J1 - J2) >> 1) * herm;
+    neg = ((J1 - J2) >> 1) + (herm < 0);
   }
   if (!d_tri(J1, J2, T.rank)) return false;
   const int ja = D.jj[a], jb = D.jj[b], jc = D.jj[c], jd = D.jj[d];
@@ -97,32 +94,31 @@ __device__ bool d_tref(const DevLayout& D, const DevTLayout& T, int herm, int ax
   if (q < 0 || T.q1[q] < 0) return false;
   const int g = d_tg(D.con[a] + D.con[b], D.con[c] + D.con[d]);
   const int N = D.N, NJ = D.NJ;
-  double pre = 1.0;
   int i1, i2;
   if (a > b) {
     i1 = D.pairpos[(b * N + a) * NJ + (J1 >> 1)];
-    pre = d_sgn(1 + ((ja + jb - J1) >> 1));
+    neg += 1 + ((ja + jb - J1) >> 1);
   } else {
-    if (a == b) pre = 1.4142135623730951;
+    nsq = a == b;
     i1 = D.pairpos[(a * N + b) * NJ + (J1 >> 1)];
   }
   if (c > d) {
     i2 = D.pairpos[(d * N + c) * NJ + (J2 >> 1)];
-    pre *= d_sgn(1 + ((jc + jd - J2) >> 1));
+    neg += 1 + ((jc + jd - J2) >> 1);
   } else {
-    if (c == d) pre *= 1.4142135623730951;
+    nsq += c == d;
     i2 = D.pairpos[(c * N + d) * NJ + (J2 >> 1)];
   }
   const int k = q * 9 + g;
   r.idx = T.goff[k] + i1 + (int64_t)i2 * T.n1[k];
-  r.f = pre * phase;
+  r.f = d_pair_factor(neg & 1, nsq);
   return true;
 }
 
 __device__ __forceinline__ double d_telem(const DevLayout& D, const DevTLayout& T, const double* op, int herm, int a,
                                           int b, int c, int d, int J1, int J2) {
   TRef r;
-  return d_tref(D, T, herm, a, b, c, d, J1, J2, r) ? op[r.idx] * r.f : 0.0;
+  return d_tref(D, T, herm, a, b, c, d, J1, J2, r) ? d_times(op[r.idx], r.f) : 0.0;
 }
 
 // f_tensor_elem (src/basic_IMSRG.f90:1261-1290)
@@ -131,7 +127,8 @@ __device__ __forceinline__ double d_ftelem(const DevLayout& D, const DevTLayout&
   const int c1 = D.con[a], c2 = D.con[b];
   if (c1 + c2 == 0) return op[T.off_fpp + D.loc[a] + (int64_t)D.loc[b] * D.P];
   if (c1 + c2 == 2) return op[T.off_fhh + D.loc[a] + (int64_t)D.loc[b] * D.A];
-  if (c1 > c2) return op[T.off_fph + D.loc[b] + (int64_t)D.loc[a] * D.P] * herm * d_sgn((D.jj[a] - D.jj[b]) >> 1);
+  if (c1 > c2)
+    return d_flip(op[T.off_fph + D.loc[b] + (int64_t)D.loc[a] * D.P], (herm < 0) != (((D.jj[a] - D.jj[b]) >> 1) & 1));
   return op[T.off_fph + D.loc[a] + (int64_t)D.loc[b] * D.P];
 }
 
@@ -246,11 +243,11 @@ __global__ void k_ts121(DevLayout D, DevTLayout T, const double* __restrict__ L,
     double smx = 0.0, smy = 0.0;
     for (int J2 = abs(ji - jq); J2 <= ji + jq; J2 += 2)
       for (int J1 = abs(ja - jp); J1 <= ja + jp; J1 += 2)
-        smx += d_telem(D, T, R, hR, ak, pk, ik, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * d_sgn(J1 >> 1) *
+        smx += d_flip(d_telem(D, T, R, hR, ak, pk, ik, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]), (J1 >> 1) & 1) *
                d_six_t(T, J1, J2, jq, jp, ji);
     for (int J1 = abs(ji - jp); J1 <= ji + jp; J1 += 2)
       for (int J2 = abs(ja - jq); J2 <= ja + jq; J2 += 2)
-        smy += d_telem(D, T, R, hR, ik, pk, ak, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]) * d_sgn(J1 >> 1) *
+        smy += d_flip(d_telem(D, T, R, hR, ik, pk, ak, qk, J1, J2) * (T.sq[J1 >> 1] * T.sq[J2 >> 1]), (J1 >> 1) & 1) *
                d_six_t(T, J1, J2, jq, jp, ji);
     sm += L[D.off_fph + a + (int64_t)i * D.P] * (hL * smx - smy) * d_sgn((rank + jq + ji) >> 1);
   }
@@ -364,7 +361,9 @@ __global__ void k_ts122(DevLayout D, DevTLayout T, const double* __restrict__ L,
       const int i = D.same_list[s0 + t];
       sm -= d_f_elem(D, L, hL, i, d) * d_telem(D, T, R, hR, a, b, c, i, J1, J2);
     }
-    RES[T.goff[0] + e] = sm / sqrt(1.0 + (a == b ? 1.0 : 0.0)) / sqrt(1.0 + (c == d ? 1.0 : 0.0));
+    if (a == b) sm /= 1.4142135623730951;
+    if (c == d) sm /= 1.4142135623730951;
+    RES[T.goff[0] + e] = sm;
   }
 }
 
@@ -396,10 +395,13 @@ __global__ void k_ts212(DevLayout D, DevTLayout T, const double* __restrict__ L,
       const int i = T.tnb_list[s0 + t];
       s4 -= d_six_t(T, J1, J2, jc, D.jj[i], jd) * d_ftelem(D, T, R, hR, i, c) * d_v_elem(D, L, hL, a, b, d, i, J1);
     }
-    const double sm = s1 * d_sgn((ja + jb - J2) >> 1) + s2 * d_sgn((J1 + J2) >> 1) + s3 * d_sgn((jc + jd - J1) >> 1) +
-                      s4 * d_sgn((J2 + J1) >> 1);
-    RES[T.goff[0] + e] += sm * sqrt((J1 + 1.0) * (J2 + 1.0) / (1.0 + (a == b ? 1.0 : 0.0)) /
-                                    (1.0 + (c == d ? 1.0 : 0.0))) * d_sgn(rank >> 1);
+    const double sm = d_flip(s1, ((ja + jb - J2) >> 1) & 1) + d_flip(s2, ((J1 + J2) >> 1) & 1) +
+                      d_flip(s3, ((jc + jd - J1) >> 1) & 1) + d_flip(s4, ((J2 + J1) >> 1) & 1);
+    // (J1 + 1)(J2 + 1) over 2 for each pair of equal orbits: exact
+    double w = d_int(J1 + 1) * d_int(J2 + 1);
+    if (a == b) w *= 0.5;
+    if (c == d) w *= 0.5;
+    RES[T.goff[0] + e] += d_flip(sm * sqrt(w), (rank >> 1) & 1);
   }
 }
 
@@ -543,7 +545,7 @@ namespace {
 //
 // One loop for the four sums and for every order of the orbits, its signs linear in J1 / 2 and J2 / 2: written out, the sixteen
 // cases took the warps through sixteen copies of the loop and past the instruction cache, 55% of the time between two issues
-// (first term of the eMax 4 observable: before 704 us).
+// (first term of the eMax 4 observable: 704 us, now 227).
 __device__ __forceinline__ void ph_scatter_elem(const DevLayout& D, const DevTLayout& T, double* RES, int J3, int J4,
                                                 int qa, int qb, int IX, int JX, double X, double Y, int hL, int hR,
                                                 double thresh, int exc) {
