@@ -410,8 +410,8 @@ imsrg_status Ctx::commutator(const double* Lp, int hL, const double* Rp, int hR,
 
 imsrg_status Ctx::fp64_commutator(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES, bool with_e0) {
   mark(kPhaseStart);
-  const bool groups = L.slab >= kGatherMinSlab;
-  if (groups) CK(gather_prepare());
+  bool groups = false;
+  CK(gather_prepare_fp64(groups));
   CK(ensure_wcc());
   // three branches that meet where RES's two-body part is added to: the one-body parts and 122, the ladder's products, and
   // (main) the cross-coupled products.  A small basis leaves most of the GPU idle in every kernel: one after the other

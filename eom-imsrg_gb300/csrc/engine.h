@@ -100,6 +100,7 @@ struct Ctx {
   double* d_gen = nullptr;  // w2 generator workspace (3 slabs)
   imsrg::TcState* tc = nullptr;
   imsrg::GatherPlan gp;  // gather kernels of the commutator (gather.cu)
+  bool gather_no_room = false;  // no device memory for them in FP64
   // FP64 products on the tensor cores (gemm_oz.cu): the digit plans of the ladder and of the cross-coupled products
   imsrg::OzPlan pphh_oz, wcc_oz;
   int oz_sms = 0;  // SMs of the device, once a plan is ready
@@ -235,6 +236,7 @@ struct Ctx {
 
   // gather plan and commutator_122 by pair groups, gather.cu
   imsrg_status gather_prepare();
+  imsrg_status gather_prepare_fp64(bool& groups);
   void gather_release();
   imsrg_status g122_set_caps(int tiny_cap, int small_cap);
   template <typename T>

@@ -11,8 +11,23 @@
 
 using namespace imsrg;
 
+// The FP64 commutator's use of the plan: wanted by the size of the basis, and left for good where the device has no room
+// for its tables (the kernels that take a thread per element need none).
+imsrg_status Ctx::gather_prepare_fp64(bool& groups) {
+  groups = L.slab >= kGatherMinSlab && !gather_no_room;
+  if (!groups) return IMSRG_OK;
+  const imsrg_status s = gather_prepare();
+  if (s != IMSRG_ERR_OUT_OF_MEMORY) return s;
+  cudaGetLastError();
+  gather_release();
+  gather_no_room = true;
+  groups = false;
+  return IMSRG_OK;
+}
+
 imsrg_status Ctx::gather_prepare() {
   if (gp.state) return IMSRG_OK;
+  gather_release();  // what a failed preparation left
   const Layout& l = L;
   if (l.JM + 1 > 26) {
     gp.why = "mixed recoupling supports 2j <= 25 (eMax <= 12)";

@@ -494,7 +494,11 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   if (macs < kOzMinMacs) {
     const std::vector<GemmTile> t = build_tiles(probs, 16, 16);
     if (t.empty()) return IMSRG_OK;
-    CK_TC(cuda(cudaMalloc(&P.tables, sizeof(GemmTile) * t.size()), "cudaMalloc(FP64 product tiles)"));
+    if (cudaMalloc(&P.tables, sizeof(GemmTile) * t.size()) != cudaSuccess) {
+      cudaGetLastError();
+      P.tables = nullptr;
+      return IMSRG_OK;
+    }
     CK_TC(cuda(cudaMemcpy(P.tables, t.data(), sizeof(GemmTile) * t.size(), cudaMemcpyHostToDevice), "cudaMemcpy(FP64 product tiles)"));
     P.d_small = static_cast<const GemmTile*>(P.tables);
     P.nsmall = (int)t.size();

@@ -307,7 +307,8 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
     if (L.cc_size) CK_TC(ensure_wcc());
     CK_TC(oz_prepare(pphh_oz, pphh_probs));
     CK_TC(oz_prepare(wcc_oz, wcc_probs));
-    if (L.slab >= kGatherMinSlab) CK_TC(gather_prepare());
+    bool groups = false;
+    CK_TC(gather_prepare_fp64(groups));
   }
   if (!sg) {
     sg = new StepGraph();
