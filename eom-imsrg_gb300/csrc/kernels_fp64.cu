@@ -8,8 +8,10 @@ namespace imsrg {
 
 // ---------------------------------------------------------------- Pandya transform
 // calculate_cross_coupled (src/cross_coupled.f90:1190-1300): one thread per CCX element,
-// CCX(q) column-major (rlen x nph), threads consecutive in the row index.
-__global__ void k_pandya(DevLayout D, const double* __restrict__ op, int herm, double* __restrict__ cc) {
+// CCX(q) column-major (rlen x nph), threads consecutive in the row index.  Bound by the latency of its table and element
+// reads (issue 45% busy at a third of the warps with 80 registers): five CTAs an SM, commutator at eMax 6 323 -> 316 us, at
+// eMax 10 8.49 -> 8.45 ms (four 321 and 8.46, six 316 and 8.45).
+__global__ void __launch_bounds__(256, 5) k_pandya(DevLayout D, const double* __restrict__ op, int herm, double* __restrict__ cc) {
   constexpr int kSq = 64;
   __shared__ double sq[kSq];  // sqrt(JC + 1): a square root costs as much as the sum of an element
   for (int k = threadIdx.x; k < kSq; k += blockDim.x) sq[k] = sqrt(2.0 * k + 1.0);
