@@ -92,10 +92,6 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_recouple_q(DevLayout D, con
   }
 }
 
-__device__ __forceinline__ double d_flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
-}
-
 // The FP64 form, on the reference's products W = LCC RCC^T: the four W elements of each J' are folded as they are read,
 //   zd(J') = Z[(k,i),(j,l)] + phase Z[(l,j),(i,k)],  Z(r, c) = hL W(r, c) - hR W(c, r),  phase = (-1)^((ji+jj+jk+jl)/2),
 // (exchange: k and l swapped), signs by integer instructions.  Bound by the W sectors it touches (four scattered reads of
