@@ -1,108 +1,196 @@
 // Grouped FP64 GEMM over a static problem/tile list on the FP64 pipe: the lists that have no digit plan
-// (gemm_oz.cu), and those with a non-finite operand.
+// (gemm_oz.cu), those with a non-finite operand, and the elements that the digits are too coarse for.
 //
 // One CTA per 64x64 output tile, 256 threads each accumulating a 4x4 sub-tile with
 // DFMA; K is staged through shared memory in chunks of 16 with loads coalesced along
 // whichever dimension is contiguous for the operand's transpose flag.  On GB300 the
 // FP64 pipe, not HBM, bounds this kernel, so the tile only has to keep DFMA busy.
 #include "gemm.h"
+#include "gemm_oz.h"
 #include "kernels.h"
 
 namespace imsrg {
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int kRestParts = 16;     // warps that share the single elements of a piece
 
 __device__ __forceinline__ double alpha_of(int code, int hL, int hR) {
   const int sel = code & 3;
   double a = (sel == kAlphaHL) ? (double)hL : (sel == kAlphaHR ? (double)hR : 1.0);
   return (code & kAlphaNeg) ? -a : a;
 }
+
+// one 64 x 64 output tile on 256 threads
+__device__ __forceinline__ void gemm_tile(const GemmProb& P, const GemmTile& tile, const GemmOperands& ops, double (&As)[BK][BM + 1],
+                                          double (&Bs)[BK][BN + 1]) {
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;
+  double acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+
+  for (int t = 0; t < P.nterm; ++t) {
+    const GemmTerm& T = P.t[t];
+    const double* A = ops.in[T.a_id] + T.a_off;
+    const double* B = ops.in[T.b_id] + T.b_off;
+    const double alpha = alpha_of(T.alpha, ops.hL, ops.hR);
+    for (int k0 = 0; k0 < T.K; k0 += BK) {
+      // A tile: op(A)(m, k), m in [m0, m0+64), k in [k0, k0+16)
+      if (T.ta == 0) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int m = tid & 63, k = (tid >> 6) + 4 * s;
+          const int gm = tile.m0 + m, gk = k0 + k;
+          As[k][m] = (gm < P.M && gk < T.K) ? alpha * A[gm + (int64_t)gk * T.lda] : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int k = tid & 15, m = (tid >> 4) + 16 * s;
+          const int gm = tile.m0 + m, gk = k0 + k;
+          As[k][m] = (gm < P.M && gk < T.K) ? alpha * A[gk + (int64_t)gm * T.lda] : 0.0;
+        }
+      }
+      // B tile: op(B)(k, n)
+      if (T.tb == 0) {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int k = tid & 15, n = (tid >> 4) + 16 * s;
+          const int gn = tile.n0 + n, gk = k0 + k;
+          Bs[k][n] = (gn < P.N && gk < T.K) ? B[gk + (int64_t)gn * T.ldb] : 0.0;
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int n = tid & 63, k = (tid >> 6) + 4 * s;
+          const int gn = tile.n0 + n, gk = k0 + k;
+          Bs[k][n] = (gn < P.N && gk < T.K) ? B[gn + (int64_t)gk * T.ldb] : 0.0;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < BK; ++kk) {
+        double a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = As[kk][tx + 16 * i];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = Bs[kk][ty + 16 * j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+      }
+      __syncthreads();
+    }
+  }
+  double* C = ops.out[P.c_id] + P.c_off;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int gm = tile.m0 + tx + 16 * i, gn = tile.n0 + ty + 16 * j;
+      if (gm < P.M && gn < P.N) {
+        double* c = C + gm + (int64_t)gn * P.ldc;
+        if (P.accum) atomicAdd(c, acc[i][j]);  // other kernels may add to the same elements
+        else *c = acc[i][j];
+      }
+    }
+}
+
 }  // namespace
 
 __global__ void __launch_bounds__(256) k_gemm_fp64(const GemmProb* __restrict__ probs,
-                                                   const GemmTile* __restrict__ tiles, int ntiles, GemmOperands ops,
-                                                   const int* __restrict__ run_if) {
+                                                   const GemmTile* __restrict__ tiles, GemmOperands ops) {
   __shared__ double As[BK][BM + 1];
   __shared__ double Bs[BK][BN + 1];
-  if (run_if && !*run_if) return;
-  for (int x = blockIdx.x; x < ntiles; x += gridDim.x) {
-    const GemmTile tile = tiles[x];
-    const GemmProb& P = probs[tile.prob];
-    const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
-    double acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+  const GemmTile tile = tiles[blockIdx.x];
+  gemm_tile(probs[tile.prob], tile, ops, As, Bs);
+}
 
-    for (int t = 0; t < P.nterm; ++t) {
-      const GemmTerm& T = P.t[t];
-      const double* A = ops.in[T.a_id] + T.a_off;
-      const double* B = ops.in[T.b_id] + T.b_off;
-      const double alpha = alpha_of(T.alpha, ops.hL, ops.hR);
-      for (int k0 = 0; k0 < T.K; k0 += BK) {
-        // A tile: op(A)(m, k), m in [m0, m0+64), k in [k0, k0+16)
-        if (T.ta == 0) {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const int m = tid & 63, k = (tid >> 6) + 4 * s;
-            const int gm = tile.m0 + m, gk = k0 + k;
-            As[k][m] = (gm < P.M && gk < T.K) ? alpha * A[gm + (int64_t)gk * T.lda] : 0.0;
-          }
-        } else {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const int k = tid & 15, m = (tid >> 4) + 16 * s;
-            const int gm = tile.m0 + m, gk = k0 + k;
-            As[k][m] = (gm < P.M && gk < T.K) ? alpha * A[gk + (int64_t)gm * T.lda] : 0.0;
-          }
-        }
-        // B tile: op(B)(k, n)
-        if (T.tb == 0) {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const int k = tid & 15, n = (tid >> 4) + 16 * s;
-            const int gn = tile.n0 + n, gk = k0 + k;
-            Bs[k][n] = (gn < P.N && gk < T.K) ? B[gk + (int64_t)gn * T.ldb] : 0.0;
-          }
-        } else {
-#pragma unroll
-          for (int s = 0; s < 4; ++s) {
-            const int n = tid & 63, k = (tid >> 6) + 4 * s;
-            const int gn = tile.n0 + n, gk = k0 + k;
-            Bs[k][n] = (gn < P.N && gk < T.K) ? B[gn + (int64_t)gk * T.ldb] : 0.0;
-          }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-          double a[4], b[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) a[i] = As[kk][tx + 16 * i];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) b[j] = Bs[kk][ty + 16 * j];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-      }
+// What the digit products of a list (gemm_oz.cu) leave: the whole list where an operand is not finite, otherwise the noted
+// elements.  A piece's few elements are shared by kRestParts warps, an element at a time with K across the lanes: a chain of
+// uncoalesced reads is what one takes, and many warps wait side by side.  A fuller piece goes to eight CTAs: a warp's lanes
+// take the rows of one column, whose reads are contiguous or broadcast, and four warps share K.  Only noted elements are
+// written.
+__global__ void __launch_bounds__(256) k_gemm_fp64_rest(const GemmProb* __restrict__ probs, const GemmTile* __restrict__ tiles,
+                                                        int ntiles, GemmOperands ops, const int* __restrict__ flags,
+                                                        const OzRedo* __restrict__ redo, int max_redo) {
+  __shared__ double sh[2][BK][BM + 1];
+  if (flags[0]) {
+    for (int x = blockIdx.x; x < ntiles; x += gridDim.x) {
+      const GemmTile tile = tiles[x];
+      gemm_tile(probs[tile.prob], tile, ops, sh[0], sh[1]);
     }
-    double* C = ops.out[P.c_id] + P.c_off;
+    return;
+  }
+  const int few = flags[1], many = flags[2], tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  auto put = [&](const GemmProb& P, int m, int c, double v) {
+    double* at = ops.out[P.c_id] + P.c_off + m + (int64_t)c * P.ldc;
+    if (P.accum) atomicAdd(at, v);
+    else *at = v;
+  };
+  for (int64_t x = blockIdx.x * 8 + warp; x < (int64_t)few * kRestParts; x += gridDim.x * 8) {
+    const OzRedo& r = redo[x / kRestParts];
+    const unsigned mask = r.mask[lane];
+    const int own = __popc(mask), count = __reduce_add_sync(0xffffffffu, own);
+    const GemmProb& P = probs[r.prob];
+    const int t0 = P.accum ? r.term : 0, t1 = P.accum ? r.term + 1 : P.nterm;
+    int before = own;  // elements of the rows before this lane's
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int gm = tile.m0 + tx + 16 * i, gn = tile.n0 + ty + 16 * j;
-        if (gm < P.M && gn < P.N) {
-          double* c = C + gm + (int64_t)gn * P.ldc;
-          if (P.accum) atomicAdd(c, acc[i][j]);  // other kernels may add to the same elements
-          else *c = acc[i][j];
-        }
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += y;
+    }
+    before -= own;
+    for (int e = (int)(x % kRestParts); e < count; e += kRestParts) {
+      const int row = 31 - __clz(__ballot_sync(0xffffffffu, before <= e));
+      unsigned bits = __shfl_sync(0xffffffffu, mask, row);
+      for (int k = e - __shfl_sync(0xffffffffu, before, row); k > 0; --k) bits &= bits - 1u;
+      const int m = r.m + row, c = r.n + __ffs((int)bits) - 1;
+      double s = 0.0;
+      for (int t = t0; t < t1; ++t) {
+        const GemmTerm& T = P.t[t];
+        const double* A = ops.in[T.a_id] + T.a_off + (T.ta ? (int64_t)m * T.lda : m);
+        const double* B = ops.in[T.b_id] + T.b_off + (T.tb ? c : (int64_t)c * T.ldb);
+        const int64_t sa = T.ta ? 1 : T.lda, sb = T.tb ? T.ldb : 1;
+        double v = 0.0;
+#pragma unroll 4
+        for (int k = lane; k < T.K; k += 32) v = fma(A[k * sa], B[k * sb], v);
+        s = fma(alpha_of(T.alpha, ops.hL, ops.hR), v, s);
       }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) put(P, m, c, s);
+    }
+  }
+  double* sums = &sh[0][0][0];
+  for (int64_t x = blockIdx.x; x < (int64_t)many * 8; x += gridDim.x) {
+    const OzRedo& r = redo[max_redo - 1 - (x >> 3)];
+    const unsigned mask = r.mask[lane];
+    const GemmProb& P = probs[r.prob];
+    const int t0 = P.accum ? r.term : 0, t1 = P.accum ? r.term + 1 : P.nterm;
+    // this thread: row `lane` and column c of the piece (clamped where it ends), every fourth K
+    const int c = 2 * (int)(x & 7) + (warp & 1), part = warp >> 1, row = min(r.m + lane, P.M - 1), col = min(r.n + c, P.N - 1);
+    double acc = 0.0;
+    for (int t = t0; t < t1; ++t) {
+      const GemmTerm& T = P.t[t];
+      const double* A = ops.in[T.a_id] + T.a_off + (T.ta ? (int64_t)row * T.lda : row);
+      const double* B = ops.in[T.b_id] + T.b_off + (T.tb ? col : (int64_t)col * T.ldb);
+      const int64_t sa = T.ta ? 1 : T.lda, sb = T.tb ? T.ldb : 1;
+      const int K = T.K;
+      double v = 0.0;
+#pragma unroll 8
+      for (int k = part; k < K; k += 4) v = fma(A[k * sa], B[k * sb], v);
+      acc = fma(alpha_of(T.alpha, ops.hL, ops.hR), v, acc);
+    }
+    sums[tid] = acc;
+    __syncthreads();
+    if (part == 0 && (mask >> c & 1u))
+      put(P, r.m + lane, r.n + c, (sums[tid] + sums[tid + 64]) + (sums[tid + 128] + sums[tid + 192]));
+    __syncthreads();
   }
 }
 

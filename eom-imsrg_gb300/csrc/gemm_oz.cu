@@ -13,11 +13,19 @@
 // i + j >= 8, together below K 2^-59 of the two powers of two (K^(1/2) 2^-62 for digits that behave as random ones),
 // against a rounding of 2^-53 of the running sum at every step of a chain of FP64 FMAs.
 //
+// The powers of two say little about an element where the large elements of a row meet the small ones of a column, and an
+// FMA chain would be far better there.  So a ninth slice holds every element's magnitude, |a| 2^-ea in BF16, and its product
+// gives each output element's sum of |a||b| 2^-(ea+eb), term by term, before the digits.  Digits are kept from
+// 2^-6 K^(1/2) on: then K 2^-59 is below K^(1/2) 2^-53 of the sum of |a||b|, within the bound of the FMAs, and K^(1/2) 2^-62
+// below what a chain of K roundings usually adds up to.  Elements below that (of random operators' products a few
+// in a million at K in the hundreds, one in 3000 at K of a few) are noted and left to k_gemm_fp64_rest.  The ninth product
+// costs 2 of 74 MMAs and a reading more of the accumulators for each term.
+//
 // Rows that hold an Inf or a NaN have no such form: the split raises a flag, this kernel then leaves the outputs alone
-// and k_gemm_fp64, launched behind it with the same flag, computes the whole list.
+// and k_gemm_fp64_rest, launched behind it with the same flag, computes the whole list.
 //
 // Measured at eMax 10 (GB300): the ladder's list (33 G multiply-adds, K up to 1291) 63.2 -> 3.0 ms, the cross-coupled
-// list (9.1 G, K up to 74) 17.7 -> 1.75 ms against k_gemm_fp64; error of W1 and W2 against extended precision at eMax 8
+// list (9.1 G, K up to 74) 17.7 -> 1.7 ms against k_gemm_fp64; error of W1 and W2 against extended precision at eMax 8
 // 6.6e-17 (norm), 6.2e-16 before.  An MMA takes about 51 clocks, near the 48 that reading its 6 KB of operands from
 // shared memory takes; a list of small K is bound by the readers' integer instructions (about 60 an output element).
 //
@@ -29,6 +37,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <queue>
@@ -49,26 +58,34 @@ constexpr int kBlockBytes = S * kSliceBytes;           // 64 KiB
 constexpr int kStageA = kBlockBytes, kStageB = kBlockBytes / 2;
 constexpr int kStageBytes = kStageA + kStageB;
 constexpr int kStages = 2;
+constexpr int kMagBlocks = S;    // K blocks of magnitudes in a stage
 constexpr int kChunkBlocks = 4;  // K blocks between two readings of the accumulators: K = 128
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = 32 * (2 + kEpiWarps);
-constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024 + 256;
+constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024 + 256 + 2 * 32 * kEpiWarps;
+
+// The accumulators in the order in which they are issued and read.  The last one holds the sums of magnitudes before a term's
+// first digits: its own digits come last, so that the readers of the tile before delay those alone.
+__host__ __device__ constexpr int oz_order(int x) { return x < S - 1 ? S - 2 - x : S - 1; }
 
 // the exponent e with |a| < 2^e of the largest high word of a row's magnitudes (subnormals count as 2^-1022)
 __device__ __forceinline__ int oz_exp(unsigned maxhi) { return max((int)(maxhi >> 20), 1) - 1022; }
 
-// a 2^(62-e) to the nearest integer, as the biased digits: byte 7 - s is d_s + 128
-__device__ __forceinline__ unsigned long long oz_digits(double a, int e) {
+// a 2^(62-e) to the nearest integer, as the biased digits: byte 7 - s is d_s + 128.  mag: |a| 2^-e rounded down to BF16, at
+// least 2^-62 unless a is zero (a product of two is then above the smallest normal number).
+__device__ __forceinline__ unsigned long long oz_digits(double a, int e, unsigned& mag) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(a);
   const int ea = (int)(b >> 52) & 0x7FF;
   const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (ea ? 1ull << 52 : 0ull);
   const int sh = max(ea, 1) - 1075 + 62 - e;  // <= 9
-  long long i;
-  if (sh >= 0) i = (long long)(m << sh);
-  else if (sh > -55) i = (long long)((m + (1ull << (-sh - 1))) >> -sh);
+  unsigned long long i;
+  if (sh >= 0) i = m << sh;
+  else if (sh > -55) i = (m + (1ull << (-sh - 1))) >> -sh;
   else i = 0;
-  if (b >> 63) i = -i;
-  return ((unsigned long long)i + 0x0080808080808080ull) ^ 0x8000000000000000ull;
+  const int z = __clzll((long long)(i | 1ull));
+  mag = m ? (unsigned)(128 - z) << 7 | ((unsigned)((i << z) >> 56) & 0x7Fu) : 0u;
+  if (b >> 63) i = 0ull - i;
+  return (i + 0x0080808080808080ull) ^ 0x8000000000000000ull;
 }
 // the BF16 values of digit s of two elements, packed (low half: the first)
 __device__ __forceinline__ unsigned oz_pair(unsigned long long x, unsigned long long y, int s) {
@@ -79,11 +96,11 @@ __device__ __forceinline__ unsigned oz_pair(unsigned long long x, unsigned long 
 
 }  // namespace
 
-// One CTA per 32 rows of an operand: the row exponents, then the digits.  Bound by memory: 8 bytes read (twice, the
-// second time from L2) and 16 written an element.
+// One CTA per 32 rows of an operand: the row exponents, then the digits and magnitudes.  Bound by memory: 8 bytes read (twice,
+// the second time from L2) and 18 written an element.
 __global__ void __launch_bounds__(256) k_oz_split(const OzOperand* __restrict__ ops, const OzChunk* __restrict__ chunks,
-                                                  GemmOperands in, char* __restrict__ buf, int* __restrict__ exps,
-                                                  int* flag) {
+                                                  GemmOperands in, char* __restrict__ buf, char* __restrict__ mag,
+                                                  int* __restrict__ exps, int* flag) {
   __shared__ unsigned mx[32];
   const OzChunk ch = chunks[blockIdx.x];
   const OzOperand o = ops[ch.op];
@@ -113,6 +130,7 @@ __global__ void __launch_bounds__(256) k_oz_split(const OzOperand* __restrict__ 
   }
   const int rb = ch.r0 >> 7, rin = ch.r0 & 127;
   char* blk = buf + (o.blk0 + (int64_t)rb * o.nkb) * kBlockBytes;
+  char* mblk = mag + (o.blk0 + (int64_t)rb * o.nkb) * kSliceBytes;
   if (o.ks == 1) {  // two rows of 32 K a warp pass, two K a thread
     const int half = lane >> 4, k2 = (lane & 15) * 2;
     for (int x = warp; x < o.nkb * 16; x += 8) {
@@ -120,11 +138,13 @@ __global__ void __launch_bounds__(256) k_oz_split(const OzOperand* __restrict__ 
       if (r >= nr) continue;
       const double* row = A + (int64_t)(ch.r0 + r) * o.rs;
       const int e = oz_exp(mx[r]);
-      const unsigned long long d0 = oz_digits(k < o.K ? row[k] : 0.0, e), d1 = oz_digits(k + 1 < o.K ? row[k + 1] : 0.0, e);
-      const int rr = rin + r;
-      char* dst = blk + (int64_t)kb * kBlockBytes + rr * 64 + (((k2 >> 3) ^ ((rr >> 1) & 3)) << 4) + (k2 & 7) * 2;
+      unsigned m0, m1;
+      const unsigned long long d0 = oz_digits(k < o.K ? row[k] : 0.0, e, m0), d1 = oz_digits(k + 1 < o.K ? row[k + 1] : 0.0, e, m1);
+      const int rr = rin + r, at = rr * 64 + (((k2 >> 3) ^ ((rr >> 1) & 3)) << 4) + (k2 & 7) * 2;
+      char* dst = blk + (int64_t)kb * kBlockBytes + at;
 #pragma unroll
       for (int s = 0; s < S; ++s) *reinterpret_cast<unsigned*>(dst + s * kSliceBytes) = oz_pair(d0, d1, s);
+      *reinterpret_cast<unsigned*>(mblk + (int64_t)kb * kSliceBytes + at) = m0 | m1 << 16;
     }
   } else if (lane < nr) {  // lanes along the rows, eight K (16 bytes of a slice's row) a thread
     const double* col = A + ch.r0 + lane;
@@ -132,13 +152,17 @@ __global__ void __launch_bounds__(256) k_oz_split(const OzOperand* __restrict__ 
     for (int x = warp; x < o.nkb * 4; x += 8) {
       const int kb = x >> 2, c = x & 3, k0 = kb * 32 + c * 8;
       unsigned long long d[8];
+      unsigned m[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) d[u] = oz_digits(k0 + u < o.K ? col[(int64_t)(k0 + u) * o.ks] : 0.0, e);
-      char* dst = blk + (int64_t)kb * kBlockBytes + rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4);
+      for (int u = 0; u < 8; ++u) d[u] = oz_digits(k0 + u < o.K ? col[(int64_t)(k0 + u) * o.ks] : 0.0, e, m[u]);
+      const int at = rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4);
+      char* dst = blk + (int64_t)kb * kBlockBytes + at;
 #pragma unroll
       for (int s = 0; s < S; ++s)
         *reinterpret_cast<uint4*>(dst + s * kSliceBytes) = make_uint4(oz_pair(d[0], d[1], s), oz_pair(d[2], d[3], s),
                                                                       oz_pair(d[4], d[5], s), oz_pair(d[6], d[7], s));
+      *reinterpret_cast<uint4*>(mblk + (int64_t)kb * kSliceBytes + at) =
+          make_uint4(m[0] | m[1] << 16, m[2] | m[3] << 16, m[4] | m[5] << 16, m[6] | m[7] << 16);
     }
   }
 }
@@ -166,6 +190,14 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
@@ -204,9 +236,9 @@ __device__ __forceinline__ void oz_mad(long long& acc, int v) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     k_oz_gemm(const OzProb* __restrict__ probs, const OzTile* __restrict__ tiles, const int* __restrict__ start, GemmOperands out,
-              const char* __restrict__ buf, const int* __restrict__ exps, const int* __restrict__ flag, int* err,
-              unsigned long long wait_ns) {
-  if (*flag) return;  // a row with an Inf or a NaN: k_gemm_fp64 computes the list
+              const char* __restrict__ buf, const char* __restrict__ mag, const int* __restrict__ exps, int* flag,
+              OzRedo* __restrict__ redo, int max_redo, int* err, unsigned long long wait_ns) {
+  if (*flag) return;  // a row with an Inf or a NaN: k_gemm_fp64_rest computes the list
   extern __shared__ uint8_t oz_smem[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(oz_smem) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)kStages * kStageBytes);
@@ -216,6 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dempty + S);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* consumed = reinterpret_cast<volatile int*>(tmem_slot + 2);
+  unsigned short* coarse = reinterpret_cast<unsigned short*>(tmem_slot + 4);  // a word for each reader's 16 elements
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -250,10 +283,21 @@ __global__ void __launch_bounds__(kThreads, 1)
         const OzProb& P = probs[tile.prob];
         for (int term = 0; term < P.nterm && ok; ++term) {
           const int nkb = P.t[term].nkb;
-          const char* a = buf + (P.t[term].a_blk + (int64_t)(tile.m0 >> 7) * nkb) * kBlockBytes;
+          const int64_t ablk = P.t[term].a_blk + (int64_t)(tile.m0 >> 7) * nkb, bblk = P.t[term].b_blk + (int64_t)(tile.n0 >> 7) * nkb;
+          const int half = ((tile.n0 >> 6) & 1) * (kSliceBytes / 2);
+          for (int kb0 = 0; kb0 < nkb; kb0 += kMagBlocks, ++it) {  // the magnitudes of up to eight K blocks in one stage
+            const int s = it % kStages, n = min(kMagBlocks, nkb - kb0);
+            if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, err, 1, wait_ns)) { ok = false; break; }
+            mbar_expect_tx(&full[s], (uint32_t)(n * (kSliceBytes + kSliceBytes / 2)));
+            const uint32_t st = smem_u32(smem + (size_t)s * kStageBytes);
+            bulk_load(st, mag + (ablk + kb0) * kSliceBytes, (uint32_t)(n * kSliceBytes), &full[s]);
+            for (int j = 0; j < n; ++j)
+              bulk_load(st + kStageA + j * (kSliceBytes / 2), mag + (bblk + kb0 + j) * kSliceBytes + half, kSliceBytes / 2, &full[s]);
+          }
+          if (!ok) break;
+          const char* a = buf + ablk * kBlockBytes;
           // a tile of 64 columns takes the upper or the lower half of every slice of its operand block
-          const char* b = buf + (P.t[term].b_blk + (int64_t)(tile.n0 >> 7) * nkb) * kBlockBytes +
-                          ((tile.n0 >> 6) & 1) * (kSliceBytes / 2);
+          const char* b = buf + bblk * kBlockBytes + half;
           for (int kb = 0; kb < nkb; ++kb, ++it) {
             const int s = it % kStages;
             if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, err, 1, wait_ns)) { ok = false; break; }
@@ -276,7 +320,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     if (elect_one()) {  // ---- MMAs
-      int it = 0, cc = 0;
+      int it = 0, cc = 0, cm = 0;  // cc: chunks so far; cm: sums of magnitudes so far
       bool ok = true;
       for (int t = t0; t < t1 && ok; ++t) {
         const OzTile tile = tiles[t];
@@ -286,6 +330,27 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tile.w >> 3) << 17) | (8u << 24);
         for (int term = 0; term < nterm && ok; ++term) {
           const int nkb = P.t[term].nkb;
+          {  // the sums of magnitudes
+            if (!mbar_wait(&dempty[S - 1], ((cc + cm) & 1) ^ 1, abort_flag, err, 2, wait_ns)) { ok = false; break; }
+            tc_fence_after();
+            for (int kb0 = 0; kb0 < nkb; kb0 += kMagBlocks, ++it) {
+              const int s = it % kStages, n = min(kMagBlocks, nkb - kb0);
+              if (!mbar_wait(&full[s], (it / kStages) & 1, abort_flag, err, 3, wait_ns)) { ok = false; break; }
+              tc_fence_after();
+              const uint32_t st = smem_u32(smem) + (uint32_t)(s * kStageBytes);
+              const uint32_t da = oz_desc_lo(st), db = oz_desc_lo(st + kStageA);
+              for (int j = 0; j < n; ++j)
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks)
+                  oz_umma(tmem_base + (S - 1) * kOzTileN, da + ((j * kSliceBytes + ks * 32) >> 4),
+                          db + ((j * (kSliceBytes / 2) + ks * 32) >> 4), idesc, (kb0 == 0 && j == 0 && ks == 0) ? 0u : 1u);
+              umma_commit(&empty[s]);
+              *consumed = it + 1;
+            }
+            if (!ok) break;
+            umma_commit(&dfull[S - 1]);
+            ++cm;
+          }
           for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
             const int s = it % kStages;
             const bool first = (kb & (kChunkBlocks - 1)) == 0, last = (kb & (kChunkBlocks - 1)) == kChunkBlocks - 1 || kb == nkb - 1;
@@ -294,9 +359,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             const uint32_t st = smem_u32(smem) + (uint32_t)(s * kStageBytes);
             const uint32_t da = oz_desc_lo(st), db = oz_desc_lo(st + kStageA);
 #pragma unroll
-            for (int d = S - 1; d >= 0; --d) {
+            for (int x = 0; x < S; ++x) {
+              const int d = oz_order(x);
               if (first) {
-                if (!mbar_wait(&dempty[d], (cc & 1) ^ 1, abort_flag, err, 2, wait_ns)) { ok = false; break; }
+                if (!mbar_wait(&dempty[d], ((d == S - 1 ? cc + cm : cc) & 1) ^ 1, abort_flag, err, 2, wait_ns)) { ok = false; break; }
                 tc_fence_after();
               }
 #pragma unroll
@@ -320,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- readers: warp (quad, grp) has rows 32 quad .. + 31 and columns 16 grp .. + 15 of the tile
     const int quad = warp & 3, grp = (warp - 2) >> 2;
     const uint32_t tm = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(grp * 16);
-    int cc = 0;
+    int cc = 0, cm = 0;
     bool ok = true;
     for (int t = t0; t < t1 && ok; ++t) {
       const OzTile tile = tiles[t];
@@ -328,21 +394,47 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int m = tile.m0 + quad * 32 + lane, n = tile.n0 + grp * 16;
       const bool mine = grp * 16 < tile.w;
       const int nterm = P.nterm;
-      double* C = out.out[P.c_id] + P.c_off + m + (int64_t)n * P.ldc;
-      const int M = P.M, N = P.N, ldc = P.ldc, nn = N - n;
-      const bool accum = P.accum != 0;
       for (int term = 0; term < nterm && ok; ++term) {
         const OzTerm& T = P.t[term];
         const int nchunk = (T.nkb + kChunkBlocks - 1) / kChunkBlocks;
-        const int ea = __ldg(exps + T.a_exp + min(m, M - 1)) - 68, eb = __ldg(exps + T.b_exp + min(n + (lane & 15), N - 1));
+        const int ea = __ldg(exps + T.a_exp + min(m, P.M - 1)) - 68, eb = __ldg(exps + T.b_exp + min(n + (lane & 15), P.N - 1));
+        // elements whose sum of magnitudes is too small for the digits: noted for k_gemm_fp64_rest
+        {
+          ok = __all_sync(0xffffffffu, mbar_wait(&dfull[S - 1], (cc + cm) & 1, abort_flag, err, 4, wait_ns));
+          if (!ok) break;
+          tc_fence_after();
+          unsigned c16 = 0u;
+          if (mine) {
+            uint32_t r[16];
+            tmem_ld16(tm + (uint32_t)((S - 1) * kOzTileN), r);
+            const unsigned least = __float_as_uint(T.least) - 1u;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) c16 |= r[j] - 1u < least ? 1u << j : 0u;  // 0 < sum < least, by the bits
+            if (c16) c16 = m < P.M ? c16 & ((1u << min(max(P.N - n, 0), 16)) - 1u) : 0u;
+            if (__any_sync(0xffffffffu, c16 != 0u)) {
+              const bool many = __reduce_add_sync(0xffffffffu, __popc(c16)) > kOzSingles;  // these from the end backwards
+              int x = 0;
+              if (lane == 0) x = many ? max_redo - 1 - atomicAdd(flag + 2, 1) : atomicAdd(flag + 1, 1);
+              x = __shfl_sync(0xffffffffu, x, 0);
+              if (lane == 0) *reinterpret_cast<int4*>(&redo[x]) = make_int4(P.src, T.src, tile.m0 + quad * 32, n);
+              redo[x].mask[lane] = (unsigned short)c16;
+            }
+            if (P.accum) coarse[threadIdx.x - 64] = (unsigned short)c16;
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&dempty[S - 1]);
+          ++cm;
+        }
         long long H[16], L[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) H[j] = L[j] = 0;
         for (int c = 0; c < nchunk && ok; ++c, ++cc) {
 #pragma unroll
-          for (int d = S - 1; d >= 0; --d) {
+          for (int x = 0; x < S; ++x) {
+            const int d = oz_order(x);
             // the warp goes on or gives up as one (the TMEM loads below are the whole warp's)
-            ok = __all_sync(0xffffffffu, mbar_wait(&dfull[d], cc & 1, abort_flag, err, 4, wait_ns));
+            ok = __all_sync(0xffffffffu, mbar_wait(&dfull[d], (d == S - 1 ? cc + cm : cc) & 1, abort_flag, err, 4, wait_ns));
             if (!ok) break;
             tc_fence_after();
             if (mine) {
@@ -374,15 +466,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (!ok) break;
         if (!mine) continue;
-        const int sel = T.alpha & 3;
-        const bool neg = ((sel == kAlphaHL && out.hL < 0) || (sel == kAlphaHR && out.hR < 0)) != ((T.alpha & kAlphaNeg) != 0);
+        const OzProb* Q = &P;  // its fields are read again here: kept from the start they cost registers, which are short
+        asm volatile("" : "+l"(Q));
+        const int M = Q->M, ldc = Q->ldc, nn = Q->N - n, sel = Q->t[term].alpha & 3, alpha_neg = Q->t[term].alpha & kAlphaNeg;
+        const bool accum = Q->accum != 0;
+        double* C = out.out[Q->c_id] + Q->c_off + m + (int64_t)n * ldc;
+        const bool neg = ((sel == kAlphaHL && out.hL < 0) || (sel == kAlphaHR && out.hR < 0)) != (alpha_neg != 0);
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           double v = oz_value(H[j], L[j], neg, ea + __shfl_sync(0xffffffffu, eb, j));
           if (m < M && j < nn) {
             double* c = C + (int64_t)j * ldc;
             if (accum) {  // a reduction: other kernels may add to the same elements
-              atomicAdd(c, v);
+              if (!((coarse[threadIdx.x - 64] >> j) & 1)) atomicAdd(c, v);
             } else {
               if (term > 0) v += *c;
               *c = v;
@@ -404,6 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // ---------------------------------------------------------------- host side
 void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
   P.ops.clear(); P.chunks.clear(); P.probs.clear(); P.tiles.clear();
+  P.max_redo = 0;
   P.blocks = 0;
   P.nexp = 0;
   std::map<std::tuple<int, int64_t, int, int, int, int>, int> seen;  // operands used by several products are split once
@@ -427,6 +524,7 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
   for (const GemmProb& g : probs) {
     if (g.M <= 0 || g.N <= 0) continue;
     OzProb p{};
+    p.src = (int)(&g - probs.data());
     p.c_off = g.c_off; p.M = g.M; p.N = g.N; p.ldc = g.ldc; p.c_id = g.c_id; p.accum = g.accum;
     for (int i = 0; i < g.nterm; ++i) {
       const GemmTerm& t = g.t[i];
@@ -438,6 +536,8 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
       o.a_exp = P.ops[a].exp0; o.b_exp = P.ops[b].exp0;
       o.nkb = P.ops[a].nkb;
       o.alpha = t.alpha;
+      o.src = i;
+      o.least = kOzLeast * std::sqrt((float)t.K);
     }
     if (!p.nterm) continue;
     const int x = (int)P.probs.size();
@@ -445,6 +545,7 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
     for (int m0 = 0; m0 < g.M; m0 += kOzTileM)
       for (int n0 = 0; n0 < g.N; n0 += kOzTileN)
         P.tiles.push_back(OzTile{x, m0, n0, std::min(kOzTileN, (g.N - n0 + 15) / 16 * 16)});
+    for (int k = 0; k < p.nterm; ++k) P.max_redo += (int64_t)((g.M + 31) / 32) * ((g.N + 15) / 16);
   }
   // every tile to the CTA with the least work so far, the longest tiles first.  The work of a tile in clocks: a K block
   // takes 72 MMAs that read 4 KB of A and w / 32 KB of B from shared memory, a reading of the accumulators about 4000.
@@ -481,7 +582,7 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
 
 using namespace imsrg;
 
-// Tables and operand blocks of a plan.  The blocks' padding (rows and K past the operand's) is zeroed here and never
+// Tables and operand blocks of a plan.  The blocks' padding (rows past the operand's) is zeroed here and never
 // written.  Where the device has no room for them the list stays on k_gemm_fp64.
 imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   if (P.state) return IMSRG_OK;
@@ -510,10 +611,11 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
   const size_t bo = al(sizeof(OzOperand) * P.ops.size()), bc = al(sizeof(OzChunk) * P.chunks.size()),
                bp = al(sizeof(OzProb) * P.probs.size()), bt = al(sizeof(OzTile) * P.tiles.size()),
-               bs = al(sizeof(int) * P.start.size()), be = al(sizeof(int) * ((size_t)P.nexp + 1));
-  const size_t bb = (size_t)P.blocks * kBlockBytes;
+               bs = al(sizeof(int) * P.start.size()), be = al(sizeof(int) * ((size_t)P.nexp + 3)),
+               br = al(sizeof(OzRedo) * (size_t)P.max_redo);
+  const size_t bb = (size_t)P.blocks * (kBlockBytes + kSliceBytes);
   char* t = nullptr;
-  if (cudaMalloc(&P.buf, bb) != cudaSuccess || cudaMalloc(&t, bo + bc + bp + bt + bs + be) != cudaSuccess) {
+  if (cudaMalloc(&P.buf, bb) != cudaSuccess || cudaMalloc(&t, bo + bc + bp + bt + bs + be + br) != cudaSuccess) {
     cudaGetLastError();
     if (P.buf) cudaFree(P.buf);
     P.buf = nullptr;
@@ -535,6 +637,8 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   P.d_start = reinterpret_cast<const int*>(t + bo + bc + bp + bt);
   P.exps = reinterpret_cast<int*>(t + bo + bc + bp + bt + bs);
   P.flag = P.exps + P.nexp;
+  P.redo = reinterpret_cast<OzRedo*>(t + bo + bc + bp + bt + bs + be);
+  P.mag = P.buf + (size_t)P.blocks * kBlockBytes;
   CK_TC(cuda(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem),
              "smem attr (FP64 products)"));
   P.state = 1;
@@ -557,15 +661,15 @@ imsrg_status Ctx::gemm_fp64(OzPlan& P, const std::vector<GemmProb>& probs, const
     return launched("k_gemm_fp64_small");
   }
   if (P.state > 0) {
-    CK_TC(cuda(cudaMemsetAsync(P.flag, 0, sizeof(int), stream), "memset(non-finite flag)"));
-    k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, P.buf, P.exps, P.flag);
+    CK_TC(cuda(cudaMemsetAsync(P.flag, 0, 3 * sizeof(int), stream), "memset(FP64 product flags)"));
+    k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, P.buf, P.mag, P.exps, P.flag);
     CK_TC(launched("k_oz_split"));
-    k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, P.buf, P.exps, P.flag, d_err,
-                                                   tc_wait_ns);
+    k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, P.buf, P.mag, P.exps, P.flag, P.redo,
+                                                   (int)P.max_redo, d_err, tc_wait_ns);
     CK_TC(launched("k_oz_gemm"));
+    k_gemm_fp64_rest<<<4 * oz_sms, 256, 0, stream>>>(d_probs, d_tiles, ntiles, ops, P.flag, P.redo, (int)P.max_redo);
+    return launched("k_gemm_fp64_rest");
   }
-  // without a plan, or with a non-finite operand
-  k_gemm_fp64<<<P.state > 0 ? std::min(ntiles, 4 * oz_sms) : ntiles, 256, 0, stream>>>(
-      d_probs, d_tiles, ntiles, ops, P.state > 0 ? P.flag : nullptr);
+  k_gemm_fp64<<<ntiles, 256, 0, stream>>>(d_probs, d_tiles, ops);
   return launched("k_gemm_fp64");
 }

@@ -18,7 +18,8 @@ constexpr double kOzMinMacs = 2e7;
 constexpr int kOzTileN = 64;     // widest output tile
 
 // One operand: op(A) as rows of M (or op(B) as rows of N) over K, cut into blocks of 128 rows x 32 K, each block
-// holding its eight digit slices one after the other.  Element (r, k) is at off + r * rs + k * ks of array id.
+// holding its eight digit slices one after the other; a ninth slice of magnitudes is kept apart, so that those of one row
+// block lie one K block after the other.  Element (r, k) is at off + r * rs + k * ks of array id.
 struct OzOperand {
   int64_t off;
   int id, rows, K, nkb;
@@ -33,12 +34,24 @@ struct OzChunk {
 struct OzTerm {
   int64_t a_blk, b_blk;
   int a_exp, b_exp, nkb, alpha;
+  int src;      // the same term of GemmProb
+  float least;  // kOzLeast sqrt(K): sums of magnitudes below it are left to FP64 FMAs
 };
 struct OzProb {
   int64_t c_off;
   int M, N, ldc, c_id, nterm, accum;
+  int src;  // the same problem of the GemmProb list
   OzTerm t[kMaxTerms];
 };
+// Elements of a 32 x 16 piece of an output that one term's digits are too coarse for (gemm_oz.cu): rows m + lane, columns
+// n + bit.  With accum that term alone is still to be added, otherwise the whole element is still to be assigned.
+struct OzRedo {
+  int prob, term, m, n;  // of the GemmProb list
+  unsigned short mask[32];
+};
+constexpr int kOzSingles = 64;  // most elements of an entry that are redone one by one
+// smallest sum of |a||b| 2^-(ea+eb) over sqrt(K) that the digits are used for
+constexpr float kOzLeast = 1.0f / 64;
 // rows m0 .. m0 + 127 and columns n0 .. n0 + w - 1 of a problem (w a multiple of 16, n0 of 64)
 struct OzTile {
   int prob, m0, n0, w;
@@ -57,9 +70,12 @@ struct OzPlan {
   int64_t blocks = 0;
   int nexp = 0;
   void* tables = nullptr;
-  char* buf = nullptr;   // operand blocks
-  int* exps = nullptr;   // row exponents, then the non-finite flag
-  int* flag = nullptr;
+  char* buf = nullptr;   // operand blocks, then their magnitude slices
+  char* mag = nullptr;
+  int* exps = nullptr;   // row exponents, then the flags
+  int* flag = nullptr;   // [0] an operand is not finite; entries of redo with [1] few and [2] many elements (from its end)
+  OzRedo* redo = nullptr;
+  int64_t max_redo = 0;
   const GemmTile* d_small = nullptr;
   int nsmall = 0;
   const OzOperand* d_ops = nullptr;

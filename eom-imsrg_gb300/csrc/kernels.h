@@ -7,6 +7,7 @@
 #include "dev.cuh"
 #include "pair_groups.h"
 #include "gemm.h"
+#include "gemm_oz.h"
 #include "tc.h"
 
 namespace imsrg {
@@ -45,9 +46,10 @@ __global__ void k_zero_runs(double* x, const int64_t* runs);
 __global__ void k_zero_runs_f(float* x, const int64_t* runs);
 __global__ void k_convert_check(const double* x, const float* y, int64_t n, float* out_f32, double* out_f64);
 
-// run_if: with a flag, nothing is done unless it is set
-__global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, int ntiles, GemmOperands ops,
-                            const int* run_if);
+__global__ void k_gemm_fp64(const GemmProb* probs, const GemmTile* tiles, GemmOperands ops);
+// what the digit products leave: flags [0] the whole list, else [1] entries from the start and [2] from the end of redo
+__global__ void k_gemm_fp64_rest(const GemmProb* probs, const GemmTile* tiles, int ntiles, GemmOperands ops, const int* flags,
+                                 const OzRedo* redo, int max_redo);
 // 16 x 16 tiles
 __global__ void k_gemm_fp64_small(const GemmProb* probs, const GemmTile* tiles, GemmOperands ops);
 

@@ -40,7 +40,8 @@ typedef int32_t imsrg_status;
 #define IMSRG_ERR_TIMEOUT 7 /* a bounded device wait ran out (the kernel stopped, the context stays usable) */
 
 /* arithmetic of the channel contractions (pp/hh ladders and cross-coupled GEMM) */
-#define IMSRG_PREC_FP64 0    /* FP64 products (exact BF16 digits on the tensor cores, rounded once) */
+#define IMSRG_PREC_FP64 0    /* FP64 products: BF16 digits on the tensor cores where they keep, element by element,
+                                the error bound of FP64 FMAs, FP64 FMAs elsewhere */
 #define IMSRG_PREC_BF16X3 1  /* 2-slice split-BF16 operands, 3 products, FP32 accumulate (tcgen05) */
 #define IMSRG_PREC_BF16X6 2  /* 3-slice split-BF16 operands, 6 products, FP32 accumulate (tcgen05) */
 #define IMSRG_PREC_TF32X3 3  /* TF32-compensated: each FP32 operand = TF32 hi + TF32 lo, 3 products
