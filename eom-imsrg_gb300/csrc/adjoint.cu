@@ -238,7 +238,7 @@ imsrg_status Ctx::dot(const double* A, const double* B, double* out) {
   CKA(launched("k_dot_partial"));
   k_sum<<<1, 1024, 0, stream>>>(adj->partial, kDotBlocks, d_scalars);
   CKA(launched("k_sum"));
-  CKA(read_scalars(1));
+  CKA(read_scalars());
   *out = h_scalars[0];
   return IMSRG_OK;
 }

@@ -495,9 +495,29 @@ imsrg_status Ctx::frob_async(const double* op, double scale, int slot) {
   return launched("k_sum_sqrt");
 }
 
-imsrg_status Ctx::read_scalars(int n) {
-  CK(cuda(cudaMemcpyAsync(h_scalars, d_scalars, sizeof(double) * n, cudaMemcpyDeviceToHost, stream), "D2H scalars"));
-  return cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+// the scalars and, in the same copy, the error word behind them
+imsrg_status Ctx::read_scalars() {
+  CK(cuda(cudaMemcpyAsync(h_scalars, d_scalars, sizeof(double) * (kErrorSlot + 1), cudaMemcpyDeviceToHost, stream), "D2H scalars"));
+  CK(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
+  return wait_error();
+}
+
+// Waits for the stream and reports a wait that ran out: the end of every call that hands results to the host, since a kernel
+// that gave up left its output incomplete.
+imsrg_status Ctx::finish() {
+  CK(cuda(cudaMemcpyAsync(h_scalars + kErrorSlot, d_scalars + kErrorSlot, sizeof(double), cudaMemcpyDeviceToHost, stream), "D2H error word"));
+  CK(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
+  return wait_error();
+}
+
+imsrg_status Ctx::wait_error() {
+  const int e = *reinterpret_cast<const int*>(h_scalars + kErrorSlot);
+  if (!e) return IMSRG_OK;
+  CK(cuda(cudaMemsetAsync(d_err, 0, sizeof(int), stream), "memset(error word)"));
+  static const char* role[] = {"", "producer (stage free)", "MMA (accumulator free)", "MMA (stage loaded)",
+                               "epilogue (accumulator ready)"};
+  return fail(IMSRG_ERR_TIMEOUT, std::string("tensor-core GEMM: a bounded wait ran out in the ") +
+                                     (e >= 1 && e <= 4 ? role[e] : "kernel") + " (code " + std::to_string(e) + ")");
 }
 
 imsrg_status Ctx::white(const double* H, int hH, double* ETA) {
@@ -553,7 +573,7 @@ imsrg_status Ctx::magnus_expand(double* DG, int hDG, const double* G, int hG, in
   double advals[8] = {0};
   CK(frob_async(DG, 1.0, 0));
   CK(frob_async(G, 1.0, 1));
-  CK(read_scalars(2));
+  CK(read_scalars());
   advals[1] = h_scalars[0];
   const double fullnorm = h_scalars[1];
   *used = 0;
@@ -571,7 +591,7 @@ imsrg_status Ctx::magnus_expand(double* DG, int hDG, const double* G, int hG, in
     CK(commutator(G, hG, ad, hDG, out, hDG, false));
     ++*used;
     CK(axpy_frob_async(DG, cof[i - 1], out, std::fabs(cof[i - 1]), 0, false));
-    CK(read_scalars(1));
+    CK(read_scalars());
     advals[i] = h_scalars[0];
   }
   return IMSRG_OK;
@@ -604,7 +624,7 @@ imsrg_status Ctx::bch_expand(double* HS, const double* G, int hG, const double* 
       CK(restore_quadrupoles(ad, hH, G, hG, int3));
     }
     CK(axpy_frob_async(HS, coef, out, coef, 0, true));
-    CK(read_scalars(1));
+    CK(read_scalars());
     if (h_scalars[0] < conv) break;
   }
   *terms = (iw > max_terms) ? max_terms - 1 : iw - 1;
@@ -750,8 +770,7 @@ imsrg_status imsrg_set_precision(imsrg_ctx* ctx, int32_t mode) {
 
 imsrg_status imsrg_synchronize(imsrg_ctx* ctx) {
   CTX(ctx);
-  CK(c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize"));
-  return c->tc_error();
+  return c->finish();
 }
 
 imsrg_status imsrg_set_wait_limit(imsrg_ctx* ctx, int64_t nanoseconds) {
@@ -889,7 +908,7 @@ imsrg_status imsrg_op_download_slab(imsrg_ctx* ctx, const imsrg_op* op, double* 
   if (!host) return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "NULL host slab");
   CK(c->cuda(cudaMemcpyAsync(host, op->d, sizeof(double) * (size_t)c->L.slab, cudaMemcpyDeviceToHost, c->stream),
              "D2H slab"));
-  return c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+  return c->finish();
 }
 
 imsrg_status imsrg_op_upload(imsrg_ctx* ctx, imsrg_op* op, const double* const* gam, const double* fhh,
@@ -921,7 +940,7 @@ imsrg_status imsrg_op_download(imsrg_ctx* ctx, const imsrg_op* op, double* const
   const Layout& L = c->L;
   std::vector<double> h((size_t)L.slab);
   CK(c->cuda(cudaMemcpyAsync(h.data(), op->d, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream), "D2H"));
-  CK(c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize"));
+  CK(c->finish());
   if (E0) *E0 = h[0];
   if (fhh && L.A) std::memcpy(fhh, &h[L.off_fhh], sizeof(double) * L.A * L.A);
   if (fpp && L.P) std::memcpy(fpp, &h[L.off_fpp], sizeof(double) * L.P * L.P);
@@ -947,7 +966,7 @@ imsrg_status imsrg_op_get_e0(imsrg_ctx* ctx, const imsrg_op* op, double* E0) {
   CK(check_op(c, op, "imsrg_op_get_e0"));
   if (!E0) return IMSRG_ERR_INVALID_ARGUMENT;
   CK(c->cuda(cudaMemcpyAsync(c->h_scalars, op->d, sizeof(double), cudaMemcpyDeviceToHost, c->stream), "D2H E0"));
-  CK(c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize"));
+  CK(c->finish());
   *E0 = c->h_scalars[0];
   return IMSRG_OK;
 }
@@ -998,7 +1017,7 @@ imsrg_status imsrg_mat_frob_norm(imsrg_ctx* ctx, const imsrg_op* op, double* out
   CK(check_op(c, op, "imsrg_mat_frob_norm"));
   if (!out) return IMSRG_ERR_INVALID_ARGUMENT;
   CK(c->frob_async(op->d, 1.0, 0));
-  CK(c->read_scalars(1));
+  CK(c->read_scalars());
   *out = c->h_scalars[0];
   return IMSRG_OK;
 }
@@ -1037,7 +1056,7 @@ imsrg_status imsrg_mbpt2(imsrg_ctx* ctx, const imsrg_op* H, double* out) {
   CK(c->launched("k_mbpt2_partial"));
   k_sum<<<1, 1024, 0, c->stream>>>(c->d_partial, c->L.nblocks, c->d_scalars);
   CK(c->launched("k_sum"));
-  CK(c->read_scalars(1));
+  CK(c->read_scalars());
   *out = c->h_scalars[0];
   return IMSRG_OK;
 }
@@ -1079,7 +1098,7 @@ imsrg_status imsrg_cc_download(imsrg_ctx* ctx, const imsrg_cc* cc, double* host)
   if (!cc || cc->owner != c || !host) return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "imsrg_cc_download");
   if (cc->n == 0) return IMSRG_OK;
   CK(c->cuda(cudaMemcpyAsync(host, cc->d, sizeof(double) * cc->n, cudaMemcpyDeviceToHost, c->stream), "D2H cc"));
-  return c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+  return c->finish();
 }
 
 imsrg_status imsrg_calculate_cross_coupled(imsrg_ctx* ctx, const imsrg_op* HS, imsrg_cc* CCME) {
@@ -1096,7 +1115,7 @@ imsrg_status imsrg_commutator_110(imsrg_ctx* ctx, const imsrg_op* L, const imsrg
   CK(check_op(c, R, "imsrg_commutator_110"));
   if (!out) return IMSRG_ERR_INVALID_ARGUMENT;
   CK(c->e0(L->d, L->herm, R->d, R->herm, nullptr, c->d_scalars));
-  CK(c->read_scalars(2));
+  CK(c->read_scalars());
   *out = c->h_scalars[0];
   return IMSRG_OK;
 }
@@ -1107,7 +1126,7 @@ imsrg_status imsrg_commutator_220(imsrg_ctx* ctx, const imsrg_op* L, const imsrg
   CK(check_op(c, R, "imsrg_commutator_220"));
   if (!out) return IMSRG_ERR_INVALID_ARGUMENT;
   CK(c->e0(L->d, L->herm, R->d, R->herm, nullptr, c->d_scalars));
-  CK(c->read_scalars(2));
+  CK(c->read_scalars());
   *out = c->h_scalars[1];
   return IMSRG_OK;
 }

@@ -61,7 +61,7 @@ constexpr int64_t kGatherMinSlab = 100000;
 // up to this size the mixed commutator runs 122 beside its GEMM (gemm_tc.cu)
 constexpr int64_t kIdleSlab = (int64_t)1 << 22;
 // the word of d_scalars (and of h_scalars) that holds the error of a bounded wait
-constexpr int kErrorSlot = 48;
+constexpr int kErrorSlot = 8;
 
 struct Ctx {
   imsrg::Layout L;
@@ -104,7 +104,7 @@ struct Ctx {
   // FP64 products on the tensor cores (gemm_oz.cu): the digit plans of the ladder and of the cross-coupled products
   imsrg::OzPlan pphh_oz, wcc_oz;
   int oz_sms = 0;  // SMs of the device, once a plan is ready
-  // error word of the tensor-core kernels' bounded waits (in d_scalars, read with tc_error)
+  // error word of the tensor-core kernels' bounded waits (in d_scalars, read with finish and read_scalars)
   int* d_err = nullptr;
   // limit of every bounded device wait of the tensor-core kernels (imsrg_set_wait_limit), and the
   // one-shot test switch that leaves one pipeline stage of the next GEMM launch unarmed
@@ -172,7 +172,9 @@ struct Ctx {
   imsrg_status axpby(const double* A, double ax, const double* B, double bx, double* C);
   imsrg_status axpy_frob_async(double* Y, double a, const double* X, double scale, int slot, bool with_e0);
   imsrg_status frob_async(const double* op, double scale, int slot);
-  imsrg_status read_scalars(int n);
+  imsrg_status read_scalars();
+  imsrg_status finish();
+  imsrg_status wait_error();
   imsrg_status white(const double* H, int hH, double* ETA);
   imsrg_status atan_generator(const double* Hden, int hden, const double* Hnum, double* ETA);
   imsrg_status w2_generator(const double* H, int hH, double* ETA);
@@ -254,7 +256,6 @@ struct Ctx {
   imsrg_status tc_wcc(const double* lcc, const double* rcc, double* wcc);
   imsrg_status tc_gemm(const imsrg::TcProb* probs, const imsrg::TcTile* tiles, int ntiles, imsrg::TcOut out, int hL,
                        int hR, int wmax);
-  imsrg_status tc_error();
   imsrg_status tc_commutator(const double* L, int hL, const double* R, int hR, double* RES, int hRES, bool with_e0);
   void tc_release();
   imsrg_status tc_gemm_on(const CUtensorMap& map, int64_t slice_rows, const imsrg::TcProb* probs,

@@ -60,6 +60,7 @@ struct imsrg_eom {
   cudaGraphExec_t gexec = nullptr;
   const double* g_H = nullptr;
   int g_prec = -1;  // the context's precision at capture (the kernels differ between modes)
+  unsigned long long g_wait = 0;  // and the limit of their waits
 };
 
 namespace {
@@ -233,7 +234,7 @@ imsrg_status Ctx::eom_matvec(imsrg_eom& E, const double* Hd, const double* d_v, 
 // (captured on first use, after one direct run that also makes the workspaces; the operands are
 // read when the graph runs)
 imsrg_status Ctx::eom_matvec_graph(imsrg_eom& E, const double* Hd) {
-  if (E.gexec && E.g_H == Hd && E.g_prec == (int)precision)
+  if (E.gexec && E.g_H == Hd && E.g_prec == (int)precision && E.g_wait == tc_wait_ns)
     return cuda(cudaGraphLaunch(E.gexec, stream), "cudaGraphLaunch(eom)");
   CKE(eom_matvec(E, Hd, E.d_v, E.d_w));
   CKE(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
@@ -254,6 +255,7 @@ imsrg_status Ctx::eom_matvec_graph(imsrg_eom& E, const double* Hd) {
   }
   E.g_H = Hd;
   E.g_prec = (int)precision;
+  E.g_wait = tc_wait_ns;
   return IMSRG_OK;  // d_w already holds the direct run's product
 }
 
@@ -263,7 +265,7 @@ imsrg_status Ctx::eom_matvec_host(imsrg_eom& E, const double* Hd, const double* 
   CKE(cuda(cudaMemcpyAsync(E.d_v, v, b, cudaMemcpyHostToDevice, stream), "H2D eom vector"));
   CKE(eom_matvec_graph(E, Hd));
   CKE(cuda(cudaMemcpyAsync(w, E.d_w, b, cudaMemcpyDeviceToHost, stream), "D2H eom vector"));
-  return cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+  return finish();
 }
 
 // LANCZOS_DIAGONALIZE (src/EOM_IMSRG.f90:164-334): the nev eigenvalues of smallest magnitude of
@@ -505,7 +507,7 @@ imsrg_status imsrg_eom_rewrap(imsrg_ctx* ctx, imsrg_eom* E, const imsrg_tensor* 
   CKE(c->launched("k_eom_rewrap"));
   CKE(c->cuda(cudaMemcpyAsync(v, E->d_w, sizeof(double) * (size_t)E->n, cudaMemcpyDeviceToHost, c->stream),
               "D2H eom vector"));
-  return c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+  return c->finish();
 }
 
 imsrg_status imsrg_eom_lanczos(imsrg_ctx* ctx, imsrg_eom* E, const imsrg_op* H, int32_t nev, double tol,

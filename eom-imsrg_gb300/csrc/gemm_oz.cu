@@ -237,7 +237,7 @@ __device__ __forceinline__ void oz_mad(long long& acc, int v) {
 __global__ void __launch_bounds__(kThreads, 1)
     k_oz_gemm(const OzProb* __restrict__ probs, const OzTile* __restrict__ tiles, const int* __restrict__ start, GemmOperands out,
               const char* __restrict__ buf, const char* __restrict__ mag, const int* __restrict__ exps, int* flag,
-              OzRedo* __restrict__ redo, int max_redo, int* err, unsigned long long wait_ns) {
+              OzRedo* __restrict__ redo, int max_redo, int* err, unsigned long long wait_ns, int unarmed_it) {
   if (*flag) return;  // a row with an Inf or a NaN: k_gemm_fp64_rest computes the list
   extern __shared__ uint8_t oz_smem[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(oz_smem) + 1023) & ~uintptr_t(1023));
@@ -288,6 +288,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int kb0 = 0; kb0 < nkb; kb0 += kMagBlocks, ++it) {  // the magnitudes of up to eight K blocks in one stage
             const int s = it % kStages, n = min(kMagBlocks, nkb - kb0);
             if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, err, 1, wait_ns)) { ok = false; break; }
+            // test switch (imsrg_test_unarmed_stage): CTA 0 issues no copy for this stage and nothing arrives on its barrier
+            if (it == unarmed_it && blockIdx.x == 0) continue;
             mbar_expect_tx(&full[s], (uint32_t)(n * (kSliceBytes + kSliceBytes / 2)));
             const uint32_t st = smem_u32(smem + (size_t)s * kStageBytes);
             bulk_load(st, mag + (ablk + kb0) * kSliceBytes, (uint32_t)(n * kSliceBytes), &full[s]);
@@ -664,8 +666,10 @@ imsrg_status Ctx::gemm_fp64(OzPlan& P, const std::vector<GemmProb>& probs, const
     CK_TC(cuda(cudaMemsetAsync(P.flag, 0, 3 * sizeof(int), stream), "memset(FP64 product flags)"));
     k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, P.buf, P.mag, P.exps, P.flag);
     CK_TC(launched("k_oz_split"));
+    const int unarmed = tc_unarmed_next ? 0 : -1;  // one-shot test switch
+    tc_unarmed_next = 0;
     k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, P.buf, P.mag, P.exps, P.flag, P.redo,
-                                                   (int)P.max_redo, d_err, tc_wait_ns);
+                                                   (int)P.max_redo, d_err, tc_wait_ns, unarmed);
     CK_TC(launched("k_oz_gemm"));
     k_gemm_fp64_rest<<<4 * oz_sms, 256, 0, stream>>>(d_probs, d_tiles, ntiles, ops, P.flag, P.redo, (int)P.max_redo);
     return launched("k_gemm_fp64_rest");

@@ -901,21 +901,6 @@ imsrg_status Ctx::tc_pphh(const double* Lp, int hL, const double* Rp, int hR, do
   return IMSRG_OK;
 }
 
-imsrg_status Ctx::tc_error() {
-  if (!tc && !oz_sms) return IMSRG_OK;
-  int& e = *reinterpret_cast<int*>(h_scalars + kErrorSlot);
-  CK_TC(cuda(cudaMemcpyAsync(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "D2H tc error"));
-  CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
-  if (e) {
-    cudaMemsetAsync(d_err, 0, sizeof(int), stream);
-    static const char* role[] = {"", "producer (stage free)", "MMA (accumulator free)", "MMA (stage loaded)",
-                                 "epilogue (accumulator ready)"};
-    return fail(IMSRG_ERR_TIMEOUT, std::string("tensor-core GEMM: a bounded wait ran out in the ") +
-                                       (e >= 1 && e <= 4 ? role[e] : "kernel") + " (code " + std::to_string(e) + ")");
-  }
-  return IMSRG_OK;
-}
-
 imsrg_status Ctx::tc_wcc(const double*, const double*, double*) {
   return fail(IMSRG_ERR_UNSUPPORTED, "the piecewise 222_ph entry point runs in FP64");
 }

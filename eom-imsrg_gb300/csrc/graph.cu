@@ -56,6 +56,7 @@ struct StepGraph {
   double* DG = nullptr;
   const double* H = nullptr;
   int hH = 0, hG = 0, precision = -1, max_terms = 0;
+  unsigned long long wait_ns = 0;
   double ds = 0, conv = 0;
 };
 
@@ -338,7 +339,7 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
     CK_TC(launched("k_mbpt2_partial"));
     k_sum<<<1, 1024, 0, stream>>>(d_partial, L.nblocks, d_scalars);
     CK_TC(launched("k_sum"));
-    CK_TC(read_scalars(1));
+    CK_TC(read_scalars());
     const double e2 = h_scalars[0];
     if (hio) {
       CK_TC(cuda(cudaMemcpyAsync(hio->hs, HS, sbytes, cudaMemcpyDeviceToHost, stream), "D2H H(s)"));
@@ -347,7 +348,7 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
     }
     double e0 = 0;
     CK_TC(cuda(cudaMemcpyAsync(h_scalars, HS, sizeof(double), cudaMemcpyDeviceToHost, stream), "D2H E0"));
-    CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
+    CK_TC(finish());
     e0 = h_scalars[0];
     if (info) {
       info->E0 = e0;
@@ -357,7 +358,6 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
       info->bch_converged = sb == IMSRG_OK ? 1 : 0;
       info->graph_rebuilt = 0;
     }
-    CK_TC(tc_error());
     if (sb != IMSRG_OK) return fail(IMSRG_ERR_NOT_CONVERGED, "BCH series did not converge within max_terms");
     return IMSRG_OK;
   }
@@ -365,7 +365,7 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
   const StepHostIO& io = hio ? *hio : none;
   const bool same = sg->exec && sg->HS == HS && sg->G == G && sg->DG == DG && sg->H == H && sg->hH == hH &&
                     sg->hG == hG && sg->ds == ds && sg->max_terms == max_terms && sg->conv == conv &&
-                    sg->precision == precision && sg->hio.hs == io.hs && sg->hio.g == io.g && sg->hio.dg == io.dg &&
+                    sg->precision == precision && sg->wait_ns == tc_wait_ns && sg->hio.hs == io.hs && sg->hio.g == io.g && sg->hio.dg == io.dg &&
                     sg->hio.h == io.h;
   if (!same) {
     if (sg->exec) cudaGraphExecDestroy(sg->exec);
@@ -375,15 +375,14 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
     CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
     CK_TC(graph_capture(HS, G, hG, DG, H, hH, ds, max_terms, conv, hio));
     sg->HS = HS; sg->G = G; sg->DG = DG; sg->H = H; sg->hH = hH; sg->hG = hG; sg->hio = io;
-    sg->ds = ds; sg->max_terms = max_terms; sg->conv = conv; sg->precision = precision;
+    sg->ds = ds; sg->max_terms = max_terms; sg->conv = conv; sg->precision = precision; sg->wait_ns = tc_wait_ns;
     rebuilt = 1;
   }
   CK_TC(cuda(cudaGraphLaunch(sg->exec, stream), "cudaGraphLaunch"));
   if (!info) return IMSRG_OK;
   CK_TC(cuda(cudaMemcpyAsync(sg->h_state, sg->d_state, sizeof(StepState), cudaMemcpyDeviceToHost, stream),
           "D2H step state"));
-  CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
-  CK_TC(tc_error());
+  CK_TC(finish());
   const StepState& st = *sg->h_state;
   info->E0 = st.e0;
   info->mbpt2 = st.mbpt2;
@@ -402,10 +401,10 @@ imsrg_status Ctx::step_counters(int64_t* commutators, int64_t* kernels, int64_t*
   }
   CK_TC(cuda(cudaMemcpyAsync(sg->h_state, sg->d_state, sizeof(StepState), cudaMemcpyDeviceToHost, stream),
           "D2H step state"));
-  CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
+  const imsrg_status s = finish();
   *commutators = sg->h_state->tot_commutators;
   *kernels = sg->h_state->tot_kernels;
   *steps = sg->h_state->tot_steps;
   *unconverged = sg->h_state->tot_unconverged;
-  return tc_error();
+  return s;
 }

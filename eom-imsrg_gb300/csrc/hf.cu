@@ -485,7 +485,7 @@ imsrg_status Ctx::hf_run(double* op, int herm, int mode, int max_iter, const dou
   std::vector<double> pre((size_t)S.prefix);
   CKH(cuda(cudaMemcpyAsync(pre.data(), op, sizeof(double) * S.prefix, cudaMemcpyDeviceToHost, stream),
            "cudaMemcpyAsync(one-body part)"));
-  CKH(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(one-body part)"));
+  CKH(finish());
   auto fref = [&](int a, int b) -> double& {  // storage of f(a,b), a, b not (hole, particle)
     if (L.con[a] + L.con[b] == 0) return pre[L.off_fpp + L.loc[a] + (int64_t)L.loc[b] * L.P];
     if (L.con[a] + L.con[b] == 2) return pre[L.off_fhh + L.loc[a] + (int64_t)L.loc[b] * L.A];

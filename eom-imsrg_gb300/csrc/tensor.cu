@@ -680,7 +680,7 @@ imsrg_status Ctx::bch_tensor(TensorState& S, const double* G, int hG, double* HS
     k_axpby<<<grid_n(S.T.slab), 256, 0, stream>>>(S.T.slab, HS, 1.0, out, coef, HS);
     CKT(launched("k_axpby"));
     CKT(tensor_frob(S, out, coef, 0));
-    CKT(read_scalars(1));
+    CKT(read_scalars());
     if (h_scalars[0] < conv) break;
   }
   *terms = (iw > max_terms) ? max_terms - 1 : iw - 1;
@@ -771,7 +771,7 @@ imsrg_status imsrg_tensor_download_slab(imsrg_ctx* ctx, const imsrg_tensor* t, d
   if (!t || t->owner != c || !host) return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "imsrg_tensor_download_slab");
   CKT(c->cuda(cudaMemcpyAsync(host, t->d, sizeof(double) * (size_t)t->ts->T.slab, cudaMemcpyDeviceToHost, c->stream),
               "D2H tensor"));
-  return c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+  return c->finish();
 }
 
 imsrg_status imsrg_tensor_commutator(imsrg_ctx* ctx, const imsrg_op* Lop, const imsrg_tensor* R, imsrg_tensor* RES,
@@ -801,7 +801,7 @@ imsrg_status imsrg_tensor_frob_norm(imsrg_ctx* ctx, const imsrg_tensor* t, doubl
   TCTX(ctx);
   if (!t || t->owner != c || !out) return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "imsrg_tensor_frob_norm");
   CKT(c->tensor_frob(*t->ts, t->d, 1.0, 0));
-  CKT(c->read_scalars(1));
+  CKT(c->read_scalars());
   *out = c->h_scalars[0];
   return IMSRG_OK;
 }

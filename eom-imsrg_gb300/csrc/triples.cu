@@ -451,7 +451,7 @@ imsrg_status Ctx::restore_triples(const double* H, const double* OM, double* e3,
     st = launched("k_triples");
   }
   if (st == IMSRG_OK) st = cuda(cudaMemcpyAsync(e3, d_out, sizeof(double), cudaMemcpyDeviceToHost, stream), "D2H triples");
-  if (st == IMSRG_OK) st = cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+  if (st == IMSRG_OK) st = finish();
   cudaFree(buf);
   return st;
 }

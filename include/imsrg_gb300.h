@@ -86,17 +86,18 @@ imsrg_status imsrg_block_pairs(const imsrg_ctx* ctx, int32_t q, int32_t cls, int
 imsrg_status imsrg_cc_info(const imsrg_ctx* ctx, int32_t* rlen, int32_t* nph, int32_t* J);
 imsrg_status imsrg_set_precision(imsrg_ctx* ctx, int32_t mode);
 /* Waits for the context's queued work.  Returns IMSRG_ERR_TIMEOUT when a bounded device wait
- * of a tensor-core kernel ran out since the last call (the reference STOPs where a loop cannot
+ * of a tensor-core kernel ran out since the last report, as every call that hands results to the
+ * host does (downloads, E0, norms, the series, the EOM product; the reference STOPs where a loop cannot
  * finish, src/IMSRG_MAGNUS.f90:232; here the kernel records a code, stops its other roles,
  * waits for its own copies in flight, frees its tensor memory and returns). */
 imsrg_status imsrg_synchronize(imsrg_ctx* ctx);
-/* Limit of every bounded device wait of the tensor-core kernels, in nanoseconds (default
- * 2 s; 0 restores the default).  No counterpart in the reference. */
+/* Limit of every bounded device wait of the tensor-core kernels (all precisions), in nanoseconds
+ * (default 2 s; 0 restores the default).  No counterpart in the reference. */
 imsrg_status imsrg_set_wait_limit(imsrg_ctx* ctx, int64_t nanoseconds);
 /* Test switch, off by default (no counterpart in the reference): with enable != 0 the next
  * tensor-core GEMM launch of this context leaves its first pipeline stage unarmed -- no copy
  * is issued for it and nothing arrives on its barrier -- so the MMA warp's wait on it runs out
- * after the wait limit and imsrg_synchronize reports IMSRG_ERR_TIMEOUT.  The switch resets
+ * after the wait limit and the next call that waits for results reports IMSRG_ERR_TIMEOUT.  The switch resets
  * after that one launch.  For testing the failure path only. */
 imsrg_status imsrg_test_unarmed_stage(imsrg_ctx* ctx, int32_t enable);
 /* The traffic of the mixed particle-hole recoupling kernel on this basis, counted exactly
