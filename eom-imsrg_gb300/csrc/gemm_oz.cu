@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* empty = full + kStages;
   uint64_t* dfull = empty + kStages;
   uint64_t* dempty = dfull + S;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dempty + S);
+  uint64_t* drain = dempty + S;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* consumed = reinterpret_cast<volatile int*>(tmem_slot + 2);
   unsigned short* coarse = reinterpret_cast<unsigned short*>(tmem_slot + 4);  // a word for each reader's 16 elements
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&dfull[d], 1);
       mbar_init(&dempty[d], kEpiWarps);
     }
+    mbar_init(drain, 1);
     *abort_flag = 0;
     *consumed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -274,9 +276,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
   const int t0 = start[blockIdx.x], t1 = start[blockIdx.x + 1];  // this CTA's tiles
 
+  int it = 0;  // stages filled (copies) or taken (MMAs)
   if (warp == 0) {
-    if (lane == 0) {  // ---- copies
-      int it = 0;
+    if (elect_one()) {  // ---- copies
       bool ok = true;
       for (int t = t0; t < t1 && ok; ++t) {
         const OzTile tile = tiles[t];
@@ -313,16 +315,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      if (!ok) {  // wait (bounded) for every copy that the MMA warp did not consume
-        const unsigned long long t0 = globaltimer();
-        for (int j = *consumed; j < it; ++j)
-          while (!mbar_test(&full[j % kStages], (j / kStages) & 1))
-            if (globaltimer() - t0 > wait_ns) break;
-      }
     }
   } else if (warp == 1) {
     if (elect_one()) {  // ---- MMAs
-      int it = 0, cc = 0, cm = 0;  // cc: chunks so far; cm: sums of magnitudes so far
+      int cc = 0, cm = 0;  // cc: chunks so far; cm: sums of magnitudes so far
       bool ok = true;
       for (int t = t0; t < t1 && ok; ++t) {
         const OzTile tile = tiles[t];
@@ -494,6 +490,16 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  __syncwarp();
+  if (*abort_flag && warp < 2 && elect_one()) {  // a wait ran out: what is in flight into or out of this CTA's memory ends first
+    if (warp == 0) {
+      for (int j = *consumed; j < it; ++j)
+        if (j != unarmed_it || blockIdx.x) mbar_drain(&full[j % kStages], (j / kStages) & 1);
+    } else {
+      umma_commit(drain);
+      mbar_drain(drain, 0);
+    }
+  }
   __syncwarp();
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");

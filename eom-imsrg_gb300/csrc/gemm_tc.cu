@@ -150,7 +150,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   uint64_t* empty = full + ST;
   uint64_t* tfull = empty + ST;
   uint64_t* tempty = tfull + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+  uint64_t* drain = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* consumed = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       mbar_init(&tfull[a], 1);
       mbar_init(&tempty[a], 8);
     }
+    mbar_init(drain, 1);
     *abort_flag = 0;
     *consumed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -179,10 +181,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  int it = 0;  // stages filled (producer) or taken (MMA issuer)
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
         const TcTile tile = tiles[t];
@@ -210,22 +212,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           }
         }
       }
-      if (!ok) {
-        // drain: wait (bounded) for every issued stage the MMA warp did not consume
-        const unsigned long long t0 = globaltimer();
-        for (int j = *consumed; j < it; ++j) {
-          while (!mbar_test(&full[j % ST], (j / ST) & 1)) {
-            if (globaltimer() - t0 > wait_ns) break;
-          }
-        }
-      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     // (one elected lane; issued from a branch on the lane index an MMA took about 80 clocks and this kernel, at eMax 10,
     // 0.48 ms in bf16x3, 0.70 in bf16x6, 0.85 in tf32x3; now 0.40, 0.63 and 0.69)
     if (elect_one()) {
-      int it = 0, local = 0;
+      int local = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++local) {
         const TcTile tile = tiles[t];
@@ -337,6 +330,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  __syncwarp();
+  if (*abort_flag && warp < 2 && elect_one()) {  // a wait ran out: what is in flight into or out of this CTA's memory ends first
+    if (warp == 0) {
+      for (int j = *consumed; j < it; ++j)
+        if (j != unarmed_it || blockIdx.x) mbar_drain(&full[j % ST], (j / ST) & 1);
+    } else {
+      umma_commit(drain);
+      mbar_drain(drain, 0);
+    }
+  }
   __syncwarp();
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * WMAX) : "memory");

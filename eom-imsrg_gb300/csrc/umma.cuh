@@ -48,7 +48,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// true in one lane of the (converged) warp.  tcgen05.mma and its commit are issued inside a branch on this: the compiler
+// Limit of the waits for a kernel's own copies and MMAs in flight after another wait has run out: they end by themselves, so this
+// is independent of the limit that the caller may set, which can be shorter than a copy takes.
+constexpr unsigned long long kDrainNs = 2000000000ull;
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = globaltimer();
+  while (!mbar_test(bar, parity))
+    if (globaltimer() - t0 > kDrainNs) break;
+}
+
+// true in one lane (the same one every time) of the (converged) warp.  tcgen05.mma and its commit are issued inside a branch on this: the compiler
 // knows that one lane runs it, where a branch on a lane index costs a loop over the lanes around every MMA.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
