@@ -198,6 +198,7 @@ struct Ctx {
   imsrg_status capture_if(cudaGraphConditionalHandle h, F&& body);
   imsrg_status step_counters(int64_t* commutators, int64_t* kernels, int64_t* steps, int64_t* unconverged);
   imsrg_status graph_release();
+  void graph_drop();
 
   // reverse mode (FP64) of the commutator, the White generator and the slab inner product (adjoint.cu)
   imsrg_status adjoint_prepare();
@@ -241,6 +242,7 @@ struct Ctx {
   imsrg_status gather_prepare_fp64(bool& groups);
   void gather_release();
   imsrg_status g122_set_caps(int tiny_cap, int small_cap);
+  imsrg_status g122_upload(int tiny_cap, int small_cap);
   template <typename T>
   imsrg_status c122_groups(const double* L, int hL, const double* R, int hR, double* RES, int hRES);
 

@@ -120,7 +120,7 @@ imsrg_status Ctx::gather_prepare() {
   CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(gather plan)"));
   // 8 lanes for a task of up to 32 elements while the warps are not all busy, up to 64 in larger bases (FP32: eMax 4 25 ->
   // 20 us, eMax 7 53 -> 50, eMax 8 91 either way, eMax 10 385 against 399)
-  CK_TC(g122_set_caps(l.slab < (int64_t)1 << 23 ? 32 : 64, 256));
+  CK_TC(g122_upload(l.slab < (int64_t)1 << 23 ? 32 : 64, 256));
   gp.state = 1;
   return IMSRG_OK;
 }
@@ -133,7 +133,7 @@ void Ctx::gather_release() {
 // Splits the 122 tasks into [tiny | warp | cta] runs by size, keeping channel order inside
 // each run, and uploads the list.  The caps must keep the per-CTA shared memory of the
 // 8-lane and warp kernels within the 48 KiB default.
-imsrg_status Ctx::g122_set_caps(int tiny_cap, int small_cap) {
+imsrg_status Ctx::g122_upload(int tiny_cap, int small_cap) {
   G122Plan& P = gp.g122;
   const int bt = P.tiny_cap, bw = P.warp_cap;
   const std::string e = g122_partition(P, tiny_cap, small_cap);
@@ -151,6 +151,13 @@ imsrg_status Ctx::g122_set_caps(int tiny_cap, int small_cap) {
   }
   CK_TC(cuda(g122_occupancy(P.smem_bytes, gp.per_sm), "occupancy (122)"));
   return IMSRG_OK;
+}
+
+// Other caps for a plan in use.  A captured step holds the counts, the grid and the shared memory of the list that is rewritten
+// here, in whatever precision it was captured: it goes first.
+imsrg_status Ctx::g122_set_caps(int tiny_cap, int small_cap) {
+  graph_drop();
+  return g122_upload(tiny_cap, small_cap);
 }
 
 // commutator_122 on pair-group sub-blocks: RES's rectangular arrays and the upper triangles of its square ones.  run_if:

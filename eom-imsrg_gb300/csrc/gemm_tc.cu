@@ -1074,6 +1074,7 @@ imsrg_status Ctx::tc_autotune(const double* Lp, int hL, const double* Rp, int hR
     return IMSRG_OK;
   };
   imsrg_status st = IMSRG_OK;
+  graph_drop();  // before the first change: an error leaves by another way than the end
   float base = 0.0f, best = 0.0f;
   do {
     if ((st = time_one(&base)) != IMSRG_OK) break;
@@ -1200,10 +1201,12 @@ extern "C" imsrg_status imsrg_set_tuning(imsrg_ctx* ctx, const imsrg_tune_info* 
     return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "imsrg_set_tuning: value out of range");
   CK_TC(c->ensure_workspace());
   CK_TC(c->tc_prepare(c->precision));
+  const int wx = cfg->gemm_wmax_x ? cfg->gemm_wmax_x : cfg->gemm_wmax;
+  for (int w : {cfg->gemm_wmax, wx})  // before anything changes
+    if (w != 128 && !(w == 256 && c->tc->S == 2)) return c->fail(IMSRG_ERR_INVALID_ARGUMENT, "unsupported tile width");
   CK_TC(c->g122_set_caps(cfg->tiny_cap, cfg->small_cap));
   {
     const bool m = cfg->gemm_merged != 0;
-    const int wx = cfg->gemm_wmax_x ? cfg->gemm_wmax_x : cfg->gemm_wmax;
     int w[3] = {cfg->gemm_wmax, wx, cfg->gemm_wmax};
     bool n[3] = {cfg->gemm_narrow != 0, (cfg->gemm_wmax_x ? cfg->gemm_narrow_x : cfg->gemm_narrow) != 0,
                  cfg->gemm_narrow != 0};

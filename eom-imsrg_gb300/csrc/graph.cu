@@ -120,10 +120,18 @@ __global__ void k_step_end(const double* HS, StepState* st, int fixed_kernels) {
 
 }  // namespace
 
-imsrg_status Ctx::graph_release() {
-  if (!sg) return IMSRG_OK;
+// The captured step goes (the next one is captured again), its counters stay.
+void Ctx::graph_drop() {
+  if (!sg) return;
   if (sg->exec) cudaGraphExecDestroy(sg->exec);
   if (sg->graph) cudaGraphDestroy(sg->graph);
+  sg->exec = nullptr;
+  sg->graph = nullptr;
+}
+
+imsrg_status Ctx::graph_release() {
+  if (!sg) return IMSRG_OK;
+  graph_drop();
   if (sg->side) cudaStreamDestroy(sg->side);
   for (cudaStream_t c : sg->cp)
     if (c) cudaStreamDestroy(c);
@@ -368,10 +376,7 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
                     sg->precision == precision && sg->wait_ns == tc_wait_ns && sg->hio.hs == io.hs && sg->hio.g == io.g && sg->hio.dg == io.dg &&
                     sg->hio.h == io.h;
   if (!same) {
-    if (sg->exec) cudaGraphExecDestroy(sg->exec);
-    if (sg->graph) cudaGraphDestroy(sg->graph);
-    sg->exec = nullptr;
-    sg->graph = nullptr;
+    graph_drop();
     CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
     CK_TC(graph_capture(HS, G, hG, DG, H, hH, ds, max_terms, conv, hio));
     sg->HS = HS; sg->G = G; sg->DG = DG; sg->H = H; sg->hH = hH; sg->hG = hG; sg->hio = io;
