@@ -579,6 +579,7 @@ struct DevPacker {
 
 void Ctx::tc_release() {
   if (!tc) return;
+  graph_drop();  // a captured mixed step holds what is freed here
   if (tc->buf) cudaFree(tc->buf);
   if (tc->d_mem) cudaFree(tc->d_mem);
   if (tc->zbuf) cudaFree(tc->zbuf);

@@ -1,5 +1,6 @@
-"""A captured Magnus step after its launch tables have changed behind it: another tuning of the mixed modes (accepted or
-rejected), which shares the 122 plan with FP64.  The step must be the eager one."""
+"""A captured Magnus step after its launch tables have changed behind it: another tuning of the mixed modes (accepted, rejected or
+broken off half-way), which shares the 122 plan with FP64, and another mixed precision and back.  The step must be the eager one."""
+import numpy as np
 import pytest
 
 from helpers import rel_err
@@ -45,3 +46,15 @@ def test_fp64_step_after_tuning(built_lib, oracles, change, accepted):
     eng.set_precision("fp64")
     for _ in range(2):
         step_both(eng, st, 1e-11)
+
+
+def test_mixed_step_after_another_precision(built_lib):
+    from imsrg_gb300 import Engine, make_basis
+    eng = Engine(make_basis(4), device=0, precision="bf16x3")
+    st = states(eng)
+    step_both(eng, st, 0.0)
+    eng.set_precision("tf32x3")
+    filler = [eng.new_op(1, np.full(eng.slab, np.nan)) for _ in range(8)]  # where the old tables lay
+    eng.set_precision("bf16x3")
+    step_both(eng, st, 0.0)
+    del filler
