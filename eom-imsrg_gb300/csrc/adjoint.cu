@@ -97,7 +97,7 @@ imsrg_status Ctx::adjoint_prepare() {
   if (!wp.empty()) std::memcpy(buf.data() + o[2], wp.data(), sizeof(GemmProb) * wp.size());
   if (!wt.empty()) std::memcpy(buf.data() + o[3], wt.data(), sizeof(GemmTile) * wt.size());
   CKA(cuda(cudaMalloc(&adj->tables, buf.size()), "cudaMalloc(adjoint tables)"));
-  CKA(cuda(cudaMemcpy(adj->tables, buf.data(), buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(adjoint tables)"));
+  CKA(put(adj->tables, buf.data(), buf.size(), "cudaMemcpy(adjoint tables)"));
   const char* base = static_cast<const char*>(adj->tables);
   adj->pphh_p = reinterpret_cast<const GemmProb*>(base + o[0]);
   adj->pphh_t = reinterpret_cast<const GemmTile*>(base + o[1]);

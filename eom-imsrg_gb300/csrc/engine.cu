@@ -208,7 +208,7 @@ imsrg_status Ctx::upload_tables() {
   pk.add(zero_runs_w2, &zr2);
 
   CK(cuda(cudaMalloc(&d_tables, pk.buf.size()), "cudaMalloc(tables)"));
-  CK(cuda(cudaMemcpy(d_tables, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tables)"));
+  CK(put(d_tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(d_tables) + f.first;
   d_pphh_probs = pp_p; d_pphh_tiles = pp_t; d_wcc_probs = wc_p; d_wcc_tiles = wc_t;
   d_seg_start = seg_s; d_seg_len = seg_l; d_seg_w = seg_w;
@@ -218,11 +218,18 @@ imsrg_status Ctx::upload_tables() {
   partial_capacity = std::max(nseg, l.nblocks) + 64;
   CK(cuda(cudaMalloc(&d_partial, sizeof(double) * partial_capacity), "cudaMalloc(partials)"));
   CK(cuda(cudaMalloc(&d_scalars, sizeof(double) * 64), "cudaMalloc(scalars)"));
-  CK(cuda(cudaMemset(d_scalars, 0, sizeof(double) * 64), "memset(scalars)"));
+  CK(cuda(cudaMemsetAsync(d_scalars, 0, sizeof(double) * 64, stream), "memset(scalars)"));
   d_err = reinterpret_cast<int*>(d_scalars + kErrorSlot);
   CK(cuda(cudaMallocHost(&h_scalars, sizeof(double) * 64), "cudaMallocHost(scalars)"));
   CK(cuda(cudaMalloc(&d_mono, sizeof(double) * (size_t)l.N * l.N), "cudaMalloc(monopole)"));
   return IMSRG_OK;
+}
+
+// A host table to the device, on the stream whose kernels read it: the context's streams do not wait for the default stream,
+// on which the last bytes of a plain copy from pageable memory may still be on their way when it returns.
+imsrg_status Ctx::put(void* dst, const void* src, size_t bytes, const char* what) {
+  CK(cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream), what));
+  return cuda(cudaStreamSynchronize(stream), what);
 }
 
 imsrg_status Ctx::ensure_workspace() {

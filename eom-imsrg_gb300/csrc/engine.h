@@ -172,6 +172,7 @@ struct Ctx {
   imsrg_status axpby(const double* A, double ax, const double* B, double bx, double* C);
   imsrg_status axpy_frob_async(double* Y, double a, const double* X, double scale, int slot, bool with_e0);
   imsrg_status frob_async(const double* op, double scale, int slot);
+  imsrg_status put(void* dst, const void* src, size_t bytes, const char* what);
   imsrg_status read_scalars();
   imsrg_status finish();
   imsrg_status wait_error();

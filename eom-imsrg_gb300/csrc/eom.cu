@@ -414,13 +414,13 @@ imsrg_status imsrg_eom_create(imsrg_ctx* ctx, int32_t rank2, int32_t dpar2, imsr
     alloc((void**)&E->d_Y[k], sb, "cudaMalloc(eom slab)");
   }
   if (st == IMSRG_OK && E->n) {
-    st = c->cuda(cudaMemcpy(E->d_pos, E->pos.data(), sizeof(int64_t) * E->n, cudaMemcpyHostToDevice), "H2D eom map");
+    st = c->cuda(cudaMemcpyAsync(E->d_pos, E->pos.data(), sizeof(int64_t) * E->n, cudaMemcpyHostToDevice, c->stream), "H2D eom map");
     if (st == IMSRG_OK)
-      st = c->cuda(cudaMemcpy(E->d_mirror, E->mirror.data(), sizeof(int64_t) * E->n, cudaMemcpyHostToDevice),
+      st = c->cuda(cudaMemcpyAsync(E->d_mirror, E->mirror.data(), sizeof(int64_t) * E->n, cudaMemcpyHostToDevice, c->stream),
                    "H2D eom map");
-    if (st == IMSRG_OK) st = c->cuda(cudaMemcpy(E->d_kind, E->kind.data(), E->n, cudaMemcpyHostToDevice), "H2D eom map");
+    if (st == IMSRG_OK) st = c->cuda(cudaMemcpyAsync(E->d_kind, E->kind.data(), E->n, cudaMemcpyHostToDevice, c->stream), "H2D eom map");
     if (st == IMSRG_OK)
-      st = c->cuda(cudaMemcpy(E->d_phase, E->phase.data(), E->n, cudaMemcpyHostToDevice), "H2D eom map");
+      st = c->cuda(cudaMemcpyAsync(E->d_phase, E->phase.data(), E->n, cudaMemcpyHostToDevice, c->stream), "H2D eom map");
   }
   for (int k = 0; k < 2 && st == IMSRG_OK; ++k) st = c->cuda(cudaMemsetAsync(E->d_S[k], 0, sb, c->stream), "memset(eom slab)");
   if (st == IMSRG_OK) st = c->cuda(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");

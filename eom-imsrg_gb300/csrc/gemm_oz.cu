@@ -608,7 +608,7 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
       P.tables = nullptr;
       return IMSRG_OK;
     }
-    CK_TC(cuda(cudaMemcpy(P.tables, t.data(), sizeof(GemmTile) * t.size(), cudaMemcpyHostToDevice), "cudaMemcpy(FP64 product tiles)"));
+    CK_TC(put(P.tables, t.data(), sizeof(GemmTile) * t.size(), "cudaMemcpy(FP64 product tiles)"));
     P.d_small = static_cast<const GemmTile*>(P.tables);
     P.nsmall = (int)t.size();
     P.state = 2;
@@ -636,7 +636,7 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   std::memcpy(h.data() + bo + bc, P.probs.data(), sizeof(OzProb) * P.probs.size());
   std::memcpy(h.data() + bo + bc + bp, P.tiles.data(), sizeof(OzTile) * P.tiles.size());
   std::memcpy(h.data() + bo + bc + bp + bt, P.start.data(), sizeof(int) * P.start.size());
-  CK_TC(cuda(cudaMemcpy(t, h.data(), h.size(), cudaMemcpyHostToDevice), "cudaMemcpy(FP64 product plan)"));
+  CK_TC(put(t, h.data(), h.size(), "cudaMemcpy(FP64 product plan)"));
   CK_TC(cuda(cudaMemsetAsync(P.buf, 0, bb, stream), "memset(FP64 product operands)"));
   P.d_ops = reinterpret_cast<const OzOperand*>(t);
   P.d_chunks = reinterpret_cast<const OzChunk*>(t + bo);

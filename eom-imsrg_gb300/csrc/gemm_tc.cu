@@ -740,9 +740,9 @@ imsrg_status Ctx::tc_prepare(int mode) {
 
   const size_t bytes = (size_t)tc_elem_bytes() * (size_t)S * tc->slice_elems;
   CK_TC(cuda(cudaMalloc(&tc->buf, std::max<size_t>(bytes, 256)), "cudaMalloc(tc operands)"));
-  CK_TC(cuda(cudaMemset(tc->buf, 0, std::max<size_t>(bytes, 256)), "memset(tc operands)"));
+  CK_TC(cuda(cudaMemsetAsync(tc->buf, 0, std::max<size_t>(bytes, 256), stream), "memset(tc operands)"));
   CK_TC(cuda(cudaMalloc(&tc->zbuf, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(X)"));
-  CK_TC(cuda(cudaMemset(tc->zbuf, 0, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "memset(X)"));
+  CK_TC(cuda(cudaMemsetAsync(tc->zbuf, 0, sizeof(float) * std::max<int64_t>(l.wcc_size, 1), stream), "memset(X)"));
   DevPacker pk;
   pk.add(tc->split_ops, &tc->d_split_ops);
   pk.add(tc->split_prefix, &tc->d_split_prefix);
@@ -763,7 +763,7 @@ imsrg_status Ctx::tc_prepare(int mode) {
   pk.add(tc->chunks, &tc->d_chunks);
 
   CK_TC(cuda(cudaMalloc(&tc->d_mem, pk.buf.size()), "cudaMalloc(tc tables)"));
-  CK_TC(cuda(cudaMemcpy(tc->d_mem, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tc tables)"));
+  CK_TC(put(tc->d_mem, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tc tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(tc->d_mem) + f.first;
   // CTAs of the recoupling: about one wave where the quadruples are few, many short ones where their lengths would
   // otherwise leave a long tail (commutator at eMax 7 212 us with 32 a SM, 207 with 8; eMax 10 1606 with 32, 1579 with 128)

@@ -393,7 +393,7 @@ imsrg_status Ctx::hf_prepare() {
   const size_t o_cg = put(mcg.data(), sizeof(int) * mcg.size());
   const size_t o_ch = put(mch.data(), sizeof(int) * mch.size());
   CKH(undo(cuda(cudaMalloc(&S->tables, std::max<size_t>(buf.size(), 16)), "cudaMalloc(HF tables)")));
-  CKH(undo(cuda(cudaMemcpy(S->tables, buf.data(), buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(HF tables)")));
+  CKH(undo(this->put(S->tables, buf.data(), buf.size(), "cudaMemcpy(HF tables)")));
   const char* base = (const char*)S->tables;
   S->dev.spb_start = (const int*)(base + o_start);
   S->dev.spb_n = (const int*)(base + o_n);

@@ -171,12 +171,12 @@ imsrg_status Ctx::quads_prepare() {
   const size_t br = sizeof(int64_t) * pre.size();
   imsrg_status st = cuda(cudaMalloc(&s->tables, bp + bt + br), "cudaMalloc(quadrupole tables)");
   if (st == IMSRG_OK && !P.empty())
-    st = cuda(cudaMemcpy(s->tables, P.data(), sizeof(GemmProb) * P.size(), cudaMemcpyHostToDevice), "H2D quads");
+    st = put(s->tables, P.data(), sizeof(GemmProb) * P.size(), "H2D quads");
   if (st == IMSRG_OK && !tiles.empty())
-    st = cuda(cudaMemcpy((char*)s->tables + bp, tiles.data(), sizeof(GemmTile) * tiles.size(), cudaMemcpyHostToDevice),
+    st = put((char*)s->tables + bp, tiles.data(), sizeof(GemmTile) * tiles.size(),
               "H2D quads");
   if (st == IMSRG_OK)
-    st = cuda(cudaMemcpy((char*)s->tables + bp + bt, pre.data(), br, cudaMemcpyHostToDevice), "H2D quads");
+    st = put((char*)s->tables + bp + bt, pre.data(), br, "H2D quads");
   s->p = reinterpret_cast<const GemmProb*>(s->tables);
   s->t = reinterpret_cast<const GemmTile*>((char*)s->tables + bp);
   s->pre = reinterpret_cast<const int64_t*>((char*)s->tables + bp + bt);
@@ -188,7 +188,7 @@ imsrg_status Ctx::quads_prepare() {
     if (st == IMSRG_OK) st = cuda(cudaMalloc(p, sb), "cudaMalloc(quadrupole workspace)");
   if (st == IMSRG_OK) st = cuda(cudaMalloc(&s->ins, std::max<size_t>(ib, 8)), "cudaMalloc(quadrupole insertions)");
   for (double* p : {s->w1, s->w2})
-    if (st == IMSRG_OK) st = cuda(cudaMemset(p, 0, sb), "memset(quadrupole workspace)");
+    if (st == IMSRG_OK) st = cuda(cudaMemsetAsync(p, 0, sb, stream), "memset(quadrupole workspace)");
   if (st != IMSRG_OK) {
     for (void* p : {s->tables, (void*)s->w1, (void*)s->w2, (void*)s->int3, (void*)s->ins})
       if (p) cudaFree(p);

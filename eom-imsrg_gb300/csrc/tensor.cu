@@ -278,7 +278,7 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
   st->pphh_probs = pphh; st->exc_probs = exc; st->x_probs = xbp;
   pk.add(T.seg_start, &st->seg_start); pk.add(T.seg_len, &st->seg_len); pk.add(T.seg_w, &st->seg_w);
   CKT(cuda(cudaMalloc(&st->tables, pk.buf.size()), "cudaMalloc(tensor tables)"));
-  CKT(cuda(cudaMemcpy(st->tables, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tensor tables)"));
+  CKT(put(st->tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tensor tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(st->tables) + f.first;
   st->n_pphh_t = (int)pphh_tiles.size();
   st->n_exc_t = (int)exc_tiles.size();
@@ -462,13 +462,13 @@ imsrg_status Ctx::tensor_tc_prepare(TensorState& S) {
     return fail(IMSRG_ERR_UNSUPPORTED, "tensor ladder operands too large for 32-bit TMA rows");
   const size_t bytes = (size_t)tc_elem_bytes() * (size_t)Sl * (size_t)S.tc_slice_elems;
   CKT(cuda(cudaMalloc(&S.tc_buf, std::max<size_t>(bytes, 256)), "cudaMalloc(tensor ladder operands)"));
-  CKT(cuda(cudaMemset(S.tc_buf, 0, std::max<size_t>(bytes, 256)), "memset(tensor ladder operands)"));
+  CKT(cuda(cudaMemsetAsync(S.tc_buf, 0, std::max<size_t>(bytes, 256), stream), "memset(tensor ladder operands)"));
   CKT(tc_encode_map(&S.tc_map, S.tc_buf, (int64_t)Sl * S.tc_slice_rows));
   Pack pk;
   pk.add(ops, &S.tc_ops); pk.add(chunks, &S.tc_chunks); pk.add(probs, &S.tc_probs); pk.add(tl, &S.tc_tiles);
   pk.add(hh, &S.hh_p); pk.add(hh_tiles, &S.hh_t);
   CKT(cuda(cudaMalloc(&S.tc_tables, pk.buf.size()), "cudaMalloc(tensor ladder tables)"));
-  CKT(cuda(cudaMemcpy(S.tc_tables, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice), "cudaMemcpy(tensor ladder)"));
+  CKT(put(S.tc_tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tensor ladder)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(S.tc_tables) + f.first;
   S.tc_nchunks = ladder_nchunks;
   S.tc_ntiles = ladder_ntiles;
