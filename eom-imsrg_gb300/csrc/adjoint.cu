@@ -74,13 +74,13 @@ imsrg_status Ctx::adjoint_prepare() {
   CKA(ensure_workspace());
   adj = new AdjointState();
   const Layout& l = L;
-  CKA(cuda(cudaMalloc(&adj->cb, sizeof(double) * (size_t)l.slab), "cudaMalloc(adjoint cb)"));
-  CKA(cuda(cudaMalloc(&adj->lccb, sizeof(double) * std::max<int64_t>(l.cc_size, 1)), "cudaMalloc(LCCb)"));
-  CKA(cuda(cudaMalloc(&adj->rccb, sizeof(double) * std::max<int64_t>(l.cc_size, 1)), "cudaMalloc(RCCb)"));
-  CKA(cuda(cudaMalloc(&adj->wccb, sizeof(double) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(WCCb)"));
-  CKA(cuda(cudaMalloc(&adj->monob, sizeof(double) * (size_t)l.N * l.N), "cudaMalloc(monopole cotangents)"));
-  CKA(cuda(cudaMalloc(&adj->partial, sizeof(double) * kDotBlocks), "cudaMalloc(dot partials)"));
-  CKA(cuda(cudaMalloc(&adj->fpart, sizeof(double) * 128 * l.same_list.size()), "cudaMalloc(one-body cotangents)"));
+  CKA(alloc(&adj->cb, sizeof(double) * (size_t)l.slab, "cudaMalloc(adjoint cb)"));
+  CKA(alloc(&adj->lccb, sizeof(double) * std::max<int64_t>(l.cc_size, 1), "cudaMalloc(LCCb)"));
+  CKA(alloc(&adj->rccb, sizeof(double) * std::max<int64_t>(l.cc_size, 1), "cudaMalloc(RCCb)"));
+  CKA(alloc(&adj->wccb, sizeof(double) * std::max<int64_t>(l.wcc_size, 1), "cudaMalloc(WCCb)"));
+  CKA(alloc(&adj->monob, sizeof(double) * (size_t)l.N * l.N, "cudaMalloc(monopole cotangents)"));
+  CKA(alloc(&adj->partial, sizeof(double) * kDotBlocks, "cudaMalloc(dot partials)"));
+  CKA(alloc(&adj->fpart, sizeof(double) * 128 * l.same_list.size(), "cudaMalloc(one-body cotangents)"));
   const auto pp = build_pphh_vjp_problems(l.nblocks, l.ncls, l.goff);
   const auto pt = build_tiles(pp, 64, 64);
   const auto wp = build_wcc_vjp_problems(l.ncc, l.cc_rlen, l.cc_nph, l.cc_off, l.wcc_off);
@@ -96,7 +96,7 @@ imsrg_status Ctx::adjoint_prepare() {
   if (!pt.empty()) std::memcpy(buf.data() + o[1], pt.data(), sizeof(GemmTile) * pt.size());
   if (!wp.empty()) std::memcpy(buf.data() + o[2], wp.data(), sizeof(GemmProb) * wp.size());
   if (!wt.empty()) std::memcpy(buf.data() + o[3], wt.data(), sizeof(GemmTile) * wt.size());
-  CKA(cuda(cudaMalloc(&adj->tables, buf.size()), "cudaMalloc(adjoint tables)"));
+  CKA(alloc(&adj->tables, buf.size(), "cudaMalloc(adjoint tables)"));
   CKA(put(adj->tables, buf.data(), buf.size(), "cudaMemcpy(adjoint tables)"));
   const char* base = static_cast<const char*>(adj->tables);
   adj->pphh_p = reinterpret_cast<const GemmProb*>(base + o[0]);
@@ -110,13 +110,18 @@ imsrg_status Ctx::adjoint_prepare() {
   return IMSRG_OK;
 }
 
+void Ctx::adjoint_release_plans() {
+  if (!adj) return;
+  oz_release(adj->pphh_oz);
+  oz_release(adj->wcc_oz);
+}
+
 void Ctx::adjoint_release() {
   if (!adj) return;
+  adjoint_release_plans();
   for (void* p : {(void*)adj->cb, (void*)adj->lccb, (void*)adj->rccb, (void*)adj->wccb, (void*)adj->monob,
                   (void*)adj->partial, (void*)adj->fpart, adj->tables})
     if (p) cudaFree(p);
-  oz_release(adj->pphh_oz);
-  oz_release(adj->wcc_oz);
   delete adj;
   adj = nullptr;
 }

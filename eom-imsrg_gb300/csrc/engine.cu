@@ -207,7 +207,7 @@ imsrg_status Ctx::upload_tables() {
   pk.add(zero_runs_w1, &zr1);
   pk.add(zero_runs_w2, &zr2);
 
-  CK(cuda(cudaMalloc(&d_tables, pk.buf.size()), "cudaMalloc(tables)"));
+  CK(alloc(&d_tables, pk.buf.size(), "cudaMalloc(tables)"));
   CK(put(d_tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(d_tables) + f.first;
   d_pphh_probs = pp_p; d_pphh_tiles = pp_t; d_wcc_probs = wc_p; d_wcc_tiles = wc_t;
@@ -216,13 +216,51 @@ imsrg_status Ctx::upload_tables() {
   d_zero_runs_w1 = zr1;
   d_zero_runs_w2 = zr2;
   partial_capacity = std::max(nseg, l.nblocks) + 64;
-  CK(cuda(cudaMalloc(&d_partial, sizeof(double) * partial_capacity), "cudaMalloc(partials)"));
-  CK(cuda(cudaMalloc(&d_scalars, sizeof(double) * 64), "cudaMalloc(scalars)"));
+  CK(alloc(&d_partial, sizeof(double) * partial_capacity, "cudaMalloc(partials)"));
+  CK(alloc(&d_scalars, sizeof(double) * 64, "cudaMalloc(scalars)"));
   CK(cuda(cudaMemsetAsync(d_scalars, 0, sizeof(double) * 64, stream), "memset(scalars)"));
   d_err = reinterpret_cast<int*>(d_scalars + kErrorSlot);
   CK(cuda(cudaMallocHost(&h_scalars, sizeof(double) * 64), "cudaMallocHost(scalars)"));
-  CK(cuda(cudaMalloc(&d_mono, sizeof(double) * (size_t)l.N * l.N), "cudaMalloc(monopole)"));
+  CK(alloc(&d_mono, sizeof(double) * (size_t)l.N * l.N, "cudaMalloc(monopole)"));
   return IMSRG_OK;
+}
+
+imsrg_status Ctx::alloc_bytes(void** p, size_t bytes, const char* what) {
+  cudaError_t e = fail_next_alloc ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+  fail_next_alloc = false;
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    release_optional();
+    e = cudaMalloc(p, bytes);
+  }
+  return cuda(e, what);
+}
+
+// What the context can do without.  A plan is made again by the next call that it serves, if there is room by then; 9j symbols are
+// evaluated where they are used from then on.
+void Ctx::release_optional() {
+  cudaStreamSynchronize(stream);
+  for (cudaStream_t b : branch_stream) cudaStreamSynchronize(b);
+  graph_drop();
+  ++plan_epoch;
+  oz_release(pphh_oz);
+  oz_release(wcc_oz);
+  adjoint_release_plans();
+  tensor_release_optional();
+  if (!tc && gp.state > 0) gather_release();  // the mixed modes cannot do without
+  for (double* p : op_pool) cudaFree(p);
+  op_pool.clear();
+}
+
+// An optional buffer takes at most half of the memory that is free, so that what is allocated next still fits.
+bool Ctx::room_for(size_t bytes) {
+  if (cache_limit >= 0) return bytes <= (size_t)cache_limit;
+  size_t avail = 0, total = 0;
+  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= avail / 2;
 }
 
 // A host table to the device, on the stream whose kernels read it: the context's streams do not wait for the default stream,
@@ -235,17 +273,17 @@ imsrg_status Ctx::put(void* dst, const void* src, size_t bytes, const char* what
 imsrg_status Ctx::ensure_workspace() {
   if (d_w1) return IMSRG_OK;
   const size_t sb = sizeof(double) * (size_t)L.slab;
-  CK(cuda(cudaMalloc(&d_w1, sb), "cudaMalloc(w1)"));
-  CK(cuda(cudaMalloc(&d_w2, sb), "cudaMalloc(w2)"));
-  CK(cuda(cudaMalloc(&d_lcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1)), "cudaMalloc(LCC)"));
-  CK(cuda(cudaMalloc(&d_rcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1)), "cudaMalloc(RCC)"));
+  CK(alloc(&d_w1, sb, "cudaMalloc(w1)"));
+  CK(alloc(&d_w2, sb, "cudaMalloc(w2)"));
+  CK(alloc(&d_lcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1), "cudaMalloc(LCC)"));
+  CK(alloc(&d_rcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1), "cudaMalloc(RCC)"));
   return IMSRG_OK;
 }
 
 // FP64 WCC workspace of the plain path (1.46 GiB at eMax=10), allocated on first use
 imsrg_status Ctx::ensure_wcc() {
   if (d_wcc) return IMSRG_OK;
-  CK(cuda(cudaMalloc(&d_wcc, sizeof(double) * std::max<int64_t>(L.wcc_size, 1)), "cudaMalloc(WCC)"));
+  CK(alloc(&d_wcc, sizeof(double) * std::max<int64_t>(L.wcc_size, 1), "cudaMalloc(WCC)"));
   CK(cuda(cudaMemsetAsync(d_wcc, 0, sizeof(double) * std::max<int64_t>(L.wcc_size, 1), stream), "memset(WCC)"));
   return IMSRG_OK;
 }
@@ -253,9 +291,9 @@ imsrg_status Ctx::ensure_wcc() {
 imsrg_status Ctx::ensure_flow_workspace() {
   if (d_int1) return IMSRG_OK;
   const size_t sb = sizeof(double) * (size_t)L.slab;
-  CK(cuda(cudaMalloc(&d_int1, sb), "cudaMalloc(INT1)"));
-  CK(cuda(cudaMalloc(&d_int2, sb), "cudaMalloc(INT2)"));
-  CK(cuda(cudaMalloc(&d_ad, sb), "cudaMalloc(AD)"));
+  CK(alloc(&d_int1, sb, "cudaMalloc(INT1)"));
+  CK(alloc(&d_int2, sb, "cudaMalloc(INT2)"));
+  CK(alloc(&d_ad, sb, "cudaMalloc(AD)"));
   return IMSRG_OK;
 }
 
@@ -558,7 +596,7 @@ imsrg_status Ctx::atan_generator(const double* Hden, int hden, const double* Hnu
 // commutator in the context's precision; three slab workspaces kept between calls
 imsrg_status Ctx::w2_generator(const double* H, int hH, double* ETA) {
   if (!d_gen) {
-    CK(cuda(cudaMalloc(&d_gen, 3 * sizeof(double) * (size_t)L.slab), "cudaMalloc(w2 generator workspace)"));
+    CK(alloc(&d_gen, 3 * sizeof(double) * (size_t)L.slab, "cudaMalloc(w2 generator workspace)"));
   }
   double* eta1 = d_gen;
   double* h2 = d_gen + L.slab;
@@ -793,6 +831,13 @@ imsrg_status imsrg_test_unarmed_stage(imsrg_ctx* ctx, int32_t enable) {
   return IMSRG_OK;
 }
 
+imsrg_status imsrg_test_memory(imsrg_ctx* ctx, int64_t cache_limit, int32_t fail_next) {
+  CTX(ctx);
+  c->cache_limit = cache_limit;
+  c->fail_next_alloc = fail_next != 0;
+  return IMSRG_OK;
+}
+
 imsrg_status imsrg_launch_count(imsrg_ctx* ctx, int64_t* count) {
   if (!ctx || !count) return IMSRG_ERR_INVALID_ARGUMENT;
   *count = reinterpret_cast<Ctx*>(ctx)->launches;
@@ -854,7 +899,7 @@ imsrg_status imsrg_op_create(imsrg_ctx* ctx, int32_t herm, imsrg_op** out) {
     op->d = c->op_pool.back();
     c->op_pool.pop_back();
   } else {
-    s = c->cuda(cudaMalloc(&op->d, sb), "cudaMalloc(operator)");
+    s = c->alloc(&op->d, sb, "cudaMalloc(operator)");
   }
   if (s == IMSRG_OK) s = c->cuda(cudaMemsetAsync(op->d, 0, sb, c->stream), "memset(operator)");
   if (s != IMSRG_OK) {
@@ -1036,7 +1081,7 @@ imsrg_status imsrg_check_conversions(imsrg_ctx* ctx, const double* host_x, const
   if (n == 0) return IMSRG_OK;
   void* d = nullptr;
   const size_t bx = sizeof(double) * (size_t)n, by = sizeof(float) * (size_t)n;
-  CK(c->cuda(cudaMalloc(&d, bx + by + 2 * by + 2 * bx), "cudaMalloc(conversion check)"));
+  CK(c->alloc(&d, bx + by + 2 * by + 2 * bx, "cudaMalloc(conversion check)"));
   // [x: n doubles | out_f64: 2n doubles | y: n floats | out_f32: 2n floats]
   double* dx = static_cast<double*>(d);
   double* dd = dx + n;
@@ -1079,7 +1124,7 @@ imsrg_status imsrg_cc_create(imsrg_ctx* ctx, int32_t kind, imsrg_cc** out) {
   cc->owner = c;
   cc->herm = 1;
   const size_t bytes = sizeof(double) * (size_t)std::max<int64_t>(cc->n, 1);
-  imsrg_status s = c->cuda(cudaMalloc(&cc->d, bytes), "cudaMalloc(cc)");
+  imsrg_status s = c->alloc(&cc->d, bytes, "cudaMalloc(cc)");
   if (s == IMSRG_OK) s = c->cuda(cudaMemsetAsync(cc->d, 0, bytes, c->stream), "memset(cc)");
   if (s != IMSRG_OK) {
     if (cc->d) cudaFree(cc->d);

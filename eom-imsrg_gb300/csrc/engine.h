@@ -103,6 +103,9 @@ struct Ctx {
   bool gather_no_room = false;  // no device memory for them in FP64
   // FP64 products on the tensor cores (gemm_oz.cu): the digit plans of the ladder and of the cross-coupled products
   imsrg::OzPlan pphh_oz, wcc_oz;
+  int plan_epoch = 0;            // how often optional buffers have gone: a captured graph holds their addresses
+  int64_t cache_limit = -1;      // test switch: most bytes of an optional buffer
+  bool fail_next_alloc = false;  // test switch
   int oz_sms = 0;  // SMs of the device, once a plan is ready
   // error word of the tensor-core kernels' bounded waits (in d_scalars, read with finish and read_scalars)
   int* d_err = nullptr;
@@ -172,6 +175,15 @@ struct Ctx {
   imsrg_status axpby(const double* A, double ax, const double* B, double bx, double* C);
   imsrg_status axpy_frob_async(double* Y, double a, const double* X, double scale, int slot, bool with_e0);
   imsrg_status frob_async(const double* op, double scale, int slot);
+  // required device memory: where there is none, the optional buffers (plans of FP64 products, 9j tables, kept operator slabs) go
+  // first
+  imsrg_status alloc_bytes(void** p, size_t bytes, const char* what);
+  template <class T>
+  imsrg_status alloc(T** p, size_t bytes, const char* what) {
+    return alloc_bytes(reinterpret_cast<void**>(p), bytes, what);
+  }
+  void release_optional();
+  bool room_for(size_t bytes);
   imsrg_status put(void* dst, const void* src, size_t bytes, const char* what);
   imsrg_status read_scalars();
   imsrg_status finish();
@@ -204,6 +216,7 @@ struct Ctx {
   // reverse mode (FP64) of the commutator, the White generator and the slab inner product (adjoint.cu)
   imsrg_status adjoint_prepare();
   void adjoint_release();
+  void adjoint_release_plans();
   imsrg_status commutator_vjp(const double* L, int hL, const double* R, int hR, int hRES, bool with_e0,
                               const double* Cb, double* Lb, double* Rb);
   imsrg_status vjp_pieces(const double* L, int hL, const double* R, int hR, int hRES, bool with_e0, const double* Cb,
@@ -215,6 +228,7 @@ struct Ctx {
   imsrg_status tensor_state(int rank, int dpar, TensorState** out);
   imsrg_status tensor_tc_prepare(TensorState& S);
   void tensor_release();
+  void tensor_release_optional();
   imsrg_status tensor_commutator(TensorState& S, const double* L, int hL, const double* R, int hR, double* RES,
                                  int pieces);
   imsrg_status tensor_pieces(TensorState& S, const double* L, int hL, const double* R, int hR, double* RES, int pieces);
@@ -239,7 +253,7 @@ struct Ctx {
                       imsrg_hf_info* info);
 
   // gather plan and commutator_122 by pair groups, gather.cu
-  imsrg_status gather_prepare();
+  imsrg_status gather_prepare(bool optional = false);
   imsrg_status gather_prepare_fp64(bool& groups);
   void gather_release();
   imsrg_status g122_set_caps(int tiny_cap, int small_cap);
@@ -248,10 +262,10 @@ struct Ctx {
   imsrg_status c122_groups(const double* L, int hL, const double* R, int hR, double* RES, int hRES);
 
   // grouped FP64 products, gemm_oz.cu
-  imsrg_status oz_prepare(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs);
+  imsrg_status oz_prepare(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs, imsrg::OzPool* pool = nullptr);
   void oz_release(imsrg::OzPlan& P);
   imsrg_status gemm_fp64(imsrg::OzPlan& P, const std::vector<imsrg::GemmProb>& probs, const imsrg::GemmProb* d_probs,
-                         const imsrg::GemmTile* d_tiles, int ntiles, const imsrg::GemmOperands& ops);
+                         const imsrg::GemmTile* d_tiles, int ntiles, const imsrg::GemmOperands& ops, imsrg::OzPool* pool = nullptr);
 
   // tensor-core (split-BF16, tcgen05) path, gemm_tc.cu
   imsrg_status tc_prepare(int mode);

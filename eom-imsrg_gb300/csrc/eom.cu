@@ -61,6 +61,7 @@ struct imsrg_eom {
   const double* g_H = nullptr;
   int g_prec = -1;  // the context's precision at capture (the kernels differ between modes)
   unsigned long long g_wait = 0;  // and the limit of their waits
+  int g_epoch = 0;
 };
 
 namespace {
@@ -234,7 +235,7 @@ imsrg_status Ctx::eom_matvec(imsrg_eom& E, const double* Hd, const double* d_v, 
 // (captured on first use, after one direct run that also makes the workspaces; the operands are
 // read when the graph runs)
 imsrg_status Ctx::eom_matvec_graph(imsrg_eom& E, const double* Hd) {
-  if (E.gexec && E.g_H == Hd && E.g_prec == (int)precision && E.g_wait == tc_wait_ns)
+  if (E.gexec && E.g_H == Hd && E.g_prec == (int)precision && E.g_wait == tc_wait_ns && E.g_epoch == plan_epoch)
     return cuda(cudaGraphLaunch(E.gexec, stream), "cudaGraphLaunch(eom)");
   CKE(eom_matvec(E, Hd, E.d_v, E.d_w));
   CKE(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
@@ -256,6 +257,7 @@ imsrg_status Ctx::eom_matvec_graph(imsrg_eom& E, const double* Hd) {
   E.g_H = Hd;
   E.g_prec = (int)precision;
   E.g_wait = tc_wait_ns;
+  E.g_epoch = plan_epoch;
   return IMSRG_OK;  // d_w already holds the direct run's product
 }
 
@@ -401,7 +403,7 @@ imsrg_status imsrg_eom_create(imsrg_ctx* ctx, int32_t rank2, int32_t dpar2, imsr
   const size_t n = (size_t)std::max<int64_t>(E->n, 1), sb = sizeof(double) * (size_t)s->T.slab;
   imsrg_status st = IMSRG_OK;
   auto alloc = [&](void** p, size_t b, const char* what) {
-    if (st == IMSRG_OK) st = c->cuda(cudaMalloc(p, b), what);
+    if (st == IMSRG_OK) st = c->alloc(p, b, what);
   };
   alloc((void**)&E->d_pos, sizeof(int64_t) * n, "cudaMalloc(eom map)");
   alloc((void**)&E->d_mirror, sizeof(int64_t) * n, "cudaMalloc(eom map)");

@@ -16,7 +16,7 @@ using namespace imsrg;
 imsrg_status Ctx::gather_prepare_fp64(bool& groups) {
   groups = L.slab >= kGatherMinSlab && !gather_no_room;
   if (!groups) return IMSRG_OK;
-  const imsrg_status s = gather_prepare();
+  const imsrg_status s = gather_prepare(true);
   if (s != IMSRG_ERR_OUT_OF_MEMORY) return s;
   cudaGetLastError();
   gather_release();
@@ -25,7 +25,7 @@ imsrg_status Ctx::gather_prepare_fp64(bool& groups) {
   return IMSRG_OK;
 }
 
-imsrg_status Ctx::gather_prepare() {
+imsrg_status Ctx::gather_prepare(bool optional) {
   if (gp.state) return IMSRG_OK;
   gather_release();  // what a failed preparation left
   const Layout& l = L;
@@ -108,7 +108,8 @@ imsrg_status Ctx::gather_prepare() {
       {nullptr, sizeof(double2) * (size_t)std::max(pg.nblk2, 1), (const void**)&gp.fb}};
   size_t total = 0;
   for (const Piece& p : pieces) total += (p.bytes + 255) & ~size_t(255);
-  CK_TC(cuda(cudaMalloc(&gp.d_mem, std::max<size_t>(total, 256)), "cudaMalloc(gather plan)"));
+  if (optional && !room_for(total)) return IMSRG_ERR_OUT_OF_MEMORY;
+  CK_TC(alloc(&gp.d_mem, std::max<size_t>(total, 256), "cudaMalloc(gather plan)"));
   char* at = static_cast<char*>(gp.d_mem);
   for (const Piece& p : pieces) {
     *p.dst = at;

@@ -590,9 +590,10 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
 
 using namespace imsrg;
 
-// Tables and operand blocks of a plan.  The blocks' padding (rows past the operand's) is zeroed here and never
-// written.  Where the device has no room for them the list stays on k_gemm_fp64.
-imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
+// Tables and operand blocks of a plan.  The blocks' padding rows hold whatever was there: a row of A or of B reaches the elements
+// of that row or column alone, and those past the problem's edge are not stored.  (Padding in K is written by the split.)  Where
+// the device has no room for them the list stays on k_gemm_fp64.
+imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs, OzPool* pool) {
   if (P.state) return IMSRG_OK;
   P.state = -1;
   cudaDeviceGetAttribute(&oz_sms, cudaDevAttrMultiProcessorCount, device);
@@ -622,13 +623,23 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
                bs = al(sizeof(int) * P.start.size()), be = al(sizeof(int) * ((size_t)P.nexp + 3)),
                br = al(sizeof(OzRedo) * (size_t)P.max_redo);
   const size_t bb = (size_t)P.blocks * (kBlockBytes + kSliceBytes);
-  char* t = nullptr;
-  if (cudaMalloc(&P.buf, bb) != cudaSuccess || cudaMalloc(&t, bo + bc + bp + bt + bs + be + br) != cudaSuccess) {
+  char *t = nullptr, *buf = nullptr;
+  const bool have = pool && pool->bytes >= bb;
+  if ((!have && (!room_for(bb) || cudaMalloc(&buf, bb) != cudaSuccess)) ||
+      cudaMalloc(&t, bo + bc + bp + bt + bs + be + br) != cudaSuccess) {
     cudaGetLastError();
-    if (P.buf) cudaFree(P.buf);
-    P.buf = nullptr;
+    if (buf) cudaFree(buf);
     return IMSRG_OK;
   }
+  if (!pool) {
+    P.own = buf;
+  } else if (!have) {  // in place of a smaller one
+    CK_TC(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize(FP64 product operands)"));
+    if (pool->buf) cudaFree(pool->buf);
+    pool->buf = buf;
+    pool->bytes = bb;
+  }
+  P.pool = pool;
   P.tables = t;
   std::vector<char> h(bo + bc + bp + bt + bs);
   std::memcpy(h.data(), P.ops.data(), sizeof(OzOperand) * P.ops.size());
@@ -637,7 +648,6 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   std::memcpy(h.data() + bo + bc + bp, P.tiles.data(), sizeof(OzTile) * P.tiles.size());
   std::memcpy(h.data() + bo + bc + bp + bt, P.start.data(), sizeof(int) * P.start.size());
   CK_TC(put(t, h.data(), h.size(), "cudaMemcpy(FP64 product plan)"));
-  CK_TC(cuda(cudaMemsetAsync(P.buf, 0, bb, stream), "memset(FP64 product operands)"));
   P.d_ops = reinterpret_cast<const OzOperand*>(t);
   P.d_chunks = reinterpret_cast<const OzChunk*>(t + bo);
   P.d_probs = reinterpret_cast<const OzProb*>(t + bo + bc);
@@ -646,7 +656,6 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
   P.exps = reinterpret_cast<int*>(t + bo + bc + bp + bt + bs);
   P.flag = P.exps + P.nexp;
   P.redo = reinterpret_cast<OzRedo*>(t + bo + bc + bp + bt + bs + be);
-  P.mag = P.buf + (size_t)P.blocks * kBlockBytes;
   CK_TC(cuda(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem),
              "smem attr (FP64 products)"));
   P.state = 1;
@@ -654,27 +663,28 @@ imsrg_status Ctx::oz_prepare(OzPlan& P, const std::vector<GemmProb>& probs) {
 }
 
 void Ctx::oz_release(OzPlan& P) {
-  if (P.buf) cudaFree(P.buf);
+  if (P.own) cudaFree(P.own);
   if (P.tables) cudaFree(P.tables);
   P = OzPlan();
 }
 
 // The grouped FP64 products of a list (d_probs, d_tiles: the same list for k_gemm_fp64).
 imsrg_status Ctx::gemm_fp64(OzPlan& P, const std::vector<GemmProb>& probs, const GemmProb* d_probs,
-                            const GemmTile* d_tiles, int ntiles, const GemmOperands& ops) {
+                            const GemmTile* d_tiles, int ntiles, const GemmOperands& ops, OzPool* pool) {
   if (!ntiles) return IMSRG_OK;
-  CK_TC(oz_prepare(P, probs));
+  CK_TC(oz_prepare(P, probs, pool));
   if (P.state == 2) {
     k_gemm_fp64_small<<<P.nsmall, 256, 0, stream>>>(d_probs, P.d_small, ops);
     return launched("k_gemm_fp64_small");
   }
   if (P.state > 0) {
     CK_TC(cuda(cudaMemsetAsync(P.flag, 0, 3 * sizeof(int), stream), "memset(FP64 product flags)"));
-    k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, P.buf, P.mag, P.exps, P.flag);
+    char *buf = P.buf(), *mag = buf + (size_t)P.blocks * kBlockBytes;
+    k_oz_split<<<(int)P.chunks.size(), 256, 0, stream>>>(P.d_ops, P.d_chunks, ops, buf, mag, P.exps, P.flag);
     CK_TC(launched("k_oz_split"));
     const int unarmed = tc_unarmed_next ? 0 : -1;  // one-shot test switch
     tc_unarmed_next = 0;
-    k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, P.buf, P.mag, P.exps, P.flag, P.redo,
+    k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, buf, mag, P.exps, P.flag, P.redo,
                                                    (int)P.max_redo, d_err, tc_wait_ns, unarmed);
     CK_TC(launched("k_oz_gemm"));
     k_gemm_fp64_rest<<<4 * oz_sms, 256, 0, stream>>>(d_probs, d_tiles, ntiles, ops, P.flag, P.redo, (int)P.max_redo);

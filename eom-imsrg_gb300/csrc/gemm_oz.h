@@ -57,6 +57,12 @@ struct OzTile {
   int prob, m0, n0, w;
 };
 
+// Operand blocks of plans that run one after the other on one stream, as large as the largest of them needs.
+struct OzPool {
+  char* buf = nullptr;
+  size_t bytes = 0;
+};
+
 // The digit plan of a problem list; `state` 0: not prepared, 1: ready, 2: a small list, for k_gemm_fp64_small (its tiles in
 // `tables`), -1: the list stays on k_gemm_fp64.
 struct OzPlan {
@@ -70,8 +76,9 @@ struct OzPlan {
   int64_t blocks = 0;
   int nexp = 0;
   void* tables = nullptr;
-  char* buf = nullptr;   // operand blocks, then their magnitude slices
-  char* mag = nullptr;
+  char* own = nullptr;   // operand blocks, then their magnitude slices; in a pool where there is one
+  OzPool* pool = nullptr;
+  char* buf() const { return pool ? pool->buf : own; }
   int* exps = nullptr;   // row exponents, then the flags
   int* flag = nullptr;   // [0] an operand is not finite; entries of redo with [1] few and [2] many elements (from its end)
   OzRedo* redo = nullptr;

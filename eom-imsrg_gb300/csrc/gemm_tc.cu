@@ -739,9 +739,9 @@ imsrg_status Ctx::tc_prepare(int mode) {
   if ((int64_t)S * tc->slice_rows >= (int64_t)1 << 31) return fail(IMSRG_ERR_UNSUPPORTED, "operand buffer too large for 32-bit TMA rows");
 
   const size_t bytes = (size_t)tc_elem_bytes() * (size_t)S * tc->slice_elems;
-  CK_TC(cuda(cudaMalloc(&tc->buf, std::max<size_t>(bytes, 256)), "cudaMalloc(tc operands)"));
+  CK_TC(alloc(&tc->buf, std::max<size_t>(bytes, 256), "cudaMalloc(tc operands)"));
   CK_TC(cuda(cudaMemsetAsync(tc->buf, 0, std::max<size_t>(bytes, 256), stream), "memset(tc operands)"));
-  CK_TC(cuda(cudaMalloc(&tc->zbuf, sizeof(float) * std::max<int64_t>(l.wcc_size, 1)), "cudaMalloc(X)"));
+  CK_TC(alloc(&tc->zbuf, sizeof(float) * std::max<int64_t>(l.wcc_size, 1), "cudaMalloc(X)"));
   CK_TC(cuda(cudaMemsetAsync(tc->zbuf, 0, sizeof(float) * std::max<int64_t>(l.wcc_size, 1), stream), "memset(X)"));
   DevPacker pk;
   pk.add(tc->split_ops, &tc->d_split_ops);
@@ -762,7 +762,7 @@ imsrg_status Ctx::tc_prepare(int mode) {
   pk.add(tc->xmask, &tc->d_xmask);
   pk.add(tc->chunks, &tc->d_chunks);
 
-  CK_TC(cuda(cudaMalloc(&tc->d_mem, pk.buf.size()), "cudaMalloc(tc tables)"));
+  CK_TC(alloc(&tc->d_mem, pk.buf.size(), "cudaMalloc(tc tables)"));
   CK_TC(put(tc->d_mem, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tc tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(tc->d_mem) + f.first;
   // CTAs of the recoupling: about one wave where the quadruples are few, many short ones where their lengths would
@@ -772,7 +772,7 @@ imsrg_status Ctx::tc_prepare(int mode) {
   tc->tile_cap_pphh = make_tiles(tc->pphh_probs, 128, false).size();
   tc->tile_cap_z = make_tiles(tc->z_probs, 128, false).size();
   tc->tile_cap_all = tc->tile_cap_pphh + tc->tile_cap_z;
-  CK_TC(cuda(cudaMalloc(&tc->d_tile_mem, sizeof(TcTile) * std::max<size_t>(tc->tile_cap_all * 2, 1)),
+  CK_TC(alloc(&tc->d_tile_mem, sizeof(TcTile) * std::max<size_t>(tc->tile_cap_all * 2, 1),
              "cudaMalloc(GEMM tiles)"));
   tc->d_pphh_tiles = tc->d_tile_mem;
   tc->d_z_tiles = tc->d_tile_mem + tc->tile_cap_pphh;

@@ -312,21 +312,21 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
                               const StepHostIO* hio) {
   CK_TC(ensure_workspace());
   CK_TC(ensure_flow_workspace());
-  if (precision == IMSRG_PREC_FP64) {
-    if (L.cc_size) CK_TC(ensure_wcc());
-    CK_TC(oz_prepare(pphh_oz, pphh_probs));
-    CK_TC(oz_prepare(wcc_oz, wcc_probs));
-    bool groups = false;
-    CK_TC(gather_prepare_fp64(groups));
-  }
   if (!sg) {
     sg = new StepGraph();
-    CK_TC(cuda(cudaMalloc(&sg->d_state, sizeof(StepState)), "cudaMalloc(step state)"));
+    CK_TC(alloc(&sg->d_state, sizeof(StepState), "cudaMalloc(step state)"));
     CK_TC(cuda(cudaMemsetAsync(sg->d_state, 0, sizeof(StepState), stream), "memset(step state)"));
     CK_TC(cuda(cudaMallocHost(&sg->h_state, sizeof(StepState)), "cudaMallocHost(step state)"));
     CK_TC(cuda(cudaStreamCreateWithFlags(&sg->side, cudaStreamNonBlocking), "cudaStreamCreate(side)"));
     for (cudaStream_t& c : sg->cp) CK_TC(cuda(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking), "cudaStreamCreate(copy)"));
     for (cudaEvent_t& e : sg->ev) CK_TC(cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate"));
+  }
+  if (precision == IMSRG_PREC_FP64) {  // the optional plans last: an allocation may release them
+    if (L.cc_size) CK_TC(ensure_wcc());
+    bool groups = false;
+    CK_TC(gather_prepare_fp64(groups));
+    CK_TC(oz_prepare(pphh_oz, pphh_probs));
+    CK_TC(oz_prepare(wcc_oz, wcc_probs));
   }
   const size_t sbytes = sizeof(double) * (size_t)L.slab;
   int rebuilt = 0;

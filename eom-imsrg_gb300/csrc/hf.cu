@@ -392,7 +392,7 @@ imsrg_status Ctx::hf_prepare() {
   const size_t o_rj = put(mrj.data(), sizeof(int) * mrj.size());
   const size_t o_cg = put(mcg.data(), sizeof(int) * mcg.size());
   const size_t o_ch = put(mch.data(), sizeof(int) * mch.size());
-  CKH(undo(cuda(cudaMalloc(&S->tables, std::max<size_t>(buf.size(), 16)), "cudaMalloc(HF tables)")));
+  CKH(undo(alloc(&S->tables, std::max<size_t>(buf.size(), 16), "cudaMalloc(HF tables)")));
   CKH(undo(this->put(S->tables, buf.data(), buf.size(), "cudaMemcpy(HF tables)")));
   const char* base = (const char*)S->tables;
   S->dev.spb_start = (const int*)(base + o_start);
@@ -408,11 +408,11 @@ imsrg_status Ctx::hf_prepare() {
   S->dev.mcol_h = (const int*)(base + o_ch);
   S->dev.nrow = S->nrow;
   S->dev.ncol = S->ncol;
-  CKH(undo(cuda(cudaMalloc(&S->d_M, sizeof(double) * std::max<int64_t>((int64_t)S->nrow * S->ncol, 1)),
+  CKH(undo(alloc(&S->d_M, sizeof(double) * std::max<int64_t>((int64_t)S->nrow * S->ncol, 1),
            "cudaMalloc(HF mean-field tensor)")));
   CKH(undo(cuda(cudaMallocHost(&S->h_M, sizeof(double) * std::max<int64_t>((int64_t)S->nrow * S->ncol, 1)),
            "cudaMallocHost(HF mean-field tensor)")));
-  CKH(undo(cuda(cudaMalloc(&S->d_dp, sizeof(double) * std::max(S->ndp, 1)), "cudaMalloc(HF coefficients)")));
+  CKH(undo(alloc(&S->d_dp, sizeof(double) * std::max(S->ndp, 1), "cudaMalloc(HF coefficients)")));
   const size_t smem = hf_cta_smem(S->nmax);
   if (S->ncta && smem > 48 * 1024)
     CKH(undo(cuda(cudaFuncSetAttribute(k_hf_transform_2b<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),

@@ -169,7 +169,7 @@ imsrg_status Ctx::quads_prepare() {
   const size_t bp = (sizeof(GemmProb) * std::max<size_t>(P.size(), 1) + 255) & ~size_t(255);
   const size_t bt = (sizeof(GemmTile) * std::max<size_t>(tiles.size(), 1) + 255) & ~size_t(255);
   const size_t br = sizeof(int64_t) * pre.size();
-  imsrg_status st = cuda(cudaMalloc(&s->tables, bp + bt + br), "cudaMalloc(quadrupole tables)");
+  imsrg_status st = alloc(&s->tables, bp + bt + br, "cudaMalloc(quadrupole tables)");
   if (st == IMSRG_OK && !P.empty())
     st = put(s->tables, P.data(), sizeof(GemmProb) * P.size(), "H2D quads");
   if (st == IMSRG_OK && !tiles.empty())
@@ -185,8 +185,8 @@ imsrg_status Ctx::quads_prepare() {
   const size_t sb = sizeof(double) * (size_t)L.slab;
   const size_t ib = sizeof(double) * (2 * (size_t)L.A * L.A + 2 * (size_t)L.P * L.P);
   for (double** p : {&s->w1, &s->w2, &s->int3})
-    if (st == IMSRG_OK) st = cuda(cudaMalloc(p, sb), "cudaMalloc(quadrupole workspace)");
-  if (st == IMSRG_OK) st = cuda(cudaMalloc(&s->ins, std::max<size_t>(ib, 8)), "cudaMalloc(quadrupole insertions)");
+    if (st == IMSRG_OK) st = alloc(p, sb, "cudaMalloc(quadrupole workspace)");
+  if (st == IMSRG_OK) st = alloc(&s->ins, std::max<size_t>(ib, 8), "cudaMalloc(quadrupole insertions)");
   for (double* p : {s->w1, s->w2})
     if (st == IMSRG_OK) st = cuda(cudaMemsetAsync(p, 0, sb, stream), "memset(quadrupole workspace)");
   if (st != IMSRG_OK) {

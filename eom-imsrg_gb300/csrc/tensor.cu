@@ -277,7 +277,7 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
   pk.add(sq, &d.sq); pk.add(nine_off, &d.nine_off);
   st->pphh_probs = pphh; st->exc_probs = exc; st->x_probs = xbp;
   pk.add(T.seg_start, &st->seg_start); pk.add(T.seg_len, &st->seg_len); pk.add(T.seg_w, &st->seg_w);
-  CKT(cuda(cudaMalloc(&st->tables, pk.buf.size()), "cudaMalloc(tensor tables)"));
+  CKT(alloc(&st->tables, pk.buf.size(), "cudaMalloc(tensor tables)"));
   CKT(put(st->tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tensor tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(st->tables) + f.first;
   st->n_pphh_t = (int)pphh_tiles.size();
@@ -287,28 +287,35 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
   st->nseg = (int)T.seg_start.size();
   const size_t tb = sizeof(double) * (size_t)T.slab;
   for (double** p : {&st->w1, &st->w2, &st->bch_a, &st->bch_b}) {
-    CKT(cuda(cudaMalloc(p, tb), "cudaMalloc(tensor workspace)"));
+    CKT(alloc(p, tb, "cudaMalloc(tensor workspace)"));
     CKT(cuda(cudaMemsetAsync(*p, 0, tb, stream), "memset(tensor workspace)"));
   }
   double** ph[] = {&st->ccr, &st->ccx, &st->wx, &st->wy};
   for (int k = 0; k < 4; ++k)
-    CKT(cuda(cudaMalloc(ph[k], sizeof(double) * (size_t)std::max<int64_t>(st->ph_sizes[std::min(k, 2)], 1)),
+    CKT(alloc(ph[k], sizeof(double) * (size_t)std::max<int64_t>(st->ph_sizes[std::min(k, 2)], 1),
              "cudaMalloc(cross-coupled tensor blocks)"));
   d.nine = nullptr;
-  if (nine_n * (int64_t)sizeof(double) <= (int64_t)1 << 30 && cudaMalloc(&st->d_nine, sizeof(double) * (size_t)nine_n) == cudaSuccess) {
-    k_tensor_nine<<<(int)nine_off.size(), 128, 0, stream>>>(d, st->d_nine);
-    CKT(launched("k_tensor_nine"));
-    d.nine = st->d_nine;
-  } else {
-    cudaGetLastError();
-    st->d_nine = nullptr;
+  for (auto& other : reg)
+    if (other.first.first == this && other.second->T.rank == T.rank && other.second->nine) st->nine = other.second->nine;
+  const size_t nine_bytes = sizeof(double) * (size_t)nine_n;
+  double* nine = nullptr;
+  if (!st->nine && nine_bytes <= (size_t)1 << 30 && room_for(nine_bytes)) {
+    if (cudaMalloc(&nine, nine_bytes) == cudaSuccess) {
+      st->nine = std::shared_ptr<double>(nine, [](double* p) { cudaFree(p); });
+      k_tensor_nine<<<(int)nine_off.size(), 128, 0, stream>>>(d, nine);
+      CKT(launched("k_tensor_nine"));
+    } else {
+      cudaGetLastError();
+    }
   }
+  d.nine = st->nine.get();
   *out = st.get();
   reg[key] = std::move(st);
   return IMSRG_OK;
 }
 
 void Ctx::tensor_release() {
+  tensor_release_optional();
   auto& reg = registry();
   for (auto it = reg.begin(); it != reg.end();) {
     if (it->first.first != this) {
@@ -318,13 +325,24 @@ void Ctx::tensor_release() {
     TensorState* s = it->second.get();
     for (void* p : {(void*)s->w1, (void*)s->w2, (void*)s->ccx, (void*)s->ccr, (void*)s->wx, (void*)s->wy,
                     (void*)s->bch_a, (void*)s->bch_b, s->tables, (void*)s->tc_buf, s->tc_tables, (void*)s->w3,
-                    (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3], (void*)s->d_nine})
+                    (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3]})
       if (p) cudaFree(p);
-    oz_release(s->pphh_oz);
-    oz_release(s->exc_oz);
-    oz_release(s->x_oz);
-    for (PhBatch& B : s->ph_batches) oz_release(B.oz);
     it = reg.erase(it);
+  }
+}
+
+void Ctx::tensor_release_optional() {
+  for (auto& e : registry()) {
+    if (e.first.first != this) continue;
+    TensorState& s = *e.second;
+    oz_release(s.pphh_oz);
+    oz_release(s.exc_oz);
+    oz_release(s.x_oz);
+    for (PhBatch& B : s.ph_batches) oz_release(B.oz);
+    if (s.ph_pool.buf) cudaFree(s.ph_pool.buf);
+    s.ph_pool = OzPool();
+    s.DT.nine = nullptr;
+    s.nine.reset();
   }
 }
 
@@ -461,19 +479,19 @@ imsrg_status Ctx::tensor_tc_prepare(TensorState& S) {
   if ((int64_t)Sl * S.tc_slice_rows >= (int64_t)1 << 31)
     return fail(IMSRG_ERR_UNSUPPORTED, "tensor ladder operands too large for 32-bit TMA rows");
   const size_t bytes = (size_t)tc_elem_bytes() * (size_t)Sl * (size_t)S.tc_slice_elems;
-  CKT(cuda(cudaMalloc(&S.tc_buf, std::max<size_t>(bytes, 256)), "cudaMalloc(tensor ladder operands)"));
+  CKT(alloc(&S.tc_buf, std::max<size_t>(bytes, 256), "cudaMalloc(tensor ladder operands)"));
   CKT(cuda(cudaMemsetAsync(S.tc_buf, 0, std::max<size_t>(bytes, 256), stream), "memset(tensor ladder operands)"));
   CKT(tc_encode_map(&S.tc_map, S.tc_buf, (int64_t)Sl * S.tc_slice_rows));
   Pack pk;
   pk.add(ops, &S.tc_ops); pk.add(chunks, &S.tc_chunks); pk.add(probs, &S.tc_probs); pk.add(tl, &S.tc_tiles);
   pk.add(hh, &S.hh_p); pk.add(hh_tiles, &S.hh_t);
-  CKT(cuda(cudaMalloc(&S.tc_tables, pk.buf.size()), "cudaMalloc(tensor ladder tables)"));
+  CKT(alloc(&S.tc_tables, pk.buf.size(), "cudaMalloc(tensor ladder tables)"));
   CKT(put(S.tc_tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tensor ladder)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(S.tc_tables) + f.first;
   S.tc_nchunks = ladder_nchunks;
   S.tc_ntiles = ladder_ntiles;
   S.n_hh_t = (int)hh_tiles.size();
-  CKT(cuda(cudaMalloc(&S.w3, sizeof(double) * (size_t)S.T.slab), "cudaMalloc(tensor w3)"));
+  CKT(alloc(&S.w3, sizeof(double) * (size_t)S.T.slab, "cudaMalloc(tensor w3)"));
   S.tc_S = Sl;
   S.tc_kind = tc_kind();
   return IMSRG_OK;
@@ -579,7 +597,7 @@ imsrg_status Ctx::tensor_pieces(TensorState& S, const double* Lp, int hL, const 
     if (S.x_nblk) {
       if (!S.x_buf[0])
         for (int k = 0; k < 4; ++k)
-          CKT(cuda(cudaMalloc(&S.x_buf[k], sizeof(double) * (size_t)std::max<int64_t>(S.x_sizes[k], 1)),
+          CKT(alloc(&S.x_buf[k], sizeof(double) * (size_t)std::max<int64_t>(S.x_sizes[k], 1),
                    "cudaMalloc(excitation ph buffers)"));
       k_tpandya_exc<<<grid_n(S.x_np), 256, 0, stream>>>(D, T, R, hR, S.x_blk, S.x_pre_p, S.x_nblk, S.d_pe, S.d_hp,
                                                          S.x_buf[0], S.x_buf[1]);
@@ -622,7 +640,7 @@ imsrg_status Ctx::tensor_pieces(TensorState& S, const double* Lp, int hL, const 
         ops.in[kOpLCC] = d_lcc; ops.in[kOpRCC] = S.ccr; ops.in[kOpWCC] = S.ccx;
         ops.out[kOpW1] = S.wx; ops.out[kOpW2] = S.wy;
         ops.hL = hL; ops.hR = hR;
-        CKT(gemm_fp64(B.oz, B.probs, S.cb_p + B.prob0, S.cb_t + B.tile0, B.ntiles, ops));
+        CKT(gemm_fp64(B.oz, B.probs, S.cb_p + B.prob0, S.cb_t + B.tile0, B.ntiles, ops, &S.ph_pool));
       }
       CKT(join(2));
       k_ts222ph_scatter<<<grid_n(B.ns), 256, 0, stream>>>(D, T, S.d_ph_blocks + B.b0, S.d_ph_pre_s + B.pre0, B.n, S.wx, S.wy,
@@ -652,7 +670,7 @@ imsrg_status Ctx::tensor_frob(TensorState& S, const double* op, double scale, in
   if (S.nseg == 0) return cuda(cudaMemsetAsync(d_scalars + slot, 0, sizeof(double), stream), "memset(norm)");
   if ((int64_t)S.nseg > partial_capacity) {  // one partial per segment: grow the buffer
     double* p = nullptr;
-    CKT(cuda(cudaMalloc(&p, sizeof(double) * (size_t)S.nseg), "cudaMalloc(partials)"));
+    CKT(alloc(&p, sizeof(double) * (size_t)S.nseg, "cudaMalloc(partials)"));
     CKT(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
     cudaFree(d_partial);
     d_partial = p;
@@ -734,7 +752,7 @@ imsrg_status imsrg_tensor_create(imsrg_ctx* ctx, int32_t rank2, int32_t dpar2, i
   imsrg_tensor* t = new (std::nothrow) imsrg_tensor();
   if (!t) return IMSRG_ERR_OUT_OF_MEMORY;
   const size_t tb = sizeof(double) * (size_t)s->T.slab;
-  imsrg_status st = c->cuda(cudaMalloc(&t->d, tb), "cudaMalloc(tensor operator)");
+  imsrg_status st = c->alloc(&t->d, tb, "cudaMalloc(tensor operator)");
   if (st == IMSRG_OK) st = c->cuda(cudaMemsetAsync(t->d, 0, tb, c->stream), "memset(tensor operator)");
   if (st != IMSRG_OK) {
     if (t->d) cudaFree(t->d);

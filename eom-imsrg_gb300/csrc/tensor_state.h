@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <memory>
 #include <vector>
 
 #include "engine.h"
@@ -85,7 +86,8 @@ struct TensorState {
   int64_t ph_sizes[3] = {0, 0, 0};  // CCR, CCX and W elements of the largest batch
   std::vector<GemmProb> pphh_probs, exc_probs, x_probs;
   imsrg::OzPlan pphh_oz, exc_oz, x_oz;
-  double* d_nine = nullptr;  // 9j table (DevTLayout::nine)
+  imsrg::OzPool ph_pool;         // operand blocks of the batches
+  std::shared_ptr<double> nine;  // 9j table (DevTLayout::nine), shared by the layouts of one rank
   const int64_t* seg_start = nullptr;
   const int* seg_len = nullptr;
   const int8_t* seg_w = nullptr;

@@ -402,7 +402,7 @@ imsrg_status Ctx::restore_triples(const double* H, const double* OM, double* e3,
                bm = al(sizeof(double) * (size_t)N * N), bf = al(sizeof(double) * N), bo = al(sizeof(double)),
                bs = al(sizeof(double) * (size_t)nsix);
   char* buf = nullptr;
-  CKR(cuda(cudaMalloc(&buf, bc + bp + bh + bl + bm + bf + bo + bs), "cudaMalloc(triples)"));
+  CKR(alloc(&buf, bc + bp + bh + bl + bm + bf + bo + bs, "cudaMalloc(triples)"));
   DevTriples T{};
   T.nh = nh; T.nJ = nJ; T.nx = nx;
   char* o = buf;

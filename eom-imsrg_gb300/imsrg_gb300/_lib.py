@@ -154,6 +154,7 @@ SIGNATURES = {
     "imsrg_set_tuning": [_vp, _vp],
     "imsrg_recouple_traffic": [_vp, _pi64, _pi64, _pi64, _pi64],
     "imsrg_test_unarmed_stage": [_vp, _i32],
+    "imsrg_test_memory": [_vp, _i64, _i32],
 }
 PHASES = ["start", "pandya", "one_body", "c122", "pphh_split", "pphh_gemm", "pphh_small", "pphh_update", "c221",
           "ph_gemm", "recouple", "mirror"]
