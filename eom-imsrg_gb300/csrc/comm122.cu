@@ -21,6 +21,7 @@
 // that the warps take in channel order from a counter, so the tasks of one channel (which
 // read the same arrays of L and R) run close together in time.
 #include "comm122.h"
+#include "kernels.h"
 
 #include <algorithm>
 #include <cmath>
@@ -287,13 +288,13 @@ template void launch_comm122<double>(int, size_t, cudaStream_t, const DevLayout&
 // shared memory limits and resident CTAs per SM of the FP32 ([0], smem bytes) and the FP64 kernel ([1], twice as many; 0
 // where a CTA cannot have that much)
 cudaError_t g122_occupancy(size_t smem, int* per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(k_comm122_sub<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_comm122_sub<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_comm122_sub<float>, kG122Threads, smem);
   if (e != cudaSuccess) return e;
   per_sm[1] = 0;
-  if (2 * smem > 227 * 1024) return cudaSuccess;
-  e = cudaFuncSetAttribute(k_comm122_sub<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * smem));
+  if (2 * smem > (size_t)kMaxDynamicSmem) return cudaSuccess;
+  e = cudaFuncSetAttribute(k_comm122_sub<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_comm122_sub<double>, kG122Threads, 2 * smem);
 }

@@ -27,6 +27,7 @@
 
 #include "../../include/imsrg_gb300.h"
 #include "engine.h"
+#include "kernels.h"
 #include "linalg.h"
 #include "pair_groups.h"
 
@@ -415,7 +416,7 @@ imsrg_status Ctx::hf_prepare() {
   CKH(undo(alloc(&S->d_dp, sizeof(double) * std::max(S->ndp, 1), "cudaMalloc(HF coefficients)")));
   const size_t smem = hf_cta_smem(S->nmax);
   if (S->ncta && smem > 48 * 1024)
-    CKH(undo(cuda(cudaFuncSetAttribute(k_hf_transform_2b<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    CKH(undo(cuda(cudaFuncSetAttribute(k_hf_transform_2b<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max((int)smem, kMaxDynamicSmem)),
              "cudaFuncSetAttribute(k_hf_transform_2b)")));
   return IMSRG_OK;
 }

@@ -12,6 +12,10 @@
 
 namespace imsrg {
 
+// Dynamic shared memory limit of a kernel whose need depends on the basis: the most that a CTA can have, for the limit belongs to
+// the process, and a context of a smaller basis must not lower that of a larger one's.
+constexpr int kMaxDynamicSmem = 227 * 1024;
+
 __global__ void k_pandya(DevLayout D, const double* op, int herm, double* cc);
 // run_if: with a flag, nothing is done unless it is set
 __global__ void k_comm122(DevLayout D, const double* L, int hL, const double* R, int hR, double* RES, int hRES,
