@@ -219,8 +219,9 @@ imsrg_status Ctx::upload_tables() {
   CK(alloc(&d_partial, sizeof(double) * partial_capacity, "cudaMalloc(partials)"));
   CK(alloc(&d_scalars, sizeof(double) * 64, "cudaMalloc(scalars)"));
   CK(cuda(cudaMemsetAsync(d_scalars, 0, sizeof(double) * 64, stream), "memset(scalars)"));
-  d_err = reinterpret_cast<int*>(d_scalars + kErrorSlot);
   CK(cuda(cudaMallocHost(&h_scalars, sizeof(double) * 64), "cudaMallocHost(scalars)"));
+  std::memset(h_scalars, 0, sizeof(double) * 64);
+  wait_err = reinterpret_cast<volatile int*>(h_scalars + kErrorSlot);
   CK(alloc(&d_mono, sizeof(double) * (size_t)l.N * l.N, "cudaMalloc(monopole)"));
   return IMSRG_OK;
 }
@@ -540,25 +541,18 @@ imsrg_status Ctx::frob_async(const double* op, double scale, int slot) {
   return launched("k_sum_sqrt");
 }
 
-// the scalars and, in the same copy, the error word behind them
 imsrg_status Ctx::read_scalars() {
-  CK(cuda(cudaMemcpyAsync(h_scalars, d_scalars, sizeof(double) * (kErrorSlot + 1), cudaMemcpyDeviceToHost, stream), "D2H scalars"));
-  CK(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
-  return wait_error();
+  CK(cuda(cudaMemcpyAsync(h_scalars, d_scalars, sizeof(double) * kErrorSlot, cudaMemcpyDeviceToHost, stream), "D2H scalars"));
+  return finish();
 }
 
 // Waits for the stream and reports a wait that ran out: the end of every call that hands results to the host, since a kernel
 // that gave up left its output incomplete.
 imsrg_status Ctx::finish() {
-  CK(cuda(cudaMemcpyAsync(h_scalars + kErrorSlot, d_scalars + kErrorSlot, sizeof(double), cudaMemcpyDeviceToHost, stream), "D2H error word"));
   CK(cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize"));
-  return wait_error();
-}
-
-imsrg_status Ctx::wait_error() {
-  const int e = *reinterpret_cast<const int*>(h_scalars + kErrorSlot);
+  const int e = *wait_err;
   if (!e) return IMSRG_OK;
-  CK(cuda(cudaMemsetAsync(d_err, 0, sizeof(int), stream), "memset(error word)"));
+  *wait_err = 0;
   static const char* role[] = {"", "producer (stage free)", "MMA (accumulator free)", "MMA (stage loaded)",
                                "epilogue (accumulator ready)"};
   return fail(IMSRG_ERR_TIMEOUT, std::string("tensor-core GEMM: a bounded wait ran out in the ") +

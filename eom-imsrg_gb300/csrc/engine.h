@@ -60,7 +60,7 @@ constexpr int64_t kGatherMinSlab = 100000;
 
 // up to this size the mixed commutator runs 122 beside its GEMM (gemm_tc.cu)
 constexpr int64_t kIdleSlab = (int64_t)1 << 22;
-// the word of d_scalars (and of h_scalars) that holds the error of a bounded wait
+// the word of h_scalars that holds the error of a bounded wait; the scalars before it
 constexpr int kErrorSlot = 8;
 
 struct Ctx {
@@ -107,8 +107,9 @@ struct Ctx {
   int64_t cache_limit = -1;      // test switch: most bytes of an optional buffer
   bool fail_next_alloc = false;  // test switch
   int oz_sms = 0;  // SMs of the device, once a plan is ready
-  // error word of the tensor-core kernels' bounded waits (in d_scalars, read with finish and read_scalars)
-  int* d_err = nullptr;
+  // error word of the tensor-core kernels' bounded waits, in pinned host memory: written by a kernel whose wait ran out, read
+  // by finish()
+  volatile int* wait_err = nullptr;
   // limit of every bounded device wait of the tensor-core kernels (imsrg_set_wait_limit), and the
   // one-shot test switch that leaves one pipeline stage of the next GEMM launch unarmed
   unsigned long long tc_wait_ns = 2000000000ull;
@@ -187,7 +188,6 @@ struct Ctx {
   imsrg_status put(void* dst, const void* src, size_t bytes, const char* what);
   imsrg_status read_scalars();
   imsrg_status finish();
-  imsrg_status wait_error();
   imsrg_status white(const double* H, int hH, double* ETA);
   imsrg_status atan_generator(const double* Hden, int hden, const double* Hnum, double* ETA);
   imsrg_status w2_generator(const double* H, int hH, double* ETA);

@@ -685,7 +685,7 @@ imsrg_status Ctx::gemm_fp64(OzPlan& P, const std::vector<GemmProb>& probs, const
     const int unarmed = tc_unarmed_next ? 0 : -1;  // one-shot test switch
     tc_unarmed_next = 0;
     k_oz_gemm<<<P.ncta, kThreads, kSmem, stream>>>(P.d_probs, P.d_tiles, P.d_start, ops, buf, mag, P.exps, P.flag, P.redo,
-                                                   (int)P.max_redo, d_err, tc_wait_ns, unarmed);
+                                                   (int)P.max_redo, const_cast<int*>(wait_err), tc_wait_ns, unarmed);
     CK_TC(launched("k_oz_gemm"));
     k_gemm_fp64_rest<<<4 * oz_sms, 256, 0, stream>>>(d_probs, d_tiles, ntiles, ops, P.flag, P.redo, (int)P.max_redo);
     return launched("k_gemm_fp64_rest");

@@ -837,7 +837,7 @@ imsrg_status Ctx::tc_gemm_on(const CUtensorMap& map, int64_t slice_rows, const T
   const int unarmed = tc_unarmed_next ? 0 : -1;  // one-shot test switch
   tc_unarmed_next = 0;
   auto go = [&](auto launcher) {
-    launcher(grid, stream, map, slice_rows, probs, tiles, ntiles, out, hL, hR, d_err, tc_wait_ns, unarmed);
+    launcher(grid, stream, map, slice_rows, probs, tiles, ntiles, out, hL, hR, const_cast<int*>(wait_err), tc_wait_ns, unarmed);
   };
   if (tc->kind == kKindTF32)
     wmax == 256 ? go(launch_tc_gemm<2, kKindTF32, 256>) : go(launch_tc_gemm<2, kKindTF32, 128>);

@@ -33,7 +33,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 }
 // Bounded wait on a barrier phase.  Returns false (after recording `code`) when it has waited
 // more than limit_ns, or when another role has already aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err,
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, volatile int* err,
                                           int code, unsigned long long limit_ns) {
   if (mbar_test(bar, parity)) return true;
   const unsigned long long t0 = globaltimer();
@@ -41,7 +41,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (mbar_test(bar, parity)) return true;
     if (*abort_flag) return false;
     if (globaltimer() - t0 > limit_ns) {
-      atomicCAS(err, 0, code);
+      *err = code;  // pinned host memory: the host reads it once the stream is done
       *abort_flag = 1;
       return false;
     }
