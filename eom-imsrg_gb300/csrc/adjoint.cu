@@ -73,6 +73,12 @@ imsrg_status Ctx::adjoint_prepare() {
   if (adj) return IMSRG_OK;
   CKA(ensure_workspace());
   adj = new AdjointState();
+  const imsrg_status s = adjoint_build();
+  if (s != IMSRG_OK) adjoint_release();  // a later call starts over
+  return s;
+}
+
+imsrg_status Ctx::adjoint_build() {
   const Layout& l = L;
   CKA(alloc(&adj->cb, sizeof(double) * (size_t)l.slab, "cudaMalloc(adjoint cb)"));
   CKA(alloc(&adj->lccb, sizeof(double) * std::max<int64_t>(l.cc_size, 1), "cudaMalloc(LCCb)"));

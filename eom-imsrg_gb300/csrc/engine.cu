@@ -227,14 +227,32 @@ imsrg_status Ctx::upload_tables() {
 }
 
 imsrg_status Ctx::alloc_bytes(void** p, size_t bytes, const char* what) {
-  cudaError_t e = fail_next_alloc ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
-  fail_next_alloc = false;
+  const bool refuse = fail_alloc == 1 || fail_alloc == -1, again = fail_alloc == -1;
+  fail_alloc -= fail_alloc > 0 ? 1 : (fail_alloc < 0 ? -1 : 0);
+  cudaError_t e = refuse ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     release_optional();
-    e = cudaMalloc(p, bytes);
+    if (!again) e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
   }
   return cuda(e, what);
+}
+
+imsrg_status Ctx::alloc_all(std::initializer_list<Want> wants) {
+  for (const Want& w : wants) {
+    const imsrg_status s = alloc(w.p, sizeof(double) * (size_t)std::max<int64_t>(w.n, 1), w.what);
+    if (s == IMSRG_OK) continue;
+    for (const Want* v = wants.begin(); v != &w; ++v) {
+      cudaFree(*v->p);
+      *v->p = nullptr;
+    }
+    return s;
+  }
+  return IMSRG_OK;
 }
 
 // What the context can do without.  A plan is made again by the next call that it serves, if there is room by then; 9j symbols are
@@ -273,12 +291,8 @@ imsrg_status Ctx::put(void* dst, const void* src, size_t bytes, const char* what
 
 imsrg_status Ctx::ensure_workspace() {
   if (d_w1) return IMSRG_OK;
-  const size_t sb = sizeof(double) * (size_t)L.slab;
-  CK(alloc(&d_w1, sb, "cudaMalloc(w1)"));
-  CK(alloc(&d_w2, sb, "cudaMalloc(w2)"));
-  CK(alloc(&d_lcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1), "cudaMalloc(LCC)"));
-  CK(alloc(&d_rcc, sizeof(double) * std::max<int64_t>(L.cc_size, 1), "cudaMalloc(RCC)"));
-  return IMSRG_OK;
+  return alloc_all({{&d_w1, L.slab, "cudaMalloc(w1)"}, {&d_w2, L.slab, "cudaMalloc(w2)"},
+                    {&d_lcc, L.cc_size, "cudaMalloc(LCC)"}, {&d_rcc, L.cc_size, "cudaMalloc(RCC)"}});
 }
 
 // FP64 WCC workspace of the plain path (1.46 GiB at eMax=10), allocated on first use
@@ -291,11 +305,7 @@ imsrg_status Ctx::ensure_wcc() {
 
 imsrg_status Ctx::ensure_flow_workspace() {
   if (d_int1) return IMSRG_OK;
-  const size_t sb = sizeof(double) * (size_t)L.slab;
-  CK(alloc(&d_int1, sb, "cudaMalloc(INT1)"));
-  CK(alloc(&d_int2, sb, "cudaMalloc(INT2)"));
-  CK(alloc(&d_ad, sb, "cudaMalloc(AD)"));
-  return IMSRG_OK;
+  return alloc_all({{&d_int1, L.slab, "cudaMalloc(INT1)"}, {&d_int2, L.slab, "cudaMalloc(INT2)"}, {&d_ad, L.slab, "cudaMalloc(AD)"}});
 }
 
 Ctx::~Ctx() {
@@ -390,6 +400,7 @@ imsrg_status Ctx::pphh_accumulate(int hL, int hR, double* RES, const double* w1,
 imsrg_status Ctx::pphh_products(const double* Lp, int hL, const double* Rp, int hR, double* w1, double* w2) {
   CK(pphh_clear(w1, w2));
   if (precision != IMSRG_PREC_FP64) {
+    CK(tc_prepare(precision));
     CK(tc_pphh(Lp, hL, Rp, hR, w1, w2));
   } else if (!pphh_tiles.empty()) {
     GemmOperands ops{};
@@ -448,6 +459,7 @@ imsrg_status Ctx::ph_recouple(int hL, int hR, double* RES, int hRES, const doubl
 
 imsrg_status Ctx::commutator(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES, bool with_e0) {
   CK(ensure_workspace());
+  if (precision != IMSRG_PREC_FP64) CK(tc_prepare(precision));  // gone if another mode found no room
   const imsrg_status s = precision != IMSRG_PREC_FP64 ? tc_commutator(Lp, hL, Rp, hR, RES, hRES, with_e0)
                                                       : fp64_commutator(Lp, hL, Rp, hR, RES, hRES, with_e0);
   for (int k = 0; k < kBranches; ++k) join(k);  // after an error: what a branch has issued is ordered all the same
@@ -828,7 +840,7 @@ imsrg_status imsrg_test_unarmed_stage(imsrg_ctx* ctx, int32_t enable) {
 imsrg_status imsrg_test_memory(imsrg_ctx* ctx, int64_t cache_limit, int32_t fail_next) {
   CTX(ctx);
   c->cache_limit = cache_limit;
-  c->fail_next_alloc = fail_next != 0;
+  c->fail_alloc = fail_next;
   return IMSRG_OK;
 }
 

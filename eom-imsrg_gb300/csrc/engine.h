@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -105,7 +106,7 @@ struct Ctx {
   imsrg::OzPlan pphh_oz, wcc_oz;
   int plan_epoch = 0;            // how often optional buffers have gone: a captured graph holds their addresses
   int64_t cache_limit = -1;      // test switch: most bytes of an optional buffer
-  bool fail_next_alloc = false;  // test switch
+  int fail_alloc = 0;            // test switch: the |n|-th required allocation from now on fails, for n < 0 also when tried again
   int oz_sms = 0;  // SMs of the device, once a plan is ready
   // error word of the tensor-core kernels' bounded waits, in pinned host memory: written by a kernel whose wait ran out, read
   // by finish()
@@ -183,6 +184,13 @@ struct Ctx {
   imsrg_status alloc(T** p, size_t bytes, const char* what) {
     return alloc_bytes(reinterpret_cast<void**>(p), bytes, what);
   }
+  // several, all or none
+  struct Want {
+    double** p;
+    int64_t n;  // doubles (at least one is allocated)
+    const char* what;
+  };
+  imsrg_status alloc_all(std::initializer_list<Want> wants);
   void release_optional();
   bool room_for(size_t bytes);
   imsrg_status put(void* dst, const void* src, size_t bytes, const char* what);
@@ -215,6 +223,7 @@ struct Ctx {
 
   // reverse mode (FP64) of the commutator, the White generator and the slab inner product (adjoint.cu)
   imsrg_status adjoint_prepare();
+  imsrg_status adjoint_build();
   void adjoint_release();
   void adjoint_release_plans();
   imsrg_status commutator_vjp(const double* L, int hL, const double* R, int hR, int hRES, bool with_e0,
@@ -269,6 +278,7 @@ struct Ctx {
 
   // tensor-core (split-BF16, tcgen05) path, gemm_tc.cu
   imsrg_status tc_prepare(int mode);
+  imsrg_status tc_build(int mode);
   imsrg_status tc_pphh(const double* L, int hL, const double* R, int hR, double* w1, double* w2);
   imsrg_status tc_wcc(const double* lcc, const double* rcc, double* wcc);
   imsrg_status tc_gemm(const imsrg::TcProb* probs, const imsrg::TcTile* tiles, int ntiles, imsrg::TcOut out, int hL,

@@ -593,6 +593,14 @@ imsrg_status Ctx::tc_prepare(int mode) {
   const int kind = (mode == IMSRG_PREC_TF32X3) ? kKindTF32 : kKindBF16;
   if (tc && tc->S == S && tc->kind == kind) return IMSRG_OK;
   tc_release();
+  const imsrg_status s = tc_build(mode);
+  if (s != IMSRG_OK) tc_release();  // a later call starts over
+  return s;
+}
+
+imsrg_status Ctx::tc_build(int mode) {
+  const int S = (mode == IMSRG_PREC_BF16X6) ? 3 : 2;
+  const int kind = (mode == IMSRG_PREC_TF32X3) ? kKindTF32 : kKindBF16;
   int cc_major = 0;
   cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, device);
   if (cc_major < 10) return fail(IMSRG_ERR_UNSUPPORTED, "tensor-core path needs a Blackwell (sm_10x) GPU");

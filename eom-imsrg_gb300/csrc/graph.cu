@@ -314,12 +314,20 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
   CK_TC(ensure_flow_workspace());
   if (!sg) {
     sg = new StepGraph();
-    CK_TC(alloc(&sg->d_state, sizeof(StepState), "cudaMalloc(step state)"));
-    CK_TC(cuda(cudaMemsetAsync(sg->d_state, 0, sizeof(StepState), stream), "memset(step state)"));
-    CK_TC(cuda(cudaMallocHost(&sg->h_state, sizeof(StepState)), "cudaMallocHost(step state)"));
-    CK_TC(cuda(cudaStreamCreateWithFlags(&sg->side, cudaStreamNonBlocking), "cudaStreamCreate(side)"));
-    for (cudaStream_t& c : sg->cp) CK_TC(cuda(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking), "cudaStreamCreate(copy)"));
-    for (cudaEvent_t& e : sg->ev) CK_TC(cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate"));
+    auto make = [&]() -> imsrg_status {
+      CK_TC(alloc(&sg->d_state, sizeof(StepState), "cudaMalloc(step state)"));
+      CK_TC(cuda(cudaMemsetAsync(sg->d_state, 0, sizeof(StepState), stream), "memset(step state)"));
+      CK_TC(cuda(cudaMallocHost(&sg->h_state, sizeof(StepState)), "cudaMallocHost(step state)"));
+      CK_TC(cuda(cudaStreamCreateWithFlags(&sg->side, cudaStreamNonBlocking), "cudaStreamCreate(side)"));
+      for (cudaStream_t& c : sg->cp) CK_TC(cuda(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking), "cudaStreamCreate(copy)"));
+      for (cudaEvent_t& e : sg->ev) CK_TC(cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate"));
+      return IMSRG_OK;
+    };
+    const imsrg_status s = make();
+    if (s != IMSRG_OK) {
+      graph_release();  // a later call starts over
+      return s;
+    }
   }
   if (precision == IMSRG_PREC_FP64) {  // the optional plans last: an allocation may release them
     if (L.cc_size) CK_TC(ensure_wcc());
@@ -327,6 +335,8 @@ imsrg_status Ctx::magnus_step(double* HS, double* G, int hG, double* DG, const d
     CK_TC(gather_prepare_fp64(groups));
     CK_TC(oz_prepare(pphh_oz, pphh_probs));
     CK_TC(oz_prepare(wcc_oz, wcc_probs));
+  } else {
+    CK_TC(tc_prepare(precision));
   }
   const size_t sbytes = sizeof(double) * (size_t)L.slab;
   int rebuilt = 0;

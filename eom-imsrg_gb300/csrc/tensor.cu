@@ -60,6 +60,14 @@ std::map<std::pair<Ctx*, int>, std::unique_ptr<TensorState>>& registry() {
   return r;
 }
 
+// what a layout holds on the device, but for its optional buffers
+void free_state(TensorState* s) {
+  for (void* p : {(void*)s->w1, (void*)s->w2, (void*)s->ccx, (void*)s->ccr, (void*)s->wx, (void*)s->wy,
+                  (void*)s->bch_a, (void*)s->bch_b, s->tables, (void*)s->tc_buf, s->tc_tables, (void*)s->w3,
+                  (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3]})
+    if (p) cudaFree(p);
+}
+
 struct Pack {
   std::vector<char> buf;
   std::vector<std::pair<size_t, const void**>> fix;
@@ -277,6 +285,12 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
   pk.add(sq, &d.sq); pk.add(nine_off, &d.nine_off);
   st->pphh_probs = pphh; st->exc_probs = exc; st->x_probs = xbp;
   pk.add(T.seg_start, &st->seg_start); pk.add(T.seg_len, &st->seg_len); pk.add(T.seg_w, &st->seg_w);
+  struct Undo {  // what has been allocated goes if the rest is not
+    TensorState* s;
+    ~Undo() {
+      if (s) free_state(s);
+    }
+  } undo{st.get()};
   CKT(alloc(&st->tables, pk.buf.size(), "cudaMalloc(tensor tables)"));
   CKT(put(st->tables, pk.buf.data(), pk.buf.size(), "cudaMemcpy(tensor tables)"));
   for (auto& f : pk.fix) *f.second = static_cast<const char*>(st->tables) + f.first;
@@ -309,6 +323,7 @@ imsrg_status Ctx::tensor_state(int rank, int dpar, TensorState** out) {
     }
   }
   d.nine = st->nine.get();
+  undo.s = nullptr;
   *out = st.get();
   reg[key] = std::move(st);
   return IMSRG_OK;
@@ -322,11 +337,7 @@ void Ctx::tensor_release() {
       ++it;
       continue;
     }
-    TensorState* s = it->second.get();
-    for (void* p : {(void*)s->w1, (void*)s->w2, (void*)s->ccx, (void*)s->ccr, (void*)s->wx, (void*)s->wy,
-                    (void*)s->bch_a, (void*)s->bch_b, s->tables, (void*)s->tc_buf, s->tc_tables, (void*)s->w3,
-                    (void*)s->x_buf[0], (void*)s->x_buf[1], (void*)s->x_buf[2], (void*)s->x_buf[3]})
-      if (p) cudaFree(p);
+    free_state(it->second.get());
     it = reg.erase(it);
   }
 }
@@ -500,7 +511,10 @@ imsrg_status Ctx::tensor_tc_prepare(TensorState& S) {
 imsrg_status Ctx::tensor_commutator(TensorState& S, const double* Lp, int hL, const double* R, int hR, double* RES,
                                     int pieces) {
   CKT(ensure_workspace());
-  if ((pieces & 96) && precision != IMSRG_PREC_FP64 && !(pieces & kTensorExcitation)) CKT(tensor_tc_prepare(S));
+  if ((pieces & 96) && precision != IMSRG_PREC_FP64 && !(pieces & kTensorExcitation)) {
+    CKT(tc_prepare(precision));
+    CKT(tensor_tc_prepare(S));
+  }
   const imsrg_status s = tensor_pieces(S, Lp, hL, R, hR, RES, pieces);
   for (int k = 0; k < kBranches; ++k) join(k);  // after an error: what a branch has issued is ordered all the same
   return s;
@@ -595,10 +609,11 @@ imsrg_status Ctx::tensor_pieces(TensorState& S, const double* Lp, int hL, const 
   }
   if ((pieces & 64) && exc) {  // excitation mode: packed CCR / CCX of all blocks (FP32 products in mixed modes)
     if (S.x_nblk) {
-      if (!S.x_buf[0])
-        for (int k = 0; k < 4; ++k)
-          CKT(alloc(&S.x_buf[k], sizeof(double) * (size_t)std::max<int64_t>(S.x_sizes[k], 1),
-                   "cudaMalloc(excitation ph buffers)"));
+      if (!S.x_buf[0]) {
+        const char* what = "cudaMalloc(excitation ph buffers)";
+        CKT(alloc_all({{&S.x_buf[0], S.x_sizes[0], what}, {&S.x_buf[1], S.x_sizes[1], what}, {&S.x_buf[2], S.x_sizes[2], what},
+                       {&S.x_buf[3], S.x_sizes[3], what}}));
+      }
       k_tpandya_exc<<<grid_n(S.x_np), 256, 0, stream>>>(D, T, R, hR, S.x_blk, S.x_pre_p, S.x_nblk, S.d_pe, S.d_hp,
                                                          S.x_buf[0], S.x_buf[1]);
       CKT(launched("k_tpandya_exc"));

@@ -102,8 +102,10 @@ imsrg_status imsrg_set_wait_limit(imsrg_ctx* ctx, int64_t nanoseconds);
 imsrg_status imsrg_test_unarmed_stage(imsrg_ctx* ctx, int32_t enable);
 /* Test switches, off by default: no optional buffer of this context (plans of the FP64 products
  * and gathers, 9j tables; half of the free device memory otherwise) above cache_limit bytes
- * (-1: off), and with fail_next != 0 the next required allocation finds no memory at first, so
- * that the optional buffers are released.  Results do not depend on either beyond rounding. */
+ * (-1: off); and the fail_next-th required allocation from now on finds no memory at first, so
+ * that the optional buffers are released (the -fail_next-th, if negative, none at all, so that
+ * the call that asked returns IMSRG_ERR_OUT_OF_MEMORY; 0: off).  Results do not depend on either
+ * beyond rounding. */
 imsrg_status imsrg_test_memory(imsrg_ctx* ctx, int64_t cache_limit, int32_t fail_next);
 /* The traffic of the mixed particle-hole recoupling kernel on this basis, counted exactly
  * from its orbit quadruples (no counterpart in the reference): X elements read and how many of
