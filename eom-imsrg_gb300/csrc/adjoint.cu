@@ -142,7 +142,8 @@ imsrg_status Ctx::commutator_vjp(const double* Lp, int hL, const double* Rp, int
 
 // The pieces carry the cotangent of RES backwards one after the other; what each makes of it for L and R goes on beside the
 // next: the WCC transposes and the Pandya transposes on the main stream, the ladder's on branch 1, 122, 121, 111 and E0 on
-// branch 2.  Everything that adds to Lb and Rb does so atomically.
+// branch 2.  The two-body parts of Lb and Rb are added to from all of them, atomically; their one-body parts from branch 2 alone
+// (111 and E0 add to those without atomics).
 imsrg_status Ctx::vjp_pieces(const double* Lp, int hL, const double* Rp, int hR, int hRES, bool with_e0, const double* Cb,
                              double* Lb, double* Rb) {
   const Layout& l = L;

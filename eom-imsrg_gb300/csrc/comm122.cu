@@ -50,9 +50,7 @@ struct G122Type<double> {
   static constexpr double kRoot2 = 1.4142135623730951, kHalfRoot2 = 0.70710678118654752;
   __device__ static double load(double x) { return x; }
   __device__ static double store(double x) { return x; }
-  __device__ static double flip(double x, bool neg) {  // an integer instruction: the FP64 pipe bounds this kernel
-    return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
-  }
+  __device__ static double flip(double x, bool neg) { return d_flip(x, neg); }
   __device__ static double f(const DevLayout& D, const double* op, int herm, int a, int b) { return d_f_elem(D, op, herm, a, b); }
 };
 

@@ -71,9 +71,10 @@ __device__ __forceinline__ double d_sgn(int n) { return (n & 1) ? -1.0 : 1.0; }
 // Phases and small factors without FP64 instructions where that can be done: the FP64 pipe takes 2 operations a clock per SM,
 // and the gather kernels spent more of them on factors of one than on the sums (same values; commutator at eMax 6
 // 351 -> 325 us, at eMax 10 8.73 -> 8.40 ms, its adjoint at eMax 6 813 -> 765 us, the eMax 4 observable 1969 -> 1832 us).
-__device__ __forceinline__ double d_flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+__device__ __forceinline__ double d_flip_bit(double x, unsigned sign) {  // sign: 0 or 0x80000000
+  return __hiloint2double(__double2hiint(x) ^ (int)sign, __double2loint(x));
 }
+__device__ __forceinline__ double d_flip(double x, bool neg) { return d_flip_bit(x, neg ? 0x80000000u : 0u); }
 // 2^(nsq/2) with a sign, nsq = 0, 1 or 2: the swap phases of an element's pairs and sqrt(2) for each pair of equal orbits
 // (the product of two rounded sqrt(2) is an ulp above 2)
 __device__ __forceinline__ double d_pair_factor(bool neg, int nsq) {

@@ -161,8 +161,8 @@ imsrg_status Ctx::g122_set_caps(int tiny_cap, int small_cap) {
   return g122_upload(tiny_cap, small_cap);
 }
 
-// commutator_122 on pair-group sub-blocks: RES's rectangular arrays and the upper triangles of its square ones.  run_if:
-// nothing is done unless that flag is zero.
+// commutator_122 on pair-group sub-blocks: RES's rectangular arrays and the upper triangles of its square ones.  In FP64 it
+// does nothing unless k_check_mirror finds both operators' lower triangles in line with the upper ones.
 template <typename T>
 imsrg_status Ctx::c122_groups(const double* Lp, int hL, const double* Rp, int hR, double* RES, int hRES) {
   const G122Plan& P = gp.g122;

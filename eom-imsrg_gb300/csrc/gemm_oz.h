@@ -11,7 +11,7 @@ namespace imsrg {
 constexpr int kOzSlices = 8;     // base-256 digits of an operand element
 constexpr int kOzBlockK = 32;    // K of an operand block (64 bytes of BF16 a row)
 constexpr int kOzTileM = 128;    // rows of an operand block and of an output tile
-// Multiply-adds of a list, in 16 x 16 tiles, from which the digits pay: the FP64 pipe does 0.6 per ns, the digit kernels take
+// Multiply-adds of a list, in 16 x 16 tiles, from which the digits pay: the FP64 pipe does 600 per ns, the digit kernels take
 // about 30 us before they have done any (ladder / cross-coupled list at eMax 4, 5 and 8 M: 56 / 30 us by digits, 32 / 20 on
 // the FP64 pipe; at eMax 5, 33 and 40 M: 74 / 43 and 86 / 74).
 constexpr double kOzMinMacs = 2e7;

@@ -107,9 +107,6 @@ __device__ __forceinline__ HFPair hf_pair(const DevLayout& D, int oi, int oj, in
   if (same_block && x > y) p.bits |= 16;
   return p;
 }
-__device__ __forceinline__ double hf_flip(double v, unsigned sign) {
-  return __hiloint2double(__double2hiint(v) ^ (int)sign, __double2loint(v));
-}
 // arrays of a channel by the hole counts of bra and ket: pp,pp 0 | pp,ph 1 | pp,hh 2 | ph,ph 3 | hh,hh 4 | ph,hh 5
 __device__ __forceinline__ int hf_array(int c1, int c2) { return c1 == 0 ? c2 : (c1 == 1 ? (c2 == 1 ? 3 : 5) : 4); }
 
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(128)
     const int i1 = tr ? s.pos : p.pos, i2 = tr ? p.pos : s.pos;
     double v = op[goff[g] + i1 + (int64_t)i2 * gn1[g]];
     if (p.same() || s.same()) v *= p.same() && s.same() ? 1.4142135623730951 * 1.4142135623730951 : 1.4142135623730951;
-    X[e] = hf_flip(v, p.neg() ^ s.neg() ^ (tr && herm < 0 ? 0x80000000u : 0u));
+    X[e] = d_flip_bit(v, p.neg() ^ s.neg() ^ (tr && herm < 0 ? 0x80000000u : 0u));
   }
   hf_sync<T>();
   hf_mode<T>(X, Y, ntot, n0, 1, dp + H.dp_off[b0], t, [&](int e) { return bra[e - ket_of(e) * nbra].x(); });
@@ -214,7 +211,7 @@ __global__ void __launch_bounds__(128)
     double v = X[e];
     if (p.same()) v *= 0.70710678118654752;
     if (s.same()) v *= 0.70710678118654752;
-    v = hf_flip(v, p.neg() ^ s.neg());
+    v = d_flip_bit(v, p.neg() ^ s.neg());
     if (p.con() <= s.con()) {
       const int g = hf_array(p.con(), s.con());
       op[goff[g] + p.pos + (int64_t)s.pos * gn1[g]] = v;

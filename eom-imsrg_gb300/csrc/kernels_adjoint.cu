@@ -257,8 +257,6 @@ __global__ void k_vjp_122(DevLayout D, const double* __restrict__ L, int hL, con
   }
 }
 
-// ---------------------------------------------------------------- 121
-// transpose of k_comm121: one warp per one-body output
 // the lanes' copies into the cotangents of f: a warp per (row or column, orbit)
 __global__ void k_vjp_122_sum(DevLayout D, const double* __restrict__ F, int nsame, int hL, int hR, double* __restrict__ Lb,
                               double* __restrict__ Rb) {
@@ -277,6 +275,8 @@ __global__ void k_vjp_122_sum(DevLayout D, const double* __restrict__ F, int nsa
   }
 }
 
+// ---------------------------------------------------------------- 121
+// transpose of k_comm121: one warp per one-body output
 __global__ void k_vjp_121(DevLayout D, const double* __restrict__ L, int hL, const double* __restrict__ R, int hR,
                           double* __restrict__ cb, int hRES, double* __restrict__ Lb, double* __restrict__ Rb) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
