@@ -13,7 +13,8 @@ namespace imsrg {
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16;
-constexpr int kRestParts = 16;     // warps that share the single elements of a piece
+constexpr int kRestParts = 16;  // warps that share the single elements of a piece
+constexpr int kRestK = 32;      // K of a stage of a fuller piece
 
 __device__ __forceinline__ double alpha_of(int code, int hL, int hR) {
   const int sel = code & 3;
@@ -110,11 +111,24 @@ __global__ void __launch_bounds__(256) k_gemm_fp64(const GemmProb* __restrict__ 
   gemm_tile(probs[tile.prob], tile, ops, As, Bs);
 }
 
+// noted elements in the rows before this lane's
+__device__ __forceinline__ int elements_before(unsigned mask, int lane) {
+  const int own = __popc(mask);
+  int n = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, n, o);
+    if (lane >= o) n += y;
+  }
+  return n - own;
+}
+
 // What the digit products of a list (gemm_oz.cu) leave: the whole list where an operand is not finite, otherwise the noted
-// elements.  A piece's few elements are shared by kRestParts warps, an element at a time with K across the lanes: a chain of
-// uncoalesced reads is what one takes, and many warps wait side by side.  A fuller piece goes to eight CTAs: a warp's lanes
-// take the rows of one column, whose reads are contiguous or broadcast, and four warps share K.  Only noted elements are
-// written.
+// elements, and those alone.  A piece's few elements are shared by kRestParts warps, an element at a time with K across the
+// lanes: a chain of uncoalesced reads is what one takes, and many warps wait side by side.  A fuller piece takes a CTA: its
+// rows and columns come through shared memory, read along their contiguous index, and a thread has one or two of the elements,
+// so that the FP64 pipe does no more than their products.  ([Omega, [Omega, H]] of an eMax 10 flow: whole columns of the
+// pieces 10.7 ms, an element a lane straight from memory 11.9, so 9.6.)
 __global__ void __launch_bounds__(256) k_gemm_fp64_rest(const GemmProb* __restrict__ probs, const GemmTile* __restrict__ tiles,
                                                         int ntiles, GemmOperands ops, const int* __restrict__ flags,
                                                         const OzRedo* __restrict__ redo, int max_redo) {
@@ -135,16 +149,10 @@ __global__ void __launch_bounds__(256) k_gemm_fp64_rest(const GemmProb* __restri
   for (int64_t x = blockIdx.x * 8 + warp; x < (int64_t)few * kRestParts; x += gridDim.x * 8) {
     const OzRedo& r = redo[x / kRestParts];
     const unsigned mask = r.mask[lane];
-    const int own = __popc(mask), count = __reduce_add_sync(0xffffffffu, own);
+    const int count = __reduce_add_sync(0xffffffffu, __popc(mask));
     const GemmProb& P = probs[r.prob];
     const int t0 = P.accum ? r.term : 0, t1 = P.accum ? r.term + 1 : P.nterm;
-    int before = own;  // elements of the rows before this lane's
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, before, o);
-      if (lane >= o) before += y;
-    }
-    before -= own;
+    const int before = elements_before(mask, lane);
     for (int e = (int)(x % kRestParts); e < count; e += kRestParts) {
       const int row = 31 - __clz(__ballot_sync(0xffffffffu, before <= e));
       unsigned bits = __shfl_sync(0xffffffffu, mask, row);
@@ -166,31 +174,77 @@ __global__ void __launch_bounds__(256) k_gemm_fp64_rest(const GemmProb* __restri
       if (lane == 0) put(P, m, c, s);
     }
   }
-  double* sums = &sh[0][0][0];
-  for (int64_t x = blockIdx.x; x < (int64_t)many * 8; x += gridDim.x) {
-    const OzRedo& r = redo[max_redo - 1 - (x >> 3)];
+  double(*As)[33] = reinterpret_cast<double(*)[33]>(&sh[0][0][0]);                // [K][row]
+  double(*Bs)[17] = reinterpret_cast<double(*)[17]>(&sh[0][0][0] + kRestK * 33);  // [K][column]
+  static_assert(kRestK * (33 + 17) <= 2 * BK * (BM + 1), "a stage fits the buffers of a tile");
+  for (int x = blockIdx.x; x < many; x += gridDim.x) {
+    const OzRedo& r = redo[max_redo - 1 - x];
     const unsigned mask = r.mask[lane];
+    const int before = elements_before(mask, lane);
+    const int count = __shfl_sync(0xffffffffu, before + __popc(mask), 31);
+    int row[2], col[2];  // this thread's elements: tid and tid + 256 of the piece's
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int e = min(tid + 256 * j, count - 1);
+      row[j] = 0;  // the last row with no more than e elements before it
+#pragma unroll
+      for (int o = 16; o; o >>= 1)
+        if (__shfl_sync(0xffffffffu, before, row[j] + o) <= e) row[j] += o;
+      unsigned bits = __shfl_sync(0xffffffffu, mask, row[j]);
+      for (int k = e - __shfl_sync(0xffffffffu, before, row[j]); k > 0; --k) bits &= bits - 1u;
+      col[j] = __ffs((int)bits) - 1;
+    }
     const GemmProb& P = probs[r.prob];
     const int t0 = P.accum ? r.term : 0, t1 = P.accum ? r.term + 1 : P.nterm;
-    // this thread: row `lane` and column c of the piece (clamped where it ends), every fourth K
-    const int c = 2 * (int)(x & 7) + (warp & 1), part = warp >> 1, row = min(r.m + lane, P.M - 1), col = min(r.n + c, P.N - 1);
-    double acc = 0.0;
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
     for (int t = t0; t < t1; ++t) {
       const GemmTerm& T = P.t[t];
-      const double* A = ops.in[T.a_id] + T.a_off + (T.ta ? (int64_t)row * T.lda : row);
-      const double* B = ops.in[T.b_id] + T.b_off + (T.tb ? col : (int64_t)col * T.ldb);
-      const int64_t sa = T.ta ? 1 : T.lda, sb = T.tb ? T.ldb : 1;
-      const int K = T.K;
-      double v = 0.0;
-#pragma unroll 8
-      for (int k = part; k < K; k += 4) v = fma(A[k * sa], B[k * sb], v);
-      acc = fma(alpha_of(T.alpha, ops.hL, ops.hR), v, acc);
+      const double* A = ops.in[T.a_id] + T.a_off;
+      const double* B = ops.in[T.b_id] + T.b_off;
+      const double alpha = alpha_of(T.alpha, ops.hL, ops.hR);
+      const int K = T.K, lda = T.lda, ldb = T.ldb, ta = T.ta, tb = T.tb;
+      double a[4], b[2];
+      auto load = [&](int k0) {  // lanes along the contiguous index of each operand
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int y = warp + 8 * i, gm = r.m + (ta ? y : lane), gk = k0 + (ta ? lane : y);
+          a[i] = (gm < P.M && gk < K) ? alpha * A[ta ? gk + (int64_t)gm * lda : gm + (int64_t)gk * lda] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int c = tb ? lane & 15 : warp + 8 * i, k = tb ? 2 * (warp + 8 * i) + (lane >> 4) : lane, gn = r.n + c, gk = k0 + k;
+          b[i] = (gn < P.N && gk < K) ? B[tb ? gn + (int64_t)gk * ldb : gk + (int64_t)gn * ldb] : 0.0;
+        }
+      };
+      load(0);
+      for (int k0 = 0; k0 < K; k0 += kRestK) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) (ta ? As[lane][warp + 8 * i] : As[warp + 8 * i][lane]) = a[i];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) (tb ? Bs[2 * (warp + 8 * i) + (lane >> 4)][lane & 15] : Bs[lane][warp + 8 * i]) = b[i];
+        __syncthreads();
+        if (k0 + kRestK < K) load(k0 + kRestK);
+        if (tid - lane < count) {
+          const int kn = min(kRestK, K - k0);
+#pragma unroll 4
+          for (int k = 0; k < kn; k += 2) {  // an odd K ends on zeros
+            acc[0][0] = fma(As[k][row[0]], Bs[k][col[0]], acc[0][0]);
+            acc[0][1] = fma(As[k + 1][row[0]], Bs[k + 1][col[0]], acc[0][1]);
+          }
+          if (tid - lane + 256 < count) {
+#pragma unroll 4
+            for (int k = 0; k < kn; k += 2) {
+              acc[1][0] = fma(As[k][row[1]], Bs[k][col[1]], acc[1][0]);
+              acc[1][1] = fma(As[k + 1][row[1]], Bs[k + 1][col[1]], acc[1][1]);
+            }
+          }
+        }
+        __syncthreads();
+      }
     }
-    sums[tid] = acc;
-    __syncthreads();
-    if (part == 0 && (mask >> c & 1u))
-      put(P, r.m + lane, r.n + c, (sums[tid] + sums[tid + 64]) + (sums[tid + 128] + sums[tid + 192]));
-    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (tid + 256 * j < count) put(P, r.m + row[j], r.n + col[j], acc[j][0] + acc[j][1]);
   }
 }
 

@@ -16,10 +16,13 @@
 // The powers of two say little about an element where the large elements of a row meet the small ones of a column, and an
 // FMA chain would be far better there.  So a ninth slice holds every element's magnitude, |a| 2^-ea in BF16, and its product
 // gives each output element's sum of |a||b| 2^-(ea+eb), term by term, before the digits.  Digits are kept from
-// 2^-6 K^(1/2) on: then K 2^-59 is below K^(1/2) 2^-53 of the sum of |a||b|, within the bound of the FMAs, and K^(1/2) 2^-62
-// below what a chain of K roundings usually adds up to.  Elements below that (of random operators' products a few
-// in a million at K in the hundreds, one in 3000 at K of a few) are noted and left to k_gemm_fp64_rest.  The ninth product
-// costs 2 of 74 MMAs and a reading more of the accumulators for each term.
+// 2^-6 on: then K 2^-59 is within K 2^-53 of the sum of |a||b|, the error bound of the FMAs, for every element (what is usual,
+// K^(1/2) 2^-62, is there at most K^(1/2) 2^-56 of the sum, where a chain of roundings usually comes to 2^-55 of it, and far below
+// that where the sum is of the size of the powers of two, as most are).  Elements below that are noted and left to
+// k_gemm_fp64_rest: fewer than one in 10^5 of random operators' products, one in 300 to 3000 of those with a flow's Omega, whose
+// elements fall off faster ([Omega, [Omega, H]] at eMax 10 9.6 ms, 8.4 with no such care; with 2^-6 K^(1/4), so that the usual
+// errors match too, 11.6; with 2^-6 K^(1/2) 14).  The ninth product costs 2 of 74 MMAs and a reading more of the accumulators for
+// each term.
 //
 // Rows that hold an Inf or a NaN have no such form: the split raises a flag, this kernel then leaves the outputs alone
 // and k_gemm_fp64_rest, launched behind it with the same flag, computes the whole list.
@@ -37,7 +40,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cmath>
 #include <cstring>
 #include <map>
 #include <queue>
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (mine) {
             uint32_t r[16];
             tmem_ld16(tm + (uint32_t)((S - 1) * kOzTileN), r);
-            const unsigned least = __float_as_uint(T.least) - 1u;
+            const unsigned least = __float_as_uint(kOzLeast) - 1u;
 #pragma unroll
             for (int j = 0; j < 16; ++j) c16 |= r[j] - 1u < least ? 1u << j : 0u;  // 0 < sum < least, by the bits
             if (c16) c16 = m < P.M ? c16 & ((1u << min(max(P.N - n, 0), 16)) - 1u) : 0u;
@@ -545,7 +547,6 @@ void build_oz_plan(const std::vector<GemmProb>& probs, int ncta, OzPlan& P) {
       o.nkb = P.ops[a].nkb;
       o.alpha = t.alpha;
       o.src = i;
-      o.least = kOzLeast * std::sqrt((float)t.K);
     }
     if (!p.nterm) continue;
     const int x = (int)P.probs.size();

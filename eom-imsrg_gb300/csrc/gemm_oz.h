@@ -34,8 +34,7 @@ struct OzChunk {
 struct OzTerm {
   int64_t a_blk, b_blk;
   int a_exp, b_exp, nkb, alpha;
-  int src;      // the same term of GemmProb
-  float least;  // kOzLeast sqrt(K): sums of magnitudes below it are left to FP64 FMAs
+  int src;  // the same term of GemmProb
 };
 struct OzProb {
   int64_t c_off;
@@ -49,9 +48,10 @@ struct OzRedo {
   int prob, term, m, n;  // of the GemmProb list
   unsigned short mask[32];
 };
-constexpr int kOzSingles = 64;  // most elements of an entry that are redone one by one
-// smallest sum of |a||b| 2^-(ea+eb) over sqrt(K) that the digits are used for
-constexpr float kOzLeast = 1.0f / 64;
+constexpr int kOzSingles = 16;  // most elements of an entry that are redone one by one
+// smallest sum of |a||b| 2^-(ea+eb) that the digits are used for: they lose at most K 8.03 2^-62 (seven digit products of 2^14 at
+// 2^-76, what follows them, and 2^-63 for each operand), FMAs K 2^-53 of the sum
+constexpr float kOzLeast = 1.01f / 64;
 // rows m0 .. m0 + 127 and columns n0 .. n0 + w - 1 of a problem (w a multiple of 16, n0 of 64)
 struct OzTile {
   int prob, m0, n0, w;

@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 
 def check(x, terms, what):
     """x against extended precision within the bound of an FP64 FMA chain, element by element.  The digits of an element that
-    keeps them are off by at most K 2^-58.9 of the two powers of two, and its sum of magnitudes is at least 2^-6 K^(1/2) of
-    those: K^(1/2) 2^-52.9 of that sum and one rounding."""
+    keeps them are off by at most K 2^-58.9 of the two powers of two, and its sum of magnitudes is at least 2^-6 of those:
+    K 2^-53 of that sum and one rounding."""
     K = sum(A.shape[1] for _, A, _ in terms)
     ref, mag = np.zeros(x.shape, np.longdouble), np.zeros(x.shape)
     for s, A, B in terms:
