@@ -217,6 +217,7 @@ imsrg_status Ctx::restore_quadrupoles(const double* X, int hX, const double* OM,
     ops.in[kOpL] = X; ops.in[kOpR] = OM;
     ops.out[kOpW1] = qs->w1; ops.out[kOpW2] = qs->w2;
     ops.hL = hX; ops.hR = hOM;
+    // once after a series of commutators, and K is a few hh pairs in half of the list, where digits would be mostly padding
     k_gemm_fp64<<<qs->nt, 256, 0, stream>>>(qs->p, qs->t, ops);
     CKQ(launched("k_gemm_fp64(quadrupole intermediates)"));
   }

@@ -537,7 +537,7 @@ imsrg_status Ctx::tensor_ladder(TensorState& S, const double* Lp, int hL, const 
     out.f64[kOpW1] = S.w1;
     out.f64[kTensorOpW3] = S.w3;
     CKT(tc_gemm_on(S.tc_map, S.tc_slice_rows, S.tc_probs, S.tc_tiles, S.tc_ntiles, out, hL, hR));
-    if (S.n_hh_t) {
+    if (S.n_hh_t) {  // K is the hh pairs of a channel, a few: blocks of digits (32 K) would be mostly padding
       k_gemm_fp64<<<S.n_hh_t, 256, 0, stream>>>(S.hh_p, S.hh_t, ops);
       CKT(launched("k_gemm_fp64(tensor hh ladder)"));
     }
